@@ -8,7 +8,10 @@
 // once per 8 rows; the reduction is cut in chunks when there are few rows), then one warp per row for the rest.
 #include <math.h>
 
+#include <type_traits>
+
 #include "dkv_common.cuh"
+#include "dkv_tma.cuh"
 
 namespace dkv {
 
@@ -233,6 +236,278 @@ __global__ void __launch_bounds__(256) gate_small_kernel(dkv_gate_args pk, dkv_g
   gate_finish_row<T>(p, row, lg, mx, lane, native, thr);
 }
 
+// ---- many 16-bit rows (a prompt): logits on the tensor core, then one warp per row with its columns in registers ----
+//
+// gate_gemm_kernel: logits = x W + b.  One CTA per 128 rows x BN columns; the reduction runs over 64-wide stages, x as
+// a K-major operand (boxes of 64 dims x 128 rows), W as it lies in memory, an MN-major operand (boxes of 64 columns x 64
+// dims), both by TMA in the 128-byte swizzle, two stages in flight; two CTAs share an SM, so that one's read-back hides
+// behind the other's products.  fp32 accumulation; the sum is rounded to the storage type only where the reference's
+// addmm writes it (native rounding), and the logits then travel in that type (half the bytes).  Bound by the tensor
+// core: 8192 rows x 1024 take 13 us of it; the CUDA-core kernel above took 1161 us.
+constexpr int GG_ROWS = 128, GG_BK = 64, GG_STAGES = 2;
+constexpr uint32_t GG_SPIN = 1u << 22;
+
+__device__ __forceinline__ uint32_t gg_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool gg_wait(unsigned long long* bar, uint32_t parity) {
+  for (uint32_t it = 0; it < GG_SPIN; ++it) {
+    uint32_t r;
+    asm volatile("{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\nselp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(r) : "r"(gg_smem(bar)), "r"(parity) : "memory");
+    if (r) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void gg_load(uint32_t dst, const CUtensorMap* map, int c0, int c1, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(gg_smem(bar)) : "memory");
+}
+// 128-byte swizzle descriptor: leading / stride byte offsets in 16-byte units
+__device__ __forceinline__ uint64_t gg_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+template <typename T>
+__device__ __forceinline__ uint32_t gg_pack(float lo, float hi) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+  } else {
+    __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+  }
+}
+
+template <typename T, int BN>
+__global__ void __launch_bounds__(128, 2) gate_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                                                           dkv_gate_args p) {
+  constexpr int A_BYTES = GG_ROWS * GG_BK * 2, B_BYTES = BN * GG_BK * 2, STAGE = A_BYTES + B_BYTES;
+  extern __shared__ unsigned char gg_raw[];
+  // the swizzle is taken on absolute shared-memory addresses: tiles start on 1024-byte boundaries
+  unsigned char* tiles = gg_raw + ((1024u - (gg_smem(gg_raw) & 1023u)) & 1023u);
+  __shared__ alignas(8) unsigned long long full[GG_STAGES], empty[GG_STAGES], done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ float bias_s[BN];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n0 = blockIdx.x * BN, row0 = blockIdx.y * GG_ROWS;
+  const int n_k = p.dim / GG_BK;
+  if (tid == 0) {
+    for (int s = 0; s < GG_STAGES; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&full[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&empty[s])));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&done)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gg_smem(&tmem_slot)), "r"(BN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  for (int e = tid; e < BN; e += 128) bias_s[e] = to_f32(reinterpret_cast<const T*>(p.b)[n0 + e]);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  if (warp == 0 && lane == 0) {
+    for (int k = 0; k < n_k; ++k) {
+      const int s = k % GG_STAGES;
+      if (k >= GG_STAGES && !gg_wait(&empty[s], (uint32_t)((k / GG_STAGES - 1) & 1))) break;
+      const uint32_t a = gg_smem(tiles) + s * STAGE, b = a + A_BYTES;
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gg_smem(&full[s])), "r"(STAGE) : "memory");
+      gg_load(a, &map_x, k * GG_BK, row0, &full[s]);
+#pragma unroll
+      for (int nb = 0; nb < BN / 64; ++nb) gg_load(b + nb * (64 * GG_BK * 2), &map_w, n0 + 64 * nb, k * GG_BK, &full[s]);
+    }
+  } else if (warp == 1 && lane == 0) {
+    const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+    // D fp32, A K-major, B MN-major (bit 16), M = 128, N = BN
+    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
+    bool ok = true;
+    for (int k = 0; k < n_k && ok; ++k) {
+      const int s = k % GG_STAGES;
+      ok = gg_wait(&full[s], (uint32_t)((k / GG_STAGES) & 1));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t a = gg_smem(tiles) + s * STAGE, b = a + A_BYTES;
+#pragma unroll
+      for (int ks = 0; ks < GG_BK / 16; ++ks) {
+        // A: 8-row groups 1024 bytes apart, k-step 32 bytes on; B: 64-column blocks 64 * GG_BK * 2 bytes apart, groups of
+        // 8 dims 1024 bytes apart, k-step two groups on
+        const uint64_t da = gg_desc(a + 32 * ks, 16, 1024), db = gg_desc(b + 2048 * ks, 64 * GG_BK * 2, 1024);
+        asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n}"
+                     ::"r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(k + ks > 0 ? 1u : 0u) : "memory");
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&empty[s])) : "memory");
+    }
+    if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&done)) : "memory");
+  }
+  __syncwarp();
+  bool ok = gg_wait(&done, 0);      // bounded; the verdict is the block's (tensor-memory loads are warp-collective)
+  ok = __syncthreads_and(ok) != 0;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (ok) {
+    const uint32_t lane_addr = tmem + ((uint32_t)(32 * warp) << 16);
+    const int row = row0 + tid;
+    const bool native = p.native_rounding != 0;
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 32) {
+      uint32_t r[32];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+          "tcgen05.wait::ld.sync.aligned;"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+            "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+            "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+            "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          : "r"(lane_addr + c) : "memory");
+      if (row < p.n_rows) {
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) + bias_s[c + i];
+        if (native) {
+          uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.workspace) + (size_t)row * p.dim + n0 + c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            o[i] = make_uint4(gg_pack<T>(v[8 * i], v[8 * i + 1]), gg_pack<T>(v[8 * i + 2], v[8 * i + 3]),
+                              gg_pack<T>(v[8 * i + 4], v[8 * i + 5]), gg_pack<T>(v[8 * i + 6], v[8 * i + 7]));
+        } else {
+          float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.workspace) + (size_t)row * p.dim + n0 + c);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
+  }
+}
+
+// gate_rows_kernel: softmax, running sum, count and masked copy of a row whose logits gate_gemm_kernel left in the
+// workspace; lane l holds columns PER l .. PER l + PER - 1 in registers.  The work is one read of the logits, one of x
+// and one write of the masked row.  8192 rows x 1024, bf16: 98 us with the columns in (bank-conflicted) shared memory.
+template <typename T, bool NATIVE, int PER>
+__global__ void __launch_bounds__(256) gate_rows_kernel(dkv_gate_args p) {
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= p.n_rows) return;
+  constexpr int d = 32 * PER;
+  const float thr = NATIVE ? to_f32(from_f32<T>(p.threshold)) : p.threshold;   // the comparison converts the scalar
+  float e[PER];
+  if (NATIVE) {
+    const uint2* src = reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(p.workspace) + (size_t)row * d + PER * lane);
+#pragma unroll
+    for (int i = 0; i < PER / 4; ++i) {
+      const uint2 v = src[i];
+      const T* t = reinterpret_cast<const T*>(&v);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) e[4 * i + k] = to_f32(t[k]);
+    }
+  } else {
+    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.workspace) + (size_t)row * d + PER * lane);
+#pragma unroll
+    for (int i = 0; i < PER / 4; ++i) {
+      const float4 v = src[i];
+      e[4 * i] = v.x; e[4 * i + 1] = v.y; e[4 * i + 2] = v.z; e[4 * i + 3] = v.w;
+    }
+  }
+  float mx = e[0];
+#pragma unroll
+  for (int i = 1; i < PER; ++i) mx = fmaxf(mx, e[i]);
+  mx = warp_max(mx);
+  float z = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) { e[i] = expf(e[i] - mx); z += e[i]; }
+  z = warp_sum(z);
+  float local = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    e[i] = e[i] / z;
+    if (NATIVE) e[i] = to_f32(from_f32<T>(e[i]));      // softmax writes the probabilities in the storage type
+    local += e[i];
+  }
+  float incl = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  float run = incl - local;
+  const int lo = d - min(max(p.low_rank, 0), d);   // only columns >= lo can count
+  int cnt = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    run += e[i];
+    const float c = NATIVE ? to_f32(from_f32<T>(run)) : run;   // cumsum writes every running sum in the storage type
+    cnt += PER * lane + i >= lo && c >= thr;
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (p.len_multiple > 1) cnt = min((cnt + p.len_multiple - 1) / p.len_multiple * p.len_multiple, d - d % p.len_multiple);
+  if (lane == 0) p.lengths[row] = cnt;
+  if (p.masked) {
+    const T* xr = reinterpret_cast<const T*>(p.x) + (size_t)row * p.x_stride;
+    T* out = reinterpret_cast<T*>(p.masked) + (size_t)row * p.masked_stride;
+    if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(xr)) & 15) == 0) {
+#pragma unroll
+      for (int i0 = 0; i0 < d; i0 += 256) {
+        const int i = i0 + 8 * lane;
+        if (i >= d) break;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (i < cnt) v = __ldcs(reinterpret_cast<const uint4*>(xr + i));
+        if (i + 8 > cnt && i < cnt) {
+          T* t = reinterpret_cast<T*>(&v);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (i + k >= cnt) t[k] = from_f32<T>(0.f);
+        }
+        __stcs(reinterpret_cast<uint4*>(out + i), v);
+      }
+    } else {
+      for (int i = lane; i < d; i += 32) out[i] = i < cnt ? xr[i] : from_f32<T>(0.f);
+    }
+  }
+}
+
+// The tensor-core path takes blocks of more than 64 rows (fewer: the reduction split over CTAs reads W at once) of 16-bit
+// types whose width is a whole number of its column tiles and that TMA can address.
+static bool gate_gemm_ok(const dkv_gate_args* a) {
+  return a->dtype != DKV_F32 && a->n_rows > 64 && (a->dim == 128 || a->dim == 256 || a->dim == 512 || a->dim == 1024) &&
+         (((uintptr_t)a->x | (uintptr_t)a->w | (uintptr_t)a->workspace) & 15) == 0 && a->x_stride % 8 == 0;
+}
+
+template <typename T, int BN>
+static cudaError_t launch_gate_gemm(const dkv_gate_args* a, const CUtensorMap& mx, const CUtensorMap& mw, cudaStream_t st) {
+  const int smem = GG_STAGES * (GG_ROWS + BN) * GG_BK * 2 + 1024;
+  const cudaError_t e = cudaFuncSetAttribute(gate_gemm_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess)
+    gate_gemm_kernel<T, BN><<<dim3(a->dim / BN, (a->n_rows + GG_ROWS - 1) / GG_ROWS), 128, smem, st>>>(mx, mw, *a);
+  return e;
+}
+template <typename T>
+static int gate_prompt(const dkv_gate_args* a) {
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
+  CUtensorMap mx, mw;
+  DKV_REQUIRE(tensor_map_16bit(&mx, a->dtype, a->x, (uint64_t)a->n_rows, (uint64_t)a->dim, (uint64_t)a->x_stride, GG_ROWS) &&
+                  tensor_map_16bit(&mw, a->dtype, a->w, (uint64_t)a->dim, (uint64_t)a->dim, (uint64_t)a->dim, GG_BK),
+              DKV_E_CUDA, "dkv_gate_lengths: tensor map encoding failed");
+  // 256-column tiles (their operand reads leave shared memory half idle) once they give every SM a CTA
+  const bool wide = a->dim % 256 == 0 && (long long)((a->n_rows + GG_ROWS - 1) / GG_ROWS) * (a->dim / 256) >= sm_count();
+  const cudaError_t e = wide ? launch_gate_gemm<T, 256>(a, mx, mw, st) : launch_gate_gemm<T, 128>(a, mx, mw, st);
+  DKV_REQUIRE(e == cudaSuccess, DKV_E_CUDA, "dkv_gate_lengths: %s", cudaGetErrorString(e));
+  const int grid = (a->n_rows + 7) / 8;
+#define ROWS(NAT)                                                                    \
+  do {                                                                               \
+    if (a->dim == 128) gate_rows_kernel<T, NAT, 4><<<grid, 256, 0, st>>>(*a);        \
+    else if (a->dim == 256) gate_rows_kernel<T, NAT, 8><<<grid, 256, 0, st>>>(*a);   \
+    else if (a->dim == 512) gate_rows_kernel<T, NAT, 16><<<grid, 256, 0, st>>>(*a);  \
+    else gate_rows_kernel<T, NAT, 32><<<grid, 256, 0, st>>>(*a);                     \
+  } while (0)
+  if (a->native_rounding) ROWS(true); else ROWS(false);
+#undef ROWS
+  DKV_CHECK_LAUNCH();
+  return DKV_OK;
+}
+
 static int gate_chunks(const dkv_gate_args* a) {
   // few rows: cut the reduction so that d/128 x d/128 CTAs share the weight read; many rows: the row tiles
   // already fill the GPU
@@ -259,6 +534,7 @@ extern "C" int dkv_gate_lengths(const dkv_gate_args* a) {
   DKV_REQUIRE(a->workspace != nullptr && a->workspace_bytes >= dkv_gate_workspace_bytes(a), DKV_E_WORKSPACE,
               "dkv_gate_lengths: workspace too small: need %zu bytes, got %zu", dkv_gate_workspace_bytes(a), a->workspace_bytes);
   DKV_REQUIRE((a->n_rows + GATE_ROWS - 1) / GATE_ROWS <= 65535, DKV_E_LIMIT, "dkv_gate_lengths: at most %d rows per call", 65535 * GATE_ROWS);
+  if (gate_gemm_ok(a)) return a->dtype == DKV_F16 ? gate_prompt<__half>(a) : gate_prompt<__nv_bfloat16>(a);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const int n_chunks = gate_chunks(a);
   const int chunk_len = n_chunks == 1 ? a->dim : GATE_TILE;

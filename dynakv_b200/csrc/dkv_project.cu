@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "dkv_common.cuh"
+#include "dkv_tma.cuh"
 
 namespace dkv {
 
@@ -171,19 +172,19 @@ pj_encode_fn pj_encoder() {
   }();
   return fn;
 }
-// [rows, cols] 16-bit matrix with a row pitch in elements, boxes of 64 columns x 128 rows in the 128-byte swizzle
-bool pj_map(CUtensorMap* m, int dtype, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch) {
+}  // namespace
+
+bool tensor_map_16bit(CUtensorMap* m, int dtype, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch, uint32_t box_rows) {
+  if (pj_encoder() == nullptr) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {pitch * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)PJ_TOK};
+  const cuuint32_t box[2] = {64, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return pj_encoder()(m, dtype == DKV_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                       const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-
-}  // namespace
 
 }  // namespace dkv
 
@@ -205,9 +206,9 @@ extern "C" int dkv_project_bulk(const dkv_project_args* a) {
   DKV_REQUIRE(pj_encoder() != nullptr, DKV_E_CUDA, "dkv_project_bulk: the driver does not export cuTensorMapEncodeTiled");
   CUtensorMap mx, mb, mo;
   const uint64_t cols = (uint64_t)a->n_heads * 128;
-  DKV_REQUIRE(pj_map(&mx, a->dtype, a->x, (uint64_t)a->n_tokens, cols, (uint64_t)a->x_stride) &&
-                  pj_map(&mb, a->dtype, a->basis, cols, 128, 128) &&
-                  pj_map(&mo, a->dtype, a->out, (uint64_t)a->n_tokens, cols, (uint64_t)a->out_stride),
+  DKV_REQUIRE(tensor_map_16bit(&mx, a->dtype, a->x, (uint64_t)a->n_tokens, cols, (uint64_t)a->x_stride, PJ_TOK) &&
+                  tensor_map_16bit(&mb, a->dtype, a->basis, cols, 128, 128, PJ_TOK) &&
+                  tensor_map_16bit(&mo, a->dtype, a->out, (uint64_t)a->n_tokens, cols, (uint64_t)a->out_stride, PJ_TOK),
               DKV_E_CUDA, "dkv_project_bulk: tensor map encoding failed");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const unsigned grid = (unsigned)(tiles * a->n_heads);

@@ -1,0 +1,27 @@
+"""The gate over many 16-bit rows (tensor-core logits): edges of the 128-row tiles, every width it takes, padded rows."""
+import pytest
+import torch
+
+from oracle import dynakv_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("rows,d,low_rank,pad", [(65, 128, 128, 0), (128, 256, 200, 8), (129, 512, 512, 0), (300, 1024, 640, 64),
+                                                 (4800, 1024, 1024, 0)])
+def test_gate_of_a_prompt_against_oracle(rows, d, low_rank, pad, dtype):
+    from dynakv_b200.kernels.compressed_attention import gate_lengths
+    gen = torch.Generator().manual_seed(rows + d)
+    wide = (torch.randn(rows, d + pad, generator=gen) * 2).to(dtype)
+    x = wide[:, :d]
+    W = (torch.randn(d, d, generator=gen) / d ** 0.5).to(dtype)
+    b = (torch.randn(d, generator=gen) * 0.5).to(dtype)
+    ref = O.gate_lengths(x.float(), W.float(), b.float(), low_rank).to(torch.int64)
+    masked, lens = gate_lengths(wide.cuda()[:, :d], W.cuda(), b.cuda(), low_rank, native_rounding=False)
+    diff = lens.cpu().to(torch.int64) - ref
+    assert int(diff.abs().max()) <= 1 and int((diff != 0).sum()) <= 1 + rows // 500     # summation order only
+    keep = torch.arange(d)[None, :] < lens.cpu()[:, None]
+    assert torch.equal(masked.cpu(), torch.where(keep, x, torch.zeros_like(x)))
+    _, lens8 = gate_lengths(wide.cuda()[:, :d], W.cuda(), b.cuda(), low_rank, native_rounding=False, len_multiple=8, return_masked=False)
+    assert torch.equal(lens8, torch.clamp((lens + 7) // 8 * 8, max=d))
