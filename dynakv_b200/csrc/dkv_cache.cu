@@ -224,6 +224,42 @@ __global__ void __launch_bounds__(256) append_project_grid_kernel(dkv_append_arg
 //     one per lane), four pieces per lane in flight; element by element otherwise.
 constexpr int SCAN_THREADS = 1024, COPY_THREADS = 256;
 
+// What the host's capacity policy asks about a block before it is packed, both sides at once: one CTA per (arena row,
+// side) writes {sum of the given lengths, sum as dkv_pack_bulk stores them, write pointer now, 0}.
+constexpr int TOTALS_THREADS = 512;
+__global__ void __launch_bounds__(TOTALS_THREADS) row_totals_kernel(dkv_pack_args pk, dkv_pack_args pv, int4* out) {
+  const dkv_pack_args& p = blockIdx.y ? pv : pk;
+  const int a = blockIdx.x, n_rows = gridDim.x, lane = threadIdx.x & 31;
+  const int32_t* nl = p.new_lens + (size_t)a * p.n_new;
+  const int n_store = p.row_counts ? min(max(p.row_counts[a / p.arenas_per_batch], 0), p.n_new) : p.n_new;
+  int raw = 0, stored = 0;
+  const int step = p.len_multiple, mask = (step & (step - 1)) == 0 ? step - 1 : -1;
+  auto add = [&](int s, int len) {
+    raw += len;
+    const bool bad = (unsigned)len > (unsigned)p.max_dim || (mask >= 0 ? (len & mask) : (len % step)) != 0;
+    if (s < n_store) stored += bad ? checked_len(len, p.max_dim, step, p.status, 0) : len;     // (lengths that are not valid are flagged here)
+  };
+  const bool vec = (reinterpret_cast<uintptr_t>(nl) & 15) == 0;
+  const int n4 = vec ? p.n_new >> 2 : 0;
+#pragma unroll 4
+  for (int q = threadIdx.x; q < n4; q += TOTALS_THREADS) {
+    const int4 v = __ldg(reinterpret_cast<const int4*>(nl) + q);
+    add(4 * q, v.x); add(4 * q + 1, v.y); add(4 * q + 2, v.z); add(4 * q + 3, v.w);
+  }
+  for (int s = 4 * n4 + threadIdx.x; s < p.n_new; s += TOTALS_THREADS) add(s, nl[s]);
+  raw = __reduce_add_sync(0xffffffffu, raw);
+  stored = __reduce_add_sync(0xffffffffu, stored);
+  __shared__ int red[2][TOTALS_THREADS / 32];
+  if (lane == 0) { red[0][threadIdx.x >> 5] = raw; red[1][threadIdx.x >> 5] = stored; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int4 r = make_int4(0, 0, p.side.ptr ? p.side.ptr[a] : 0, 0);
+#pragma unroll
+    for (int w = 0; w < TOTALS_THREADS / 32; ++w) { r.x += red[0][w]; r.y += red[1][w]; }
+    out[blockIdx.y * n_rows + a] = r;
+  }
+}
+
 struct pack_row {
   int base, n_new, pos0;
 };
@@ -380,6 +416,58 @@ __global__ void __launch_bounds__(COPY_THREADS) pack_copy_kernel(dkv_pack_args p
   }
 }
 
+// Ragged -> dense, one 16-byte piece of the dense rows per thread and step, four pieces in flight: bound by HBM (the dense
+// rows written once, the payload read once).  A piece whose source is 16-byte aligned and inside the arena row is one
+// load, the rest of it masked; other pieces (any-integer lengths) go element by element.  8 x 8 x 8192 rows of 128 bf16
+// from 29 % retention: 103 us with one element per lane, 38 us now (eight pieces in flight, streaming stores or the metadata
+// staged in shared memory are no faster).
+constexpr int DEC_ITEMS = 4;
+template <typename T>
+__global__ void __launch_bounds__(256) decompress_vec_kernel(dkv_side sd, T* dense, int n_tok, int max_dim, unsigned pieces, int shift) {
+  constexpr int E = 16 / (int)sizeof(T);          // elements of a piece
+  const int a = blockIdx.y;
+  const T* flat = reinterpret_cast<const T*>(sd.flat) + (size_t)a * sd.flat_stride;
+  const int32_t* lens = sd.lens + (size_t)a * sd.lens_stride_a;
+  const int32_t* offs = sd.offs + (size_t)a * sd.offs_stride_a;
+  const unsigned n = (unsigned)n_tok * pieces, first = blockIdx.x * (256u * DEC_ITEMS) + threadIdx.x;
+  uint4* out = reinterpret_cast<uint4*>(dense + (size_t)a * n_tok * max_dim);
+  uint4 v[DEC_ITEMS];
+#pragma unroll
+  for (int k = 0; k < DEC_ITEMS; ++k) {
+    const unsigned i = first + 256u * k;
+    v[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (i >= n) continue;
+    const unsigned s = shift >= 0 ? i >> shift : i / pieces;
+    const int e0 = (int)(i - s * pieces) * E;
+    int len = min(max(lens[(size_t)s * sd.lens_stride_s], 0), max_dim);
+    const int off = offs[(size_t)s * sd.offs_stride_s];
+    if (off < 0 || (int64_t)off + len > sd.flat_stride) len = 0;      // never read outside the arena row
+    const int keep = len - e0;                     // elements of the piece that are stored
+    if (keep <= 0) continue;
+    const T* src = flat + off + e0;
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (int64_t)off + e0 + E <= sd.flat_stride) {
+      v[k] = __ldg(reinterpret_cast<const uint4*>(src));
+      if (keep < E) {
+        T* t = reinterpret_cast<T*>(&v[k]);
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+          if (e >= keep) t[e] = T(0);
+      }
+    } else {
+      T t[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) t[e] = e < keep ? src[e] : T(0);
+      v[k] = *reinterpret_cast<const uint4*>(t);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < DEC_ITEMS; ++k) {
+    const unsigned i = first + 256u * k;
+    if (i < n) out[i] = v[k];
+  }
+}
+
+// the same for rows that are no whole number of 16-byte pieces: one warp per row
 template <typename T>
 __global__ void __launch_bounds__(256) decompress_kernel(dkv_side sd, T* dense, int n_tok, int max_dim) {
   const int a = blockIdx.y, lane = threadIdx.x & 31;
@@ -390,7 +478,7 @@ __global__ void __launch_bounds__(256) decompress_kernel(dkv_side sd, T* dense, 
   if (off < 0 || (int64_t)off + len > sd.flat_stride) { len = 0; off = 0; }   // never read outside the arena row
   const T* src = reinterpret_cast<const T*>(sd.flat) + (size_t)a * sd.flat_stride + off;
   T* dst = dense + ((size_t)a * n_tok + s) * max_dim;
-  for (int i = lane; i < max_dim; i += 32) dst[i] = i < len ? src[i] : from_f32<T>(0.f);
+  for (int i = lane; i < max_dim; i += 32) dst[i] = i < len ? src[i] : T(0);
 }
 
 static int check_side(const dkv_side& s, const char* what) {
@@ -467,6 +555,21 @@ extern "C" int dkv_pack_bulk(const dkv_pack_args* a) {
   return DKV_OK;
 }
 
+extern "C" int dkv_row_totals(const dkv_pack_args* k, const dkv_pack_args* v, int32_t* totals) {
+  DKV_REQUIRE(k != nullptr && v != nullptr && totals != nullptr, DKV_E_ARG, "dkv_row_totals: null argument");
+  DKV_REQUIRE(((uintptr_t)totals & 15) == 0, DKV_E_ALIGN, "dkv_row_totals: totals must be 16-byte aligned");
+  DKV_REQUIRE(k->batch == v->batch && k->arenas_per_batch == v->arenas_per_batch && k->n_new == v->n_new && k->stream == v->stream,
+              DKV_E_ARG, "dkv_row_totals: the two sides must agree in batch, arenas, tokens and stream");
+  for (const dkv_pack_args* a : {k, v})
+    DKV_REQUIRE(a->batch >= 0 && a->arenas_per_batch >= 1 && a->n_new >= 0 && a->max_dim >= 1 && a->len_multiple >= 1 && a->new_lens, DKV_E_ARG,
+                "dkv_row_totals: bad sizes or null lengths");
+  const int n_arena = k->batch * k->arenas_per_batch;
+  if (n_arena == 0) return DKV_OK;
+  row_totals_kernel<<<dim3(n_arena, 2), TOTALS_THREADS, 0, reinterpret_cast<cudaStream_t>(k->stream)>>>(*k, *v, reinterpret_cast<int4*>(totals));
+  DKV_CHECK_LAUNCH();
+  return DKV_OK;
+}
+
 extern "C" int dkv_decompress(int32_t dtype, int32_t n_arena, int32_t n_tok, int32_t max_dim, const dkv_side* side,
                               void* dense, void* stream) {
   DKV_REQUIRE(side && dense, DKV_E_ARG, "dkv_decompress: null argument");
@@ -475,12 +578,20 @@ extern "C" int dkv_decompress(int32_t dtype, int32_t n_arena, int32_t n_tok, int
   if (int rc = check_side(*side, "dkv_decompress side")) return rc;
   if (n_arena == 0 || n_tok == 0) return DKV_OK;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  dim3 grid((n_tok + 7) / 8, n_arena);
-  if (dtype == DKV_F32) decompress_kernel<float><<<grid, 256, 0, st>>>(*side, (float*)dense, n_tok, max_dim);
-  else if (dtype == DKV_F16) decompress_kernel<__half><<<grid, 256, 0, st>>>(*side, (__half*)dense, n_tok, max_dim);
-  else if (dtype == DKV_BF16)
-    decompress_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*side, (__nv_bfloat16*)dense, n_tok, max_dim);
-  else DKV_REQUIRE(false, DKV_E_ARG, "dkv_decompress: bad dtype %d", dtype);
+  DKV_REQUIRE(dtype >= DKV_F32 && dtype <= DKV_BF16, DKV_E_ARG, "dkv_decompress: bad dtype %d", dtype);
+  // the copy is of bits: 16-bit types share one instance
+  const int row_bytes = max_dim * (dtype == DKV_F32 ? 4 : 2);
+  if (row_bytes % 16 == 0 && ((uintptr_t)dense & 15) == 0 && (int64_t)n_tok * (row_bytes / 16) < (1ll << 31)) {
+    const unsigned pieces = row_bytes / 16;
+    const int shift = (pieces & (pieces - 1)) == 0 ? __builtin_ctz(pieces) : -1;
+    const dim3 grid(((unsigned)n_tok * pieces + 256 * DEC_ITEMS - 1) / (256 * DEC_ITEMS), n_arena);
+    if (dtype == DKV_F32) decompress_vec_kernel<float><<<grid, 256, 0, st>>>(*side, (float*)dense, n_tok, max_dim, pieces, shift);
+    else decompress_vec_kernel<uint16_t><<<grid, 256, 0, st>>>(*side, (uint16_t*)dense, n_tok, max_dim, pieces, shift);
+  } else {
+    const dim3 grid((n_tok + 7) / 8, n_arena);
+    if (dtype == DKV_F32) decompress_kernel<float><<<grid, 256, 0, st>>>(*side, (float*)dense, n_tok, max_dim);
+    else decompress_kernel<uint16_t><<<grid, 256, 0, st>>>(*side, (uint16_t*)dense, n_tok, max_dim);
+  }
   DKV_CHECK_LAUNCH();
   return DKV_OK;
 }

@@ -166,21 +166,19 @@ class CustomDynamicCache:
             cache[0] = new
 
     # ------------------------------------------------------------------ update
-    def _prepare(self, cache_list, layer_idx, new_states, new_len, max_dim, is_decode, n_new):
-        """Host-side capacity policy of the reference (_update_layer_cache, compressed_cache.py:96-168)."""
+    def _prepare(self, cache_list, layer_idx, new_states, new_len, max_dim):
+        """Host-side capacity policy of the reference for one new token (_update_layer_cache, compressed_cache.py:96-168)."""
         while len(cache_list) <= layer_idx:
             cache_list.append(None)
         rows = new_len.shape[0]
         if cache_list[layer_idx] is None:
             # first use: exact fit (one synchronising reduction, as in the reference)
             init_flat = int(new_len.sum(dim=1).max().item())
-            cache_list[layer_idx] = self._new_state(rows, _round8(init_flat), n_new, new_states.dtype,
-                                                    new_states.device)
+            cache_list[layer_idx] = self._new_state(rows, _round8(init_flat), 1, new_states.dtype, new_states.device)
         cache = cache_list[layer_idx]
-        seq_ptr = cache[4]
-        if seq_ptr + n_new > cache[1].shape[1]:
-            self._ensure_capacity(cache, cache[0].shape[1], max(cache[1].shape[1] + EXPAND_SEQ_STEP, seq_ptr + n_new))
-        max_added = n_new * max_dim if is_decode else int(new_len.sum(dim=1).max().item())
+        if cache[4] + 1 > cache[1].shape[1]:
+            self._ensure_capacity(cache, cache[0].shape[1], cache[1].shape[1] + EXPAND_SEQ_STEP)
+        max_added = max_dim
         if max(cache[5]) + max_added > cache[0].shape[1]:
             real = cache[3].cpu().tolist()          # resynchronise the conservative bound
             cache[5] = real
@@ -223,63 +221,121 @@ class CustomDynamicCache:
             return t.contiguous()
 
         kl, vl = lens2d(key_len), lens2d(value_len)
-        ck, _ = self._prepare(self.key_cache_sp, layer_idx, key_states, kl, width, is_decode, n_new)
-        cv, max_added = self._prepare(self.value_cache_sp, layer_idx, value_states, vl, width, is_decode, n_new)
+        if not is_decode or token_counts is not None:
+            return self._update_block(key_states, kl, value_states, vl, row_dim, width, layer_idx, token_counts)
+        ck, _ = self._prepare(self.key_cache_sp, layer_idx, key_states, kl, width)
+        cv, max_added = self._prepare(self.value_cache_sp, layer_idx, value_states, vl, width)
         seq_ptr = ck[4]
+        row_counter = self._row_counter(layer_idx, B, dev, seq_ptr, token_counts)
+        ks = key_states.contiguous()
+        vs = value_states.contiguous()
+        a = _lib.AppendArgs()
+        a.dtype, a.batch, a.arenas_per_batch, a.max_dim = _lib.dtype_code(key_states.dtype), B, A, row_dim
+        a.new_k, a.new_v, a.len_k, a.len_v = ks.data_ptr(), vs.data_ptr(), kl.data_ptr(), vl.data_ptr()
+        a.k, a.v = self._side(ck), self._side(cv)
+        a.seq_pos, a.seq_capacity = seq_ptr, ck[1].shape[1]
+        a.seq_lens = _lib.ptr(row_counter)   # ragged: write at the row's own count, kernel advances it
+        a.len_multiple, a.status, a.stream = self.len_multiple, status_word(dev).data_ptr(), _lib.stream_ptr(dev)
+        _lib.check(lib.dkv_append_decode(C.byref(a)), "dkv_append_decode")
+        if row_counter is not None:
+            self._seq_lens_host[layer_idx] = [n + 1 for n in self._seq_lens_host[layer_idx]]
+        for cache in (ck, cv):
+            cache[4] = seq_ptr + 1
+            cache[5] = [p_ + max_added for p_ in cache[5]]
+        s = ck[4]
+        return ck[0], cv[0], ck[1][:, :s], cv[1][:, :s], ck[2][:, :s], cv[2][:, :s]
+
+    def _row_counter(self, layer_idx, batch, dev, seq_ptr, token_counts):
+        """Device row counters of a ragged layer (created by the first update with ``token_counts``), else None."""
         while len(self._seq_lens) <= layer_idx:
             self._seq_lens.append(None)
             self._seq_lens_host.append(None)
-        ragged = token_counts is not None or self._seq_lens[layer_idx] is not None
-        if ragged and self._seq_lens[layer_idx] is None:
+        if token_counts is not None and self._seq_lens[layer_idx] is None:
             if seq_ptr != 0:
                 raise ValueError("token_counts must be given from the first update of a layer on")
-            self._seq_lens[layer_idx] = torch.zeros(B, dtype=torch.int32, device=dev)
-            self._seq_lens_host[layer_idx] = [0] * B
-        row_counter = self._seq_lens[layer_idx]
-        st = status_word(dev)
-        stream = _lib.stream_ptr(dev)
-        dt = _lib.dtype_code(key_states.dtype)
+            self._seq_lens[layer_idx] = torch.zeros(batch, dtype=torch.int32, device=dev)
+            self._seq_lens_host[layer_idx] = [0] * batch
+        return self._seq_lens[layer_idx]
 
-        if is_decode and token_counts is None:
-            ks = key_states.contiguous()
-            vs = value_states.contiguous()
-            a = _lib.AppendArgs()
-            a.dtype, a.batch, a.arenas_per_batch, a.max_dim = dt, B, A, row_dim
-            a.new_k, a.new_v, a.len_k, a.len_v = ks.data_ptr(), vs.data_ptr(), kl.data_ptr(), vl.data_ptr()
-            a.k, a.v = self._side(ck), self._side(cv)
-            a.seq_pos, a.seq_capacity = seq_ptr, ck[1].shape[1]
-            a.seq_lens = _lib.ptr(row_counter)   # ragged: write at the row's own count, kernel advances it
-            a.len_multiple, a.status, a.stream = self.len_multiple, st.data_ptr(), stream
-            _lib.check(lib.dkv_append_decode(C.byref(a)), "dkv_append_decode")
-            if ragged:
-                self._seq_lens_host[layer_idx] = [n + 1 for n in self._seq_lens_host[layer_idx]]
-        else:
-            counts_dev = None
-            if token_counts is not None:
-                counts_dev = torch.tensor(list(token_counts), dtype=torch.int32, device=dev)
-            for states, lens, cache in ((key_states, kl, ck), (value_states, vl, cv)):
-                if states.stride(2) != 1:
-                    states = states.contiguous()
-                p = _lib.PackArgs()
-                p.dtype, p.batch, p.arenas_per_batch, p.n_new, p.max_dim = dt, B, A, n_new, row_dim
-                p.states, p.stride_b, p.stride_j, p.stride_s = states.data_ptr(), states.stride(0), row_dim, states.stride(1)
-                p.new_lens = lens.data_ptr()
-                p.row_counts = _lib.ptr(counts_dev)
-                p.seq_lens = _lib.ptr(row_counter)
-                p.side = self._side(cache)
-                p.seq_pos, p.seq_capacity, p.len_multiple = seq_ptr, cache[1].shape[1], self.len_multiple
-                p.status, p.stream = st.data_ptr(), stream
-                _lib.check(lib.dkv_pack_bulk(C.byref(p)), "dkv_pack_bulk")
-            if ragged:
-                counts = list(token_counts) if token_counts is not None else [n_new] * B
-                row_counter.add_(counts_dev if counts_dev is not None else n_new)
-                self._seq_lens_host[layer_idx] = [a_ + int(c) for a_, c in zip(self._seq_lens_host[layer_idx], counts)]
+    def _update_block(self, key_states, kl, value_states, vl, row_dim, width, layer_idx, token_counts):
+        """A block of tokens (prefill).  The capacity policy of _update_layer_cache (compressed_cache.py:143-209) needs the
+        rows' totals and write pointers on the host: one kernel collects them for both sides, one copy brings them over,
+        and when the layer already has buffers the pack is queued behind that copy without waiting for it -- a block that
+        does not fit leaves nothing behind that the repeated pack into the grown buffers does not overwrite."""
+        lib, A, dev = _lib.load(), self.arenas_per_batch, key_states.device
+        B, n_new = key_states.shape[0], key_states.shape[1]
+        rows, dt, stream = B * A, _lib.dtype_code(key_states.dtype), _lib.stream_ptr(dev)
+        st = status_word(dev).data_ptr()
+        lists = (self.key_cache_sp, self.value_cache_sp)
+        for cache_list in lists:
+            while len(cache_list) <= layer_idx:
+                cache_list.append(None)
+        fresh = [lst[layer_idx] is None for lst in lists]
+        seq_ptr = 0 if fresh[0] else lists[0][layer_idx][4]
+        counts = None if token_counts is None else [int(c) for c in token_counts]
+        row_counter = self._row_counter(layer_idx, B, dev, seq_ptr, token_counts)
+        counts_dev = None
+        if counts is not None and any(c != n_new for c in counts):
+            counts_dev = torch.tensor(counts, dtype=torch.int32, device=dev)
+        for lst, new in zip(lists, fresh):
+            if not new and lst[layer_idx][4] + n_new > lst[layer_idx][1].shape[1]:
+                c = lst[layer_idx]
+                self._ensure_capacity(c, c[0].shape[1], max(c[1].shape[1] + EXPAND_SEQ_STEP, c[4] + n_new))
+        args = []
+        keep = []
+        for states, lens in ((key_states, kl), (value_states, vl)):
+            if states.stride(2) != 1:
+                states = states.contiguous()
+            keep.append(states)
+            p = _lib.PackArgs()
+            p.dtype, p.batch, p.arenas_per_batch, p.n_new, p.max_dim = dt, B, A, n_new, row_dim
+            p.states, p.stride_b, p.stride_j, p.stride_s = states.data_ptr(), states.stride(0), row_dim, states.stride(1)
+            p.new_lens = lens.data_ptr()
+            p.row_counts = _lib.ptr(counts_dev)
+            p.seq_lens = _lib.ptr(row_counter)
+            p.seq_pos, p.len_multiple, p.status, p.stream = seq_ptr, self.len_multiple, st, stream
+            args.append(p)
 
-        for cache in (ck, cv):
+        def pack(side, status):
+            cache, p = lists[side][layer_idx], args[side]
+            p.side, p.seq_capacity, p.status = self._side(cache), cache[1].shape[1], status
+            _lib.check(lib.dkv_pack_bulk(C.byref(p)), "dkv_pack_bulk")
+
+        for side in (0, 1):
+            if not fresh[side]:
+                args[side].side = self._side(lists[side][layer_idx])
+        totals = torch.empty((2, rows, 4), dtype=torch.int32, device=dev)
+        _lib.check(lib.dkv_row_totals(C.byref(args[0]), C.byref(args[1]), totals.data_ptr()), "dkv_row_totals")
+        host = torch.empty((2, rows, 4), dtype=torch.int32, pin_memory=True)
+        host.copy_(totals, non_blocking=True)
+        here = torch.cuda.Event()
+        here.record(torch.cuda.current_stream(dev))
+        for side in (0, 1):
+            if not fresh[side]:
+                pack(side, None)
+        here.synchronize()
+        for side, lst in enumerate(lists):
+            raw, stored, now, _ = host[side].t().tolist()
+            if fresh[side]:
+                lst[layer_idx] = self._new_state(rows, _round8(max(raw)), n_new, key_states.dtype, dev)      # exact fit
+            cache = lst[layer_idx]
+            max_added = max(raw) if n_new > 1 else width
+            grow = max(now) + max_added > cache[0].shape[1]
+            if grow:
+                step = EXPAND_SEQ_STEP * (width // 2)
+                self._ensure_capacity(cache, _round8(max(cache[0].shape[1] + step, max(now) + max_added)), cache[1].shape[1])
+                cache[3].copy_(host[side, :, 2].contiguous())     # rows of the first attempt that did fit moved on
+            cap = cache[0].shape[1]
+            if fresh[side] or grow:
+                pack(side, st)
+            elif max(n + s_ for n, s_ in zip(now, stored)) > cap:     # lengths made valid no longer fit: recorded as empty
+                status_word(dev).bitwise_or_(_lib.ST_OVERFLOW)
             cache[4] = seq_ptr + n_new
-            if is_decode:
-                cache[5] = [p_ + max_added for p_ in cache[5]]
-            else:
-                cache[5] = cache[3].cpu().tolist()
+            cache[5] = [n + s_ if n + s_ <= cap else n for n, s_ in zip(now, stored)]
+        if row_counter is not None:
+            row_counter.add_(counts_dev if counts_dev is not None else n_new)
+            self._seq_lens_host[layer_idx] = [n + (counts[b] if counts is not None else n_new)
+                                              for b, n in enumerate(self._seq_lens_host[layer_idx])]
+        ck, cv = lists[0][layer_idx], lists[1][layer_idx]
         s = ck[4]
         return ck[0], cv[0], ck[1][:, :s], cv[1][:, :s], ck[2][:, :s], cv[2][:, :s]

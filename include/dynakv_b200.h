@@ -202,6 +202,13 @@ typedef struct dkv_pack_args {
  * Replaces the per-row python loop of _update_layer_cache (compressed_cache.py:184-209). */
 int dkv_pack_bulk(const dkv_pack_args* a);
 
+/* What the host's capacity policy asks about a block before it is packed (_update_layer_cache's sums and write pointers,
+ * compressed_cache.py:143-168), both sides in one launch: totals[side][arena row] = {sum of the lengths given, sum as
+ * dkv_pack_bulk would store them (first row_counts tokens, lengths made valid), side.ptr now (0 when NULL), 0}.
+ * Only batch, arenas_per_batch, n_new, max_dim, len_multiple, new_lens, row_counts, side.ptr, status (lengths that are
+ * not valid are flagged) and stream are read. */
+int dkv_row_totals(const dkv_pack_args* k, const dkv_pack_args* v, int32_t* totals /* [2, n_arena, 4], 16-byte aligned */);
+
 /* Diagnostic, no counterpart in the reference: clock cycles per 128-token tile that the tensor pipe of one SM is
  * held by the decode kernel's tcgen05.mma chains, issued back to back by one thread over zero operands with nothing
  * else running on the SM.  `products` is a mask: 1 = K reconstruction (8 x M128 N128 K16), 2 = scores (8 x M128 N16
