@@ -1,10 +1,8 @@
-// Generic (CUDA-core, fp32-accumulate) decode attention over the ragged compressed cache.
+// Generic decode attention in one kernel, one CTA per (row, query head): the path of callers that give no workspace.
 //
 // Handles every layout the reference API can express: any element type, rank R up to 1024,
 // any integer lengths, lens/offs as strided views, joint latent rows shared by all heads or
-// per-KV-head arenas.  It is the path for fp32 inputs and for caches that do not meet the
-// alignment contract of the tensor-core path, and it implements the reference's stage-1 /
-// stage-2 operators (scores, softmax.V) with their exact conventions.
+// per-KV-head arenas; with a workspace the kernels of dkv_tiles.cu take these caches.
 //
 // Math (reference: src/dynakv/kernels/fused.py:28-142, two_stage.py:52-157, 211-281):
 //   k_s = x^k_s . Bk[g]            (first len_s coefficients only)
@@ -19,20 +17,16 @@
 
 namespace dkv {
 
-enum { MODE_ATTN = 0, MODE_SCORES = 1, MODE_SOFTMAX_V = 2, MODE_ATTN_SPLIT = 3 };
-// MODE_ATTN_SPLIT: blockIdx.z takes a slice of the tokens and leaves a partial record (m, l, latent accumulator) in
-// the workspace; generic_combine_kernel merges the records of a (row, head) and projects through Bv.
+enum { MODE_ATTN = 0, MODE_SOFTMAX_V = 2 };
 
 constexpr int GD = 128;       // head_dim
 constexpr int GTT = 32;       // tokens per tile
 constexpr int GRC = 64;       // latent coefficients staged per step
 constexpr int GTHREADS = 256;
-constexpr int GZ_TOKENS = 256;  // tokens per blockIdx.z slice in MODE_SCORES
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(GTHREADS)
-generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t sc_sb, int64_t sc_sh, float log_theta,
-                      int split_tokens) {
+generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t sc_sb, int64_t sc_sh, float log_theta) {
   __shared__ float q_s[GD];
   __shared__ float k_s[GTT][GD + 1];
   // staging: fp32 path = x tile [GTT][GRC] floats; 16-bit path = x tile [GTT][GRC + 8] and basis chunk
@@ -50,18 +44,10 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
   const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank;
   const int g = h / (Hq / p.n_basis_groups);
   const int a = b * A + (h * A) / Hq;
-  if ((MODE == MODE_ATTN || MODE == MODE_ATTN_SPLIT) && row_routed_out(p, b)) return;   // the row belongs to the other kernel
+  if (MODE == MODE_ATTN && row_routed_out(p, b)) return;   // the row belongs to the other kernel
   int S = p.seq_len;
   if (p.seq_lens) S = min(S, max(p.seq_lens[b], 0));
-  int t_begin = 0, t_end = S;
-  if (MODE == MODE_SCORES) {
-    t_begin = blockIdx.z * GZ_TOKENS;
-    t_end = min(p.seq_len, t_begin + GZ_TOKENS);  // scores are written for every column
-  }
-  if (MODE == MODE_ATTN_SPLIT) {
-    t_begin = min(S, (int)blockIdx.z * split_tokens);
-    t_end = min(S, t_begin + split_tokens);
-  }
+  const int t_begin = 0, t_end = S;
 
   const T* kflat = reinterpret_cast<const T*>(p.k.flat) + (size_t)a * p.k.flat_stride;
   const T* vflat = reinterpret_cast<const T*>(p.v.flat) + (size_t)a * p.v.flat_stride;
@@ -102,7 +88,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
             lk = 0; ok = 0;
           }
         }
-        if (MODE != MODE_SCORES) {
+        {
           lv = p.v.lens[(size_t)a * p.v.lens_stride_a + (size_t)s * p.v.lens_stride_s];
           ov = p.v.offs[(size_t)a * p.v.offs_stride_a + (size_t)s * p.v.offs_stride_s];
           lv = min(max(lv, 0), R);
@@ -271,13 +257,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
         part = warp_sum(part);
         if (lane == 0) {
           const bool in = s < t_end;
-          if (MODE == MODE_SCORES) {
-            if (in) {
-              const float v = (lenk_s[t] > 0 ? part : -1.0e4f) * scale;
-              T* op = reinterpret_cast<T*>(p.out) + (size_t)b * p.out_stride_b + (size_t)h * p.out_stride_h;
-              op[s] = from_f32<T>(v);
-            }
-          } else {
+          {
             sc_s[t] = (in && lenk_s[t] > 0) ? part * scale : -INFINITY;
           }
         }
@@ -291,7 +271,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
       __syncthreads();
     }
 
-    if (MODE != MODE_SCORES) {
+    {
       // ---- online softmax over the tile (warp 0) ----
       if (warp == 0) {
         const float sc = sc_s[lane];
@@ -333,20 +313,6 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
     }
   }
 
-  if (MODE == MODE_SCORES) return;
-  if (MODE == MODE_ATTN_SPLIT) {
-    // partial record of this slice: [m, l, acc[R]] at ((row, head), slice)
-    float* rec = reinterpret_cast<float*>(p.workspace) +
-                 (((size_t)blockIdx.x * Hq + h) * gridDim.z + blockIdx.z) * (size_t)(2 + R);
-    if (tid == 0) { rec[0] = m_run; rec[1] = l_s; }      // warp 0 owns the running maximum
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = tid + i * GTHREADS;
-      if (r < R) rec[2 + r] = acc_lat[i];
-    }
-    return;
-  }
-
   // ---- normalise and project the latent accumulator through Bv ----
   float* lat_s = &k_s[0][0];  // >= 1024 floats
   const float l = l_s;
@@ -375,97 +341,6 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
   }
 }
 
-// Merge the slices' partial records of one (row, head) and project through Bv (MODE_ATTN_SPLIT's second half).
-template <typename T>
-__global__ void __launch_bounds__(GTHREADS) generic_combine_kernel(dkv_attn_args p, int n_split) {
-  __shared__ float lat_s[1024];
-  __shared__ float w_s[64];
-  __shared__ float red_s[16][GD];
-  __shared__ float L_s;
-  const int tid = threadIdx.x, h = blockIdx.y, Hq = p.n_q_heads, R = p.rank;
-  const int b = p.batch_index ? p.batch_index[blockIdx.x] : blockIdx.x;
-  if (row_routed_out(p, b)) return;
-  const int g = h / (Hq / p.n_basis_groups);
-  const float* rec0 = reinterpret_cast<const float*>(p.workspace) + (((size_t)blockIdx.x * Hq + h) * n_split) * (size_t)(2 + R);
-  if (tid < 32) {
-    float M = -INFINITY;
-    for (int k = tid; k < n_split; k += 32) M = fmaxf(M, rec0[(size_t)k * (2 + R)]);
-    M = warp_max(M);
-    float L = 0.f;
-    for (int k = tid; k < n_split; k += 32) {
-      const float m = rec0[(size_t)k * (2 + R)];
-      const float w = (m == -INFINITY) ? 0.f : __expf(m - M);
-      w_s[k] = w;
-      L = fmaf(w, rec0[(size_t)k * (2 + R) + 1], L);
-    }
-    L = warp_sum(L);
-    if (tid == 0) L_s = L;
-  }
-  __syncthreads();
-  const float L = L_s;
-  if (L <= 0.f && tid == 0) set_status(p.status, DKV_ST_EMPTY_ROW);
-  const float inv = L > 0.f ? 1.f / L : 0.f;
-  for (int r = tid; r < R; r += GTHREADS) {
-    float v = 0.f;
-    for (int k = 0; k < n_split; ++k)
-      if (w_s[k] != 0.f) v = fmaf(w_s[k], rec0[(size_t)k * (2 + R) + 2 + r], v);
-    lat_s[r] = v * inv;
-  }
-  __syncthreads();
-  // projection through Bv: thread (rg, dg) takes latent rows rg, rg + 16, ... and the 8 output dims 8 dg..8 dg + 7
-  // (one 16-byte load per row, eight rows in flight); the 16 row groups are added up through shared memory
-  const T* vup = reinterpret_cast<const T*>(p.v_up) + (size_t)g * R * GD;
-  const int dg = tid & 15, rg = tid >> 4;
-  const bool vec = (reinterpret_cast<uintptr_t>(p.v_up) & 15) == 0 && sizeof(T) == 2;
-  float acc8[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) acc8[e] = 0.f;
-  if (vec) {
-#pragma unroll 8
-    for (int r = rg; r < R; r += 16) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(vup + (size_t)r * GD) + dg);
-      const T* vp = reinterpret_cast<const T*>(&v);
-      const float lr = lat_s[r];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc8[e] = fmaf(lr, to_f32(vp[e]), acc8[e]);
-    }
-  } else {
-#pragma unroll 4
-    for (int r = rg; r < R; r += 16) {
-      const float lr = lat_s[r];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc8[e] = fmaf(lr, to_f32(vup[(size_t)r * GD + 8 * dg + e]), acc8[e]);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < 8; ++e) red_s[rg][8 * dg + e] = acc8[e];
-  __syncthreads();
-  if (tid < GD) {
-    float o = 0.f;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) o += red_s[k][tid];
-    T* op = reinterpret_cast<T*>(p.out) + (size_t)b * p.out_stride_b + (size_t)h * p.out_stride_h;
-    op[tid] = from_f32<T>(o);
-  }
-}
-
-// Slices of the token axis for the two-stage entry on caches that take this path: at least 128 tokens each, at most 64.
-static int generic_split_tokens(const dkv_attn_args* a) {
-  int t = (a->seq_len + 63) / 64;
-  t = (t + GTT - 1) / GTT * GTT;
-  return t < 128 ? 128 : t;
-}
-static int generic_n_split(const dkv_attn_args* a) {
-  const int t = generic_split_tokens(a);
-  const int n = (a->seq_len + t - 1) / t;
-  return n < 1 ? 1 : n;
-}
-size_t generic_split_workspace_bytes(const dkv_attn_args* a) {
-  const int n = generic_n_split(a);
-  if (n <= 1) return 0;
-  return (size_t)a->batch * a->n_q_heads * n * (size_t)(2 + a->rank) * sizeof(float);
-}
-
 int check_attn_args(const dkv_attn_args* a, const char* who, bool need_q, bool need_k, bool need_v) {
   DKV_REQUIRE(a != nullptr, DKV_E_ARG, "%s: null args", who);
   DKV_REQUIRE(a->dtype >= DKV_F32 && a->dtype <= DKV_BF16, DKV_E_ARG, "%s: bad dtype %d", who, a->dtype);
@@ -489,45 +364,27 @@ template <int MODE>
 static int launch_generic(const dkv_attn_args* a, const void* scores, int64_t sb, int64_t sh) {
   if (a->batch == 0) return DKV_OK;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
-  dim3 grid(a->batch, a->n_q_heads, 1);
-  if (MODE == MODE_SCORES) {
-    if (a->seq_len == 0) return DKV_OK;
-    grid.z = (a->seq_len + GZ_TOKENS - 1) / GZ_TOKENS;
-    DKV_REQUIRE(grid.z <= 65535, DKV_E_LIMIT, "dkv_scores: seq_len too large");
-  }
+  const dim3 grid(a->batch, a->n_q_heads);
   const float log_theta = (float)log((double)a->theta);
-  int split_tokens = 0, n_split = 1;
-  if (MODE == MODE_ATTN_SPLIT) {
-    split_tokens = generic_split_tokens(a);
-    n_split = generic_n_split(a);
-    grid.z = n_split;
-  }
   if (a->dtype == DKV_F32)
-    generic_decode_kernel<float, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const float*)scores, sb, sh, log_theta, split_tokens);
+    generic_decode_kernel<float, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const float*)scores, sb, sh, log_theta);
   else if (a->dtype == DKV_F16)
-    generic_decode_kernel<__half, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const __half*)scores, sb, sh, log_theta, split_tokens);
+    generic_decode_kernel<__half, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const __half*)scores, sb, sh, log_theta);
   else
-    generic_decode_kernel<__nv_bfloat16, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const __nv_bfloat16*)scores, sb, sh,
-                                                                        log_theta, split_tokens);
+    generic_decode_kernel<__nv_bfloat16, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const __nv_bfloat16*)scores, sb, sh, log_theta);
   DKV_CHECK_LAUNCH();
-  if (MODE == MODE_ATTN_SPLIT) {
-    const dim3 cgrid(a->batch, a->n_q_heads);
-    if (a->dtype == DKV_F32) generic_combine_kernel<float><<<cgrid, GTHREADS, 0, st>>>(*a, n_split);
-    else if (a->dtype == DKV_F16) generic_combine_kernel<__half><<<cgrid, GTHREADS, 0, st>>>(*a, n_split);
-    else generic_combine_kernel<__nv_bfloat16><<<cgrid, GTHREADS, 0, st>>>(*a, n_split);
-    DKV_CHECK_LAUNCH();
-  }
   return DKV_OK;
 }
 
-int generic_attention(const dkv_attn_args* a) { return launch_generic<MODE_ATTN>(a, nullptr, 0, 0); }
+// implemented in dkv_tiles.cu
+bool tiles_ok(const dkv_attn_args* a, bool with_scores);
+int tiles_scores(const dkv_attn_args* a);
+int tiles_attention(const dkv_attn_args* a);
+int tiles_softmax_v(const dkv_attn_args* a, const void* scores, int64_t sb, int64_t sh);
 
-// Two-stage entry on this path: slices of the token axis + merge when the caller's workspace holds the records,
-// one CTA per (row, head) otherwise.
-int generic_two_stage(const dkv_attn_args* a) {
-  const size_t need = generic_split_workspace_bytes(a);
-  if (need == 0 || a->workspace == nullptr || a->workspace_bytes < need) return generic_attention(a);
-  return launch_generic<MODE_ATTN_SPLIT>(a, nullptr, 0, 0);
+// Both entries on caches that take this path: tile kernels when the caller's workspace holds their scores and records.
+int generic_attention(const dkv_attn_args* a) {
+  return tiles_ok(a, true) ? tiles_attention(a) : launch_generic<MODE_ATTN>(a, nullptr, 0, 0);
 }
 
 }  // namespace dkv
@@ -536,11 +393,12 @@ using namespace dkv;
 
 extern "C" int dkv_scores(const dkv_attn_args* a) {
   if (int rc = check_attn_args(a, "dkv_scores", true, true, false)) return rc;
-  return launch_generic<MODE_SCORES>(a, nullptr, 0, 0);
+  return tiles_scores(a);
 }
 
 extern "C" int dkv_softmax_v(const dkv_attn_args* a, const void* scores, int64_t sc_stride_b, int64_t sc_stride_h) {
   if (int rc = check_attn_args(a, "dkv_softmax_v", false, false, true)) return rc;
   DKV_REQUIRE(scores != nullptr, DKV_E_ARG, "dkv_softmax_v: null scores");
+  if (tiles_ok(a, false)) return tiles_softmax_v(a, scores, sc_stride_b, sc_stride_h);
   return launch_generic<MODE_SOFTMAX_V>(a, scores, sc_stride_b, sc_stride_h);
 }

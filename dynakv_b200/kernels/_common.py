@@ -2,13 +2,12 @@
 from __future__ import annotations
 
 import ctypes as C
-from typing import Dict, Optional, Tuple
+from typing import Dict
 
 import torch
 
 from .. import _lib
 
-_workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 _status: Dict[int, torch.Tensor] = {}
 _n_sm: Dict[int, int] = {}
 
@@ -37,17 +36,6 @@ def read_status(device: torch.device, clear: bool = True) -> int:
     return v
 
 
-def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Grow-only scratch buffer per device, reused by every split-path call on the current stream."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    key = (idx, 0)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
-
-
 def arena_rows(t: torch.Tensor, what: str) -> torch.Tensor:
     """View [B, H, X] as [B*H, X] without copying; 2-D tensors pass through."""
     if t.dim() == 2:
@@ -62,8 +50,10 @@ def arena_rows(t: torch.Tensor, what: str) -> torch.Tensor:
 
 def build_attn_args(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, theta, *, out, seq_lens=None,
                     batch_index=None, k_norm_weight=None, k_norm_eps=1e-6, len_multiple=1, need_workspace=False,
-                    route_min_tokens=0, route_max_tokens=0):
-    """Fill a dkv_attn_args from torch tensors; returns (args, keepalive)."""
+                    route_min_tokens=0, route_max_tokens=0, workspace=None):
+    """Fill a dkv_attn_args from torch tensors; returns (args, keepalive).  With ``need_workspace`` the call's scratch is
+    ``workspace`` when that is large enough (a caller that keeps one must order the calls that share it), else a tensor
+    of its own."""
     lib = _lib.load()
     _lib.require_cuda(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, out)
     dev = out.device
@@ -138,7 +128,9 @@ def build_attn_args(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, theta, *,
     if need_workspace:
         nbytes = lib.dkv_split_workspace_bytes(C.byref(a))
         if nbytes:
-            ws = workspace(dev, nbytes)
+            ws = workspace
+            if ws is None or ws.numel() < nbytes:
+                ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)     # stream-ordered: calls on other streams do not share it
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
             keep.append(ws)
     return a, keep

@@ -214,24 +214,27 @@ class CompressedDecodeLayer:
 
     def attend(self, cache: CustomDynamicCache, q: torch.Tensor, out: torch.Tensor, row_counter: torch.Tensor,
                seq_columns: int, route: str, route_min_tokens: int = 0, route_max_tokens: int = 0,
-               prepare_only: bool = False) -> None:
+               prepare_only: bool = False, workspace: Optional[torch.Tensor] = None) -> int:
         """Attention of all batch rows through one kernel (``route``); with routing bounds the kernel skips the rows
-        whose current length (read from ``row_counter`` on the device) belongs to the other kernel."""
+        whose current length (read from ``row_counter`` on the device) belongs to the other kernel.  ``workspace`` is
+        scratch the caller keeps for calls that follow one another on one stream; the bytes the call needs are returned
+        (``prepare_only``: nothing else happens)."""
         ck, cv = cache.key_cache_sp[self.layer_idx], cache.value_cache_sp[self.layer_idx]
         args, keep = build_attn_args(
             q, ck[0], self.k_up, cv[0], self.v_up, ck[1][:, :seq_columns], ck[2][:, :seq_columns],
             cv[1][:, :seq_columns], cv[2][:, :seq_columns], self.theta, out=out, seq_lens=row_counter,
             k_norm_weight=self.k_norm_weight, k_norm_eps=self.k_norm_eps,
-            len_multiple=cache.len_multiple, need_workspace=(route == "long_two_stage"),
-            route_min_tokens=route_min_tokens, route_max_tokens=route_max_tokens)
+            len_multiple=cache.len_multiple, need_workspace=not prepare_only,
+            route_min_tokens=route_min_tokens, route_max_tokens=route_max_tokens, workspace=workspace)
         lib = _lib.load()
-        if prepare_only:     # only size and allocate what the call needs (workspace, status word)
-            return
+        if prepare_only:
+            return int(lib.dkv_split_workspace_bytes(C.byref(args)))
         if route == "short_fused":
             _lib.check(lib.dkv_fused_decode(C.byref(args)), "dkv_fused_decode")
         else:
             _lib.check(lib.dkv_two_stage_decode(C.byref(args)), "dkv_two_stage_decode")
         del keep
+        return int(args.workspace_bytes)
 
 
 class DecodeGraph:
@@ -272,9 +275,12 @@ class DecodeGraph:
                 _scratch(self.device, 8 * batch * Hkv * 128)
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         status_word(self.device)
-        self._run_layers(prepare_only=True)   # allocate the split workspace before any capture
+        # one scratch for all layers' attention, before any capture: they follow one another
+        self._workspace: Optional[torch.Tensor] = None
+        self._workspace = torch.empty(max(self._run_layers(prepare_only=True), 16), dtype=torch.uint8, device=self.device)
 
-    def _run_layers(self, prepare_only: bool = False) -> None:
+    def _run_layers(self, prepare_only: bool = False) -> int:
+        need = 0
         for li, layer in enumerate(self.layers):
             ck = self.cache.key_cache_sp[layer.layer_idx]
             counter = self.cache.seq_lens(layer.layer_idx)
@@ -285,18 +291,27 @@ class DecodeGraph:
                 layer.append(self.cache, self.new_k[li], self.new_v[li], self.len_k[li], self.len_v[li], counter, cap)
             both = self._has_short and self._has_long
             if self._has_short:
-                layer.attend(self.cache, self.q[li], self.out[li], counter, cap, "short_fused",
-                             route_max_tokens=self._switch if both else 0, prepare_only=prepare_only)
+                need = max(need, layer.attend(self.cache, self.q[li], self.out[li], counter, cap, "short_fused",
+                                              route_max_tokens=self._switch if both else 0, prepare_only=prepare_only,
+                                              workspace=self._workspace))
             if self._has_long:
-                layer.attend(self.cache, self.q[li], self.out[li], counter, cap, "long_two_stage",
-                             route_min_tokens=self._switch if both else 0, prepare_only=prepare_only)
+                need = max(need, layer.attend(self.cache, self.q[li], self.out[li], counter, cap, "long_two_stage",
+                                              route_min_tokens=self._switch if both else 0, prepare_only=prepare_only,
+                                              workspace=self._workspace))
+        return need
 
     def capture(self) -> None:
         """Capture one decode step.  Nothing is executed: the cache is left as it is."""
         torch.cuda.synchronize(self.device)
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):
-            self._run_layers()
+        # not through torch.cuda.graph(): that collects garbage and empties the allocator's cache first (up to 0.3 s with
+        # a few GB cached), and this step allocates nothing
+        with torch.cuda.stream(torch.cuda.Stream(self.device)):
+            g.capture_begin()
+            try:
+                self._run_layers()
+            finally:
+                g.capture_end()
         self.graph = g
 
     def step(self) -> torch.Tensor:

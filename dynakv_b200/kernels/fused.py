@@ -32,8 +32,8 @@ def fused_attention_dispatch(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, 
         out = torch.empty((q3.shape[0], q3.shape[1], q3.shape[2]), dtype=q3.dtype, device=q3.device)
     args, keep = build_attn_args(q3, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, theta, out=out,
                                  seq_lens=seq_lens, batch_index=batch_index, k_norm_weight=k_norm_weight,
-                                 k_norm_eps=k_norm_eps, len_multiple=len_multiple, route_min_tokens=route_min_tokens,
-                                 route_max_tokens=route_max_tokens)
+                                 k_norm_eps=k_norm_eps, len_multiple=len_multiple, need_workspace=True,
+                                 route_min_tokens=route_min_tokens, route_max_tokens=route_max_tokens)
     _lib.check(_lib.load().dkv_fused_decode(C.byref(args)), "dkv_fused_decode")
     del keep
     return out

@@ -79,7 +79,8 @@ def avx(a: torch.Tensor, x_flat: torch.Tensor, v_up: torch.Tensor, l_vec: torch.
         a = a.contiguous()
     batch, heads, _ = a.shape
     out = torch.empty((batch, heads, v_up.shape[-1]), dtype=a.dtype, device=a.device)
-    args, keep = build_attn_args(None, None, None, x_flat, v_up, None, None, l_vec, offsets, 10000.0, out=out)
+    args, keep = build_attn_args(None, None, None, x_flat, v_up, None, None, l_vec, offsets, 10000.0, out=out,
+                                 need_workspace=True)
     _lib.check(_lib.load().dkv_softmax_v(C.byref(args), a.data_ptr(), a.stride(0), a.stride(1)), "dkv_softmax_v")
     del keep
     return out

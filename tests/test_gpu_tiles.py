@@ -1,0 +1,75 @@
+"""Tile kernels (any layout with a workspace): tile and slice edges, odd ranks, one and many heads per group or arena,
+rows that start at any element, bases that are not 16-byte aligned."""
+import pytest
+import torch
+
+from dynakv_b200.kernels import _common
+from dynakv_b200.kernels.fused import fused_attention_dispatch
+from dynakv_b200.kernels.two_stage import abx_sparse, avx, two_stage_attention
+from oracle import dynakv_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(seed, B, S, R, Hq, groups, arenas, dtype):
+    gen = torch.Generator().manual_seed(seed)
+    t = {"q": torch.randn(B, Hq, 128, generator=gen).to(dtype)}
+    for side in "kv":
+        lens = torch.randint(0, R + 1, (B * arenas, S), generator=gen, dtype=torch.int32)
+        lens[:, 0].clamp_(min=1)
+        offs = (torch.cumsum(lens.long(), 1) - lens.long()).to(torch.int32)
+        cap = int(lens.long().sum(1).max()) + 3
+        sigma = torch.exp(-torch.arange(R, dtype=torch.float32) / max(R / 4, 1))
+        t["flat_" + side] = (torch.randn(B * arenas, cap, generator=gen) * sigma[torch.arange(cap) % R]).to(dtype)
+        t["lens_" + side], t["offs_" + side] = lens, offs
+        t[side + "_up"] = (torch.randn(groups, R, 128, generator=gen) / R ** 0.5).to(dtype)
+    return t
+
+
+def _dev(t, shift):
+    d = {k: v.cuda() for k, v in t.items()}
+    if shift:       # bases that start two bytes past a 16-byte boundary
+        for k in ("k_up", "v_up"):
+            buf = torch.empty(d[k].numel() + 1, dtype=d[k].dtype, device="cuda")
+            buf[1:].copy_(d[k].view(-1))
+            d[k] = buf[1:].view(d[k].shape)
+    return d
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("B,S,R,Hq,groups,arenas,shift", [
+    (1, 1, 8, 4, 1, 1, 0), (2, 127, 63, 8, 2, 2, 0), (1, 129, 64, 12, 1, 1, 1), (3, 33, 819, 32, 8, 1, 0), (1, 300, 1024, 40, 40, 1, 0),
+    (1, 130, 513, 36, 4, 1, 1)])
+def test_tile_kernels_against_oracle(B, S, R, Hq, groups, arenas, shift, dtype):
+    t = _case(S + R, B, S, R, Hq, groups, arenas, dtype)
+    d = _dev(t, shift)
+    knw = 1.0 + 0.1 * torch.randn(128, generator=torch.Generator().manual_seed(1)) if S == 33 else None
+    ref = O.compact_attention(*(t[k] for k in ("q", "flat_k", "k_up", "flat_v", "v_up", "lens_k", "offs_k", "lens_v", "offs_v")), 10000.0,
+                              k_norm_weight=knw)
+    args = [d[k] for k in ("q", "flat_k", "k_up", "flat_v", "v_up", "lens_k", "offs_k", "lens_v", "offs_v")]
+    kw = {} if knw is None else dict(k_norm_weight=knw.cuda())
+    tol = 1e-4 if dtype == torch.float32 else 2e-2
+    for fn in (fused_attention_dispatch, two_stage_attention):
+        out = fn(*args, 10000.0, **kw).float().cpu()
+        assert float((out - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
+    if knw is None:
+        # the stage operators chained: scores in the query type, then the softmax over them
+        sc = abx_sparse(d["q"], d["k_up"], d["flat_k"], d["lens_k"], offsets=d["offs_k"], theta=10000.0)
+        out = avx(sc, d["flat_v"], d["v_up"], d["lens_v"], d["offs_v"]).float().cpu()
+        loose = tol if dtype == torch.float32 else 4e-2
+        assert float((out - ref).abs().max()) <= loose * max(1.0, float(ref.abs().max()))
+    assert _common.read_status(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+def test_ragged_rows_over_several_slices(dtype):
+    # 9000 tokens: 64 slices of more than one tile, a short row whose other slices are empty, an empty row
+    t = _case(5, 3, 9000, 24, 8, 2, 1, dtype)
+    d = _dev(t, 0)
+    seq = [9000, 150, 0]
+    ref = O.compact_attention(*(t[k] for k in ("q", "flat_k", "k_up", "flat_v", "v_up", "lens_k", "offs_k", "lens_v", "offs_v")), 500000.0,
+                              seq_lens=seq)
+    args = [d[k] for k in ("q", "flat_k", "k_up", "flat_v", "v_up", "lens_k", "offs_k", "lens_v", "offs_v")]
+    out = two_stage_attention(*args, 500000.0, seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda")).float().cpu()
+    assert float((out - torch.nan_to_num(ref)).abs().max()) <= (2e-4 if dtype == torch.float32 else 2e-2)
+    assert _common.read_status(torch.device("cuda")) == 4       # the empty row is reported
