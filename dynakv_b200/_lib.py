@@ -95,6 +95,23 @@ class GateArgs(C.Structure):
 
 
 _lib: Optional[C.CDLL] = None
+_host = None
+HOST_PATH = os.path.join(_HERE, "_host.so")
+
+
+def host():
+    """The native host side (argument marshalling of the hot entry points); raises, like ``load``, when it is missing."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m dynakv_b200.build`")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("_host", HOST_PATH)
+        _host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_host)
+    return _host
+
 
 
 def load() -> C.CDLL:

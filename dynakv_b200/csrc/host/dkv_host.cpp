@@ -1,0 +1,313 @@
+// Native host side of the Python entry points: turns torch tensors into the C ABI's argument structs and launches.
+//
+// A decode step is two short kernels per layer; marshalling them through ctypes costs 25-45 us of Python per call, more
+// than the kernels take on small caches.  The functions here do the same work in 3-5 us.  Each of them handles the plain
+// case -- CUDA tensors of the documented shapes, types and layouts -- and returns None for anything else, without having
+// launched or changed anything; the Python callers then take their own path, which copies what has to be copied and
+// raises what has to be raised.  No state is kept between calls but the address of each device's status word.
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/ops/empty.h>
+#include <ATen/ops/empty_like.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/Exceptions.h>
+
+#include "../../../include/dynakv_b200.h"
+
+namespace {
+
+constexpr int MAX_DEVICES = 64;
+int32_t* g_status[MAX_DEVICES];
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return DKV_F32;
+    case at::kHalf: return DKV_F16;
+    case at::kBFloat16: return DKV_BF16;
+    default: return -1;
+  }
+}
+
+bool is_tensor(PyObject* o) { return THPVariable_Check(o); }
+const at::Tensor& unpack(PyObject* o) { return THPVariable_Unpack(o); }
+// a plain CUDA tensor on `dev` (no subclass that wants to see the call, no gradient to record)
+bool plain(PyObject* o, int dev) {
+  if (!THPVariable_CheckExact(o)) return false;
+  const at::Tensor& t = unpack(o);
+  return t.is_cuda() && t.get_device() == dev && !t.requires_grad();
+}
+void* stream_of(int dev) { return at::cuda::getCurrentCUDAStream(dev).stream(); }
+
+// [rows, X] or [B, H, X] whose first two axes fold into one without a copy
+bool fold(const at::Tensor& t, int64_t& rows, int64_t& cols, int64_t& stride_r, int64_t& stride_c) {
+  if (t.dim() == 2) {
+    rows = t.size(0); cols = t.size(1); stride_r = t.stride(0); stride_c = t.stride(1);
+    return true;
+  }
+  if (t.dim() != 3 || (t.size(0) > 1 && t.stride(0) != t.size(1) * t.stride(1))) return false;
+  rows = t.size(0) * t.size(1); cols = t.size(2); stride_r = t.stride(1); stride_c = t.stride(2);
+  return true;
+}
+
+bool fill_side(dkv_side& s, const at::Tensor& flat, const at::Tensor& lens, const at::Tensor& offs, int64_t& rows, int64_t& tokens) {
+  int64_t fr, fc, fs, fe, or_, oc, os, oe, ls, le;
+  if (!fold(flat, fr, fc, fs, fe) || !fold(lens, rows, tokens, ls, le) || !fold(offs, or_, oc, os, oe)) return false;
+  if (fe != 1 || fr != rows || or_ != rows || oc != tokens || lens.scalar_type() != at::kInt || offs.scalar_type() != at::kInt) return false;
+  s.flat = flat.data_ptr();
+  s.flat_stride = fs;
+  s.lens = static_cast<int32_t*>(lens.data_ptr());
+  s.lens_stride_a = ls;
+  s.lens_stride_s = tokens > 1 ? le : 1;
+  s.offs = static_cast<int32_t*>(offs.data_ptr());
+  s.offs_stride_a = os;
+  s.offs_stride_s = tokens > 1 ? oe : 1;
+  s.ptr = nullptr;
+  return true;
+}
+
+PyObject* fail(const char* what, int rc) {
+  PyErr_Format(PyExc_RuntimeError, "%s failed (code %d): %s", what, rc, dkv_last_error());
+  return nullptr;
+}
+
+// attend(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, theta, out|None, seq_lens|None, batch_index|None,
+//        k_norm_weight|None, k_norm_eps, len_multiple, route_min, route_max, two_stage) -> out
+PyObject* attend(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 19 || !is_tensor(v[0]) || !unpack(v[0]).is_cuda()) Py_RETURN_NONE;
+  const int dev = unpack(v[0]).get_device();
+  if (dev < 0 || dev >= MAX_DEVICES || g_status[dev] == nullptr) Py_RETURN_NONE;
+  for (int i = 0; i < 9; ++i)
+    if (!plain(v[i], dev)) Py_RETURN_NONE;
+  for (int i = 10; i < 14; ++i)
+    if (v[i] != Py_None && !plain(v[i], dev)) Py_RETURN_NONE;
+  const at::Tensor &q = unpack(v[0]), &k_up = unpack(v[2]), &v_up = unpack(v[4]), &k_flat = unpack(v[1]), &v_flat = unpack(v[3]);
+  const auto dt = q.scalar_type();
+  dkv_attn_args a = {};
+  a.dtype = dtype_code(dt);
+  const bool q4 = q.dim() == 4;
+  if (a.dtype < 0 || !(q.dim() == 3 || (q4 && q.size(2) == 1)) || q.stride(-1) != 1) Py_RETURN_NONE;
+  if (k_up.dim() != 3 || v_up.sizes() != k_up.sizes() || !k_up.is_contiguous() || !v_up.is_contiguous()) Py_RETURN_NONE;
+  if (k_flat.scalar_type() != dt || v_flat.scalar_type() != dt || k_up.scalar_type() != dt || v_up.scalar_type() != dt) Py_RETURN_NONE;
+  const int64_t B = q.size(0), Hq = q.size(1), D = q.size(q4 ? 3 : 2);
+  if (B == 0 || k_up.size(2) != D) Py_RETURN_NONE;
+  int64_t rows_k, rows_v, S_k, S_v;
+  if (!fill_side(a.k, k_flat, unpack(v[5]), unpack(v[6]), rows_k, S_k) || !fill_side(a.v, v_flat, unpack(v[7]), unpack(v[8]), rows_v, S_v)) Py_RETURN_NONE;
+  if (rows_k != rows_v || S_k != S_v || rows_k % B != 0) Py_RETURN_NONE;
+  a.n_q_heads = (int32_t)Hq;
+  a.n_basis_groups = (int32_t)k_up.size(0);
+  a.head_dim = (int32_t)D;
+  a.rank = (int32_t)k_up.size(1);
+  a.arenas_per_batch = (int32_t)(rows_k / B);
+  a.seq_len = (int32_t)S_k;
+  a.q = q.data_ptr();
+  a.q_stride_b = q.stride(0);
+  a.q_stride_h = q.stride(1);
+  a.k_up = k_up.data_ptr();
+  a.v_up = v_up.data_ptr();
+  a.theta = (float)PyFloat_AsDouble(v[9]);
+  a.batch = (int32_t)B;
+  if (v[11] != Py_None) {
+    const at::Tensor& t = unpack(v[11]);
+    if (t.scalar_type() != at::kInt || t.numel() != B || !t.is_contiguous()) Py_RETURN_NONE;
+    a.seq_lens = static_cast<const int32_t*>(t.data_ptr());
+  }
+  if (v[12] != Py_None) {
+    const at::Tensor& t = unpack(v[12]);
+    if (t.scalar_type() != at::kInt || !t.is_contiguous()) Py_RETURN_NONE;
+    a.batch_index = static_cast<const int32_t*>(t.data_ptr());
+    a.batch = (int32_t)t.numel();
+  }
+  if (v[13] != Py_None) {
+    const at::Tensor& t = unpack(v[13]);
+    if (t.scalar_type() != at::kFloat || !t.is_contiguous()) Py_RETURN_NONE;
+    a.k_norm_weight = static_cast<const float*>(t.data_ptr());
+  }
+  a.k_norm_eps = (float)PyFloat_AsDouble(v[14]);
+  a.len_multiple = (int32_t)PyLong_AsLong(v[15]);
+  a.route_min_tokens = (int32_t)PyLong_AsLong(v[16]);
+  a.route_max_tokens = (int32_t)PyLong_AsLong(v[17]);
+  if (PyErr_Occurred()) return nullptr;
+  if ((a.route_min_tokens || a.route_max_tokens) && a.seq_lens == nullptr) Py_RETURN_NONE;
+  a.status = g_status[dev];
+  a.stream = stream_of(dev);
+  at::Tensor out;
+  if (v[10] != Py_None) {
+    out = unpack(v[10]);
+    if (out.scalar_type() != dt || out.dim() != 3 || out.stride(2) != 1) Py_RETURN_NONE;
+  } else {
+    out = at::empty({B, Hq, D}, q.options());
+  }
+  a.out = out.data_ptr();
+  a.out_stride_b = out.stride(0);
+  a.out_stride_h = out.stride(1);
+  const size_t need = dkv_split_workspace_bytes(&a);
+  at::Tensor ws;
+  if (need) {
+    ws = at::empty({(int64_t)need}, q.options().dtype(at::kByte));
+    a.workspace = ws.data_ptr();
+    a.workspace_bytes = need;
+  }
+  const bool two_stage = v[18] == Py_True;
+  const int rc = two_stage ? dkv_two_stage_decode(&a) : dkv_fused_decode(&a);
+  if (rc) return fail(two_stage ? "dkv_two_stage_decode" : "dkv_fused_decode", rc);
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+long long_max(PyObject* list) {
+  long m = 0;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) m = std::max(m, PyLong_AsLong(PyList_GET_ITEM(list, i)));
+  return m;
+}
+
+// append_token(k_state, v_state, key_states, key_len, value_states, value_len, arenas, width, len_multiple, row_counter|None)
+//   -> (flat_k, flat_v, lens_k, lens_v, offs_k, offs_v) and the states advanced by one token, or None (nothing done) when
+//   a buffer may have to grow
+PyObject* append_token(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 10 || !PyList_Check(v[0]) || !PyList_Check(v[1]) || !is_tensor(v[2]) || !unpack(v[2]).is_cuda()) Py_RETURN_NONE;
+  const int dev = unpack(v[2]).get_device();
+  if (dev < 0 || dev >= MAX_DEVICES || g_status[dev] == nullptr) Py_RETURN_NONE;
+  for (int i = 2; i < 6; ++i)
+    if (!plain(v[i], dev)) Py_RETURN_NONE;
+  const at::Tensor &ks = unpack(v[2]), &kl = unpack(v[3]), &vs = unpack(v[4]), &vl = unpack(v[5]);
+  const long A = PyLong_AsLong(v[6]), width = PyLong_AsLong(v[7]), mult = PyLong_AsLong(v[8]);
+  if (PyErr_Occurred()) return nullptr;
+  if (ks.dim() != 3 || ks.size(1) != 1 || ks.size(2) % A != 0 || vs.sizes() != ks.sizes() || !ks.is_contiguous() || !vs.is_contiguous()) Py_RETURN_NONE;
+  const int64_t B = ks.size(0), rows = B * A;
+  for (const at::Tensor* t : {&kl, &vl})
+    if (t->scalar_type() != at::kInt || t->numel() != rows || !t->is_contiguous() || !(t->dim() == 2 || t->dim() == 3)) Py_RETURN_NONE;
+  dkv_append_args a = {};
+  a.dtype = dtype_code(ks.scalar_type());
+  if (a.dtype < 0 || vs.scalar_type() != ks.scalar_type()) Py_RETURN_NONE;
+  at::Tensor view[2][3];
+  int64_t pos = 0;
+  PyObject* bounds[2];
+  for (int sd = 0; sd < 2; ++sd) {
+    PyObject* st = v[sd];
+    if (PyList_GET_SIZE(st) != 6) Py_RETURN_NONE;
+    for (int i = 0; i < 4; ++i)
+      if (!plain(PyList_GET_ITEM(st, i), dev)) Py_RETURN_NONE;
+    const at::Tensor &flat = unpack(PyList_GET_ITEM(st, 0)), &lens = unpack(PyList_GET_ITEM(st, 1)), &offs = unpack(PyList_GET_ITEM(st, 2)),
+                     &ptr = unpack(PyList_GET_ITEM(st, 3));
+    bounds[sd] = PyList_GET_ITEM(st, 5);
+    if (!PyLong_Check(PyList_GET_ITEM(st, 4)) || !PyList_Check(bounds[sd])) Py_RETURN_NONE;
+    const int64_t seq = PyLong_AsLong(PyList_GET_ITEM(st, 4));
+    if (sd == 0) pos = seq;
+    dkv_side& s = sd ? a.v : a.k;
+    int64_t r, cap;
+    if (flat.scalar_type() != ks.scalar_type() || !fill_side(s, flat, lens, offs, r, cap) || r != rows || ptr.scalar_type() != at::kInt ||
+        ptr.numel() != rows || !ptr.is_contiguous() || seq != pos || seq + 1 > cap || long_max(bounds[sd]) + width > flat.size(1))
+      Py_RETURN_NONE;
+    s.ptr = static_cast<int32_t*>(ptr.data_ptr());
+    a.seq_capacity = (int32_t)(sd ? std::min<int64_t>(a.seq_capacity, cap) : cap);
+    view[sd][0] = flat;
+    view[sd][1] = lens.narrow(1, 0, seq + 1);
+    view[sd][2] = offs.narrow(1, 0, seq + 1);
+  }
+  if (v[9] != Py_None) {
+    if (!plain(v[9], dev)) Py_RETURN_NONE;
+    const at::Tensor& t = unpack(v[9]);
+    if (t.scalar_type() != at::kInt || t.numel() != B || !t.is_contiguous()) Py_RETURN_NONE;
+    a.seq_lens = static_cast<int32_t*>(t.data_ptr());
+  }
+  a.batch = (int32_t)B;
+  a.arenas_per_batch = (int32_t)A;
+  a.max_dim = (int32_t)(ks.size(2) / A);
+  a.new_k = ks.data_ptr();
+  a.new_v = vs.data_ptr();
+  a.len_k = static_cast<const int32_t*>(kl.data_ptr());
+  a.len_v = static_cast<const int32_t*>(vl.data_ptr());
+  a.seq_pos = (int32_t)pos;
+  a.len_multiple = (int32_t)mult;
+  a.status = g_status[dev];
+  a.stream = stream_of(dev);
+  if (int rc = dkv_append_decode(&a)) return fail("dkv_append_decode", rc);
+  for (int sd = 0; sd < 2; ++sd) {
+    PyList_SetItem(v[sd], 4, PyLong_FromLongLong(pos + 1));
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(bounds[sd]); ++i)
+      PyList_SetItem(bounds[sd], i, PyLong_FromLong(PyLong_AsLong(PyList_GET_ITEM(bounds[sd], i)) + width));
+  }
+  PyObject* r = PyTuple_New(6);
+  for (int i = 0; i < 3; ++i)
+    for (int sd = 0; sd < 2; ++sd) PyTuple_SET_ITEM(r, 2 * i + sd, THPVariable_Wrap(view[sd][i]));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// gate(states, weight, bias, low_rank, threshold, return_masked, len_multiple, native_rounding) -> (masked|None, lengths)
+PyObject* gate(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 8 || !is_tensor(v[0]) || !unpack(v[0]).is_cuda()) Py_RETURN_NONE;
+  const int dev = unpack(v[0]).get_device();
+  for (int i = 0; i < 3; ++i)
+    if (!plain(v[i], dev)) Py_RETURN_NONE;
+  const at::Tensor &x = unpack(v[0]), &w = unpack(v[1]), &b = unpack(v[2]);
+  const auto dt = x.scalar_type();
+  dkv_gate_args a = {};
+  a.dtype = dtype_code(dt);
+  if (a.dtype < 0 || x.dim() < 1 || !x.is_contiguous() || !w.is_contiguous() || !b.is_contiguous() || w.scalar_type() != dt || b.scalar_type() != dt) Py_RETURN_NONE;
+  const int64_t d = x.size(-1);
+  if (d == 0 || w.dim() != 2 || w.size(0) != d || w.size(1) != d || b.numel() != d) Py_RETURN_NONE;
+  a.n_rows = (int32_t)(x.numel() / d);
+  a.dim = (int32_t)d;
+  a.low_rank = (int32_t)PyLong_AsLong(v[3]);
+  a.threshold = (float)PyFloat_AsDouble(v[4]);
+  const bool want = v[5] == Py_True;
+  a.len_multiple = (int32_t)PyLong_AsLong(v[6]);
+  a.native_rounding = v[7] == Py_True ? 1 : 0;
+  if (PyErr_Occurred()) return nullptr;
+  a.x = x.data_ptr();
+  a.x_stride = d;
+  a.w = w.data_ptr();
+  a.b = b.data_ptr();
+  at::Tensor lengths = at::empty(x.sizes().slice(0, x.dim() - 1), x.options().dtype(at::kInt)), masked;
+  a.lengths = static_cast<int32_t*>(lengths.data_ptr());
+  if (want) {
+    masked = at::empty(x.sizes(), x.options());
+    a.masked = masked.data_ptr();
+    a.masked_stride = d;
+  }
+  const size_t need = std::max<size_t>(dkv_gate_workspace_bytes(&a), 16);
+  at::Tensor ws = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
+  a.workspace = ws.data_ptr();
+  a.workspace_bytes = need;
+  a.stream = stream_of(dev);
+  if (int rc = dkv_gate_lengths(&a)) return fail("dkv_gate_lengths", rc);
+  PyObject* r = PyTuple_New(2);
+  if (want) {
+    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(masked));
+  } else {
+    Py_INCREF(Py_None);
+    PyTuple_SET_ITEM(r, 0, Py_None);
+  }
+  PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(lengths));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// set_status(device index, address): where kernels on that device report their DKV_ST_* conditions
+PyObject* set_status_word(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  if (n != 2) {
+    PyErr_SetString(PyExc_TypeError, "set_status(device, address)");
+    return nullptr;
+  }
+  const long dev = PyLong_AsLong(v[0]);
+  void* p = PyLong_AsVoidPtr(v[1]);
+  if (PyErr_Occurred()) return nullptr;
+  if (dev >= 0 && dev < MAX_DEVICES) g_status[dev] = static_cast<int32_t*>(p);
+  Py_RETURN_NONE;
+}
+
+#define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)), METH_FASTCALL
+PyMethodDef methods[] = {{"attend", FAST(attend), "decode attention"},
+                         {"append_token", FAST(append_token), "decode append"},
+                         {"gate", FAST(gate), "cutoff gate of one side"},
+                         {"set_status", FAST(set_status_word), "status word of a device"},
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host side of dynakv_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }

@@ -24,6 +24,7 @@ def status_word(device: torch.device) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     if idx not in _status:
         _status[idx] = torch.zeros(1, dtype=torch.int32, device=device)
+        _lib.host().set_status(idx, _status[idx].data_ptr())
     return _status[idx]
 
 

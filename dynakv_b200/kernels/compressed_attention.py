@@ -80,6 +80,10 @@ def gate_lengths(states: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
     """
     if not states.is_cuda:
         raise RuntimeError("dynakv_b200 has no CPU path: the gate needs CUDA tensors")
+    if out_lengths is None:
+        done = _lib.host().gate(states, weight, bias, low_rank, threshold, return_masked, len_multiple, bool(native_rounding))
+        if done is not None:        # else: tensors that have to be copied first, or refused
+            return done
     d = states.shape[-1]
     if weight.shape != (d, d) or bias.numel() != d:
         raise ValueError(f"gate weight must be [{d}, {d}] and bias [{d}], got {tuple(weight.shape)} and {tuple(bias.shape)}")

@@ -203,9 +203,19 @@ class CustomDynamicCache:
         are stored.  Returns ``(flat_k, flat_v, lens_k, lens_v, offs_k, offs_v)`` with the metadata
         sliced to the tokens stored, exactly as the reference's ``update_sp``.
         """
+        A = self.arenas_per_batch
+        if token_counts is None and isinstance(tensor_d, int) and layer_idx < len(self.key_cache_sp) and key_states.shape[1] == 1 \
+                and self.key_cache_sp[layer_idx] is not None:
+            counter = self.seq_lens(layer_idx)
+            views = _lib.host().append_token(self.key_cache_sp[layer_idx], self.value_cache_sp[layer_idx], key_states, key_len,
+                                             value_states, value_len, A, min(tensor_d, key_states.shape[2] // A), self.len_multiple,
+                                             counter)
+            if views is not None:       # else: a buffer has to grow, or tensors have to be copied first
+                if counter is not None:
+                    self._seq_lens_host[layer_idx] = [n + 1 for n in self._seq_lens_host[layer_idx]]
+                return views
         lib = _lib.load()
         _lib.require_cuda(key_states, value_states, key_len, value_len)
-        A = self.arenas_per_batch
         B, n_new = key_states.shape[0], key_states.shape[1]
         is_decode = n_new == 1
         row_dim = key_states.shape[2] // A
