@@ -959,10 +959,15 @@ __global__ void __launch_bounds__(512) split_combine_kernel(dkv_attn_args p) {
   // units [u_lo, u_hi) each left one partial record at entry (row + k).
   int k_lo = 0, k_hi = -1;
   if (u_hi > u_lo && total_units > 0) {
+    // first CTA that ends past u_lo, first that begins at or past u_hi: two divisions and a step or two (a division per
+    // record was a third of this kernel's time on small batches)
     k_lo = (int)(((long long)u_lo * n_cta) / total_units);
-    while (k_lo > 0 && unit_begin(k_lo, n_cta, total_units) > u_lo) --k_lo;
-    k_hi = min(n_cta - 1, (int)(((long long)u_hi * n_cta + total_units - 1) / total_units));
+    while (unit_begin(k_lo + 1, n_cta, total_units) <= u_lo) ++k_lo;
+    k_hi = min(n_cta - 1, (int)(((long long)u_hi * n_cta) / total_units));
+    while (unit_begin(k_hi, n_cta, total_units) >= u_hi) --k_hi;
   }
+  // with at least one unit per CTA every CTA of the range has a record; with fewer units some have none
+  const bool dense = total_units >= n_cta;
   const float* rec0 = ws + (((size_t)g * entries_per_group + (size_t)i) * HP + h) * PART_STRIDE;
   const size_t rec_step = (size_t)HP * PART_STRIDE;   // record k sits at rec0 + k * rec_step
   float M = -INFINITY, L = 0.f, v = 0.f;
@@ -974,8 +979,7 @@ __global__ void __launch_bounds__(512) split_combine_kernel(dkv_attn_args p) {
         const int k = base + j;
         m[j] = -INFINITY; l[j] = 0.f; x[j] = 0.f;
         if (k <= k_hi) {
-          const int ub = unit_begin(k, n_cta, total_units), ue = unit_begin(k + 1, n_cta, total_units);
-          if (ue > ub && ub < u_hi && ue > u_lo) {
+          if (dense || unit_begin(k + 1, n_cta, total_units) > unit_begin(k, n_cta, total_units)) {
             const float* rec = rec0 + (size_t)k * rec_step;
             m[j] = __ldcg(rec); l[j] = __ldcg(rec + 1); x[j] = __ldcg(rec + 2 + r);
           }

@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
   const int t_end = sink.ws ? row_len(p, b) : p.seq_len;     // the operator writes every column
   if (t0 >= t_end) return;
   const int a = b * A + (g * G * A) / Hq;
+  pdl_launch_dependents();      // the latent-sum kernel may set itself up meanwhile
   if (tid == 0) {
     sm.rmax = 0;
     for (int s = 0; s < TS_STAGES; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ts_smem(&sm.done[s])));
@@ -398,10 +399,12 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
   const int rb = blockIdx.y % r_blocks, head0 = j * HA + (blockIdx.y / r_blocks) * NH, nh = min(NH, (j + 1) * HA - head0);
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
   if (row_routed_out(p, b)) return;
+  pdl_launch_dependents();
   const int S = row_len(p, b), t0 = sl * slice, t1 = min(S, t0 + slice);
   float* my_rec = rec + (((size_t)i_row * Hq + head0) * n_split + sl) * (size_t)(2 + R);     // + h * n_split * (2 + R)
   const size_t rec_h = (size_t)n_split * (2 + R);
   if (t0 >= t1) {
+    pdl_wait();
     if (rb == 0 && tid < nh) { my_rec[tid * rec_h] = -INFINITY; my_rec[tid * rec_h + 1] = 0.f; }
     return;
   }
@@ -417,6 +420,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
   }
   if (tid < NH) sm.l[tid] = 0.f;
   for (int e = tid; e < 2 * TS_TOK * NH; e += TS_THREADS) reinterpret_cast<uint32_t*>(sm.pt)[e] = 0u;     // columns of heads that are not there
+  pdl_wait();        // the scores (and, in a chain of layers, the workspace) are the kernel's before this one
   slice_maxima(src, i_row, b, Hq, head0, nh, t0, t1, sm.m);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -537,6 +541,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   const int t_end = sink.ws ? row_len(p, b) : p.seq_len;
   if (t0 >= t_end) return;
   const int a = b * A + (g * G * A) / Hq;
+  pdl_launch_dependents();
   if (warp == 0) {
     int len = 0, off = 0;
     if (lane < TF_TOK) {
@@ -559,7 +564,6 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   for (int r0 = 0; r0 < rmax; r0 += TS_CHUNK) {
-    float bv[TS_CHUNK / 8][8];
     const int nr = min(TS_CHUNK, rmax - r0);
     for (int e = tid; e < TS_CHUNK * TF_TOK; e += TS_THREADS) {
       const int t = e >> 6, r = e & 63;
@@ -568,14 +572,14 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
     __syncthreads();
 #pragma unroll 1
     for (int rr = 0; rr < nr; rr += 16) {
+      float w[16];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) bv[u >> 3][u & 7] = r0 + rr + u < R ? __ldg(kup + (size_t)(r0 + rr + u) * TD + d) : 0.f;
+      for (int u = 0; u < 16; ++u) w[u] = r0 + rr + u < rmax ? __ldg(kup + (size_t)(r0 + rr + u) * TD + d) : 0.f;
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const float4 x0 = *reinterpret_cast<const float4*>(&x_s[rr + u][8 * th]), x1 = *reinterpret_cast<const float4*>(&x_s[rr + u][8 * th + 4]);
-        const float w = bv[u >> 3][u & 7];
-        acc[0] = fmaf(x0.x, w, acc[0]); acc[1] = fmaf(x0.y, w, acc[1]); acc[2] = fmaf(x0.z, w, acc[2]); acc[3] = fmaf(x0.w, w, acc[3]);
-        acc[4] = fmaf(x1.x, w, acc[4]); acc[5] = fmaf(x1.y, w, acc[5]); acc[6] = fmaf(x1.z, w, acc[6]); acc[7] = fmaf(x1.w, w, acc[7]);
+        acc[0] = fmaf(x0.x, w[u], acc[0]); acc[1] = fmaf(x0.y, w[u], acc[1]); acc[2] = fmaf(x0.z, w[u], acc[2]); acc[3] = fmaf(x0.w, w[u], acc[3]);
+        acc[4] = fmaf(x1.x, w[u], acc[4]); acc[5] = fmaf(x1.y, w[u], acc[5]); acc[6] = fmaf(x1.z, w[u], acc[6]); acc[7] = fmaf(x1.w, w[u], acc[7]);
       }
     }
     __syncthreads();
@@ -633,15 +637,18 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_f32_kernel(dkv_attn_args p
   const int rb = blockIdx.y % r_blocks, head0 = j * HA + (blockIdx.y / r_blocks) * NH, nh = min(NH, (j + 1) * HA - head0);
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
   if (row_routed_out(p, b)) return;
+  pdl_launch_dependents();
   const int S = row_len(p, b), t0 = sl * slice, t1 = min(S, t0 + slice);
   float* my_rec = rec + (((size_t)i_row * Hq + head0) * n_split + sl) * (size_t)(2 + R);
   const size_t rec_h = (size_t)n_split * (2 + R);
   if (t0 >= t1) {
+    pdl_wait();
     if (rb == 0 && tid < nh) { my_rec[tid * rec_h] = -INFINITY; my_rec[tid * rec_h + 1] = 0.f; }
     return;
   }
   const int a = b * A + j;
   if (tid < NH) l_s[tid] = 0.f;
+  pdl_wait();
   slice_maxima(src, i_row, b, Hq, head0, nh, t0, t1, m_s);
   const float* flat = reinterpret_cast<const float*>(p.v.flat) + (size_t)a * p.v.flat_stride;
   const int r = 128 * rb + (tid & 127), half = tid >> 7;
@@ -709,6 +716,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_combine_kernel(dkv_attn_args 
   if (row_routed_out(p, b)) return;      // (uniform over the cluster)
   if (RS > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");     // the others' shared memory is there once they have started
   const int g = h / (Hq / p.n_basis_groups);
+  pdl_wait();
   const float* rec0 = rec + (((size_t)blockIdx.x * Hq + h) * n_split) * (size_t)(2 + R);
   if (tid < 32) {
     float M = -INFINITY;
@@ -841,11 +849,11 @@ int launch_pv(const dkv_attn_args* a, const ScoreSource<T>& src, float* rec) {
   DKV_REQUIRE(ctas <= 2147483647LL && (long long)r_blocks * ((heads + NH - 1) / NH) <= 65535, DKV_E_LIMIT, "too many rows or heads");
   const dim3 grid((unsigned)ctas, r_blocks * ((heads + NH - 1) / NH));
   if constexpr (std::is_same<T, float>::value) {
-    tile_pv_f32_kernel<NH><<<grid, TS_THREADS, 0, st>>>(*a, src, rec, slice_tokens(a), n_split, r_blocks);
+    launch_pdl(tile_pv_f32_kernel<NH>, grid, dim3(TS_THREADS), 0, st, *a, src, rec, slice_tokens(a), n_split, r_blocks);
   } else {
     const int smem = (int)sizeof(PvSmem<NH>) + 128;
     if (int rc = opt_in(tile_pv_kernel<T, NH>, smem)) return rc;
-    tile_pv_kernel<T, NH><<<grid, TS_THREADS, smem, st>>>(*a, src, rec, slice_tokens(a), n_split, r_blocks);
+    launch_pdl(tile_pv_kernel<T, NH>, grid, dim3(TS_THREADS), smem, st, *a, src, rec, slice_tokens(a), n_split, r_blocks);
   }
   DKV_CHECK_LAUNCH();
   return DKV_OK;
@@ -858,12 +866,14 @@ int launch_merge(const dkv_attn_args* a, const float* rec) {
   cfg.gridDim = dim3(a->batch, a->n_q_heads, rs);
   cfg.blockDim = dim3(TS_THREADS);
   cfg.stream = reinterpret_cast<cudaStream_t>(a->stream);
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = rs;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = rs;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = rs > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, tile_combine_kernel<T, OPERATOR>, *a, rec, n_slices(a));
   DKV_REQUIRE(e == cudaSuccess, DKV_E_CUDA, "launch of the merge kernel failed: %s", cudaGetErrorString(e));
   DKV_CHECK_LAUNCH();
@@ -899,7 +909,13 @@ size_t tiles_workspace_bytes(const dkv_attn_args* a) {
   if (a->batch <= 0 || a->seq_len <= 0) return 0;
   return score_bytes(a) + record_bytes(a);
 }
+// Whether a call takes the tile kernels: it has the workspace, and is not one of the small calls where three kernels cost
+// more than one -- a single 32-token tile of the one-kernel path, CTAs enough for every (row, head) at once (measured,
+// bf16: 8.7-13 us against 18-22 at up to 32 tokens, 19-20 against 18-23 at 48; B * Hq = 1024: 42-51 against 28), and for
+// fp32 a rank up to 256 (1024: 57 against 41).
 bool tiles_ok(const dkv_attn_args* a, bool with_scores) {
+  if (with_scores && a->seq_len <= 32 && (long long)a->batch * a->n_q_heads <= 4LL * sm_count() && (a->dtype != DKV_F32 || a->rank <= 256))
+    return false;
   return a->batch > 0 && a->seq_len > 0 && a->workspace != nullptr && ((uintptr_t)a->workspace & 15) == 0 &&
          a->workspace_bytes >= record_bytes(a) + (with_scores ? score_bytes(a) : 0);
 }
