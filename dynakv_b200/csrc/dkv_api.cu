@@ -34,6 +34,8 @@ size_t tiles_workspace_bytes(const dkv_attn_args* a);
 bool mma_path_ok(const dkv_attn_args* a);
 size_t mma_split_workspace_bytes(const dkv_attn_args* a);
 int mma_fused(const dkv_attn_args* a);
+bool short_ok(const dkv_attn_args* a);
+int short_fused(const dkv_attn_args* a);
 int mma_split(const dkv_attn_args* a);
 int mma_combine(const dkv_attn_args* a);
 int mma_two_stage_noalloc(const dkv_attn_args* a);
@@ -48,7 +50,7 @@ extern "C" const char* dkv_last_error(void) { return g_err; }
 
 extern "C" int dkv_fused_decode(const dkv_attn_args* a) {
   if (int rc = check_attn_args(a, "dkv_fused_decode", true, true, true)) return rc;
-  if (mma_path_ok(a)) return mma_fused(a);
+  if (mma_path_ok(a)) return short_ok(a) ? short_fused(a) : mma_fused(a);
   return generic_attention(a);
 }
 

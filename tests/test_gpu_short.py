@@ -1,0 +1,46 @@
+"""Short-cache fused kernel: tile and cluster edges (one to four CTAs, rows walked in several rounds), one to four query
+heads per group, bases of fewer coefficients, rows of other lengths in the launch, rows without tokens."""
+import pytest
+import torch
+
+from dynakv_b200 import synthetic
+from dynakv_b200.kernels import _common
+from dynakv_b200.kernels.fused import fused_attention_dispatch
+from oracle import dynakv_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(seq, dtype, hq, hkv, knorm=False, rank=128, shift=False):
+    c = synthetic.make_layer_case(sum(seq) + hq, seq, "beta:2,5", 5e5, dtype, "cpu", n_q_heads=hq, n_kv_heads=hkv)
+    fk, fv, lk, lv, ok, ov = c.views()
+    k_up, v_up = c.k_up, c.v_up
+    if rank < 128:
+        lk, lv = lk.clamp(max=rank), lv.clamp(max=rank)
+        k_up, v_up = k_up[:, :rank].contiguous(), v_up[:, :rank].contiguous()
+    knw = 1.0 + 0.1 * torch.randn(128, generator=torch.Generator().manual_seed(1)) if knorm else None
+    ref = O.compact_attention(c.q, fk, k_up, fv, v_up, lk, ok, lv, ov, c.theta, seq_lens=seq, k_norm_weight=knw)
+    d = [t.cuda() for t in (c.q, fk, k_up, fv, v_up, lk, ok, lv, ov)]
+    if shift:       # a V basis that starts two bytes past a 16-byte boundary
+        buf = torch.empty(v_up.numel() + 1, dtype=dtype, device="cuda")
+        buf[1:].copy_(v_up.cuda().view(-1))
+        d[4] = buf[1:].view(v_up.shape)
+    kw = {} if knw is None else dict(k_norm_weight=knw.cuda())
+    out = fused_attention_dispatch(*d, c.theta, seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda"), len_multiple=8, **kw).float().cpu()
+    assert float((out - torch.nan_to_num(ref)).abs().max()) <= 2e-2 * max(1.0, float(torch.nan_to_num(ref).abs().max()))
+    assert _common.read_status(torch.device("cuda")) == (4 if 0 in seq else 0)      # an empty row is reported
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("seq", [[1], [127, 128], [129, 1, 256], [257, 384, 128, 0], [500, 385], [1100, 512, 513, 3]], ids=str)
+def test_tile_and_cluster_edges(seq, dtype):
+    _run(seq, dtype, 32, 8, knorm=len(seq) == 3)
+
+
+@pytest.mark.parametrize("hq,rank,shift", [(2, 128, False), (4, 64, False), (6, 40, True), (8, 128, True)])
+def test_heads_per_group_and_bases(hq, rank, shift):
+    _run([300, 70], torch.bfloat16, hq, 2, rank=rank, shift=shift)
+
+
+def test_one_tile_rows_of_more_ctas_than_the_gpu_holds():
+    _run([128] * 150 + [5] * 50, torch.bfloat16, 16, 4)
