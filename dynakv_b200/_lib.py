@@ -23,6 +23,7 @@ EXPORTS = (
     "dkv_version", "dkv_last_error", "dkv_fused_decode", "dkv_split_workspace_bytes", "dkv_split_decode",
     "dkv_split_combine", "dkv_two_stage_decode", "dkv_two_stage_decode_noalloc", "dkv_scores", "dkv_softmax_v", "dkv_append_decode",
     "dkv_pack_bulk", "dkv_row_totals", "dkv_decompress", "dkv_gate_lengths", "dkv_gate_workspace_bytes", "dkv_gate_lengths_pair", "dkv_project_bulk", "dkv_probe_tensor_pipe",
+    "dkv_norm_rows", "dkv_split_qkv", "dkv_silu_mul", "dkv_argmax_rows",
 )
 
 
@@ -94,6 +95,15 @@ class GateArgs(C.Structure):
     ]
 
 
+class NormArgs(C.Structure):
+    _fields_ = [
+        ("dtype", C.c_int32), ("n_rows", C.c_int32), ("dim", C.c_int32),
+        ("h", C.c_void_p), ("y", C.c_void_p), ("weight", C.c_void_p), ("eps", C.c_float), ("x", C.c_void_p),
+        ("w_cut", C.c_void_p), ("n_cut", C.c_int32), ("cut_bias", C.c_float), ("len_k", C.c_void_p), ("len_v", C.c_void_p),
+        ("stream", C.c_void_p),
+    ]
+
+
 _lib: Optional[C.CDLL] = None
 _host = None
 HOST_PATH = os.path.join(_HERE, "_host.so")
@@ -153,6 +163,12 @@ def load() -> C.CDLL:
     lib.dkv_project_bulk.restype = C.c_int
     lib.dkv_probe_tensor_pipe.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.dkv_probe_tensor_pipe.restype = C.c_int
+    lib.dkv_norm_rows.argtypes = [C.POINTER(NormArgs)]
+    lib.dkv_split_qkv.argtypes = [C.c_int32] * 4 + [C.c_void_p, C.c_int64, C.c_void_p, C.c_float] + [C.c_void_p] * 4
+    lib.dkv_silu_mul.argtypes = [C.c_int32] * 3 + [C.c_void_p] * 3
+    lib.dkv_argmax_rows.argtypes = [C.c_int32] * 3 + [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
+    for name in ("dkv_norm_rows", "dkv_split_qkv", "dkv_silu_mul", "dkv_argmax_rows"):
+        getattr(lib, name).restype = C.c_int
     _lib = lib
     return lib
 

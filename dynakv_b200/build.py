@@ -16,7 +16,7 @@ LIB = os.path.join(HERE, "libdynakv_b200.so")
 HOST = os.path.join(HERE, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host", "dkv_host.cpp")
 HEADER = os.path.join(HERE, "..", "include", "dynakv_b200.h")
-SOURCES = ["dkv_api.cu", "dkv_cache.cu", "dkv_generic.cu", "dkv_tiles.cu", "dkv_gate.cu", "dkv_mma_decode.cu", "dkv_short.cu", "dkv_project.cu", "dkv_pipe_probe.cu"]
+SOURCES = ["dkv_api.cu", "dkv_cache.cu", "dkv_generic.cu", "dkv_tiles.cu", "dkv_gate.cu", "dkv_mma_decode.cu", "dkv_short.cu", "dkv_layer.cu", "dkv_project.cu", "dkv_pipe_probe.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--shared", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=default", "-cudart", "shared",

@@ -3,9 +3,9 @@
 Stands in for the reference's model wrappers (src/dynakv/custom_llama.py:36-85 swaps the decoder layers of a
 Hugging Face Llama for ``CustomAttention``; scripts/benchmark_throughput.py:37-81 times ``generate``), which need
 a checkpoint, a tokenizer and transformers 4.53.  Here the model is random-init at the given shape; embeddings,
-RMSNorm, the QKV / output / MLP GEMMs, RoPE of the query and greedy sampling are plain torch (library GEMMs), and
-everything that touches the cache is this package: bulk projection + pack for the prompt, the projecting append
-and the routed attention kernels for every generated token.
+RMSNorm, RoPE and the GEMMs of the prompt are plain torch (library GEMMs), and so are the QKV / output / MLP GEMMs of a
+generated token; the row operators between those (csrc/dkv_layer.cu) and everything that touches the cache is this
+package: bulk projection + pack for the prompt, the projecting append and the routed attention kernels.
 
 Partitioning (no collective inside attention): data parallel = each rank runs its own sequences with its own
 caches; tensor parallel by KV head = rank r owns KV heads [r*Hkv/N, (r+1)*Hkv/N) with their query heads, their
@@ -14,6 +14,7 @@ row-parallel ``o_proj`` and ``down_proj`` are all-reduced (NCCL on GPUs), once e
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
@@ -22,7 +23,7 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 
-from . import synthetic
+from . import _lib, synthetic
 from .kernels.compressed_attention import CompressedDecodeLayer, project_bulk
 from .kernels.compressed_cache import CustomDynamicCache
 from .kernels.router import KernelPolicy
@@ -62,7 +63,49 @@ def rope(x: torch.Tensor, pos: torch.Tensor, theta: float) -> torch.Tensor:
 
 
 class _LayerWeights:
-    __slots__ = ("wq", "wk", "wv", "wo", "wg", "wu", "wd", "norm1", "norm2", "k_up", "v_up", "w_cut")
+    # wq, wk, wv are column ranges of wqkv and wg, wu of wgu: one GEMM each in a decode step
+    __slots__ = ("wqkv", "wq", "wk", "wv", "wo", "wgu", "wg", "wu", "wd", "norm1", "norm2", "k_up", "v_up", "w_cut")
+
+
+# Row operators between the GEMMs of a decode step, one kernel each (csrc/dkv_layer.cu).
+def _norm_rows(h, y, weight, eps, w_cut=None, cut_bias=0.0):
+    """``h += y`` in place (when given), RMSNorm of the rows, and with a cutoff head the kept lengths of the new rows."""
+    x = torch.empty_like(h)
+    a = _lib.NormArgs()
+    a.dtype, a.n_rows, a.dim = _lib.dtype_code(h.dtype), h.shape[0], h.shape[1]
+    a.h, a.y, a.weight, a.eps, a.x = h.data_ptr(), _lib.ptr(y), weight.data_ptr(), eps, x.data_ptr()
+    len_k = len_v = None
+    if w_cut is not None:
+        len_k = torch.empty(h.shape[0], w_cut.shape[0] // 2, dtype=torch.int32, device=h.device)
+        len_v = torch.empty_like(len_k)
+        a.w_cut, a.n_cut, a.cut_bias = w_cut.data_ptr(), w_cut.shape[0], cut_bias
+        a.len_k, a.len_v = len_k.data_ptr(), len_v.data_ptr()
+    a.stream = _lib.stream_ptr(h.device)
+    _lib.check(_lib.load().dkv_norm_rows(C.byref(a)), "dkv_norm_rows")
+    return x, len_k, len_v
+
+
+def _split_qkv(qkv, n_q, n_kv, positions, theta):
+    """Rotated queries and the pre-RoPE K and V rows of a merged projection."""
+    B = qkv.shape[0]
+    q, k, v = (torch.empty(B, n, 128, dtype=qkv.dtype, device=qkv.device) for n in (n_q, n_kv, n_kv))
+    _lib.check(_lib.load().dkv_split_qkv(_lib.dtype_code(qkv.dtype), B, n_q, n_kv, qkv.data_ptr(), qkv.stride(0), positions.data_ptr(), theta,
+                                         q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.stream_ptr(qkv.device)), "dkv_split_qkv")
+    return q, k, v
+
+
+def _silu_mul(gu):
+    out = torch.empty(gu.shape[0], gu.shape[1] // 2, dtype=gu.dtype, device=gu.device)
+    _lib.check(_lib.load().dkv_silu_mul(_lib.dtype_code(gu.dtype), gu.shape[0], out.shape[1], gu.data_ptr(), out.data_ptr(),
+                                        _lib.stream_ptr(gu.device)), "dkv_silu_mul")
+    return out
+
+
+def _argmax_rows(x):
+    out = torch.empty(x.shape[0], dtype=torch.int64, device=x.device)
+    _lib.check(_lib.load().dkv_argmax_rows(_lib.dtype_code(x.dtype), x.shape[0], x.shape[1], x.data_ptr(), x.stride(0), out.data_ptr(),
+                                           _lib.stream_ptr(x.device)), "dkv_argmax_rows")
+    return out
 
 
 class MiniLlama:
@@ -101,12 +144,13 @@ class MiniLlama:
         self.layers: List[_LayerWeights] = []
         for li in range(s.layers):
             w = _LayerWeights()
-            w.wq = normal(s.hidden, s.n_q_heads * D)[:, kv_lo * G * D: kv_hi * G * D].contiguous()
-            w.wk = normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D].contiguous()
-            w.wv = normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D].contiguous()
+            w.wqkv = torch.cat((normal(s.hidden, s.n_q_heads * D)[:, kv_lo * G * D: kv_hi * G * D],
+                                normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D],
+                                normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D]), dim=1)
+            w.wq, w.wk, w.wv = w.wqkv.split((self.q_local * D, self.kv_local * D, self.kv_local * D), dim=1)
             w.wo = normal(s.n_q_heads * D, s.hidden)[kv_lo * G * D: kv_hi * G * D].contiguous()
-            w.wg = normal(s.hidden, s.mlp)[:, m_lo:m_hi].contiguous()
-            w.wu = normal(s.hidden, s.mlp)[:, m_lo:m_hi].contiguous()
+            w.wgu = torch.cat((normal(s.hidden, s.mlp)[:, m_lo:m_hi], normal(s.hidden, s.mlp)[:, m_lo:m_hi]), dim=1)
+            w.wg, w.wu = w.wgu.split(m_hi - m_lo, dim=1)
             w.wd = normal(s.mlp, s.hidden)[m_lo:m_hi].contiguous()
             w.norm1 = torch.ones(s.hidden, dtype=dtype, device=self.device)
             w.norm2 = torch.ones(s.hidden, dtype=dtype, device=self.device)
@@ -201,18 +245,17 @@ class MiniLlama:
         return (last @ self.lm_head).argmax(dim=-1)
 
     # ------------------------------------------------------------------ one generated token
-    def _attention_part(self, li: int, h: torch.Tensor) -> torch.Tensor:
+    # (h, y): the residual stream and the part that is still to be added to it, which the next row operator does
+    def _attention_part(self, li: int, h: torch.Tensor, y: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Layer ``li`` from the residual stream to this rank's partial sum of the output projection [B, H]."""
         s, D, B = self.shape, self.shape.head_dim, h.shape[0]
         w = self.layers[li]
         has_short = any(n + 1 < self.policy.switch_tokens for n in self.seq_lens_host)
         counter = self.cache.seq_lens(li)                  # tokens stored per row = position of the new token
         cap = self.cache.key_cache_sp[li][1].shape[1]
-        x = rms_norm(h, w.norm1, s.rms_eps)
-        q = rope((x @ w.wq).view(B, self.q_local, D), counter, s.theta)
-        new_k = (x @ w.wk).view(B, self.kv_local, D)       # pre-RoPE: the append projects them onto the bases
-        new_v = (x @ w.wv).view(B, self.kv_local, D)
-        len_k, len_v = self._cutoffs(w, x)
+        x, len_k, len_v = _norm_rows(h, y, w.norm1, s.rms_eps, w.w_cut, self.cutoff_bias)
+        # new_k, new_v stay pre-RoPE: the append projects them onto the bases
+        q, new_k, new_v = _split_qkv(x @ w.wqkv, self.q_local, self.kv_local, counter, s.theta)
         out = torch.empty(B, self.q_local, D, dtype=self.dtype, device=self.device)
         layer = self.attn[li]
         layer.append(self.cache, new_k, new_v, len_k, len_v, counter, cap)
@@ -227,16 +270,20 @@ class MiniLlama:
             self.trace.append((li, q.clone(), out.clone()))
         return out.view(B, -1) @ w.wo
 
-    def _mlp_part(self, li: int, h: torch.Tensor) -> torch.Tensor:
+    def _mlp_part(self, li: int, h: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         w = self.layers[li]
-        return (F.silu((x := rms_norm(h, w.norm2, self.shape.rms_eps)) @ w.wg) * (x @ w.wu)) @ w.wd
+        x, _, _ = _norm_rows(h, y, w.norm2, self.shape.rms_eps)
+        return _silu_mul(x @ w.wgu) @ w.wd
+
+    def _head(self, h: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+        return _norm_rows(h, y, self.final_norm, self.shape.rms_eps)[0] @ self.lm_head
 
     def _decode_layers(self, ids: torch.Tensor) -> torch.Tensor:
-        h = self.embed[ids]                                    # [B, H]
+        h, y = self.embed[ids], None                           # [B, H]
         for li in range(len(self.layers)):
-            h = h + self._all_reduce(self._attention_part(li, h))
-            h = h + self._all_reduce(self._mlp_part(li, h))
-        return rms_norm(h, self.final_norm, self.shape.rms_eps) @ self.lm_head
+            y = self._all_reduce(self._attention_part(li, h, y))
+            y = self._all_reduce(self._mlp_part(li, h, y))
+        return self._head(h, y)
 
     # Tensor-parallel replay: the step is cut at its all-reduces.  Each piece between two all-reduces (a layer's
     # attention part, a layer's MLP part, the head) is its own CUDA graph on static buffers; the all-reduces run
@@ -261,19 +308,16 @@ class MiniLlama:
         capture(first)
         for li in range(len(self.layers)):
             def mlp(li=li):
-                self._h.add_(self._y)
-                self._y.copy_(self._mlp_part(li, self._h))
+                self._y.copy_(self._mlp_part(li, self._h, self._y))
             capture(mlp)
             if li + 1 < len(self.layers):
                 def attn(li=li + 1):
-                    self._h.add_(self._y)
-                    self._y.copy_(self._attention_part(li, self._h))
+                    self._y.copy_(self._attention_part(li, self._h, self._y))
                 capture(attn)
 
         def head():
-            self._h.add_(self._y)
-            self.logits = rms_norm(self._h, self.final_norm, self.shape.rms_eps) @ self.lm_head
-            self._next = self.logits.argmax(dim=-1)
+            self.logits = self._head(self._h, self._y)
+            self._next = _argmax_rows(self.logits)
         capture(head)
 
     def _replay_segments(self) -> None:
@@ -311,7 +355,7 @@ class MiniLlama:
                     g = torch.cuda.CUDAGraph()
                     with torch.cuda.graph(g):
                         self.logits = self._decode_layers(self._ids)
-                        self._next = self.logits.argmax(dim=-1)
+                        self._next = _argmax_rows(self.logits)
                     self._graph = g
                 else:
                     self._capture_segments(ids)
@@ -323,7 +367,7 @@ class MiniLlama:
             nxt = self._next
         else:
             self.logits = self._decode_layers(ids)
-            nxt = self.logits.argmax(dim=-1)
+            nxt = _argmax_rows(self.logits)
         self.seq_lens_host = [n + 1 for n in self.seq_lens_host]
         return nxt
 

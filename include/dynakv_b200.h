@@ -285,6 +285,40 @@ int dkv_gate_lengths(const dkv_gate_args* args);
  * argument blocks must agree in dtype, dim, n_rows and stream; workspace fields are ignored. */
 int dkv_gate_lengths_pair(const dkv_gate_args* k, const dkv_gate_args* v);
 
+/* ---- row operators of a Llama-shaped decode step ------------------------ */
+/* (No counterpart among the reference's kernels: its model wrapper, src/dynakv/custom_llama.py, runs these as torch ops.) */
+
+/* h += y (optional; rounded to the type), x = round(h * rsqrt(mean(h^2) + eps)) * weight, rounded; with n_cut > 0 also the
+ * kept lengths 8 clamp(ceil(16 sigmoid(x . w_cut[o] + cut_bias)), 1, 16), fp32 sums: len_k [n_rows, n_cut / 2] from the
+ * first half of the outputs, len_v from the second. dim <= 49152. */
+typedef struct dkv_norm_args {
+  int32_t dtype;
+  int32_t n_rows, dim;
+  void* h;              /* [n_rows, dim] residual stream, updated when y is given */
+  const void* y;        /* [n_rows, dim] or NULL */
+  const void* weight;   /* [dim] */
+  float eps;
+  void* x;              /* out [n_rows, dim] */
+  const float* w_cut;   /* [n_cut, dim] or NULL */
+  int32_t n_cut;
+  float cut_bias;
+  int32_t* len_k;
+  int32_t* len_v;
+  void* stream;
+} dkv_norm_args;
+int dkv_norm_rows(const dkv_norm_args* args);
+
+/* qkv [n_rows, (n_q + 2 n_kv) * 128] (row stride in elements): q heads rotated by positions[row] (rotate-half RoPE, fp32)
+ * to q [n_rows, n_q, 128], k and v heads copied to [n_rows, n_kv, 128]. */
+int dkv_split_qkv(int32_t dtype, int32_t n_rows, int32_t n_q_heads, int32_t n_kv_heads, const void* qkv, int64_t stride,
+                  const int32_t* positions, float theta, void* q, void* k, void* v, void* stream);
+
+/* out [n_rows, m] = round(silu(gu[:, :m])) * gu[:, m:], rounded. */
+int dkv_silu_mul(int32_t dtype, int32_t n_rows, int32_t m, const void* gu, void* out, void* stream);
+
+/* out[row] = index of the row's maximum (the first of equals). */
+int dkv_argmax_rows(int32_t dtype, int32_t n_rows, int32_t n, const void* x, int64_t stride, int64_t* out, void* stream);
+
 /* ---- misc -------------------------------------------------------------- */
 int dkv_version(void);
 const char* dkv_last_error(void);
