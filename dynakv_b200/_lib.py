@@ -20,9 +20,9 @@ ST_OVERFLOW, ST_BAD_LENGTH, ST_EMPTY_ROW, ST_TIMEOUT = 1, 2, 4, 8
 _DTYPES = {torch.float32: DKV_F32, torch.float16: DKV_F16, torch.bfloat16: DKV_BF16}
 
 EXPORTS = (
-    "dkv_version", "dkv_last_error", "dkv_fused_decode", "dkv_split_workspace_bytes", "dkv_split_decode",
+    "dkv_version", "dkv_last_error", "dkv_fused_decode", "dkv_split_workspace_bytes", "dkv_fused_workspace_bytes", "dkv_split_decode",
     "dkv_split_combine", "dkv_two_stage_decode", "dkv_two_stage_decode_noalloc", "dkv_scores", "dkv_softmax_v", "dkv_append_decode",
-    "dkv_pack_bulk", "dkv_row_totals", "dkv_decompress", "dkv_gate_lengths", "dkv_gate_workspace_bytes", "dkv_gate_lengths_pair", "dkv_project_bulk", "dkv_probe_tensor_pipe",
+    "dkv_pack_bulk", "dkv_pack_pair", "dkv_row_totals", "dkv_decompress", "dkv_gate_lengths", "dkv_gate_workspace_bytes", "dkv_gate_lengths_pair", "dkv_project_bulk", "dkv_probe_tensor_pipe",
     "dkv_norm_rows", "dkv_split_qkv", "dkv_silu_mul", "dkv_argmax_rows",
 )
 
@@ -141,14 +141,17 @@ def load() -> C.CDLL:
         fn = getattr(lib, name)
         fn.argtypes = [C.POINTER(AttnArgs)]
         fn.restype = C.c_int
-    lib.dkv_split_workspace_bytes.argtypes = [C.POINTER(AttnArgs)]
-    lib.dkv_split_workspace_bytes.restype = C.c_size_t
+    for fn in (lib.dkv_split_workspace_bytes, lib.dkv_fused_workspace_bytes):
+        fn.argtypes = [C.POINTER(AttnArgs)]
+        fn.restype = C.c_size_t
     lib.dkv_softmax_v.argtypes = [C.POINTER(AttnArgs), C.c_void_p, C.c_int64, C.c_int64]
     lib.dkv_softmax_v.restype = C.c_int
     lib.dkv_append_decode.argtypes = [C.POINTER(AppendArgs)]
     lib.dkv_append_decode.restype = C.c_int
     lib.dkv_pack_bulk.argtypes = [C.POINTER(PackArgs)]
     lib.dkv_pack_bulk.restype = C.c_int
+    lib.dkv_pack_pair.argtypes = [C.POINTER(PackArgs)] * 2
+    lib.dkv_pack_pair.restype = C.c_int
     lib.dkv_row_totals.argtypes = [C.POINTER(PackArgs), C.POINTER(PackArgs), C.c_void_p]
     lib.dkv_row_totals.restype = C.c_int
     lib.dkv_decompress.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.POINTER(Side), C.c_void_p, C.c_void_p]

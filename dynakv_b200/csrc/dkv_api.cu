@@ -60,6 +60,10 @@ extern "C" size_t dkv_split_workspace_bytes(const dkv_attn_args* a) {
   return mma_split_workspace_bytes(a);
 }
 
+extern "C" size_t dkv_fused_workspace_bytes(const dkv_attn_args* a) {
+  return a == nullptr || mma_path_ok(a) ? 0 : tiles_workspace_bytes(a);
+}
+
 extern "C" int dkv_split_decode(const dkv_attn_args* a) {
   if (int rc = check_attn_args(a, "dkv_split_decode", true, true, true)) return rc;
   DKV_REQUIRE(mma_path_ok(a), DKV_E_ARG,

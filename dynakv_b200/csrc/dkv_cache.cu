@@ -274,7 +274,9 @@ __device__ __forceinline__ bool positions_fit(const dkv_pack_args& p, const pack
   return r.pos0 >= 0 && r.pos0 + r.n_new <= p.seq_capacity;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) pack_scan_kernel(dkv_pack_args p) {
+// Both kernels of a pack run over one side or over both at once (grid.z).
+__global__ void __launch_bounds__(SCAN_THREADS) pack_scan_kernel(const __grid_constant__ dkv_pack_args pk, const __grid_constant__ dkv_pack_args pv) {
+  const dkv_pack_args& p = blockIdx.z ? pv : pk;
   __shared__ int red[2 * SCAN_THREADS / 32];
   __shared__ int warp_tot[SCAN_THREADS / 32];
   const int a = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -354,7 +356,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) pack_scan_kernel(dkv_pack_args p
 }
 
 template <typename T>
-__global__ void __launch_bounds__(COPY_THREADS) pack_copy_kernel(dkv_pack_args p, int vec16) {
+__global__ void __launch_bounds__(COPY_THREADS) pack_copy_kernel(const __grid_constant__ dkv_pack_args pk, const __grid_constant__ dkv_pack_args pv, int vec16) {
+  const dkv_pack_args& p = blockIdx.z ? pv : pk;
+  pdl_wait();       // lengths and offsets come from the scan
   const int a = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b = a / p.arenas_per_batch, j = a - b * p.arenas_per_batch;
   const dkv_side& sd = p.side;
@@ -378,7 +382,7 @@ __global__ void __launch_bounds__(COPY_THREADS) pack_copy_kernel(dkv_pack_args p
                   (size_t)s0 * p.stride_s;
   T* flat = reinterpret_cast<T*>(sd.flat) + (size_t)a * sd.flat_stride + first_off;
   const int pre = s < n_new ? off - first_off : run;         // elements of the run before this row
-  if (vec16 && (first_off & 7) == 0) {
+  if ((vec16 >> blockIdx.z & 1) && (first_off & 7) == 0) {
     const int n_pieces = run >> 3, pre8 = pre >> 3;
     uint4* dst = reinterpret_cast<uint4*>(flat);
     for (int g0 = 0; g0 < n_pieces; g0 += 128) {
@@ -529,7 +533,7 @@ extern "C" int dkv_append_decode(const dkv_append_args* a) {
   return DKV_OK;
 }
 
-extern "C" int dkv_pack_bulk(const dkv_pack_args* a) {
+static int check_pack(const dkv_pack_args* a) {
   DKV_REQUIRE(a != nullptr, DKV_E_ARG, "dkv_pack_bulk: null args");
   DKV_REQUIRE(a->batch >= 0 && a->arenas_per_batch >= 1 && a->n_new >= 0 && a->max_dim >= 1 && a->max_dim <= 1024,
               DKV_E_ARG, "dkv_pack_bulk: bad sizes");
@@ -537,22 +541,44 @@ extern "C" int dkv_pack_bulk(const dkv_pack_args* a) {
   DKV_REQUIRE(a->states && a->new_lens && a->side.ptr, DKV_E_ARG, "dkv_pack_bulk: null input");
   DKV_REQUIRE(a->len_multiple >= 1, DKV_E_ARG, "dkv_pack_bulk: len_multiple must be >= 1");
   if (int rc = check_side(a->side, "dkv_pack_bulk side")) return rc;
+  DKV_REQUIRE((int64_t)a->batch * a->arenas_per_batch <= 65535, DKV_E_LIMIT, "dkv_pack_bulk: at most 65535 arena rows per call");
+  return DKV_OK;
+}
+
+// 16-byte copies when every row start is 16-byte aligned on both sides: 16-bit elements, lengths declared as
+// multiples of 8 (offsets are then multiples of 8 too), aligned bases and strides
+static int pack_vec16(const dkv_pack_args* a) {
+  return a->dtype != DKV_F32 && a->len_multiple % 8 == 0 && (((uintptr_t)a->states | (uintptr_t)a->side.flat) & 15) == 0 &&
+         a->stride_b % 8 == 0 && a->stride_j % 8 == 0 && a->stride_s % 8 == 0 && a->side.flat_stride % 8 == 0;
+}
+
+static int launch_pack(const dkv_pack_args* a, const dkv_pack_args* b, unsigned sides) {
   const int n_arena = a->batch * a->arenas_per_batch;
   if (n_arena == 0 || a->n_new == 0) return DKV_OK;
-  DKV_REQUIRE(n_arena <= 65535, DKV_E_LIMIT, "dkv_pack_bulk: at most 65535 arena rows per call");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
-  // 16-byte copies when every row start is 16-byte aligned on both sides: 16-bit elements, lengths declared as
-  // multiples of 8 (offsets are then multiples of 8 too), aligned bases and strides
-  const bool two_byte = a->dtype != DKV_F32;
-  const int vec16 = two_byte && a->len_multiple % 8 == 0 && (((uintptr_t)a->states | (uintptr_t)a->side.flat) & 15) == 0 &&
-                    a->stride_b % 8 == 0 && a->stride_j % 8 == 0 && a->stride_s % 8 == 0 && a->side.flat_stride % 8 == 0;
-  const dim3 scan_grid((unsigned)((a->n_new + SCAN_THREADS - 1) / SCAN_THREADS), (unsigned)n_arena);
-  pack_scan_kernel<<<scan_grid, SCAN_THREADS, 0, st>>>(*a);
-  const dim3 grid((unsigned)((a->n_new + COPY_THREADS - 1) / COPY_THREADS), (unsigned)n_arena);
-  if (a->dtype == DKV_F32) pack_copy_kernel<float><<<grid, COPY_THREADS, 0, st>>>(*a, 0);
-  else pack_copy_kernel<uint16_t><<<grid, COPY_THREADS, 0, st>>>(*a, vec16);
+  const int vec16 = pack_vec16(a) | pack_vec16(b) << 1;
+  const dim3 scan_grid((unsigned)((a->n_new + SCAN_THREADS - 1) / SCAN_THREADS), (unsigned)n_arena, sides);
+  pack_scan_kernel<<<scan_grid, SCAN_THREADS, 0, st>>>(*a, *b);
+  DKV_CHECK_LAUNCH();
+  const dim3 grid((unsigned)((a->n_new + COPY_THREADS - 1) / COPY_THREADS), (unsigned)n_arena, sides);
+  const cudaError_t e = a->dtype == DKV_F32 ? launch_pdl(pack_copy_kernel<float>, grid, dim3(COPY_THREADS), 0, st, *a, *b, 0)
+                                            : launch_pdl(pack_copy_kernel<uint16_t>, grid, dim3(COPY_THREADS), 0, st, *a, *b, vec16);
+  DKV_REQUIRE(e == cudaSuccess, DKV_E_CUDA, "launch of the pack failed: %s", cudaGetErrorString(e));
   DKV_CHECK_LAUNCH();
   return DKV_OK;
+}
+
+extern "C" int dkv_pack_bulk(const dkv_pack_args* a) {
+  if (int rc = check_pack(a)) return rc;
+  return launch_pack(a, a, 1);
+}
+
+extern "C" int dkv_pack_pair(const dkv_pack_args* k, const dkv_pack_args* v) {
+  if (int rc = check_pack(k)) return rc;
+  if (int rc = check_pack(v)) return rc;
+  DKV_REQUIRE(k->dtype == v->dtype && k->batch == v->batch && k->arenas_per_batch == v->arenas_per_batch && k->n_new == v->n_new && k->stream == v->stream,
+              DKV_E_ARG, "dkv_pack_pair: the sides differ in type, sizes or stream");
+  return launch_pack(k, v, 2);
 }
 
 extern "C" int dkv_row_totals(const dkv_pack_args* k, const dkv_pack_args* v, int32_t* totals) {

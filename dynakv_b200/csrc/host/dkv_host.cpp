@@ -6,6 +6,7 @@
 // launched or changed anything; the Python callers then take their own path, which copies what has to be copied and
 // raises what has to be raised.  No state is kept between calls but the address of each device's status word.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -63,6 +64,19 @@ bool fill_side(dkv_side& s, const at::Tensor& flat, const at::Tensor& lens, cons
   s.offs_stride_s = tokens > 1 ? oe : 1;
   s.ptr = nullptr;
   return true;
+}
+
+at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev) {
+  return at::Tensor(at::detail::empty_cuda(sizes, dt, dev, std::nullopt));
+}
+
+// A [rows, cols] view of int or data rows inside `base` (no autograd here: a tensor over the same storage is all a view has
+// to be, and costs a tenth of what a dispatched narrow() does).
+at::Tensor rows_view(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes, at::IntArrayRef strides) {
+  at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(base.storage()), base.key_set(), base.dtype());
+  t.unsafeGetTensorImpl()->set_storage_offset(base.storage_offset() + offset);
+  t.unsafeGetTensorImpl()->set_sizes_and_strides(sizes, strides);
+  return t;
 }
 
 PyObject* fail(const char* what, int rc) {
@@ -136,19 +150,19 @@ PyObject* attend(PyObject*, PyObject* const* v, Py_ssize_t n) {
     out = unpack(v[10]);
     if (out.scalar_type() != dt || out.dim() != 3 || out.stride(2) != 1) Py_RETURN_NONE;
   } else {
-    out = at::empty({B, Hq, D}, q.options());
+    out = empty({B, Hq, D}, dt, q.device());
   }
   a.out = out.data_ptr();
   a.out_stride_b = out.stride(0);
   a.out_stride_h = out.stride(1);
-  const size_t need = dkv_split_workspace_bytes(&a);
+  const bool two_stage = v[18] == Py_True;
+  const size_t need = two_stage ? dkv_split_workspace_bytes(&a) : dkv_fused_workspace_bytes(&a);
   at::Tensor ws;
   if (need) {
-    ws = at::empty({(int64_t)need}, q.options().dtype(at::kByte));
+    ws = empty({(int64_t)need}, at::kByte, q.device());
     a.workspace = ws.data_ptr();
     a.workspace_bytes = need;
   }
-  const bool two_stage = v[18] == Py_True;
   const int rc = two_stage ? dkv_two_stage_decode(&a) : dkv_fused_decode(&a);
   if (rc) return fail(two_stage ? "dkv_two_stage_decode" : "dkv_fused_decode", rc);
   return THPVariable_Wrap(out);
@@ -203,8 +217,13 @@ PyObject* append_token(PyObject*, PyObject* const* v, Py_ssize_t n) {
     s.ptr = static_cast<int32_t*>(ptr.data_ptr());
     a.seq_capacity = (int32_t)(sd ? std::min<int64_t>(a.seq_capacity, cap) : cap);
     view[sd][0] = flat;
-    view[sd][1] = lens.narrow(1, 0, seq + 1);
-    view[sd][2] = offs.narrow(1, 0, seq + 1);
+    if (lens.dim() == 2) {
+      view[sd][1] = rows_view(lens, 0, {rows, seq + 1}, lens.strides());
+      view[sd][2] = rows_view(offs, 0, {rows, seq + 1}, offs.strides());
+    } else {
+      view[sd][1] = lens.narrow(1, 0, seq + 1);
+      view[sd][2] = offs.narrow(1, 0, seq + 1);
+    }
   }
   if (v[9] != Py_None) {
     if (!plain(v[9], dev)) Py_RETURN_NONE;
@@ -233,6 +252,60 @@ PyObject* append_token(PyObject*, PyObject* const* v, Py_ssize_t n) {
   for (int i = 0; i < 3; ++i)
     for (int sd = 0; sd < 2; ++sd) PyTuple_SET_ITEM(r, 2 * i + sd, THPVariable_Wrap(view[sd][i]));
   return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// new_state(flat [rows, capacity], seq_capacity) -> [flat, lens, offs, ptr, 0, [0] * rows], all zero: the three index buffers
+// are views of one allocation, so that a new layer costs two fills and not four of each side
+PyObject* new_state(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2 || !is_tensor(v[0]) || !unpack(v[0]).is_cuda()) Py_RETURN_NONE;
+  const at::Tensor& flat = unpack(v[0]);
+  const int64_t seq = PyLong_AsLong(v[1]);
+  if (PyErr_Occurred()) return nullptr;
+  if (flat.dim() != 2 || !flat.is_contiguous() || flat.requires_grad() || seq < 0 || seq % 4) Py_RETURN_NONE;
+  const int64_t rows = flat.size(0);
+  c10::cuda::CUDAGuard guard(flat.device());
+  cudaStream_t st = at::cuda::getCurrentCUDAStream(flat.get_device()).stream();
+  const at::Tensor ints = empty({2 * rows * seq + rows}, at::kInt, flat.device());
+  cudaError_t e = cudaMemsetAsync(flat.data_ptr(), 0, flat.nbytes(), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ints.data_ptr(), 0, ints.nbytes(), st);
+  if (e != cudaSuccess) {
+    PyErr_Format(PyExc_RuntimeError, "zeroing a new cache layer failed: %s", cudaGetErrorString(e));
+    return nullptr;
+  }
+  PyObject* zeros = PyList_New(rows);
+  for (int64_t i = 0; i < rows; ++i) PyList_SET_ITEM(zeros, i, PyLong_FromLong(0));
+  PyObject* r = PyList_New(6);
+  Py_INCREF(v[0]);
+  PyList_SET_ITEM(r, 0, v[0]);
+  for (int i = 0; i < 2; ++i) PyList_SET_ITEM(r, 1 + i, THPVariable_Wrap(rows_view(ints, i * rows * seq, {rows, seq}, {seq, 1})));
+  PyList_SET_ITEM(r, 3, THPVariable_Wrap(rows_view(ints, 2 * rows * seq, {rows}, {1})));
+  PyList_SET_ITEM(r, 4, PyLong_FromLong(0));
+  PyList_SET_ITEM(r, 5, zeros);
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// grow(buffer [rows, cols], new_cols) -> [rows, new_cols] that holds the old columns and zeros behind them
+PyObject* grow(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2 || !is_tensor(v[0]) || !unpack(v[0]).is_cuda()) Py_RETURN_NONE;
+  const at::Tensor& t = unpack(v[0]);
+  const int64_t cols = PyLong_AsLong(v[1]);
+  if (PyErr_Occurred()) return nullptr;
+  if (t.dim() != 2 || t.stride(1) != 1 || t.requires_grad() || cols < t.size(1) || t.numel() == 0) Py_RETURN_NONE;
+  c10::cuda::CUDAGuard guard(t.device());
+  cudaStream_t st = at::cuda::getCurrentCUDAStream(t.get_device()).stream();
+  const at::Tensor r = empty({t.size(0), cols}, t.scalar_type(), t.device());
+  const size_t es = t.element_size(), had = t.size(1) * es, pitch = cols * es;
+  cudaError_t e = cudaMemcpy2DAsync(r.data_ptr(), pitch, t.data_ptr(), t.stride(0) * es, had, t.size(0), cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess && pitch > had) e = cudaMemset2DAsync(static_cast<char*>(r.data_ptr()) + had, pitch, 0, pitch - had, t.size(0), st);
+  if (e != cudaSuccess) {
+    PyErr_Format(PyExc_RuntimeError, "growing a cache buffer failed: %s", cudaGetErrorString(e));
+    return nullptr;
+  }
+  return THPVariable_Wrap(r);
   END_HANDLE_TH_ERRORS
 }
 
@@ -303,6 +376,8 @@ PyObject* set_status_word(PyObject*, PyObject* const* v, Py_ssize_t n) {
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)), METH_FASTCALL
 PyMethodDef methods[] = {{"attend", FAST(attend), "decode attention"},
                          {"append_token", FAST(append_token), "decode append"},
+                         {"new_state", FAST(new_state), "buffers of a new cache layer"},
+                         {"grow", FAST(grow), "a cache buffer with more columns"},
                          {"gate", FAST(gate), "cutoff gate of one side"},
                          {"set_status", FAST(set_status_word), "status word of a device"},
                          {nullptr, nullptr, 0, nullptr}};

@@ -143,30 +143,38 @@ class CustomDynamicCache:
 
     @staticmethod
     def _new_state(rows, flat_cap, seq_cap, dtype, device):
+        seq_cap = _round4(max(seq_cap, 1))
+        if torch.device(device).type == "cuda":
+            state = _lib.host().new_state(torch.empty((rows, max(flat_cap, 8)), dtype=dtype, device=device), seq_cap)
+            if state is not None:
+                return state
         return [
             torch.zeros((rows, max(flat_cap, 8)), dtype=dtype, device=device),
-            torch.zeros((rows, _round4(max(seq_cap, 1))), dtype=torch.int32, device=device),
-            torch.zeros((rows, _round4(max(seq_cap, 1))), dtype=torch.int32, device=device),
+            torch.zeros((rows, seq_cap), dtype=torch.int32, device=device),
+            torch.zeros((rows, seq_cap), dtype=torch.int32, device=device),
             torch.zeros(rows, dtype=torch.int32, device=device),
             0,
             [0] * rows,
         ]
 
     @staticmethod
-    def _ensure_capacity(cache, flat_cap, seq_cap):
-        flat_buf, lens_buf, offs_buf = cache[0], cache[1], cache[2]
-        if seq_cap > lens_buf.shape[1]:
+    def _grown(buf, cols):
+        new = _lib.host().grow(buf, cols) if buf.is_cuda else None
+        if new is None:
+            new = buf.new_zeros(buf.shape[0], cols)
+            new[:, : buf.shape[1]].copy_(buf)
+        return new
+
+    @classmethod
+    def _ensure_capacity(cls, cache, flat_cap, seq_cap):
+        if seq_cap > cache[1].shape[1]:
             for i in (1, 2):
-                new = cache[i].new_zeros(cache[i].shape[0], _round4(seq_cap))
-                new[:, : cache[i].shape[1]].copy_(cache[i])
-                cache[i] = new
-        if flat_cap > flat_buf.shape[1]:
-            new = flat_buf.new_zeros(flat_buf.shape[0], flat_cap)
-            new[:, : flat_buf.shape[1]].copy_(flat_buf)
-            cache[0] = new
+                cache[i] = cls._grown(cache[i], _round4(seq_cap))
+        if flat_cap > cache[0].shape[1]:
+            cache[0] = cls._grown(cache[0], flat_cap)
 
     # ------------------------------------------------------------------ update
-    def _prepare(self, cache_list, layer_idx, new_states, new_len, max_dim):
+    def _prepare(self, cache_list, layer_idx, new_states, new_len, max_dim, exact=False):
         """Host-side capacity policy of the reference for one new token (_update_layer_cache, compressed_cache.py:96-168)."""
         while len(cache_list) <= layer_idx:
             cache_list.append(None)
@@ -180,7 +188,7 @@ class CustomDynamicCache:
             self._ensure_capacity(cache, cache[0].shape[1], cache[1].shape[1] + EXPAND_SEQ_STEP)
         max_added = max_dim
         if max(cache[5]) + max_added > cache[0].shape[1]:
-            real = cache[3].cpu().tolist()          # resynchronise the conservative bound
+            real = cache[5] if exact else cache[3].cpu().tolist()          # resynchronise the conservative bound
             cache[5] = real
             if max(real) + max_added > cache[0].shape[1]:
                 step = EXPAND_SEQ_STEP * (max_dim // 2)
@@ -233,8 +241,12 @@ class CustomDynamicCache:
         kl, vl = lens2d(key_len), lens2d(value_len)
         if not is_decode or token_counts is not None:
             return self._update_block(key_states, kl, value_states, vl, row_dim, width, layer_idx, token_counts)
-        ck, _ = self._prepare(self.key_cache_sp, layer_idx, key_states, kl, width)
-        cv, max_added = self._prepare(self.value_cache_sp, layer_idx, value_states, vl, width)
+        both = [lst[layer_idx] if layer_idx < len(lst) else None for lst in (self.key_cache_sp, self.value_cache_sp)]
+        exact = all(c is not None and max(c[5]) + width > c[0].shape[1] for c in both)
+        if exact:       # both bounds have run out, as they do together: one synchronising copy instead of two
+            both[0][5], both[1][5] = torch.stack((both[0][3], both[1][3])).tolist()
+        ck, _ = self._prepare(self.key_cache_sp, layer_idx, key_states, kl, width, exact)
+        cv, max_added = self._prepare(self.value_cache_sp, layer_idx, value_states, vl, width, exact)
         seq_ptr = ck[4]
         row_counter = self._row_counter(layer_idx, B, dev, seq_ptr, token_counts)
         ks = key_states.contiguous()
@@ -306,10 +318,14 @@ class CustomDynamicCache:
             p.seq_pos, p.len_multiple, p.status, p.stream = seq_ptr, self.len_multiple, st, stream
             args.append(p)
 
-        def pack(side, status):
-            cache, p = lists[side][layer_idx], args[side]
-            p.side, p.seq_capacity, p.status = self._side(cache), cache[1].shape[1], status
-            _lib.check(lib.dkv_pack_bulk(C.byref(p)), "dkv_pack_bulk")
+        def pack(sides, status):
+            for side in sides:
+                cache, p = lists[side][layer_idx], args[side]
+                p.side, p.seq_capacity, p.status = self._side(cache), cache[1].shape[1], status
+            if len(sides) == 2:
+                _lib.check(lib.dkv_pack_pair(C.byref(args[0]), C.byref(args[1])), "dkv_pack_pair")
+            elif sides:
+                _lib.check(lib.dkv_pack_bulk(C.byref(args[sides[0]])), "dkv_pack_bulk")
 
         for side in (0, 1):
             if not fresh[side]:
@@ -320,9 +336,8 @@ class CustomDynamicCache:
         host.copy_(totals, non_blocking=True)
         here = torch.cuda.Event()
         here.record(torch.cuda.current_stream(dev))
-        for side in (0, 1):
-            if not fresh[side]:
-                pack(side, None)
+        pack([side for side in (0, 1) if not fresh[side]], None)
+        again = []
         here.synchronize()
         for side, lst in enumerate(lists):
             raw, stored, now, _ = host[side].t().tolist()
@@ -337,11 +352,12 @@ class CustomDynamicCache:
                 cache[3].copy_(host[side, :, 2].contiguous())     # rows of the first attempt that did fit moved on
             cap = cache[0].shape[1]
             if fresh[side] or grow:
-                pack(side, st)
+                again.append(side)
             elif max(n + s_ for n, s_ in zip(now, stored)) > cap:     # lengths made valid no longer fit: recorded as empty
                 status_word(dev).bitwise_or_(_lib.ST_OVERFLOW)
             cache[4] = seq_ptr + n_new
             cache[5] = [n + s_ if n + s_ <= cap else n for n, s_ in zip(now, stored)]
+        pack(again, st)
         if row_counter is not None:
             row_counter.add_(counts_dev if counts_dev is not None else n_new)
             self._seq_lens_host[layer_idx] = [n + (counts[b] if counts is not None else n_new)

@@ -16,6 +16,8 @@ from typing import Optional, Sequence
 
 import torch
 
+from . import fused as _fused, two_stage as _two_stage
+
 
 @dataclass(frozen=True)
 class KernelPolicy:
@@ -36,6 +38,9 @@ class KernelPolicy:
         return short, long_
 
 
+DEFAULT_POLICY = KernelPolicy()
+
+
 def compressed_decode_attention(
     *, q, k_flat, k_up, v_flat, v_up, key_lengths, key_offsets,
     value_lengths, value_offsets, theta: float, cache_length: int,
@@ -47,18 +52,14 @@ def compressed_decode_attention(
     len_multiple: int = 1,
 ):
     """Run the kernel selected from the current physical cache length; returns [B, Hq, D]."""
-    from .fused import fused_attention_dispatch
-    from .two_stage import two_stage_attention
-
-    policy = policy or KernelPolicy()
-    common = dict(k_norm_weight=k_norm_weight, k_norm_eps=k_norm_eps, len_multiple=len_multiple, seq_lens=seq_lens)
     args = (q, k_flat, k_up, v_flat, v_up, key_lengths, key_offsets, value_lengths, value_offsets, theta)
+    policy = policy or DEFAULT_POLICY
     if seq_lens is None:
         if seq_lens_host is not None:
             raise ValueError("seq_lens_host needs the matching device tensor seq_lens")
-        if policy.select(cache_length) == "short_fused":
-            return fused_attention_dispatch(*args, **common)
-        return two_stage_attention(*args, **common)
+        run = _fused.fused_attention_dispatch if policy.select(cache_length) == "short_fused" else _two_stage.two_stage_attention
+        return run(*args, k_norm_weight=k_norm_weight, k_norm_eps=k_norm_eps, len_multiple=len_multiple)
+    common = dict(k_norm_weight=k_norm_weight, k_norm_eps=k_norm_eps, len_multiple=len_multiple, seq_lens=seq_lens)
 
     # per-row routing on the device
     q3 = q.squeeze(2) if q.dim() == 4 else q
@@ -68,7 +69,7 @@ def compressed_decode_attention(
         short, long_ = policy.partition(seq_lens_host)
         any_short, any_long = bool(short), bool(long_)
     if any_short:
-        fused_attention_dispatch(*args, out=out, route_max_tokens=policy.switch_tokens if any_long else 0, **common)
+        _fused.fused_attention_dispatch(*args, out=out, route_max_tokens=policy.switch_tokens if any_long else 0, **common)
     if any_long:
-        two_stage_attention(*args, out=out, route_min_tokens=policy.switch_tokens if any_short else 0, **common)
+        _two_stage.two_stage_attention(*args, out=out, route_min_tokens=policy.switch_tokens if any_short else 0, **common)
     return out

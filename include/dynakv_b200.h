@@ -113,6 +113,10 @@ int dkv_fused_decode(const dkv_attn_args* a);
  * Replaces the abx_sparse -> avx pair as the router uses it (src/dynakv/kernels/router.py:50-59,
  * two_stage.py:159-189,283-324). dkv_two_stage_decode = dkv_split_decode then dkv_split_combine. */
 size_t dkv_split_workspace_bytes(const dkv_attn_args* a);
+
+/* The scratch that dkv_fused_decode uses: 0 on the packed path, where dkv_split_workspace_bytes is what the long-cache
+ * calls need. */
+size_t dkv_fused_workspace_bytes(const dkv_attn_args* a);
 int dkv_split_decode(const dkv_attn_args* a);
 int dkv_split_combine(const dkv_attn_args* a);
 int dkv_two_stage_decode(const dkv_attn_args* a);
@@ -201,6 +205,9 @@ typedef struct dkv_pack_args {
  * positions would pass seq_capacity sets DKV_ST_OVERFLOW and is not touched at all.
  * Replaces the per-row python loop of _update_layer_cache (compressed_cache.py:184-209). */
 int dkv_pack_bulk(const dkv_pack_args* a);
+
+/* The same for both sides of a block in one pair of launches; the sides agree in dtype, batch, arenas, n_new and stream. */
+int dkv_pack_pair(const dkv_pack_args* k, const dkv_pack_args* v);
 
 /* What the host's capacity policy asks about a block before it is packed (_update_layer_cache's sums and write pointers,
  * compressed_cache.py:143-168), both sides in one launch: totals[side][arena row] = {sum of the lengths given, sum as
