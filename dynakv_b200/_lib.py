@@ -22,7 +22,7 @@ _DTYPES = {torch.float32: DKV_F32, torch.float16: DKV_F16, torch.bfloat16: DKV_B
 EXPORTS = (
     "dkv_version", "dkv_last_error", "dkv_fused_decode", "dkv_split_workspace_bytes", "dkv_fused_workspace_bytes", "dkv_split_decode",
     "dkv_split_combine", "dkv_two_stage_decode", "dkv_two_stage_decode_noalloc", "dkv_scores", "dkv_softmax_v", "dkv_append_decode",
-    "dkv_pack_bulk", "dkv_pack_pair", "dkv_row_totals", "dkv_decompress", "dkv_gate_lengths", "dkv_gate_workspace_bytes", "dkv_gate_lengths_pair", "dkv_project_bulk", "dkv_probe_tensor_pipe",
+    "dkv_pack_bulk", "dkv_pack_pair", "dkv_row_totals", "dkv_decompress", "dkv_gate_lengths", "dkv_gate_lengths_both", "dkv_gate_workspace_bytes", "dkv_gate_lengths_pair", "dkv_project_bulk", "dkv_probe_tensor_pipe",
     "dkv_norm_rows", "dkv_split_qkv", "dkv_silu_mul", "dkv_argmax_rows",
 )
 
@@ -160,6 +160,8 @@ def load() -> C.CDLL:
     lib.dkv_gate_lengths.restype = C.c_int
     lib.dkv_gate_workspace_bytes.argtypes = [C.POINTER(GateArgs)]
     lib.dkv_gate_workspace_bytes.restype = C.c_size_t
+    lib.dkv_gate_lengths_both.argtypes = [C.POINTER(GateArgs), C.POINTER(GateArgs)]
+    lib.dkv_gate_lengths_both.restype = C.c_int
     lib.dkv_gate_lengths_pair.argtypes = [C.POINTER(GateArgs), C.POINTER(GateArgs)]
     lib.dkv_gate_lengths_pair.restype = C.c_int
     lib.dkv_project_bulk.argtypes = [C.POINTER(ProjectArgs)]

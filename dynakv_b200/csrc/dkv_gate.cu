@@ -238,13 +238,16 @@ __global__ void __launch_bounds__(256) gate_small_kernel(dkv_gate_args pk, dkv_g
 
 // ---- many 16-bit rows (a prompt): logits on the tensor core, then one warp per row with its columns in registers ----
 //
-// gate_gemm_kernel: logits = x W + b.  One CTA per 128 rows x BN columns; the reduction runs over 64-wide stages, x as
-// a K-major operand (boxes of 64 dims x 128 rows), W as it lies in memory, an MN-major operand (boxes of 64 columns x 64
-// dims), both by TMA in the 128-byte swizzle, two stages in flight; two CTAs share an SM, so that one's read-back hides
-// behind the other's products.  fp32 accumulation; the sum is rounded to the storage type only where the reference's
-// addmm writes it (native rounding), and the logits then travel in that type (half the bytes).  Bound by the tensor
-// core: 8192 rows x 1024 take 13 us of it; the CUDA-core kernel above took 1161 us.
-constexpr int GG_ROWS = 128, GG_BK = 64, GG_STAGES = 2;
+// gate_gemm_kernel: logits = x W + b, of one side or of both in one launch.  Tiles of 128 rows x BN columns; the reduction
+// runs over 64-wide stages, x as a K-major operand (boxes of 64 dims x 128 rows), W as it lies in memory, an MN-major
+// operand (boxes of 64 columns x 64 dims), both by TMA in the 128-byte swizzle, as many stages in flight as shared memory
+// holds.  One CTA per SM walks the tiles with two accumulators in tensor memory, so that a tile is read back and written
+// while the next one is multiplied, and no wave is left half empty.  fp32 accumulation; the sum is rounded to the storage
+// type only where the reference's addmm writes it (native rounding), and the logits then travel in that type (half the
+// bytes).  Bound by the operands' way from L2 (48 KB per stage, ~45 bytes per SM and clock), before the tensor core: both
+// sides of 8192 rows x 1024 take 36 us (2 x 21.6 with a CTA per tile, two stages and two CTAs an SM; 2 x 1161 on the CUDA
+// cores); the products alone are 21 us.
+constexpr int GG_ROWS = 128, GG_BK = 64, GG_RING = 192 * 1024, GG_THREADS = 192;
 constexpr uint32_t GG_SPIN = 1u << 22;
 
 __device__ __forceinline__ uint32_t gg_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -277,131 +280,179 @@ __device__ __forceinline__ uint32_t gg_pack(float lo, float hi) {
 }
 
 template <typename T, int BN>
-__global__ void __launch_bounds__(128, 2) gate_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                                                           dkv_gate_args p) {
-  constexpr int A_BYTES = GG_ROWS * GG_BK * 2, B_BYTES = BN * GG_BK * 2, STAGE = A_BYTES + B_BYTES;
+__global__ void __launch_bounds__(GG_THREADS) gate_gemm_kernel(const __grid_constant__ CUtensorMap map_xk, const __grid_constant__ CUtensorMap map_wk,
+                                                               const __grid_constant__ CUtensorMap map_xv, const __grid_constant__ CUtensorMap map_wv,
+                                                               const __grid_constant__ dkv_gate_args pk, const __grid_constant__ dkv_gate_args pv, int n_tiles) {
+  constexpr int A_BYTES = GG_ROWS * GG_BK * 2, B_BYTES = BN * GG_BK * 2, STAGE = A_BYTES + B_BYTES, STAGES = GG_RING / STAGE;
   extern __shared__ unsigned char gg_raw[];
   // the swizzle is taken on absolute shared-memory addresses: tiles start on 1024-byte boundaries
-  unsigned char* tiles = gg_raw + ((1024u - (gg_smem(gg_raw) & 1023u)) & 1023u);
-  __shared__ alignas(8) unsigned long long full[GG_STAGES], empty[GG_STAGES], done;
+  unsigned char* ring = gg_raw + ((1024u - (gg_smem(gg_raw) & 1023u)) & 1023u);
+  __shared__ alignas(8) unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ float bias_s[BN];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * BN, row0 = blockIdx.y * GG_ROWS;
-  const int n_k = p.dim / GG_BK;
+  const int n_k = pk.dim / GG_BK, cols = pk.dim / BN, per_side = cols * ((pk.n_rows + GG_ROWS - 1) / GG_ROWS);
   if (tid == 0) {
-    for (int s = 0; s < GG_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&full[s])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&empty[s])));
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&done)));
+    for (int s = 0; s < 2; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gg_smem(&acc_full[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gg_smem(&acc_empty[s])), "n"(4));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gg_smem(&tmem_slot)), "r"(BN));
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gg_smem(&tmem_slot)), "r"(2 * BN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  for (int e = tid; e < BN; e += 128) bias_s[e] = to_f32(reinterpret_cast<const T*>(p.b)[n0 + e]);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  if (warp == 0 && lane == 0) {
-    for (int k = 0; k < n_k; ++k) {
-      const int s = k % GG_STAGES;
-      if (k >= GG_STAGES && !gg_wait(&empty[s], (uint32_t)((k / GG_STAGES - 1) & 1))) break;
-      const uint32_t a = gg_smem(tiles) + s * STAGE, b = a + A_BYTES;
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gg_smem(&full[s])), "r"(STAGE) : "memory");
-      gg_load(a, &map_x, k * GG_BK, row0, &full[s]);
+  pdl_launch_dependents();
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      int s = 0;
+      uint32_t turn = 0;      // rounds of the ring
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+        const int side = t >= per_side, u = t - side * per_side, n0 = (u % cols) * BN, row0 = (u / cols) * GG_ROWS;
+        const CUtensorMap *mx = side ? &map_xv : &map_xk, *mw = side ? &map_wv : &map_wk;
+        for (int k = 0; k < n_k; ++k) {
+          if (turn > 0 && !(ok = gg_wait(&empty[s], (turn - 1) & 1))) break;
+          const uint32_t a = gg_smem(ring) + s * STAGE, b = a + A_BYTES;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gg_smem(&full[s])), "r"(STAGE) : "memory");
+          gg_load(a, mx, k * GG_BK, row0, &full[s]);
 #pragma unroll
-      for (int nb = 0; nb < BN / 64; ++nb) gg_load(b + nb * (64 * GG_BK * 2), &map_w, n0 + 64 * nb, k * GG_BK, &full[s]);
-    }
-  } else if (warp == 1 && lane == 0) {
-    const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-    // D fp32, A K-major, B MN-major (bit 16), M = 128, N = BN
-    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
-    bool ok = true;
-    for (int k = 0; k < n_k && ok; ++k) {
-      const int s = k % GG_STAGES;
-      ok = gg_wait(&full[s], (uint32_t)((k / GG_STAGES) & 1));
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a = gg_smem(tiles) + s * STAGE, b = a + A_BYTES;
-#pragma unroll
-      for (int ks = 0; ks < GG_BK / 16; ++ks) {
-        // A: 8-row groups 1024 bytes apart, k-step 32 bytes on; B: 64-column blocks 64 * GG_BK * 2 bytes apart, groups of
-        // 8 dims 1024 bytes apart, k-step two groups on
-        const uint64_t da = gg_desc(a + 32 * ks, 16, 1024), db = gg_desc(b + 2048 * ks, 64 * GG_BK * 2, 1024);
-        asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n}"
-                     ::"r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(k + ks > 0 ? 1u : 0u) : "memory");
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&empty[s])) : "memory");
-    }
-    if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&done)) : "memory");
-  }
-  __syncwarp();
-  bool ok = gg_wait(&done, 0);      // bounded; the verdict is the block's (tensor-memory loads are warp-collective)
-  ok = __syncthreads_and(ok) != 0;
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok) {
-    const uint32_t lane_addr = tmem + ((uint32_t)(32 * warp) << 16);
-    const int row = row0 + tid;
-    const bool native = p.native_rounding != 0;
-#pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
-      uint32_t r[32];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-          "tcgen05.wait::ld.sync.aligned;"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-            "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-            "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-            "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-          : "r"(lane_addr + c) : "memory");
-      if (row < p.n_rows) {
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) + bias_s[c + i];
-        if (native) {
-          uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.workspace) + (size_t)row * p.dim + n0 + c);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            o[i] = make_uint4(gg_pack<T>(v[8 * i], v[8 * i + 1]), gg_pack<T>(v[8 * i + 2], v[8 * i + 3]),
-                              gg_pack<T>(v[8 * i + 4], v[8 * i + 5]), gg_pack<T>(v[8 * i + 6], v[8 * i + 7]));
-        } else {
-          float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.workspace) + (size_t)row * p.dim + n0 + c);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          for (int nb = 0; nb < BN / 64; ++nb) gg_load(b + nb * (64 * GG_BK * 2), mw, n0 + 64 * nb, k * GG_BK, &full[s]);
+          if (++s == STAGES) { s = 0; ++turn; }
         }
       }
     }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+      // D fp32, A K-major, B MN-major (bit 16), M = 128, N = BN
+      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
+      bool ok = true;
+      int s = 0, j = 0;
+      uint32_t turn = 0;
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
+        if (j >= 2 && !(ok = gg_wait(&acc_empty[j & 1], (uint32_t)((j >> 1) - 1) & 1))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int k = 0; k < n_k; ++k) {
+          if (!(ok = gg_wait(&full[s], turn & 1))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = gg_smem(ring) + s * STAGE, b = a + A_BYTES;
+#pragma unroll
+          for (int ks = 0; ks < GG_BK / 16; ++ks) {
+            // A: 8-row groups 1024 bytes apart, k-step 32 bytes on; B: 64-column blocks 64 * GG_BK * 2 bytes apart, groups of
+            // 8 dims 1024 bytes apart, k-step two groups on
+            const uint64_t da = gg_desc(a + 32 * ks, 16, 1024), db = gg_desc(b + 2048 * ks, 64 * GG_BK * 2, 1024);
+            asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n}"
+                         ::"r"(tmem + (j & 1) * BN), "l"(da), "l"(db), "r"(idesc), "r"(k + ks > 0 ? 1u : 0u) : "memory");
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&empty[s])) : "memory");
+          if (++s == STAGES) { s = 0; ++turn; }
+        }
+        if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&acc_full[j & 1])) : "memory");
+      }
+    }
+  } else {
+    const int quarter = warp & 3;         // the quarter of tensor memory that the warp may read
+    unsigned char* const stage = ring + GG_RING + (warp - 2) * 4096;
+    int j = 0;
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++j) {
+      const int side = t >= per_side, u = t - side * per_side, n0 = (u % cols) * BN, row = (u / cols) * GG_ROWS + 32 * quarter + lane;
+      const dkv_gate_args& p = side ? pv : pk;
+      const T* bias = reinterpret_cast<const T*>(p.b) + n0;
+      const bool native = p.native_rounding != 0;
+      if (!__all_sync(0xffffffffu, gg_wait(&acc_full[j & 1], (uint32_t)(j >> 1) & 1))) break;      // bounded
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t lane_addr = tmem + (j & 1) * BN + ((uint32_t)(32 * quarter) << 16);
+      // 32 columns of the thread's row at a time go through the warp's 4 KB of shared memory and leave as whole 128-byte
+      // lines (16-byte pieces of 32 rows per store made the read-back as long as the products); 16-byte piece q of row r
+      // lies at (q ^ r % 8) * 16 of the row
+      const int row_base = row - lane;
+      const size_t es = native ? sizeof(T) : sizeof(float), pitch = (size_t)p.dim * es;
+      unsigned char* const out = reinterpret_cast<unsigned char*>(p.workspace) + (size_t)row_base * pitch + (size_t)n0 * es;
+      auto flush = [&](int c) {        // 128 bytes of each row from column c on
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = 4 * i + (lane >> 3), q = lane & 7;
+          if (row_base + r < p.n_rows)
+            *reinterpret_cast<uint4*>(out + r * pitch + c * es + 16 * q) = *reinterpret_cast<const uint4*>(stage + r * 128 + ((q ^ (r & 7)) << 4));
+        }
+        __syncwarp();
+      };
+#pragma unroll 1
+      for (int c = 0; c < BN; c += 32) {
+        uint32_t r[32];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+            "tcgen05.wait::ld.sync.aligned;"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+              "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+              "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+              "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+            : "r"(lane_addr + c) : "memory");
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) + to_f32(__ldg(bias + c + i));
+        if (native) {      // two rounds make a line
+          const int q0 = (c & 32) >> 3;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(stage + lane * 128 + (((q0 + i) ^ (lane & 7)) << 4)) =
+                make_uint4(gg_pack<T>(v[8 * i], v[8 * i + 1]), gg_pack<T>(v[8 * i + 2], v[8 * i + 3]),
+                           gg_pack<T>(v[8 * i + 4], v[8 * i + 5]), gg_pack<T>(v[8 * i + 6], v[8 * i + 7]));
+          if (c & 32) flush(c - 32);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<float4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          flush(c);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gg_smem(&acc_empty[j & 1])) : "memory");
+    }
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 2) {
+  if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN));
   }
 }
 
 // gate_rows_kernel: softmax, running sum, count and masked copy of a row whose logits gate_gemm_kernel left in the
 // workspace; lane l holds columns PER l .. PER l + PER - 1 in registers.  The work is one read of the logits, one of x
-// and one write of the masked row.  8192 rows x 1024, bf16: 98 us with the columns in (bank-conflicted) shared memory.
+// and one write of the masked row.  Both sides of 8192 rows x
+// 1024, bf16: 2 x 98 us with the columns in (bank-conflicted) shared memory, 2 x 15.6 in registers, 30 us in one launch;
+// bound by the ~900 instructions of a row (exp, division and the roundings that the reference makes).
 template <typename T, bool NATIVE, int PER>
-__global__ void __launch_bounds__(256) gate_rows_kernel(dkv_gate_args p) {
+__global__ void __launch_bounds__(256) gate_rows_kernel(const __grid_constant__ dkv_gate_args pk, const __grid_constant__ dkv_gate_args pv) {
+  const dkv_gate_args& p = blockIdx.y ? pv : pk;
   const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= p.n_rows) return;
+  pdl_wait();       // the logits come from gate_gemm_kernel
   constexpr int d = 32 * PER;
   const float thr = NATIVE ? to_f32(from_f32<T>(p.threshold)) : p.threshold;   // the comparison converts the scalar
   float e[PER];
   if (NATIVE) {
-    const uint2* src = reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(p.workspace) + (size_t)row * d + PER * lane);
+    constexpr int W = PER < 8 ? PER : 8;           // columns of a load
+    struct alignas(2 * W) Piece { T t[W]; };
+    const Piece* src = reinterpret_cast<const Piece*>(reinterpret_cast<const T*>(p.workspace) + (size_t)row * d + PER * lane);
 #pragma unroll
-    for (int i = 0; i < PER / 4; ++i) {
-      const uint2 v = src[i];
-      const T* t = reinterpret_cast<const T*>(&v);
+    for (int i = 0; i < PER / W; ++i) {
+      const Piece v = src[i];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) e[4 * i + k] = to_f32(t[k]);
+      for (int k = 0; k < W; ++k) e[W * i + k] = to_f32(v.t[k]);
     }
   } else {
     const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.workspace) + (size_t)row * d + PER * lane);
@@ -476,34 +527,43 @@ static bool gate_gemm_ok(const dkv_gate_args* a) {
 }
 
 template <typename T, int BN>
-static cudaError_t launch_gate_gemm(const dkv_gate_args* a, const CUtensorMap& mx, const CUtensorMap& mw, cudaStream_t st) {
-  const int smem = GG_STAGES * (GG_ROWS + BN) * GG_BK * 2 + 1024;
+static cudaError_t launch_gate_gemm(const dkv_gate_args* a, const dkv_gate_args* b, const CUtensorMap (&m)[4], int row_tiles, cudaStream_t st) {
+  const int smem = GG_RING + 4 * 4096 + 1024, n_tiles = row_tiles * (a->dim / BN);
   const cudaError_t e = cudaFuncSetAttribute(gate_gemm_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    gate_gemm_kernel<T, BN><<<dim3(a->dim / BN, (a->n_rows + GG_ROWS - 1) / GG_ROWS), 128, smem, st>>>(mx, mw, *a);
+  if (e == cudaSuccess) gate_gemm_kernel<T, BN><<<min(n_tiles, sm_count()), GG_THREADS, smem, st>>>(m[0], m[1], m[2], m[3], *a, *b, n_tiles);
   return e;
 }
+// one side (b == a), or two sides of one shape in one launch each
 template <typename T>
-static int gate_prompt(const dkv_gate_args* a) {
+static int gate_prompt(const dkv_gate_args* a, const dkv_gate_args* b) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
-  CUtensorMap mx, mw;
-  DKV_REQUIRE(tensor_map_16bit(&mx, a->dtype, a->x, (uint64_t)a->n_rows, (uint64_t)a->dim, (uint64_t)a->x_stride, GG_ROWS) &&
-                  tensor_map_16bit(&mw, a->dtype, a->w, (uint64_t)a->dim, (uint64_t)a->dim, (uint64_t)a->dim, GG_BK),
-              DKV_E_CUDA, "dkv_gate_lengths: tensor map encoding failed");
-  // 256-column tiles (their operand reads leave shared memory half idle) once they give every SM a CTA
-  const bool wide = a->dim % 256 == 0 && (long long)((a->n_rows + GG_ROWS - 1) / GG_ROWS) * (a->dim / 256) >= sm_count();
-  const cudaError_t e = wide ? launch_gate_gemm<T, 256>(a, mx, mw, st) : launch_gate_gemm<T, 128>(a, mx, mw, st);
+  const int sides = a == b ? 1 : 2;
+  CUtensorMap m[4];
+  for (int i = 0; i < 2; ++i) {
+    const dkv_gate_args* s = i ? b : a;
+    DKV_REQUIRE(tensor_map_16bit(&m[2 * i], s->dtype, s->x, (uint64_t)s->n_rows, (uint64_t)s->dim, (uint64_t)s->x_stride, GG_ROWS) &&
+                    tensor_map_16bit(&m[2 * i + 1], s->dtype, s->w, (uint64_t)s->dim, (uint64_t)s->dim, (uint64_t)s->dim, GG_BK),
+                DKV_E_CUDA, "dkv_gate_lengths: tensor map encoding failed");
+  }
+  // 256-column tiles (a quarter less through L2 per product) once they give every SM one; 256 x 256 ones, which leave no
+  // second accumulator, were slower (39 against 36 us)
+  const int row_tiles = sides * ((a->n_rows + GG_ROWS - 1) / GG_ROWS);
+  const bool wide = a->dim % 256 == 0 && (long long)row_tiles * (a->dim / 256) >= sm_count();
+  const cudaError_t e = wide ? launch_gate_gemm<T, 256>(a, b, m, row_tiles, st) : launch_gate_gemm<T, 128>(a, b, m, row_tiles, st);
   DKV_REQUIRE(e == cudaSuccess, DKV_E_CUDA, "dkv_gate_lengths: %s", cudaGetErrorString(e));
-  const int grid = (a->n_rows + 7) / 8;
-#define ROWS(NAT)                                                                    \
-  do {                                                                               \
-    if (a->dim == 128) gate_rows_kernel<T, NAT, 4><<<grid, 256, 0, st>>>(*a);        \
-    else if (a->dim == 256) gate_rows_kernel<T, NAT, 8><<<grid, 256, 0, st>>>(*a);   \
-    else if (a->dim == 512) gate_rows_kernel<T, NAT, 16><<<grid, 256, 0, st>>>(*a);  \
-    else gate_rows_kernel<T, NAT, 32><<<grid, 256, 0, st>>>(*a);                     \
+  DKV_CHECK_LAUNCH();
+  const dim3 grid((a->n_rows + 7) / 8, sides);
+  cudaError_t r = cudaSuccess;
+#define ROWS(NAT)                                                                                       \
+  do {                                                                                                  \
+    if (a->dim == 128) r = launch_pdl(gate_rows_kernel<T, NAT, 4>, grid, dim3(256), 0, st, *a, *b);       \
+    else if (a->dim == 256) r = launch_pdl(gate_rows_kernel<T, NAT, 8>, grid, dim3(256), 0, st, *a, *b);  \
+    else if (a->dim == 512) r = launch_pdl(gate_rows_kernel<T, NAT, 16>, grid, dim3(256), 0, st, *a, *b); \
+    else r = launch_pdl(gate_rows_kernel<T, NAT, 32>, grid, dim3(256), 0, st, *a, *b);                    \
   } while (0)
   if (a->native_rounding) ROWS(true); else ROWS(false);
 #undef ROWS
+  DKV_REQUIRE(r == cudaSuccess, DKV_E_CUDA, "dkv_gate_lengths: %s", cudaGetErrorString(r));
   DKV_CHECK_LAUNCH();
   return DKV_OK;
 }
@@ -521,7 +581,7 @@ extern "C" size_t dkv_gate_workspace_bytes(const dkv_gate_args* a) {
   return (size_t)dkv::gate_chunks(a) * (size_t)a->n_rows * (size_t)a->dim * sizeof(float);
 }
 
-extern "C" int dkv_gate_lengths(const dkv_gate_args* a) {
+static int check_gate(const dkv_gate_args* a) {
   using namespace dkv;
   DKV_REQUIRE(a != nullptr, DKV_E_ARG, "dkv_gate_lengths: null args");
   DKV_REQUIRE(a->dtype >= DKV_F32 && a->dtype <= DKV_BF16, DKV_E_ARG, "dkv_gate_lengths: bad dtype %d", a->dtype);
@@ -530,11 +590,17 @@ extern "C" int dkv_gate_lengths(const dkv_gate_args* a) {
   DKV_REQUIRE(a->x && a->w && a->b && a->lengths, DKV_E_ARG, "dkv_gate_lengths: null input");
   DKV_REQUIRE(a->x_stride >= a->dim && (!a->masked || a->masked_stride >= a->dim), DKV_E_ARG,
               "dkv_gate_lengths: row strides must be at least dim");
-  if (a->n_rows == 0) return DKV_OK;
-  DKV_REQUIRE(a->workspace != nullptr && a->workspace_bytes >= dkv_gate_workspace_bytes(a), DKV_E_WORKSPACE,
+  DKV_REQUIRE(a->n_rows == 0 || (a->workspace != nullptr && a->workspace_bytes >= dkv_gate_workspace_bytes(a)), DKV_E_WORKSPACE,
               "dkv_gate_lengths: workspace too small: need %zu bytes, got %zu", dkv_gate_workspace_bytes(a), a->workspace_bytes);
   DKV_REQUIRE((a->n_rows + GATE_ROWS - 1) / GATE_ROWS <= 65535, DKV_E_LIMIT, "dkv_gate_lengths: at most %d rows per call", 65535 * GATE_ROWS);
-  if (gate_gemm_ok(a)) return a->dtype == DKV_F16 ? gate_prompt<__half>(a) : gate_prompt<__nv_bfloat16>(a);
+  return DKV_OK;
+}
+
+extern "C" int dkv_gate_lengths(const dkv_gate_args* a) {
+  using namespace dkv;
+  if (int rc = check_gate(a)) return rc;
+  if (a->n_rows == 0) return DKV_OK;
+  if (gate_gemm_ok(a)) return a->dtype == DKV_F16 ? gate_prompt<__half>(a, a) : gate_prompt<__nv_bfloat16>(a, a);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const int n_chunks = gate_chunks(a);
   const int chunk_len = n_chunks == 1 ? a->dim : GATE_TILE;
@@ -557,6 +623,18 @@ extern "C" int dkv_gate_lengths(const dkv_gate_args* a) {
 #undef LAUNCH
   DKV_CHECK_LAUNCH();
   return DKV_OK;
+}
+
+extern "C" int dkv_gate_lengths_both(const dkv_gate_args* k, const dkv_gate_args* v) {
+  using namespace dkv;
+  if (int rc = check_gate(k)) return rc;
+  if (int rc = check_gate(v)) return rc;
+  // one shape and rounding, and scratch of their own: one launch of each kernel takes both sides
+  if (k->n_rows > 0 && k->dtype == v->dtype && k->dim == v->dim && k->n_rows == v->n_rows && k->stream == v->stream &&
+      k->native_rounding == v->native_rounding && k->workspace != v->workspace && gate_gemm_ok(k) && gate_gemm_ok(v))
+    return k->dtype == DKV_F16 ? gate_prompt<__half>(k, v) : gate_prompt<__nv_bfloat16>(k, v);
+  if (int rc = dkv_gate_lengths(k)) return rc;
+  return dkv_gate_lengths(v);
 }
 
 extern "C" int dkv_gate_lengths_pair(const dkv_gate_args* k, const dkv_gate_args* v) {

@@ -309,53 +309,87 @@ PyObject* grow(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// gate(states, weight, bias, low_rank, threshold, return_masked, len_multiple, native_rounding) -> (masked|None, lengths)
-PyObject* gate(PyObject*, PyObject* const* v, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
-  if (n != 8 || !is_tensor(v[0]) || !unpack(v[0]).is_cuda()) Py_RETURN_NONE;
-  const int dev = unpack(v[0]).get_device();
-  for (int i = 0; i < 3; ++i)
-    if (!plain(v[i], dev)) Py_RETURN_NONE;
-  const at::Tensor &x = unpack(v[0]), &w = unpack(v[1]), &b = unpack(v[2]);
-  const auto dt = x.scalar_type();
+// One side of the gate: argument struct from tensors, outputs and scratch allocated; false for anything but the plain case.
+struct GateSide {
   dkv_gate_args a = {};
+  at::Tensor lengths, masked, ws;
+};
+bool gate_side(GateSide& g, PyObject* const* t, long low_rank, double threshold, bool want, long len_multiple, bool native) {
+  if (!is_tensor(t[0]) || !unpack(t[0]).is_cuda()) return false;
+  const int dev = unpack(t[0]).get_device();
+  for (int i = 0; i < 3; ++i)
+    if (!plain(t[i], dev)) return false;
+  const at::Tensor &x = unpack(t[0]), &w = unpack(t[1]), &b = unpack(t[2]);
+  const auto dt = x.scalar_type();
+  dkv_gate_args& a = g.a;
   a.dtype = dtype_code(dt);
-  if (a.dtype < 0 || x.dim() < 1 || !x.is_contiguous() || !w.is_contiguous() || !b.is_contiguous() || w.scalar_type() != dt || b.scalar_type() != dt) Py_RETURN_NONE;
+  if (a.dtype < 0 || x.dim() < 1 || !x.is_contiguous() || !w.is_contiguous() || !b.is_contiguous() || w.scalar_type() != dt || b.scalar_type() != dt) return false;
   const int64_t d = x.size(-1);
-  if (d == 0 || w.dim() != 2 || w.size(0) != d || w.size(1) != d || b.numel() != d) Py_RETURN_NONE;
+  if (d == 0 || w.dim() != 2 || w.size(0) != d || w.size(1) != d || b.numel() != d) return false;
   a.n_rows = (int32_t)(x.numel() / d);
   a.dim = (int32_t)d;
-  a.low_rank = (int32_t)PyLong_AsLong(v[3]);
-  a.threshold = (float)PyFloat_AsDouble(v[4]);
-  const bool want = v[5] == Py_True;
-  a.len_multiple = (int32_t)PyLong_AsLong(v[6]);
-  a.native_rounding = v[7] == Py_True ? 1 : 0;
-  if (PyErr_Occurred()) return nullptr;
+  a.low_rank = (int32_t)low_rank;
+  a.threshold = (float)threshold;
+  a.len_multiple = (int32_t)len_multiple;
+  a.native_rounding = native ? 1 : 0;
   a.x = x.data_ptr();
   a.x_stride = d;
   a.w = w.data_ptr();
   a.b = b.data_ptr();
-  at::Tensor lengths = at::empty(x.sizes().slice(0, x.dim() - 1), x.options().dtype(at::kInt)), masked;
-  a.lengths = static_cast<int32_t*>(lengths.data_ptr());
+  g.lengths = empty(x.sizes().slice(0, x.dim() - 1), at::kInt, x.device());
+  a.lengths = static_cast<int32_t*>(g.lengths.data_ptr());
   if (want) {
-    masked = at::empty(x.sizes(), x.options());
-    a.masked = masked.data_ptr();
+    g.masked = empty(x.sizes(), dt, x.device());
+    a.masked = g.masked.data_ptr();
     a.masked_stride = d;
   }
   const size_t need = std::max<size_t>(dkv_gate_workspace_bytes(&a), 16);
-  at::Tensor ws = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
-  a.workspace = ws.data_ptr();
+  g.ws = empty({(int64_t)need}, at::kByte, x.device());
+  a.workspace = g.ws.data_ptr();
   a.workspace_bytes = need;
   a.stream = stream_of(dev);
-  if (int rc = dkv_gate_lengths(&a)) return fail("dkv_gate_lengths", rc);
+  return true;
+}
+
+// gate(states, weight, bias, low_rank, threshold, return_masked, len_multiple, native_rounding) -> (masked|None, lengths)
+PyObject* gate(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 8) Py_RETURN_NONE;
+  const long low_rank = PyLong_AsLong(v[3]), len_multiple = PyLong_AsLong(v[6]);
+  const double threshold = PyFloat_AsDouble(v[4]);
+  if (PyErr_Occurred()) return nullptr;
+  const bool want = v[5] == Py_True;
+  GateSide g;
+  if (!gate_side(g, v, low_rank, threshold, want, len_multiple, v[7] == Py_True)) Py_RETURN_NONE;
+  if (int rc = dkv_gate_lengths(&g.a)) return fail("dkv_gate_lengths", rc);
   PyObject* r = PyTuple_New(2);
   if (want) {
-    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(masked));
+    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(g.masked));
   } else {
     Py_INCREF(Py_None);
     PyTuple_SET_ITEM(r, 0, Py_None);
   }
-  PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(lengths));
+  PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(g.lengths));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// gate_both(k, Wk, bk, v, Wv, bv, low_rank, threshold, len_multiple) -> (masked k, masked v, lengths k, lengths v)
+PyObject* gate_both(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 9) Py_RETURN_NONE;
+  const long low_rank = PyLong_AsLong(v[6]), len_multiple = PyLong_AsLong(v[8]);
+  const double threshold = PyFloat_AsDouble(v[7]);
+  if (PyErr_Occurred()) return nullptr;
+  GateSide g[2];
+  for (int i = 0; i < 2; ++i)
+    if (!gate_side(g[i], v + 3 * i, low_rank, threshold, true, len_multiple, true)) Py_RETURN_NONE;
+  if (int rc = dkv_gate_lengths_both(&g[0].a, &g[1].a)) return fail("dkv_gate_lengths_both", rc);
+  PyObject* r = PyTuple_New(4);
+  for (int i = 0; i < 2; ++i) {
+    PyTuple_SET_ITEM(r, i, THPVariable_Wrap(g[i].masked));
+    PyTuple_SET_ITEM(r, 2 + i, THPVariable_Wrap(g[i].lengths));
+  }
   return r;
   END_HANDLE_TH_ERRORS
 }
@@ -379,6 +413,7 @@ PyMethodDef methods[] = {{"attend", FAST(attend), "decode attention"},
                          {"new_state", FAST(new_state), "buffers of a new cache layer"},
                          {"grow", FAST(grow), "a cache buffer with more columns"},
                          {"gate", FAST(gate), "cutoff gate of one side"},
+                         {"gate_both", FAST(gate_both), "cutoff gate of both sides"},
                          {"set_status", FAST(set_status_word), "status word of a device"},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host side of dynakv_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};

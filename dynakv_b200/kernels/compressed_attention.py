@@ -154,6 +154,10 @@ def kv_process_fused(key_states: torch.Tensor, value_states: torch.Tensor, Wk, b
                      len_multiple: int = 1):
     """Drop-in for the reference module method of the same name (kernels/compressed_attention.py:84-119):
     returns (k_out, v_out, len_k, len_v, 1, 1) for key_states / value_states [B, S, d]."""
+    if key_states.is_cuda:
+        done = _lib.host().gate_both(key_states, Wk, bk, value_states, Wv, bv, low_rank, 0.1, len_multiple)
+        if done is not None:        # else: tensors that have to be copied first, or refused
+            return *done, 1, 1
     k_out, len_k = gate_lengths(key_states, Wk, bk, low_rank, len_multiple=len_multiple)
     v_out, len_v = gate_lengths(value_states, Wv, bv, low_rank, len_multiple=len_multiple)
     return k_out, v_out, len_k, len_v, 1, 1

@@ -286,6 +286,10 @@ typedef struct dkv_gate_args {
 size_t dkv_gate_workspace_bytes(const dkv_gate_args* args);
 int dkv_gate_lengths(const dkv_gate_args* args);
 
+/* dkv_gate_lengths of two sides (kv_process_fused); sides of one shape over many 16-bit rows share their launches.  Each
+ * side has a workspace of its own. */
+int dkv_gate_lengths_both(const dkv_gate_args* k, const dkv_gate_args* v);
+
 /* The gate for narrow rows (dim <= 128: one row per (sequence, KV head), the decode shape of the per-head layout),
  * K and V sides in ONE launch and without a workspace: same arithmetic, in the same order, as dkv_gate_lengths on
  * each side (kv_process_fused computes both sides in one call too, compressed_attention.py:92-114).  The two

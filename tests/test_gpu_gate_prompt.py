@@ -25,3 +25,15 @@ def test_gate_of_a_prompt_against_oracle(rows, d, low_rank, pad, dtype):
     assert torch.equal(masked.cpu(), torch.where(keep, x, torch.zeros_like(x)))
     _, lens8 = gate_lengths(wide.cuda()[:, :d], W.cuda(), b.cuda(), low_rank, native_rounding=False, len_multiple=8, return_masked=False)
     assert torch.equal(lens8, torch.clamp((lens + 7) // 8 * 8, max=d))
+
+
+@pytest.mark.parametrize("rows,d", [(70, 128), (1000, 512), (3000, 1024)])
+def test_both_sides_in_one_launch_give_what_each_gives(rows, d):
+    from dynakv_b200.kernels.compressed_attention import gate_lengths, kv_process_fused
+    gen = torch.Generator().manual_seed(rows)
+    side = lambda: (torch.randn(2, rows // 2, d, generator=gen).bfloat16().cuda(), (torch.randn(d, d, generator=gen) / d ** 0.5).bfloat16().cuda(),
+                    torch.randn(1, d, generator=gen).bfloat16().cuda())
+    (k, wk, bk), (v, wv, bv) = side(), side()
+    k_out, v_out, len_k, len_v, _, _ = kv_process_fused(k, v, wk, bk, wv, bv, d)
+    for (out, lens), got in ((gate_lengths(k, wk, bk, d), (k_out, len_k)), (gate_lengths(v, wv, bv, d), (v_out, len_v))):
+        assert torch.equal(out, got[0]) and torch.equal(lens, got[1])

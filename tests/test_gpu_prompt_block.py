@@ -18,7 +18,7 @@ def test_blocks_grow_and_expand_like_the_layout_oracle(R, step, dtype):
     cache = CustomDynamicCache(arenas_per_batch=A, len_multiple=step)
     cache.reserve(0, B, 8 * R, 64, dtype, "cuda")           # the second block does not fit: the buffers grow behind it
     lays = [O.LayoutOracle(B * A, np.float32) for _ in range(2)]
-    for n_new, counts in ((5, None), (37, None), (1, None), (300, None)):
+    for n_new, counts in ((5, None), (37, None), (1, None), (300, None), (4200, None)):
         rows = [torch.randn(B, n_new, A * R, generator=gen).to(dtype) for _ in range(2)]
         lens = [(torch.randint(0, R // step + 1, (B, A, n_new), generator=gen) * step).to(torch.int32) for _ in range(2)]
         cache.update_sp(rows[0].cuda(), lens[0].cuda(), rows[1].cuda(), lens[1].cuda(), A * R, 0, R, token_counts=counts)
