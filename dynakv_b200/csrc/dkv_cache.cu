@@ -151,31 +151,51 @@ __global__ void __launch_bounds__(256) append_project_grid_kernel(dkv_append_arg
   const int b = blockIdx.y, item = blockIdx.x, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int A = p.arenas_per_batch;
+  const int side_idx = item / A, j = item - side_idx * A;
+  const dkv_side& sd = side_idx ? p.v : p.k;
+  const int a = b * A + j;
+  const T* src = reinterpret_cast<const T*>(side_idx ? p.new_v : p.new_k) + (size_t)a * 128;
+  const T* basis = reinterpret_cast<const T*>(side_idx ? p.v_basis : p.k_basis) + (size_t)j * 128 * 128;
+  // The row, the basis rows of the first round and the metadata are asked for together: one trip to memory, not three
+  // (decode step of 4 short rows through 32 layers: 748 -> 660 us).
+  struct alignas(4 * sizeof(T)) Four { T t[4]; };
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(basis)) & (sizeof(Four) - 1)) == 0;
+  auto load4 = [&](const T* at) {
+    Four f;
+    if (vec) {
+      f = *reinterpret_cast<const Four*>(at);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f.t[e] = at[e];
+    }
+    return f;
+  };
+  Four xr = load4(src + lane * 4), rows[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) rows[u] = load4(basis + (size_t)(warp * 8 + u) * 128 + lane * 4);
   const int pos = p.seq_lens ? p.seq_lens[b] : p.seq_pos;
+  const int off = sd.ptr[a], given = (side_idx ? p.len_v : p.len_k)[a];
   const bool pos_ok = pos >= 0 && pos < p.seq_capacity;
   if (!pos_ok && tid == 0 && item == 0) set_status(p.status, DKV_ST_OVERFLOW);
   if (pos_ok) {
-    const int side_idx = item / A, j = item - side_idx * A;
-    const dkv_side& sd = side_idx ? p.v : p.k;
-    const int a = b * A + j;
-    const T* src = reinterpret_cast<const T*>(side_idx ? p.new_v : p.new_k) + (size_t)a * 128;
-    const int len = checked_len((side_idx ? p.len_v : p.len_k)[a], 128, p.len_multiple, p.status, tid);
-    const int off = sd.ptr[a];
+    const int len = checked_len(given, 128, p.len_multiple, p.status, tid);
     const bool fits = (int64_t)off + len <= sd.flat_stride;
     if (fits) {
       T* dst = reinterpret_cast<T*>(sd.flat) + (size_t)a * sd.flat_stride + off;
-      const T* basis = reinterpret_cast<const T*>(side_idx ? p.v_basis : p.k_basis) + (size_t)j * 128 * 128;
       float x[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) x[e] = to_f32(src[lane * 4 + e]);
+      for (int e = 0; e < 4; ++e) x[e] = to_f32(xr.t[e]);
       for (int r0 = warp * 8; r0 < len; r0 += 64) {
+        if (r0 != warp * 8) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) rows[u] = load4(basis + (size_t)(r0 + u) * 128 + lane * 4);   // r0 + u < 128 always (len <= 128, step 8)
+        }
         float acc[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const T* row = basis + (size_t)(r0 + u) * 128 + lane * 4;   // r0 + u < 128 always (len <= 128, step 8)
           float s = 0.f;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s = fmaf(x[e], to_f32(row[e]), s);
+          for (int e = 0; e < 4; ++e) s = fmaf(x[e], to_f32(rows[u].t[e]), s);
           acc[u] = s;
         }
 #pragma unroll
