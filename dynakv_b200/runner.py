@@ -144,13 +144,16 @@ class MiniLlama:
         self.layers: List[_LayerWeights] = []
         for li in range(s.layers):
             w = _LayerWeights()
-            w.wqkv = torch.cat((normal(s.hidden, s.n_q_heads * D)[:, kv_lo * G * D: kv_hi * G * D],
-                                normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D],
-                                normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D]), dim=1)
+            w.wqkv = torch.empty(s.hidden, (self.q_local + 2 * self.kv_local) * D, dtype=dtype, device=self.device)
             w.wq, w.wk, w.wv = w.wqkv.split((self.q_local * D, self.kv_local * D, self.kv_local * D), dim=1)
+            w.wq.copy_(normal(s.hidden, s.n_q_heads * D)[:, kv_lo * G * D: kv_hi * G * D])
+            w.wk.copy_(normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D])
+            w.wv.copy_(normal(s.hidden, s.n_kv_heads * D)[:, kv_lo * D: kv_hi * D])
             w.wo = normal(s.n_q_heads * D, s.hidden)[kv_lo * G * D: kv_hi * G * D].contiguous()
-            w.wgu = torch.cat((normal(s.hidden, s.mlp)[:, m_lo:m_hi], normal(s.hidden, s.mlp)[:, m_lo:m_hi]), dim=1)
+            w.wgu = torch.empty(s.hidden, 2 * (m_hi - m_lo), dtype=dtype, device=self.device)
             w.wg, w.wu = w.wgu.split(m_hi - m_lo, dim=1)
+            w.wg.copy_(normal(s.hidden, s.mlp)[:, m_lo:m_hi])
+            w.wu.copy_(normal(s.hidden, s.mlp)[:, m_lo:m_hi])
             w.wd = normal(s.mlp, s.hidden)[m_lo:m_hi].contiguous()
             w.norm1 = torch.ones(s.hidden, dtype=dtype, device=self.device)
             w.norm2 = torch.ones(s.hidden, dtype=dtype, device=self.device)
