@@ -309,6 +309,166 @@ PyObject* grow(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// A cache layer's state list [flat, lens, offs, ptr, tokens, bounds] of plain tensors on `dev`, as a side of the C ABI.
+bool state_side(PyObject* st, int dev, at::ScalarType dt, int64_t rows, dkv_side& s, int64_t& cap) {
+  if (!PyList_Check(st) || PyList_GET_SIZE(st) != 6) return false;
+  for (int i = 0; i < 4; ++i)
+    if (!plain(PyList_GET_ITEM(st, i), dev)) return false;
+  const at::Tensor& ptr = unpack(PyList_GET_ITEM(st, 3));
+  int64_t r;
+  const at::Tensor& flat = unpack(PyList_GET_ITEM(st, 0));
+  if (flat.scalar_type() != dt || !fill_side(s, flat, unpack(PyList_GET_ITEM(st, 1)), unpack(PyList_GET_ITEM(st, 2)), r, cap) || r != rows ||
+      ptr.scalar_type() != at::kInt || ptr.numel() != rows || !ptr.is_contiguous())
+    return false;
+  s.ptr = static_cast<int32_t*>(ptr.data_ptr());
+  return true;
+}
+
+// The arguments that both block calls share: k_state|None, v_state|None, key_states, key_len, value_states, value_len, arenas,
+// row width, len_multiple, first position, row counts|None, row counter|None.
+constexpr Py_ssize_t BLOCK_ARGS = 12;
+bool block_sides(PyObject* const* v, dkv_pack_args (&a)[2]) {
+  if (!is_tensor(v[2]) || !unpack(v[2]).is_cuda()) return false;
+  const int dev = unpack(v[2]).get_device();
+  if (dev < 0 || dev >= MAX_DEVICES || g_status[dev] == nullptr) return false;
+  const int64_t A = PyLong_AsLong(v[6]);
+  for (int sd = 0; sd < 2; ++sd) {
+    if (!plain(v[2 + 2 * sd], dev) || !plain(v[3 + 2 * sd], dev)) return false;
+    const at::Tensor &x = unpack(v[2 + 2 * sd]), &l = unpack(v[3 + 2 * sd]);
+    dkv_pack_args& p = a[sd];
+    p = {};
+    p.dtype = dtype_code(x.scalar_type());
+    if (p.dtype < 0 || x.dim() != 3 || x.stride(2) != 1 || x.sizes() != unpack(v[2]).sizes() || l.dim() != 2 || l.size(0) != x.size(0) * A ||
+        l.size(1) != x.size(1) || l.scalar_type() != at::kInt || !l.is_contiguous())
+      return false;
+    p.batch = (int32_t)x.size(0);
+    p.arenas_per_batch = (int32_t)A;
+    p.n_new = (int32_t)x.size(1);
+    p.max_dim = (int32_t)PyLong_AsLong(v[7]);
+    p.states = x.data_ptr();
+    p.stride_b = x.stride(0);
+    p.stride_j = p.max_dim;
+    p.stride_s = x.stride(1);
+    p.new_lens = static_cast<const int32_t*>(l.data_ptr());
+    p.len_multiple = (int32_t)PyLong_AsLong(v[8]);
+    p.seq_pos = (int32_t)PyLong_AsLong(v[9]);
+    if (v[10] != Py_None) p.row_counts = static_cast<const int32_t*>(unpack(v[10]).data_ptr());
+    if (v[11] != Py_None) p.seq_lens = static_cast<const int32_t*>(unpack(v[11]).data_ptr());
+    p.status = g_status[dev];
+    p.stream = stream_of(dev);
+    if (v[sd] != Py_None) {
+      int64_t cap;
+      if (!state_side(v[sd], dev, x.scalar_type(), l.size(0), p.side, cap)) return false;
+      p.seq_capacity = (int32_t)cap;
+    }
+  }
+  return true;
+}
+int pack_sides(const dkv_pack_args (&a)[2], long sides) {
+  return sides == 3 ? dkv_pack_pair(&a[0], &a[1]) : sides == 1 ? dkv_pack_bulk(&a[0]) : sides == 2 ? dkv_pack_bulk(&a[1]) : 0;
+}
+
+// block_begin(...) -> per side (largest sum of lengths given, largest write pointer, largest end, write pointers, ends): the
+// rows' totals on the host.  Sides that have a state are packed behind the copy (nothing flagged), before it is waited for.
+PyObject* block_begin(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  dkv_pack_args a[2];
+  if (n != BLOCK_ARGS || !block_sides(v, a)) Py_RETURN_NONE;
+  if (PyErr_Occurred()) return nullptr;
+  const at::Tensor& x = unpack(v[2]);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t rows = (int64_t)a[0].batch * a[0].arenas_per_batch;
+  const at::Tensor totals = empty({2, rows, 4}, at::kInt, x.device());
+  const at::Tensor host = at::empty({2, rows, 4}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  cudaStream_t st = static_cast<cudaStream_t>(a[0].stream);
+  if (int rc = dkv_row_totals(&a[0], &a[1], static_cast<int32_t*>(totals.data_ptr()))) return fail("dkv_row_totals", rc);
+  cudaEvent_t here = nullptr;
+  cudaError_t e = cudaMemcpyAsync(host.data_ptr(), totals.data_ptr(), host.nbytes(), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&here, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(here, st);
+  int rc = 0;
+  if (e == cudaSuccess) {
+    for (dkv_pack_args& p : a) p.status = nullptr;
+    rc = pack_sides(a, (v[0] != Py_None ? 1 : 0) | (v[1] != Py_None ? 2 : 0));
+    Py_BEGIN_ALLOW_THREADS
+    e = cudaEventSynchronize(here);
+    Py_END_ALLOW_THREADS
+  }
+  if (here) cudaEventDestroy(here);
+  if (rc) return fail("dkv_pack_bulk", rc);
+  if (e != cudaSuccess) {
+    PyErr_Format(PyExc_RuntimeError, "reading a block's totals failed: %s", cudaGetErrorString(e));
+    return nullptr;
+  }
+  PyObject* r = PyTuple_New(2);
+  for (int sd = 0; sd < 2; ++sd) {
+    const int32_t* t = static_cast<const int32_t*>(host.data_ptr()) + sd * rows * 4;
+    long raw = 0, now = 0, end = 0;
+    PyObject *ptrs = PyList_New(rows), *ends = PyList_New(rows);
+    for (int64_t i = 0; i < rows; ++i) {
+      const long p = t[4 * i + 2], q = p + t[4 * i + 1];
+      raw = std::max(raw, (long)t[4 * i]);
+      now = std::max(now, p);
+      end = std::max(end, q);
+      PyList_SET_ITEM(ptrs, i, PyLong_FromLong(p));
+      PyList_SET_ITEM(ends, i, PyLong_FromLong(q));
+    }
+    PyTuple_SET_ITEM(r, sd, Py_BuildValue("(lllNN)", raw, now, end, ptrs, ends));
+  }
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// block_pack(..., sides): 1 = K, 2 = V, 3 = both
+PyObject* block_pack(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  dkv_pack_args a[2];
+  if (n != BLOCK_ARGS + 1 || !block_sides(v, a)) Py_RETURN_NONE;
+  const long sides = PyLong_AsLong(v[BLOCK_ARGS]);
+  if (PyErr_Occurred()) return nullptr;
+  if (int rc = pack_sides(a, sides)) return fail("dkv_pack_bulk", rc);
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+// views(k_state, v_state) -> (flat_k, flat_v, lens_k, lens_v, offs_k, offs_v), metadata cut at the tokens stored
+PyObject* views(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2) Py_RETURN_NONE;
+  at::Tensor t[6];
+  for (int sd = 0; sd < 2; ++sd) {
+    if (!PyList_Check(v[sd]) || PyList_GET_SIZE(v[sd]) != 6) Py_RETURN_NONE;
+    const int64_t s = PyLong_AsLong(PyList_GET_ITEM(v[sd], 4));
+    for (int i = 0; i < 3; ++i) {
+      PyObject* o = PyList_GET_ITEM(v[sd], i);
+      if (!THPVariable_CheckExact(o) || unpack(o).dim() != 2 || unpack(o).requires_grad() || (i && unpack(o).size(1) < s)) Py_RETURN_NONE;
+      t[2 * i + sd] = i ? rows_view(unpack(o), 0, {unpack(o).size(0), s}, unpack(o).strides()) : unpack(o);
+    }
+  }
+  if (PyErr_Occurred()) return nullptr;
+  PyObject* r = PyTuple_New(6);
+  for (int i = 0; i < 6; ++i) PyTuple_SET_ITEM(r, i, THPVariable_Wrap(t[i]));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// expand(state, max_dim) -> dense zero-padded rows [rows, tokens stored, max_dim]
+PyObject* expand(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2 || !PyList_Check(v[0]) || PyList_GET_SIZE(v[0]) != 6 || !is_tensor(PyList_GET_ITEM(v[0], 0)) || !unpack(PyList_GET_ITEM(v[0], 0)).is_cuda()) Py_RETURN_NONE;
+  const at::Tensor& flat = unpack(PyList_GET_ITEM(v[0], 0));
+  const int64_t s = PyLong_AsLong(PyList_GET_ITEM(v[0], 4)), dim = PyLong_AsLong(v[1]), rows = flat.size(0);
+  if (PyErr_Occurred()) return nullptr;
+  dkv_side side = {};
+  int64_t cap;
+  if (dim < 1 || dtype_code(flat.scalar_type()) < 0 || !state_side(v[0], flat.get_device(), flat.scalar_type(), rows, side, cap) || s > cap) Py_RETURN_NONE;
+  const at::Tensor dense = empty({rows, s, dim}, flat.scalar_type(), flat.device());
+  if (int rc = dkv_decompress(dtype_code(flat.scalar_type()), (int32_t)rows, (int32_t)s, (int32_t)dim, &side, dense.data_ptr(), stream_of(flat.get_device())))
+    return fail("dkv_decompress", rc);
+  return THPVariable_Wrap(dense);
+  END_HANDLE_TH_ERRORS
+}
+
 // One side of the gate: argument struct from tensors, outputs and scratch allocated; false for anything but the plain case.
 struct GateSide {
   dkv_gate_args a = {};
@@ -412,6 +572,10 @@ PyMethodDef methods[] = {{"attend", FAST(attend), "decode attention"},
                          {"append_token", FAST(append_token), "decode append"},
                          {"new_state", FAST(new_state), "buffers of a new cache layer"},
                          {"grow", FAST(grow), "a cache buffer with more columns"},
+                         {"block_begin", FAST(block_begin), "totals of a block of tokens, first attempt at its pack"},
+                         {"block_pack", FAST(block_pack), "pack of a block of tokens"},
+                         {"views", FAST(views), "a layer's tensors, cut at the tokens stored"},
+                         {"expand", FAST(expand), "dense rows of a layer's side"},
                          {"gate", FAST(gate), "cutoff gate of one side"},
                          {"gate_both", FAST(gate_both), "cutoff gate of both sides"},
                          {"set_status", FAST(set_status_word), "status word of a device"},

@@ -105,6 +105,10 @@ class CustomDynamicCache:
 
     def get_origin_states(self, max_dim, layer_idx):
         c_k, c_v = self.key_cache_sp[layer_idx], self.value_cache_sp[layer_idx]
+        if c_k[0].is_cuda:
+            dense = [_lib.host().expand(c, max_dim) for c in (c_k, c_v)]
+            if dense[0] is not None and dense[1] is not None:
+                return tuple(dense)
         seq = c_k[4]
         k = simple_decompress(c_k[0], c_k[1][:, :seq], max_dim, c_k[2][:, :seq])
         v = simple_decompress(c_v[0], c_v[1][:, :seq], max_dim, c_v[2][:, :seq])
@@ -284,84 +288,60 @@ class CustomDynamicCache:
         rows' totals and write pointers on the host: one kernel collects them for both sides, one copy brings them over,
         and when the layer already has buffers the pack is queued behind that copy without waiting for it -- a block that
         does not fit leaves nothing behind that the repeated pack into the grown buffers does not overwrite."""
-        lib, A, dev = _lib.load(), self.arenas_per_batch, key_states.device
+        A, dev, host = self.arenas_per_batch, key_states.device, _lib.host()
         B, n_new = key_states.shape[0], key_states.shape[1]
-        rows, dt, stream = B * A, _lib.dtype_code(key_states.dtype), _lib.stream_ptr(dev)
-        st = status_word(dev).data_ptr()
+        status_word(dev)
         lists = (self.key_cache_sp, self.value_cache_sp)
         for cache_list in lists:
             while len(cache_list) <= layer_idx:
                 cache_list.append(None)
-        fresh = [lst[layer_idx] is None for lst in lists]
-        seq_ptr = 0 if fresh[0] else lists[0][layer_idx][4]
+        states = [lst[layer_idx] for lst in lists]
+        seq_ptr = 0 if states[0] is None else states[0][4]
         counts = None if token_counts is None else [int(c) for c in token_counts]
         row_counter = self._row_counter(layer_idx, B, dev, seq_ptr, token_counts)
         counts_dev = None
         if counts is not None and any(c != n_new for c in counts):
             counts_dev = torch.tensor(counts, dtype=torch.int32, device=dev)
-        for lst, new in zip(lists, fresh):
-            if not new and lst[layer_idx][4] + n_new > lst[layer_idx][1].shape[1]:
-                c = lst[layer_idx]
+        for c in states:
+            if c is not None and c[4] + n_new > c[1].shape[1]:
                 self._ensure_capacity(c, c[0].shape[1], max(c[1].shape[1] + EXPAND_SEQ_STEP, c[4] + n_new))
-        args = []
-        keep = []
-        for states, lens in ((key_states, kl), (value_states, vl)):
-            if states.stride(2) != 1:
-                states = states.contiguous()
-            keep.append(states)
-            p = _lib.PackArgs()
-            p.dtype, p.batch, p.arenas_per_batch, p.n_new, p.max_dim = dt, B, A, n_new, row_dim
-            p.states, p.stride_b, p.stride_j, p.stride_s = states.data_ptr(), states.stride(0), row_dim, states.stride(1)
-            p.new_lens = lens.data_ptr()
-            p.row_counts = _lib.ptr(counts_dev)
-            p.seq_lens = _lib.ptr(row_counter)
-            p.seq_pos, p.len_multiple, p.status, p.stream = seq_ptr, self.len_multiple, st, stream
-            args.append(p)
-
-        def pack(sides, status):
-            for side in sides:
-                cache, p = lists[side][layer_idx], args[side]
-                p.side, p.seq_capacity, p.status = self._side(cache), cache[1].shape[1], status
-            if len(sides) == 2:
-                _lib.check(lib.dkv_pack_pair(C.byref(args[0]), C.byref(args[1])), "dkv_pack_pair")
-            elif sides:
-                _lib.check(lib.dkv_pack_bulk(C.byref(args[sides[0]])), "dkv_pack_bulk")
-
-        for side in (0, 1):
-            if not fresh[side]:
-                args[side].side = self._side(lists[side][layer_idx])
-        totals = torch.empty((2, rows, 4), dtype=torch.int32, device=dev)
-        _lib.check(lib.dkv_row_totals(C.byref(args[0]), C.byref(args[1]), totals.data_ptr()), "dkv_row_totals")
-        host = torch.empty((2, rows, 4), dtype=torch.int32, pin_memory=True)
-        host.copy_(totals, non_blocking=True)
-        here = torch.cuda.Event()
-        here.record(torch.cuda.current_stream(dev))
-        pack([side for side in (0, 1) if not fresh[side]], None)
-        again = []
-        here.synchronize()
-        for side, lst in enumerate(lists):
-            raw, stored, now, _ = host[side].t().tolist()
-            if fresh[side]:
-                lst[layer_idx] = self._new_state(rows, _round8(max(raw)), n_new, key_states.dtype, dev)      # exact fit
-            cache = lst[layer_idx]
-            max_added = max(raw) if n_new > 1 else width
-            grow = max(now) + max_added > cache[0].shape[1]
+        # plain detached tensors, dense in the last axis: what the native side takes
+        block = [t if t.stride(2) == 1 else t.contiguous() for t in (key_states.detach(), value_states.detach())]
+        if not all(type(t) is torch.Tensor for t in (*block, kl, vl)):
+            block = [t.as_subclass(torch.Tensor) for t in block]
+            kl, vl = kl.detach().as_subclass(torch.Tensor), vl.detach().as_subclass(torch.Tensor)
+        block = (block[0], kl, block[1], vl, A, row_dim, self.len_multiple, seq_ptr, counts_dev, row_counter)
+        totals = host.block_begin(*states, *block)
+        if totals is None:
+            raise ValueError("a block needs key and value states of one shape and dtype, on the device and in the dtype of the layer")
+        again = 0
+        for side, (raw, now, end, ptrs, ends) in enumerate(totals):
+            cache = states[side]
+            if fresh := cache is None:
+                cache = lists[side][layer_idx] = self._new_state(B * A, _round8(raw), n_new, key_states.dtype, dev)      # exact fit
+                states[side] = cache
+            max_added = raw if n_new > 1 else width
+            grow = now + max_added > cache[0].shape[1]
             if grow:
                 step = EXPAND_SEQ_STEP * (width // 2)
-                self._ensure_capacity(cache, _round8(max(cache[0].shape[1] + step, max(now) + max_added)), cache[1].shape[1])
-                cache[3].copy_(host[side, :, 2].contiguous())     # rows of the first attempt that did fit moved on
+                self._ensure_capacity(cache, _round8(max(cache[0].shape[1] + step, now + max_added)), cache[1].shape[1])
+                cache[3].copy_(torch.tensor(ptrs, dtype=torch.int32))     # rows of the first attempt that did fit moved on
             cap = cache[0].shape[1]
-            if fresh[side] or grow:
-                again.append(side)
-            elif max(n + s_ for n, s_ in zip(now, stored)) > cap:     # lengths made valid no longer fit: recorded as empty
+            if fresh or grow:
+                again |= 1 << side
+            elif end > cap:     # lengths made valid no longer fit: recorded as empty
                 status_word(dev).bitwise_or_(_lib.ST_OVERFLOW)
             cache[4] = seq_ptr + n_new
-            cache[5] = [n + s_ if n + s_ <= cap else n for n, s_ in zip(now, stored)]
-        pack(again, st)
+            cache[5] = ends if end <= cap else [e if e <= cap else n for n, e in zip(ptrs, ends)]
+        if again:
+            host.block_pack(*states, *block, again)
         if row_counter is not None:
             row_counter.add_(counts_dev if counts_dev is not None else n_new)
             self._seq_lens_host[layer_idx] = [n + (counts[b] if counts is not None else n_new)
                                               for b, n in enumerate(self._seq_lens_host[layer_idx])]
-        ck, cv = lists[0][layer_idx], lists[1][layer_idx]
+        ck, cv = states
+        done = host.views(ck, cv)
+        if done is not None:
+            return done
         s = ck[4]
         return ck[0], cv[0], ck[1][:, :s], cv[1][:, :s], ck[2][:, :s], cv[2][:, :s]
