@@ -48,9 +48,26 @@ extern "C" int dkv_version(void) { return DKV_VERSION; }
 
 extern "C" const char* dkv_last_error(void) { return g_err; }
 
+namespace dkv {
+// Whether the fused entry is better off as split + merge.  One-kernel paths take whole rows and queue them up, the split grid
+// cuts the same tiles evenly: better once the (row, KV head) pairs fill the SMs twice for the short kernel, of which two fit
+// an SM (8 KV heads, 128 tokens: 32 rows 15.9 against 19.6 us, 64 rows 32 against 28.5), and once for the fused pipeline
+// (499 tokens: 16 rows 17 against 20 us, 32 rows 32 against 26, 64 rows 65 against 40).
+static bool fused_by_split(const dkv_attn_args* a) {
+  const int n_sm = a->n_sm > 0 ? a->n_sm : sm_count();
+  return (long long)a->batch * a->n_basis_groups > (short_ok(a) ? 2LL : 1LL) * n_sm;
+}
+}  // namespace dkv
+
 extern "C" int dkv_fused_decode(const dkv_attn_args* a) {
   if (int rc = check_attn_args(a, "dkv_fused_decode", true, true, true)) return rc;
-  if (mma_path_ok(a)) return short_ok(a) ? short_fused(a) : mma_fused(a);
+  if (mma_path_ok(a)) {
+    if (fused_by_split(a) && a->workspace != nullptr && a->workspace_bytes >= mma_split_workspace_bytes(a) && ((uintptr_t)a->workspace & 15) == 0) {
+      if (int rc = mma_split(a)) return rc;
+      return mma_combine(a);
+    }
+    return short_ok(a) ? short_fused(a) : mma_fused(a);
+  }
   return generic_attention(a);
 }
 
@@ -61,7 +78,9 @@ extern "C" size_t dkv_split_workspace_bytes(const dkv_attn_args* a) {
 }
 
 extern "C" size_t dkv_fused_workspace_bytes(const dkv_attn_args* a) {
-  return a == nullptr || mma_path_ok(a) ? 0 : tiles_workspace_bytes(a);
+  if (a == nullptr) return 0;
+  if (!mma_path_ok(a)) return tiles_workspace_bytes(a);
+  return fused_by_split(a) ? mma_split_workspace_bytes(a) : 0;
 }
 
 extern "C" int dkv_split_decode(const dkv_attn_args* a) {
@@ -84,6 +103,20 @@ extern "C" int dkv_two_stage_decode(const dkv_attn_args* a) {
   if (!mma_path_ok(a)) return generic_attention(a);
   if (int rc = mma_split(a)) return rc;
   return mma_combine(a);
+}
+
+extern "C" int dkv_routed_decode(const dkv_attn_args* a, int32_t switch_tokens) {
+  if (int rc = check_attn_args(a, "dkv_routed_decode", true, true, true)) return rc;
+  DKV_REQUIRE(a->seq_lens != nullptr && switch_tokens > 0, DKV_E_ARG, "dkv_routed_decode: needs seq_lens and a switch point");
+  dkv_attn_args s = *a, l = *a;
+  s.route_min_tokens = l.route_max_tokens = 0;
+  s.route_max_tokens = l.route_min_tokens = switch_tokens;
+  if (mma_path_ok(a) && fused_by_split(&s)) {      // the short rows would go through split and merge as well: one pass for all
+    l.route_min_tokens = 0;
+    return dkv_two_stage_decode(&l);
+  }
+  if (int rc = dkv_fused_decode(&s)) return rc;
+  return dkv_two_stage_decode(&l);
 }
 
 extern "C" int dkv_two_stage_decode_noalloc(const dkv_attn_args* a) {

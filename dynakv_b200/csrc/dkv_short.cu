@@ -8,7 +8,8 @@
 // cluster has CTAs are walked with a running softmax.)  Everything that does not depend on the kernel before this one
 // (basis, tensor memory, barriers) is set up before griddepcontrol.wait.
 // Per launch in a chain (8 KV heads, bf16), against the warp-specialised pipeline of dkv_mma_decode.cu, one CTA per row:
-// B = 1, 499 tokens 16.1 -> 10.7 us; B = 4, 1 token 12.1 -> 10.2, 499 tokens 16.3 -> 12.0; B = 64, 128 tokens 49.5 -> 32.1.
+// B = 1, 499 tokens 16.1 -> 10.7 us; B = 4, 1 token 12.1 -> 10.2, 499 tokens 16.3 -> 12.0; B = 64, 128 tokens 49.5 -> 32.1 (with a
+// workspace such batches go through the split kernel).
 //
 // Reference math: src/dynakv/kernels/fused.py:28-142.
 #include <math.h>

@@ -85,7 +85,8 @@ PyObject* fail(const char* what, int rc) {
 }
 
 // attend(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, theta, out|None, seq_lens|None, batch_index|None,
-//        k_norm_weight|None, k_norm_eps, len_multiple, route_min, route_max, two_stage) -> out
+//        k_norm_weight|None, k_norm_eps, len_multiple, route_min, route_max, two_stage) -> out; an integer in place of the last
+// is a switch point: every row through the kernel of its own length
 PyObject* attend(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 19 || !is_tensor(v[0]) || !unpack(v[0]).is_cuda()) Py_RETURN_NONE;
@@ -155,16 +156,19 @@ PyObject* attend(PyObject*, PyObject* const* v, Py_ssize_t n) {
   a.out = out.data_ptr();
   a.out_stride_b = out.stride(0);
   a.out_stride_h = out.stride(1);
-  const bool two_stage = v[18] == Py_True;
-  const size_t need = two_stage ? dkv_split_workspace_bytes(&a) : dkv_fused_workspace_bytes(&a);
+  const bool two_stage = v[18] == Py_True, routed = !PyBool_Check(v[18]);
+  const long switch_tokens = routed ? PyLong_AsLong(v[18]) : 0;
+  if (PyErr_Occurred()) return nullptr;
+  if (routed && a.seq_lens == nullptr) Py_RETURN_NONE;
+  const size_t need = two_stage || routed ? dkv_split_workspace_bytes(&a) : dkv_fused_workspace_bytes(&a);
   at::Tensor ws;
   if (need) {
     ws = empty({(int64_t)need}, at::kByte, q.device());
     a.workspace = ws.data_ptr();
     a.workspace_bytes = need;
   }
-  const int rc = two_stage ? dkv_two_stage_decode(&a) : dkv_fused_decode(&a);
-  if (rc) return fail(two_stage ? "dkv_two_stage_decode" : "dkv_fused_decode", rc);
+  const int rc = routed ? dkv_routed_decode(&a, (int32_t)switch_tokens) : two_stage ? dkv_two_stage_decode(&a) : dkv_fused_decode(&a);
+  if (rc) return fail(routed ? "dkv_routed_decode" : two_stage ? "dkv_two_stage_decode" : "dkv_fused_decode", rc);
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }

@@ -222,11 +222,12 @@ class CompressedDecodeLayer:
 
     def attend(self, cache: CustomDynamicCache, q: torch.Tensor, out: torch.Tensor, row_counter: torch.Tensor,
                seq_columns: int, route: str, route_min_tokens: int = 0, route_max_tokens: int = 0,
-               prepare_only: bool = False, workspace: Optional[torch.Tensor] = None) -> int:
-        """Attention of all batch rows through one kernel (``route``); with routing bounds the kernel skips the rows
-        whose current length (read from ``row_counter`` on the device) belongs to the other kernel.  ``workspace`` is
+               prepare_only: bool = False, workspace: Optional[torch.Tensor] = None):
+        """Attention of all batch rows through one kernel (``route``), or with ``"routed"`` every row through the kernel of
+        its current length (read from ``row_counter`` on the device) by the policy's switch point.  With routing bounds a
+        single kernel skips the rows that belong to the other one.  ``workspace`` is
         scratch the caller keeps for calls that follow one another on one stream; the bytes the call needs are returned
-        (``prepare_only``: nothing else happens)."""
+        (``prepare_only``: nothing is launched, and the number of launches is returned beside them)."""
         ck, cv = cache.key_cache_sp[self.layer_idx], cache.value_cache_sp[self.layer_idx]
         args, keep = build_attn_args(
             q, ck[0], self.k_up, cv[0], self.v_up, ck[1][:, :seq_columns], ck[2][:, :seq_columns],
@@ -236,8 +237,14 @@ class CompressedDecodeLayer:
             route_min_tokens=route_min_tokens, route_max_tokens=route_max_tokens, workspace=workspace)
         lib = _lib.load()
         if prepare_only:
-            return int(lib.dkv_split_workspace_bytes(C.byref(args)))
-        if route == "short_fused":
+            need = int(lib.dkv_split_workspace_bytes(C.byref(args)))
+            if route == "routed":
+                args.route_max_tokens = self.policy.switch_tokens
+            by_split = lib.dkv_fused_workspace_bytes(C.byref(args)) > 0       # short rows through split and merge
+            return need, {"long_two_stage": 2, "short_fused": 2 if by_split else 1, "routed": 2 if by_split else 3}[route]
+        if route == "routed":
+            _lib.check(lib.dkv_routed_decode(C.byref(args), self.policy.switch_tokens), "dkv_routed_decode")
+        elif route == "short_fused":
             _lib.check(lib.dkv_fused_decode(C.byref(args)), "dkv_fused_decode")
         else:
             _lib.check(lib.dkv_two_stage_decode(C.byref(args)), "dkv_two_stage_decode")
@@ -275,8 +282,6 @@ class DecodeGraph:
         self._has_short = any(int(n) + 1 < switch for n in seq_lens_host)
         self._has_long = reach >= switch
         self._switch = switch
-        self.kernel_launches_per_step = L * (1 + (1 if self._has_short else 0) + (2 if self._has_long else 0)) + \
-            sum(1 for l in self.layers if l.gate is not None)     # the gate of both sides is one launch
         for l in self.layers:       # size the gate's scratch and the append's tickets before any capture
             l.prepare(batch, self.device)
             if l.gate is not None:
@@ -285,10 +290,12 @@ class DecodeGraph:
         status_word(self.device)
         # one scratch for all layers' attention, before any capture: they follow one another
         self._workspace: Optional[torch.Tensor] = None
-        self._workspace = torch.empty(max(self._run_layers(prepare_only=True), 16), dtype=torch.uint8, device=self.device)
+        need, launches = self._run_layers(prepare_only=True)
+        self._workspace = torch.empty(max(need, 16), dtype=torch.uint8, device=self.device)
+        self.kernel_launches_per_step = launches + L + sum(1 for l in self.layers if l.gate is not None)     # appends; the gate of both sides is one launch
 
-    def _run_layers(self, prepare_only: bool = False) -> int:
-        need = 0
+    def _run_layers(self, prepare_only: bool = False):
+        need, launches = 0, 0
         for li, layer in enumerate(self.layers):
             ck = self.cache.key_cache_sp[layer.layer_idx]
             counter = self.cache.seq_lens(layer.layer_idx)
@@ -297,16 +304,12 @@ class DecodeGraph:
             cap = ck[1].shape[1]
             if not prepare_only:
                 layer.append(self.cache, self.new_k[li], self.new_v[li], self.len_k[li], self.len_v[li], counter, cap)
-            both = self._has_short and self._has_long
-            if self._has_short:
-                need = max(need, layer.attend(self.cache, self.q[li], self.out[li], counter, cap, "short_fused",
-                                              route_max_tokens=self._switch if both else 0, prepare_only=prepare_only,
-                                              workspace=self._workspace))
-            if self._has_long:
-                need = max(need, layer.attend(self.cache, self.q[li], self.out[li], counter, cap, "long_two_stage",
-                                              route_min_tokens=self._switch if both else 0, prepare_only=prepare_only,
-                                              workspace=self._workspace))
-        return need
+            route = "routed" if self._has_short and self._has_long else "short_fused" if self._has_short else "long_two_stage"
+            used = layer.attend(self.cache, self.q[li], self.out[li], counter, cap, route, prepare_only=prepare_only,
+                                workspace=self._workspace)
+            if prepare_only:
+                need, launches = max(need, used[0]), launches + used[1]
+        return need, launches
 
     def capture(self) -> None:
         """Capture one decode step.  Nothing is executed: the cache is left as it is."""

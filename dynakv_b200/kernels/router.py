@@ -16,6 +16,7 @@ from typing import Optional, Sequence
 
 import torch
 
+from .. import _lib
 from . import fused as _fused, two_stage as _two_stage
 
 
@@ -62,12 +63,16 @@ def compressed_decode_attention(
     common = dict(k_norm_weight=k_norm_weight, k_norm_eps=k_norm_eps, len_multiple=len_multiple, seq_lens=seq_lens)
 
     # per-row routing on the device
-    q3 = q.squeeze(2) if q.dim() == 4 else q
-    out = torch.empty((q3.shape[0], q3.shape[1], q3.shape[2]), dtype=q3.dtype, device=q3.device)
     any_short, any_long = True, True
     if seq_lens_host is not None:
         short, long_ = policy.partition(seq_lens_host)
         any_short, any_long = bool(short), bool(long_)
+    if any_short and any_long and q.is_cuda:
+        done = _lib.host().attend(*args, None, seq_lens, None, k_norm_weight, k_norm_eps, len_multiple, 0, 0, int(policy.switch_tokens))
+        if done is not None:        # else: tensors that have to be copied first, or refused
+            return done
+    q3 = q.squeeze(2) if q.dim() == 4 else q
+    out = torch.empty((q3.shape[0], q3.shape[1], q3.shape[2]), dtype=q3.dtype, device=q3.device)
     if any_short:
         _fused.fused_attention_dispatch(*args, out=out, route_max_tokens=policy.switch_tokens if any_long else 0, **common)
     if any_long:

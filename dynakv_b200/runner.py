@@ -262,13 +262,11 @@ class MiniLlama:
         out = torch.empty(B, self.q_local, D, dtype=self.dtype, device=self.device)
         layer = self.attn[li]
         layer.append(self.cache, new_k, new_v, len_k, len_v, counter, cap)
-        routes = [("long_two_stage", dict(route_min_tokens=self.policy.switch_tokens if has_short else 0))]
-        if has_short:     # rows only grow: the long kernels are always there, the short one while a row needs it
-            routes.insert(0, ("short_fused", dict(route_max_tokens=self.policy.switch_tokens)))
-        for route, bounds in routes:      # the layers follow one another: one scratch for all of them, sized by the first calls
-            used = layer.attend(self.cache, q, out, counter, cap, route, workspace=self._workspace, **bounds)
-            if (self._workspace is None or self._workspace.numel() < used) and not torch.cuda.is_current_stream_capturing():
-                self._workspace = torch.empty(used, dtype=torch.uint8, device=self.device)
+        # rows only grow: the long kernels are always there, the short one while a row needs it; the layers follow one another:
+        # one scratch for all of them, sized by the first calls
+        used = layer.attend(self.cache, q, out, counter, cap, "routed" if has_short else "long_two_stage", workspace=self._workspace)
+        if (self._workspace is None or self._workspace.numel() < used) and not torch.cuda.is_current_stream_capturing():
+            self._workspace = torch.empty(used, dtype=torch.uint8, device=self.device)
         if self.trace is not None:
             self.trace.append((li, q.clone(), out.clone()))
         return out.view(B, -1) @ w.wo

@@ -44,3 +44,21 @@ def test_heads_per_group_and_bases(hq, rank, shift):
 
 def test_one_tile_rows_of_more_ctas_than_the_gpu_holds():
     _run([128] * 150 + [5] * 50, torch.bfloat16, 16, 4)
+
+
+@pytest.mark.parametrize("seq", [[1, 130, 499, 500, 640] * 8, [256] * 40], ids=["straddling", "short"])
+def test_batches_whose_rows_go_through_the_split(seq):
+    # 40 rows x 8 KV heads of more than one tile: past the line where the fused entry becomes split and merge
+    from dynakv_b200.kernels.router import compressed_decode_attention
+    c = synthetic.make_layer_case(5, seq, "beta:2,5", 5e5, torch.bfloat16, "cpu")
+    fk, fv, lk, lv, ok, ov = c.views()
+    ref = O.compact_attention(c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov, c.theta, seq_lens=seq)
+    d = [t.cuda() for t in (c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov)]
+    lens = torch.tensor(seq, dtype=torch.int32, device="cuda")
+    outs = [fused_attention_dispatch(*d, c.theta, seq_lens=lens, len_multiple=8)]
+    outs.append(compressed_decode_attention(q=d[0], k_flat=d[1], k_up=d[2], v_flat=d[3], v_up=d[4], key_lengths=d[5], key_offsets=d[6],
+                                            value_lengths=d[7], value_offsets=d[8], theta=c.theta, cache_length=max(seq), seq_lens=lens,
+                                            len_multiple=8))
+    for out in outs:
+        assert float((out.float().cpu() - ref).abs().max()) <= 2e-2
+    assert _common.read_status(torch.device("cuda")) == 0
