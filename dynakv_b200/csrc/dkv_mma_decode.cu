@@ -957,15 +957,25 @@ __global__ void __launch_bounds__(512, 2) split_combine_kernel(dkv_attn_args p) 
   if (p.route_min_tokens > 0 || p.route_max_tokens > 0) {      // launched behind the split kernel: the row may belong to the other kernel
     if (row_routed_out(p, p.batch_index ? p.batch_index[i] : i)) return;
   }
-  // Bv pieces of this thread: rows tid/16 + 32 j, columns 8 (tid % 16) .. +8
+  // Bv pieces of this thread: rows tid/16 + 32 j, columns 8 (tid % 16) .. +8; element by element when the basis does not
+  // start on a 16-byte boundary (every row does when the first one does)
   const int c8 = tid & 15, row0 = tid >> 4;
   uint4 bv[4];
   {
     const T* vup = reinterpret_cast<const T*>(p.v_up) + (size_t)g * R * D;
+    const bool vec = (reinterpret_cast<uintptr_t>(p.v_up) & 15) == 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int row = row0 + 32 * j;
-      bv[j] = row < R ? __ldg(reinterpret_cast<const uint4*>(vup + (size_t)row * D) + c8) : make_uint4(0u, 0u, 0u, 0u);
+      bv[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < R) {
+        if (vec) {
+          bv[j] = __ldg(reinterpret_cast<const uint4*>(vup + (size_t)row * D) + c8);
+        } else {
+          const uint16_t* e = reinterpret_cast<const uint16_t*>(vup + (size_t)row * D + 8 * c8);
+          bv[j] = make_uint4(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16, e[4] | (uint32_t)e[5] << 16, e[6] | (uint32_t)e[7] << 16);
+        }
+      }
     }
   }
   pdl_wait();

@@ -6,12 +6,13 @@ import torch
 from dynakv_b200 import synthetic
 from dynakv_b200.kernels import _common
 from dynakv_b200.kernels.fused import fused_attention_dispatch
+from dynakv_b200.kernels.two_stage import two_stage_attention
 from oracle import dynakv_oracle as O
 
 pytestmark = pytest.mark.gpu
 
 
-def _run(seq, dtype, hq, hkv, knorm=False, rank=128, shift=False):
+def _run(seq, dtype, hq, hkv, knorm=False, rank=128, shift=False, entry=fused_attention_dispatch):
     c = synthetic.make_layer_case(sum(seq) + hq, seq, "beta:2,5", 5e5, dtype, "cpu", n_q_heads=hq, n_kv_heads=hkv)
     fk, fv, lk, lv, ok, ov = c.views()
     k_up, v_up = c.k_up, c.v_up
@@ -26,7 +27,7 @@ def _run(seq, dtype, hq, hkv, knorm=False, rank=128, shift=False):
         buf[1:].copy_(v_up.cuda().view(-1))
         d[4] = buf[1:].view(v_up.shape)
     kw = {} if knw is None else dict(k_norm_weight=knw.cuda())
-    out = fused_attention_dispatch(*d, c.theta, seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda"), len_multiple=8, **kw).float().cpu()
+    out = entry(*d, c.theta, seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda"), len_multiple=8, **kw).float().cpu()
     assert float((out - torch.nan_to_num(ref)).abs().max()) <= 2e-2 * max(1.0, float(torch.nan_to_num(ref).abs().max()))
     assert _common.read_status(torch.device("cuda")) == (4 if 0 in seq else 0)      # an empty row is reported
 
@@ -40,6 +41,17 @@ def test_tile_and_cluster_edges(seq, dtype):
 @pytest.mark.parametrize("hq,rank,shift", [(2, 128, False), (4, 64, False), (6, 40, True), (8, 128, True)])
 def test_heads_per_group_and_bases(hq, rank, shift):
     _run([300, 70], torch.bfloat16, hq, 2, rank=rank, shift=shift)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("rows,rank", [(18, 128), (19, 128), (40, 120)])
+def test_shifted_bases_on_both_sides_of_the_split(rows, rank, dtype):
+    # 8 KV heads, 300 tokens: one kernel up to 148 (row, head) pairs, split and merge past them
+    _run([300, 140] * (rows // 2) + [1] * (rows % 2), dtype, 32, 8, rank=rank, shift=True)
+
+
+def test_shifted_bases_of_one_long_row():
+    _run([3000], torch.bfloat16, 8, 2, shift=True, entry=two_stage_attention)
 
 
 def test_one_tile_rows_of_more_ctas_than_the_gpu_holds():
