@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(AM_THREADS) argmax_rows_kernel(const T* x, int
   __shared__ int mi[AM_THREADS / 32], ci[AM_CLUSTER];
   const int r = blockIdx.x / parts, part = blockIdx.x - r * parts;
   const T* row = x + (size_t)r * stride;
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");     // the first CTA's shared memory is there once it has started
   float best = -INFINITY;
   int at = n;
   auto take = [&](float v, int i) {
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(AM_THREADS) argmax_rows_kernel(const T* x, int
   over_lanes();
   if ((threadIdx.x & 31) == 0) { mv[threadIdx.x >> 5] = best; mi[threadIdx.x >> 5] = at; }
   __syncthreads();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   if (threadIdx.x < 32) {
     best = -INFINITY;
     at = n;

@@ -51,3 +51,11 @@ def test_silu_and_argmax(rows, n, dtype):
     _close(runner._silu_mul(gu), F.silu(gu[:, :n]) * gu[:, n:], dtype)
     x = gu[:, :n]           # 16-bit rows of odd lengths start off a 16-byte boundary; few values, so many ties
     assert torch.equal(runner._argmax_rows(x).cpu(), torch.tensor([int((r == r.max()).nonzero()[0]) for r in x.float().cpu()]))
+
+
+def test_argmax_of_more_clusters_than_the_gpu_holds():
+    # 1500 rows x 4 CTAs: the CTAs of a cluster start while others of the launch still run
+    x = torch.randint(-50, 50, (1500, 30000), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    x[torch.arange(1500), torch.arange(1500) * 19 % 30000] = 60.0
+    for _ in range(3):
+        assert torch.equal(runner._argmax_rows(x).cpu(), torch.arange(1500) * 19 % 30000)
