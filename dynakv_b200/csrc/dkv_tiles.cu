@@ -397,6 +397,9 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
   const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, HA = Hq / A;
   const int row_arena = blockIdx.x / n_split, sl = blockIdx.x - row_arena * n_split, i_row = row_arena / A, j = row_arena - i_row * A;
   const int rb = blockIdx.y % r_blocks, head0 = j * HA + (blockIdx.y / r_blocks) * NH, nh = min(NH, (j + 1) * HA - head0);
+  // Behind the score kernel, which started when everything before it had ended, the rows' indices and lengths may be read
+  // at once; the operator follows whatever the caller ran last -- an append, say, that moves seq_lens on.
+  if (src.ws == nullptr) pdl_wait();
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
   if (row_routed_out(p, b)) return;
   pdl_launch_dependents();
@@ -635,6 +638,9 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_f32_kernel(dkv_attn_args p
   const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, HA = Hq / A;
   const int row_arena = blockIdx.x / n_split, sl = blockIdx.x - row_arena * n_split, i_row = row_arena / A, j = row_arena - i_row * A;
   const int rb = blockIdx.y % r_blocks, head0 = j * HA + (blockIdx.y / r_blocks) * NH, nh = min(NH, (j + 1) * HA - head0);
+  // Behind the score kernel, which started when everything before it had ended, the rows' indices and lengths may be read
+  // at once; the operator follows whatever the caller ran last -- an append, say, that moves seq_lens on.
+  if (src.ws == nullptr) pdl_wait();
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
   if (row_routed_out(p, b)) return;
   pdl_launch_dependents();

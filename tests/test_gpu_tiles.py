@@ -73,3 +73,36 @@ def test_ragged_rows_over_several_slices(dtype):
     out = two_stage_attention(*args, 500000.0, seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda")).float().cpu()
     assert float((out - torch.nan_to_num(ref)).abs().max()) <= (2e-4 if dtype == torch.float32 else 2e-2)
     assert _common.read_status(torch.device("cuda")) == 4       # the empty row is reported
+
+
+def test_softmax_operator_reads_the_counter_behind_an_append():
+    # the append lets the kernel behind it start early and moves the rows' counters on at its end
+    import ctypes as C
+
+    from dynakv_b200 import _lib, synthetic
+    from dynakv_b200.kernels._common import build_attn_args
+    from dynakv_b200.kernels.compressed_attention import CompressedDecodeLayer
+    from dynakv_b200.kernels.compressed_cache import CustomDynamicCache
+    B, H, n, steps = 4, 8, 20, 12
+    c = synthetic.make_layer_case(9, [n] * B, "beta:2,5", 5e5, torch.bfloat16, "cuda", extra_tokens=steps)
+    cache = CustomDynamicCache(arenas_per_batch=H, len_multiple=8)
+    cache.adopt(0, (c.k.flat, c.k.lens, c.k.offs, c.k.ptr), (c.v.flat, c.v.lens, c.v.offs, c.v.ptr), [n] * B)
+    layer = CompressedDecodeLayer(0, c.k_up, c.v_up, 5e5, project_new_rows=True)
+    layer.prepare(B, "cuda")
+    flat, lens, offs = cache.value_cache_sp[0][:3]
+    cap, counter = lens.shape[1], cache.seq_lens(0)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    scores = torch.arange(cap, device="cuda").float().expand(B, 32, cap).contiguous().bfloat16()      # the last token weighs most
+    lengths = torch.full((B, H), 64, dtype=torch.int32, device="cuda")
+    for step in range(1, steps + 1):
+        new = torch.randn(B, H, 128, generator=gen, device="cuda").bfloat16()
+        out = torch.empty(B, 32, 128, dtype=torch.bfloat16, device="cuda")
+        args, keep = build_attn_args(None, None, None, flat, c.v_up, None, None, lens, offs, 1e4, out=out, seq_lens=counter, need_workspace=True)
+        torch.cuda.synchronize()
+        layer.append(cache, new, new, lengths, lengths, counter, cap)
+        _lib.check(_lib.load().dkv_softmax_v(C.byref(args), scores.data_ptr(), scores.stride(0), scores.stride(1)), "dkv_softmax_v")
+        del keep
+        s = n + step
+        ref = O.softmax_v_reference(scores[:, :, :s].float().cpu(), flat.float().cpu(), c.v_up.float().cpu(), lens[:, :s].cpu(), offs[:, :s].cpu())
+        assert float((out.float().cpu() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
+    assert _common.read_status(torch.device("cuda")) == 0
