@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(256) decompress_vec_kernel(dkv_side sd, T* den
           if (e >= keep) t[e] = T(0);
       }
     } else {
-      T t[E];
+      __align__(16) T t[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) t[e] = e < keep ? src[e] : T(0);
       v[k] = *reinterpret_cast<const uint4*>(t);

@@ -142,7 +142,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
               if (vec) {
                 v = __ldg(reinterpret_cast<const uint4*>(kup + (size_t)r * GD) + c);
               } else {
-                T tmp[8];
+                __align__(16) T tmp[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) tmp[i] = kup[(size_t)r * GD + 8 * c + i];
                 v = *reinterpret_cast<const uint4*>(tmp);

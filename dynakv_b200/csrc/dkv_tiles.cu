@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
       if (b_vec) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ts_smem(dst)), "l"(kup + (size_t)min(r, R - 1) * TD + 8 * d), "r"(r < R ? 16 : 0) : "memory");
       } else {
-        T v[8];
+        __align__(16) T v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = r < R ? kup[(size_t)r * TD + 8 * d + k] : from_f32<T>(0.f);
         *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
