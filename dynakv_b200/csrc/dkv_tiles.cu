@@ -1,7 +1,7 @@
 // Attention over caches that the packed tensor-core kernel does not take: fp32, the joint latent row shared by all heads
 // (rank up to 1024), any integer lengths, strided metadata.  Three kernels instead of one CTA per (row, query head):
-//   1. scores, one CTA per (batch row, token tile, basis group): the tile's K is reconstructed once for all query heads of
-//      the group, rotated and multiplied with each of them; fp32 scores go to the workspace (or, for the score operator,
+//   1. scores, one CTA per (batch row, token tile, heads that share a basis and an arena): the tile's K is reconstructed once
+//      for these query heads, rotated and multiplied with each of them; fp32 scores go to the workspace (or, for the score operator,
 //      out in the query type);
 //   2. latent sum, one CTA per (token slice, block of 128 latent coefficients, arena): the V rows are read once for all
 //      heads of the arena; a slice leaves a partial record (m, l, latent accumulator) per head;
@@ -17,6 +17,7 @@
 // the single-kernel path for callers without a workspace.
 #include <math.h>
 
+#include <numeric>
 #include <type_traits>
 
 #include "dkv_common.cuh"
@@ -122,6 +123,7 @@ __device__ __forceinline__ void token_meta(const dkv_attn_args& p, const dkv_sid
 struct ScoreSink {
   float* ws;             // fp32 workspace [batch, Hq, pitch], or NULL: out in the query type, masked as the reference does
   int64_t pitch;
+  int heads;             // consecutive query heads of a CTA, all of one basis group and one arena
 };
 
 // --------------------------------------------------------------- 1. scores, 16-bit types
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tile = (p.seq_len + TS_TOK - 1) / TS_TOK, i_row = blockIdx.x / n_tile, g = blockIdx.y, t0 = (blockIdx.x - i_row * n_tile) * TS_TOK;
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
-  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = Hq / p.n_basis_groups;
+  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = sink.heads;
   if (sink.ws && row_routed_out(p, b)) return;
   const int t_end = sink.ws ? row_len(p, b) : p.seq_len;     // the operator writes every column
   if (t0 >= t_end) return;
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
   const uint32_t tmem = sm.tmem;
   const int rmax = sm.rmax, n_chunk = (rmax + TS_CHUNK - 1) / TS_CHUNK;
   const T* flat = reinterpret_cast<const T*>(p.k.flat) + (size_t)a * p.k.flat_stride;
-  const T* kup = reinterpret_cast<const T*>(p.k_up) + (size_t)g * R * TD;
+  const T* kup = reinterpret_cast<const T*>(p.k_up) + (size_t)(g * G / (Hq / p.n_basis_groups)) * R * TD;
   const bool b_vec = (reinterpret_cast<uintptr_t>(p.k_up) & 15) == 0;
   // X pieces of this thread: tokens (tid & 7) + 8 * (tid >> 5) + 64 u', pieces ((tid >> 3) & 3) + 4 u: eight lanes with
   // consecutive tokens write 128 consecutive bytes, four lanes read 64 consecutive bytes of a row
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tile = (p.seq_len + TF_TOK - 1) / TF_TOK, i_row = blockIdx.x / n_tile, g = blockIdx.y, t0 = (blockIdx.x - i_row * n_tile) * TF_TOK;
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
-  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = Hq / p.n_basis_groups;
+  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = sink.heads;
   if (sink.ws && row_routed_out(p, b)) return;
   const int t_end = sink.ws ? row_len(p, b) : p.seq_len;
   if (t0 >= t_end) return;
@@ -561,7 +563,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   }
   __syncthreads();
   const float* flat = reinterpret_cast<const float*>(p.k.flat) + (size_t)a * p.k.flat_stride;
-  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)g * R * TD;
+  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(g * G / (Hq / p.n_basis_groups)) * R * TD;
   const int d = tid & 127, th = tid >> 7, rmax = rmax_s;
   float acc[8];
 #pragma unroll
@@ -828,11 +830,12 @@ int launch_scores(const dkv_attn_args* a, float* ws) {
   if (a->batch == 0 || a->seq_len == 0) return DKV_OK;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const float log_theta = (float)log((double)a->theta);
-  const ScoreSink sink{ws, score_pitch(a)};
+  const int heads = std::gcd(a->n_q_heads / a->n_basis_groups, a->n_q_heads / a->arenas_per_batch);
+  const ScoreSink sink{ws, score_pitch(a), heads};
   const int tok = a->dtype == DKV_F32 ? TF_TOK : TS_TOK;
   const long long ctas = (long long)a->batch * ((a->seq_len + tok - 1) / tok);
-  DKV_REQUIRE(ctas <= 2147483647LL && a->n_basis_groups <= 65535, DKV_E_LIMIT, "too many tokens or basis groups");
-  const dim3 grid((unsigned)ctas, a->n_basis_groups);
+  DKV_REQUIRE(ctas <= 2147483647LL, DKV_E_LIMIT, "too many tokens");
+  const dim3 grid((unsigned)ctas, a->n_q_heads / heads);      // (n_q_heads <= 65535)
   const int smem = (int)sizeof(ScoreSmem) + 128;
   if (a->dtype == DKV_F32) {
     tile_scores_f32_kernel<<<grid, TS_THREADS, 0, st>>>(*a, sink, log_theta);

@@ -39,7 +39,9 @@ def _dev(t, shift):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
 @pytest.mark.parametrize("B,S,R,Hq,groups,arenas,shift", [
     (1, 1, 8, 4, 1, 1, 0), (2, 127, 63, 8, 2, 2, 0), (1, 129, 64, 12, 1, 1, 1), (3, 33, 819, 32, 8, 1, 0), (1, 300, 1024, 40, 40, 1, 0),
-    (1, 130, 513, 36, 4, 1, 1)])
+    (1, 130, 513, 36, 4, 1, 1),
+    # one basis for several arenas, basis groups that straddle arenas
+    (2, 70, 24, 8, 1, 4, 0), (1, 150, 100, 12, 2, 3, 0), (2, 129, 64, 24, 4, 3, 1), (1, 260, 128, 32, 2, 32, 0)])
 def test_tile_kernels_against_oracle(B, S, R, Hq, groups, arenas, shift, dtype):
     t = _case(S + R, B, S, R, Hq, groups, arenas, dtype)
     d = _dev(t, shift)
