@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
 
   // A routed launch may have nothing to do (split: no row of the batch is long; fused: this row is): such a CTA leaves
   // before the set-up, which costs it ~6 us -- a launch of 148 idle CTAs took 7.8 us of every layer of a short batch.
-  if (FUSED ? p.route_max_tokens > 0 : p.route_min_tokens > 0) {
+  // (A fused CTA has one row: either bound may rule it out, and then nothing of it is written or reported.)
+  if (p.route_min_tokens > 0 || (FUSED && p.route_max_tokens > 0)) {
     pdl_wait();
     if (FUSED) {
       if (row_routed_out(p, p.batch_index ? p.batch_index[blockIdx.x] : (int)blockIdx.x)) return;

@@ -74,3 +74,24 @@ def test_batches_whose_rows_go_through_the_split(seq):
     for out in outs:
         assert float((out.float().cpu() - ref).abs().max()) <= 2e-2
     assert _common.read_status(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("bounds", [dict(route_min_tokens=200), dict(route_max_tokens=200), dict(route_min_tokens=100, route_max_tokens=300)],
+                         ids=["min", "max", "both"])
+@pytest.mark.parametrize("rows", [2, 16, 24])
+def test_rows_out_of_bounds_are_left_alone(rows, bounds):
+    # 499 columns, 8 KV heads: the short kernel's cluster, the pipeline of one CTA per row, split and merge
+    seq = [(0, 60, 199, 200, 299, 300, 499)[i % 7] for i in range(rows)]
+    c = synthetic.make_layer_case(7, seq, "beta:2,5", 5e5, torch.bfloat16, "cpu")
+    fk, fv, lk, lv, ok, ov = c.views()
+    ref = O.compact_attention(c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov, c.theta, seq_lens=seq)
+    out = torch.full(c.q.shape, 7.0, dtype=torch.bfloat16, device="cuda")
+    fused_attention_dispatch(*(t.cuda() for t in (c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov)), c.theta, out=out, len_multiple=8,
+                             seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda"), **bounds)
+    lo, hi = bounds.get("route_min_tokens", 0), bounds.get("route_max_tokens", 1 << 30)
+    for b, n in enumerate(seq):
+        if lo <= n < hi:
+            assert float((out[b].float().cpu() - torch.nan_to_num(ref[b])).abs().max()) <= 2e-2
+        else:
+            assert bool((out[b] == 7.0).all())
+    assert _common.read_status(torch.device("cuda")) == (4 if lo == 0 and 0 in seq else 0)      # only a row that takes part is reported
