@@ -342,16 +342,19 @@ bool block_sides(PyObject* const* v, dkv_pack_args (&a)[2]) {
     dkv_pack_args& p = a[sd];
     p = {};
     p.dtype = dtype_code(x.scalar_type());
-    if (p.dtype < 0 || x.dim() != 3 || x.stride(2) != 1 || x.sizes() != unpack(v[2]).sizes() || l.dim() != 2 || l.size(0) != x.size(0) * A ||
-        l.size(1) != x.size(1) || l.scalar_type() != at::kInt || !l.is_contiguous())
+    if (p.dtype < 0 || x.dim() != 3 || x.stride(2) != 1 || unpack(v[2]).dim() != 3 || x.size(0) != unpack(v[2]).size(0) || x.size(1) != unpack(v[2]).size(1) ||
+        l.dim() != 2 || l.size(0) != x.size(0) * A || l.size(1) != x.size(1) || l.scalar_type() != at::kInt || !l.is_contiguous())
       return false;
+    // the sides may differ in type and, within bounds, in width: the row width is the keys', values of a joint row may have fewer
+    const int64_t row_dim = PyLong_AsLong(v[7]);
+    if (A != 1 && x.size(2) < A * row_dim) return false;
     p.batch = (int32_t)x.size(0);
     p.arenas_per_batch = (int32_t)A;
     p.n_new = (int32_t)x.size(1);
-    p.max_dim = (int32_t)PyLong_AsLong(v[7]);
+    p.max_dim = (int32_t)(A == 1 ? std::min(row_dim, x.size(2)) : row_dim);
     p.states = x.data_ptr();
     p.stride_b = x.stride(0);
-    p.stride_j = p.max_dim;
+    p.stride_j = row_dim;
     p.stride_s = x.stride(1);
     p.new_lens = static_cast<const int32_t*>(l.data_ptr());
     p.len_multiple = (int32_t)PyLong_AsLong(v[8]);
@@ -369,6 +372,10 @@ bool block_sides(PyObject* const* v, dkv_pack_args (&a)[2]) {
   return true;
 }
 int pack_sides(const dkv_pack_args (&a)[2], long sides) {
+  if (sides == 3 && a[0].dtype != a[1].dtype) {
+    const int rc = dkv_pack_bulk(&a[0]);
+    return rc ? rc : dkv_pack_bulk(&a[1]);
+  }
   return sides == 3 ? dkv_pack_pair(&a[0], &a[1]) : sides == 1 ? dkv_pack_bulk(&a[0]) : sides == 2 ? dkv_pack_bulk(&a[1]) : 0;
 }
 

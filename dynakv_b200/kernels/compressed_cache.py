@@ -313,12 +313,13 @@ class CustomDynamicCache:
         block = (block[0], kl, block[1], vl, A, row_dim, self.len_multiple, seq_ptr, counts_dev, row_counter)
         totals = host.block_begin(*states, *block)
         if totals is None:
-            raise ValueError("a block needs key and value states of one shape and dtype, on the device and in the dtype of the layer")
+            raise ValueError("a block needs key and value states of one batch and token count, on the device and each in the dtype of "
+                             "its side of the layer, with a length for every arena row and token")
         again = 0
         for side, (raw, now, end, ptrs, ends) in enumerate(totals):
             cache = states[side]
             if fresh := cache is None:
-                cache = lists[side][layer_idx] = self._new_state(B * A, _round8(raw), n_new, key_states.dtype, dev)      # exact fit
+                cache = lists[side][layer_idx] = self._new_state(B * A, _round8(raw), n_new, block[2 * side].dtype, dev)      # exact fit
                 states[side] = cache
             max_added = raw if n_new > 1 else width
             grow = now + max_added > cache[0].shape[1]
@@ -333,8 +334,8 @@ class CustomDynamicCache:
                 status_word(dev).bitwise_or_(_lib.ST_OVERFLOW)
             cache[4] = seq_ptr + n_new
             cache[5] = ends if end <= cap else [e if e <= cap else n for n, e in zip(ptrs, ends)]
-        if again:
-            host.block_pack(*states, *block, again)
+        if again and not host.block_pack(*states, *block, again):
+            raise RuntimeError("the buffers of a cache layer do not fit the block that they were made for")
         if row_counter is not None:
             row_counter.add_(counts_dev if counts_dev is not None else n_new)
             self._seq_lens_host[layer_idx] = [n + (counts[b] if counts is not None else n_new)

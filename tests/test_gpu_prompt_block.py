@@ -48,3 +48,34 @@ def test_ragged_block_keeps_each_rows_count():
     stored = torch.stack([lens[0, :, :7].sum(1), lens[1].sum(1)]).view(-1)
     assert cache.key_cache_sp[0][3].tolist() == stored.tolist() == cache.key_cache_sp[0][5]
     assert _common.read_status(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("k_type,v_type,k_dim,v_dim", [(torch.bfloat16, torch.float16, 128, 128), (torch.float32, torch.bfloat16, 128, 128),
+                                                       (torch.bfloat16, torch.bfloat16, 64, 128), (torch.float16, torch.float16, 128, 72)])
+def test_sides_of_other_types_and_widths(k_type, v_type, k_dim, v_dim):
+    # a fresh layer, a block that fits and one that grows it; the joint layout's row width is the keys'
+    gen = torch.Generator().manual_seed(k_dim + v_dim)
+    B, width = 2, min(k_dim, v_dim)
+    cache = CustomDynamicCache(len_multiple=8)
+    types, lays = (k_type, v_type), [O.LayoutOracle(B, np.float32) for _ in range(2)]
+    for n_new in (9, 3, 200):
+        rows = [torch.randn(B, n_new, d, generator=gen).to(t) for d, t in zip((k_dim, v_dim), types)]
+        lens = [(torch.randint(0, width // 8 + 1, (B, n_new), generator=gen) * 8).to(torch.int32) for _ in range(2)]
+        cache.update_sp(rows[0].cuda(), lens[0].cuda(), rows[1].cuda(), lens[1].cuda(), k_dim, 0, k_dim)
+        for lay, x, n in zip(lays, rows, lens):
+            lay.update(x[:, :, :width].float().numpy(), n.numpy())
+    for lay, state, t in zip(lays, (cache.key_cache_sp[0], cache.value_cache_sp[0]), types):
+        assert state[0].dtype == t and state[4] == 212 and np.array_equal(state[3].cpu().numpy(), lay.ptr)
+        assert np.array_equal(state[1][:, :212].cpu().numpy(), lay.lens)
+        for r in range(B):
+            assert np.array_equal(state[0][r, : lay.ptr[r]].float().cpu().numpy(), lay.flat[r])
+    assert _common.read_status(torch.device("cuda")) == 0
+
+
+def test_values_narrower_than_the_arenas_are_refused():
+    x = torch.randn(1, 4, 256, dtype=torch.float32, device="cuda")
+    lens = torch.full((1, 2, 4), 8, dtype=torch.int32, device="cuda")
+    cache = CustomDynamicCache(arenas_per_batch=2, len_multiple=8)
+    with pytest.raises(ValueError):
+        cache.update_sp(x, lens, x[:, :, :128].contiguous(), lens, 256, 0, 128)
+    assert cache.get_seq_length(0) == 0
