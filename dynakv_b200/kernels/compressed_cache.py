@@ -315,27 +315,34 @@ class CustomDynamicCache:
         if totals is None:
             raise ValueError("a block needs key and value states of one batch and token count, on the device and each in the dtype of "
                              "its side of the layer, with a length for every arena row and token")
-        again = 0
-        for side, (raw, now, end, ptrs, ends) in enumerate(totals):
-            cache = states[side]
-            if fresh := cache is None:
-                cache = lists[side][layer_idx] = self._new_state(B * A, _round8(raw), n_new, block[2 * side].dtype, dev)      # exact fit
-                states[side] = cache
-            max_added = raw if n_new > 1 else width
-            grow = now + max_added > cache[0].shape[1]
-            if grow:
-                step = EXPAND_SEQ_STEP * (width // 2)
-                self._ensure_capacity(cache, _round8(max(cache[0].shape[1] + step, now + max_added)), cache[1].shape[1])
-                cache[3].copy_(torch.tensor(ptrs, dtype=torch.int32))     # rows of the first attempt that did fit moved on
+        again, first = 0, [c is not None for c in states]      # (sides that the first attempt packed)
+        try:        # every allocation, before anything of the layer moves on
+            for side, (raw, now, _, _, _) in enumerate(totals):
+                if states[side] is None:
+                    states[side] = self._new_state(B * A, _round8(raw), n_new, block[2 * side].dtype, dev)      # exact fit
+                    again |= 1 << side
+                cache, max_added = states[side], raw if n_new > 1 else width
+                if now + max_added > cache[0].shape[1]:
+                    step = EXPAND_SEQ_STEP * (width // 2)
+                    self._ensure_capacity(cache, _round8(max(cache[0].shape[1] + step, now + max_added)), cache[1].shape[1])
+                    again |= 1 << side
+        except BaseException:
+            for cache, packed, (_, _, _, ptrs, _) in zip(states, first, totals):
+                if packed:
+                    cache[3].copy_(torch.tensor(ptrs, dtype=torch.int32))
+            raise
+        for side, (_, _, _, ptrs, _) in enumerate(totals):
+            if again >> side & 1 and first[side]:
+                states[side][3].copy_(torch.tensor(ptrs, dtype=torch.int32))     # rows of the first attempt that did fit moved on
+        if again and not host.block_pack(*states, *block, again):
+            raise RuntimeError("the buffers of a cache layer do not fit the block that they were made for")
+        for side, (_, _, end, ptrs, ends) in enumerate(totals):
+            cache = lists[side][layer_idx] = states[side]
             cap = cache[0].shape[1]
-            if fresh or grow:
-                again |= 1 << side
-            elif end > cap:     # lengths made valid no longer fit: recorded as empty
+            if end > cap and not again >> side & 1:     # lengths made valid no longer fit: recorded as empty
                 status_word(dev).bitwise_or_(_lib.ST_OVERFLOW)
             cache[4] = seq_ptr + n_new
             cache[5] = ends if end <= cap else [e if e <= cap else n for n, e in zip(ptrs, ends)]
-        if again and not host.block_pack(*states, *block, again):
-            raise RuntimeError("the buffers of a cache layer do not fit the block that they were made for")
         if row_counter is not None:
             row_counter.add_(counts_dev if counts_dev is not None else n_new)
             self._seq_lens_host[layer_idx] = [n + (counts[b] if counts is not None else n_new)

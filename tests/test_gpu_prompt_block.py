@@ -79,3 +79,42 @@ def test_values_narrower_than_the_arenas_are_refused():
     with pytest.raises(ValueError):
         cache.update_sp(x, lens, x[:, :, :128].contiguous(), lens, 256, 0, 128)
     assert cache.get_seq_length(0) == 0
+
+
+@pytest.mark.parametrize("fresh", [False, True])
+def test_a_block_whose_growth_fails_leaves_the_layer_as_it_was(fresh, monkeypatch):
+    # K fits, the V buffer cannot grow (or be made): the block can be given again
+    gen = torch.Generator().manual_seed(4)
+    B, A, R = 2, 2, 128
+    cache = CustomDynamicCache(arenas_per_batch=A, len_multiple=8)
+    lays = [O.LayoutOracle(B * A, np.float32) for _ in range(2)]
+    if not fresh:
+        cache.reserve(0, B, 4000, 64, torch.bfloat16, "cuda")
+    allocate = CustomDynamicCache._new_state if fresh else CustomDynamicCache._ensure_capacity
+    for n_new, fails in ((20, fresh), (25, not fresh)):
+        rows = [torch.randn(B, n_new, A * R, generator=gen).to(torch.bfloat16) for _ in range(2)]
+        lens = [torch.full((B, A, n_new), n, dtype=torch.int32) for n in (16, 128)]
+        args = (rows[0].cuda(), lens[0].cuda(), rows[1].cuda(), lens[1].cuda(), A * R, 0, R)
+        if fails:
+            calls = []
+
+            def failing(*a):
+                calls.append(a)
+                if (len(calls) == 2 if fresh else a[0] is cache.value_cache_sp[0]):
+                    raise torch.cuda.OutOfMemoryError("no memory")
+                return allocate(*a)
+            with monkeypatch.context() as m:
+                m.setattr(cache, "_new_state" if fresh else "_ensure_capacity", failing)
+                with pytest.raises(torch.cuda.OutOfMemoryError):
+                    cache.update_sp(*args)
+            for lst, lay in zip((cache.key_cache_sp, cache.value_cache_sp), lays):
+                assert lst[0] is None if fresh else (lst[0][4] == 20 and np.array_equal(lst[0][3].cpu().numpy(), lay.ptr))
+        cache.update_sp(*args)
+        for lay, x, n in zip(lays, rows, lens):
+            lay.update(x.float().view(B, n_new, A, R).permute(0, 2, 1, 3).reshape(B * A, n_new, R).numpy(), n.view(B * A, n_new).numpy())
+    for lay, state in zip(lays, (cache.key_cache_sp[0], cache.value_cache_sp[0])):
+        assert state[4] == 45 and np.array_equal(state[3].cpu().numpy(), lay.ptr)
+        assert np.array_equal(state[1][:, :45].cpu().numpy(), lay.lens) and np.array_equal(state[2][:, :45].cpu().numpy(), lay.offs)
+        for r in range(B * A):
+            assert np.array_equal(state[0][r, : lay.ptr[r]].float().cpu().numpy(), lay.flat[r])
+    assert _common.read_status(torch.device("cuda")) == 0
