@@ -732,10 +732,11 @@ __global__ void __launch_bounds__(TS_THREADS) tile_combine_kernel(dkv_attn_args 
     M = warp_max(M);
     float L = 0.f;
     for (int k = tid; k < n_split; k += 32) {
-      const float m = rec0[(size_t)k * (2 + R)];
-      const float w = (m == -INFINITY) ? 0.f : __expf(m - M);
+      // (a slice whose scores are all NaN leaves the maximum of no score and a sum that is NaN, which its weight takes on)
+      const float m = rec0[(size_t)k * (2 + R)], l = rec0[(size_t)k * (2 + R) + 1];
+      const float w = l != l ? l : m == -INFINITY ? 0.f : __expf(m - M);
       w_s[k] = w;
-      L = fmaf(w, rec0[(size_t)k * (2 + R) + 1], L);
+      L = fmaf(w, l, L);
     }
     L = warp_sum(L);
     if (tid == 0) L_s = L;

@@ -108,3 +108,26 @@ def test_softmax_operator_reads_the_counter_behind_an_append():
         ref = O.softmax_v_reference(scores[:, :, :s].float().cpu(), flat.float().cpu(), c.v_up.float().cpu(), lens[:, :s].cpu(), offs[:, :s].cpu())
         assert float((out.float().cpu() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
     assert _common.read_status(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("poison", ["query", "key", "key_inf", "value"])
+def test_what_is_not_finite_stays_so(poison, dtype):
+    # 300 tokens, none of them empty: a NaN query leaves no score that is a number in any slice
+    t = _case(3, 1, 300, 64, 8, 2, 1, dtype)
+    for side in "kv":
+        t["lens_" + side] = t["lens_" + side].clamp(min=1)
+        t["offs_" + side] = (torch.cumsum(t["lens_" + side], 1) - t["lens_" + side]).to(torch.int32)
+        t["flat_" + side] = torch.randn(1, int(t["lens_" + side].sum()), generator=torch.Generator().manual_seed(8)).to(dtype)
+    where, at, value = {"query": ("q", (0, 3, 5), "nan"), "key": ("flat_k", (0, 40), "nan"), "key_inf": ("flat_k", (0, 40), "inf"),
+                        "value": ("flat_v", (0, 0), "nan")}[poison]
+    t[where][at] = float(value)
+    want = torch.zeros(8, dtype=torch.bool)
+    want[3 if poison == "query" else slice(None)] = True
+    d = _dev(t, 0)
+    args = [d[k] for k in ("q", "flat_k", "k_up", "flat_v", "v_up", "lens_k", "offs_k", "lens_v", "offs_v")]
+    outs = [fn(*args, 10000.0) for fn in (fused_attention_dispatch, two_stage_attention)]
+    outs.append(avx(abx_sparse(d["q"], d["k_up"], d["flat_k"], d["lens_k"], offsets=d["offs_k"]), d["flat_v"], d["v_up"], d["lens_v"], d["offs_v"]))
+    for out in outs:
+        assert torch.equal(out[0].isnan().any(-1).cpu(), want)
+    _common.read_status(torch.device("cuda"))
