@@ -107,9 +107,13 @@ extern "C" int dkv_two_stage_decode(const dkv_attn_args* a) {
 
 extern "C" int dkv_routed_decode(const dkv_attn_args* a, int32_t switch_tokens) {
   if (int rc = check_attn_args(a, "dkv_routed_decode", true, true, true)) return rc;
-  DKV_REQUIRE(a->seq_lens != nullptr && switch_tokens > 0, DKV_E_ARG, "dkv_routed_decode: needs seq_lens and a switch point");
+  DKV_REQUIRE(a->seq_lens != nullptr, DKV_E_ARG, "dkv_routed_decode: needs seq_lens");
   dkv_attn_args s = *a, l = *a;
   s.route_min_tokens = l.route_max_tokens = 0;
+  if (switch_tokens <= 0) {      // no row is short
+    l.route_min_tokens = 0;
+    return dkv_two_stage_decode(&l);
+  }
   s.route_max_tokens = l.route_min_tokens = switch_tokens;
   if (mma_path_ok(a) && fused_by_split(&s)) {      // the short rows would go through split and merge as well: one pass for all
     l.route_min_tokens = 0;

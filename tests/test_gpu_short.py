@@ -95,3 +95,19 @@ def test_rows_out_of_bounds_are_left_alone(rows, bounds):
         else:
             assert bool((out[b] == 7.0).all())
     assert _common.read_status(torch.device("cuda")) == (4 if lo == 0 and 0 in seq else 0)      # only a row that takes part is reported
+
+
+@pytest.mark.parametrize("switch", [0, -1, 1])
+@pytest.mark.parametrize("mult", [8, 1], ids=["packed", "any_length"])
+def test_router_whose_policy_makes_every_row_long(switch, mult):
+    from dynakv_b200.kernels.router import KernelPolicy, compressed_decode_attention
+    seq = [100, 700, 1]
+    c = synthetic.make_layer_case(11, seq, "beta:2,5", 5e5, torch.bfloat16, "cpu")
+    fk, fv, lk, lv, ok, ov = c.views()
+    ref = O.compact_attention(c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov, c.theta, seq_lens=seq)
+    d = [t.cuda() for t in (c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov)]
+    out = compressed_decode_attention(q=d[0], k_flat=d[1], k_up=d[2], v_flat=d[3], v_up=d[4], key_lengths=d[5], key_offsets=d[6],
+                                      value_lengths=d[7], value_offsets=d[8], theta=c.theta, cache_length=700, len_multiple=mult,
+                                      seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda"), policy=KernelPolicy(switch_tokens=switch))
+    assert float((out.float().cpu() - ref).abs().max()) <= 2e-2
+    assert _common.read_status(torch.device("cuda")) == 0
