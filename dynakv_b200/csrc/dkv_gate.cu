@@ -354,6 +354,11 @@ __global__ void __launch_bounds__(GG_THREADS) gate_gemm_kernel(const __grid_cons
           if (++s == STAGES) { s = 0; ++turn; }
         }
       }
+      if (!ok) {      // given up: reported, and the copies in flight waited for
+        set_status(pk.status, DKV_ST_TIMEOUT);
+        for (int i = 0; i < STAGES; ++i)
+          if (i < s || turn > 0) gg_wait(&full[i], (i < s ? turn : turn - 1) & 1);
+      }
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -383,6 +388,10 @@ __global__ void __launch_bounds__(GG_THREADS) gate_gemm_kernel(const __grid_cons
         }
         if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gg_smem(&acc_full[j & 1])) : "memory");
       }
+      if (!ok) {      // given up: reported, and the products in flight waited for
+        set_status(pk.status, DKV_ST_TIMEOUT);
+        if (s > 0 || turn > 0) gg_wait(&empty[s > 0 ? s - 1 : STAGES - 1], (s > 0 ? turn : turn - 1) & 1);
+      }
     }
   } else {
     const int quarter = warp & 3;         // the quarter of tensor memory that the warp may read
@@ -393,7 +402,10 @@ __global__ void __launch_bounds__(GG_THREADS) gate_gemm_kernel(const __grid_cons
       const dkv_gate_args& p = side ? pv : pk;
       const T* bias = reinterpret_cast<const T*>(p.b) + n0;
       const bool native = p.native_rounding != 0;
-      if (!__all_sync(0xffffffffu, gg_wait(&acc_full[j & 1], (uint32_t)(j >> 1) & 1))) break;      // bounded
+      if (!__all_sync(0xffffffffu, gg_wait(&acc_full[j & 1], (uint32_t)(j >> 1) & 1))) {
+        if (lane == 0) set_status(p.status, DKV_ST_TIMEOUT);
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem + (j & 1) * BN + ((uint32_t)(32 * quarter) << 16);
       // 32 columns of the thread's row at a time go through the warp's 4 KB of shared memory and leave as whole 128-byte

@@ -488,6 +488,7 @@ struct GateSide {
 bool gate_side(GateSide& g, PyObject* const* t, long low_rank, double threshold, bool want, long len_multiple, bool native) {
   if (!is_tensor(t[0]) || !unpack(t[0]).is_cuda()) return false;
   const int dev = unpack(t[0]).get_device();
+  if (dev < 0 || dev >= MAX_DEVICES || g_status[dev] == nullptr) return false;
   for (int i = 0; i < 3; ++i)
     if (!plain(t[i], dev)) return false;
   const at::Tensor &x = unpack(t[0]), &w = unpack(t[1]), &b = unpack(t[2]);
@@ -503,6 +504,7 @@ bool gate_side(GateSide& g, PyObject* const* t, long low_rank, double threshold,
   a.threshold = (float)threshold;
   a.len_multiple = (int32_t)len_multiple;
   a.native_rounding = native ? 1 : 0;
+  a.status = g_status[dev];
   a.x = x.data_ptr();
   a.x_stride = d;
   a.w = w.data_ptr();

@@ -110,7 +110,7 @@ def gate_lengths(states: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
     scratch = _scratch(states.device, max(need, 4) // 4)
     a.workspace, a.workspace_bytes = scratch.data_ptr(), scratch.numel() * 4
     a.len_multiple, a.native_rounding = int(len_multiple), int(bool(native_rounding))
-    a.stream = _lib.stream_ptr(states.device)
+    a.status, a.stream = status_word(states.device).data_ptr(), _lib.stream_ptr(states.device)
     _lib.check(lib.dkv_gate_lengths(C.byref(a)), "dkv_gate_lengths")
     lead = states.shape[:-1]
     return (masked.reshape(*lead, d) if return_masked else None), lengths.reshape(lead)
@@ -143,7 +143,7 @@ def gate_lengths_pair(k_rows: torch.Tensor, Wk: torch.Tensor, bk: torch.Tensor, 
         a.x, a.x_stride, a.w, a.b = x.data_ptr(), x.stride(0), wc.data_ptr(), bc.data_ptr()
         a.lengths, a.masked, a.masked_stride = out.data_ptr(), None, 0
         a.len_multiple, a.native_rounding = int(len_multiple), int(bool(native_rounding))
-        a.stream = _lib.stream_ptr(rows.device)
+        a.status, a.stream = status_word(rows.device).data_ptr(), _lib.stream_ptr(rows.device)
         args.append(a)
         keep += [x, wc, bc]
     _lib.check(_lib.load().dkv_gate_lengths_pair(C.byref(args[0]), C.byref(args[1])), "dkv_gate_lengths_pair")

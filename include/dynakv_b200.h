@@ -287,6 +287,7 @@ typedef struct dkv_gate_args {
   void* stream;
   int32_t len_multiple;   /* 0 or 1: exact counts */
   int32_t native_rounding;
+  int32_t* status;        /* device word for DKV_ST_TIMEOUT, or NULL */
 } dkv_gate_args;
 size_t dkv_gate_workspace_bytes(const dkv_gate_args* args);
 int dkv_gate_lengths(const dkv_gate_args* args);

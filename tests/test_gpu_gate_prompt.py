@@ -37,3 +37,23 @@ def test_both_sides_in_one_launch_give_what_each_gives(rows, d):
     k_out, v_out, len_k, len_v, _, _ = kv_process_fused(k, v, wk, bk, wv, bv, d)
     for (out, lens), got in ((gate_lengths(k, wk, bk, d), (k_out, len_k)), (gate_lengths(v, wv, bv, d), (v_out, len_v))):
         assert torch.equal(out, got[0]) and torch.equal(lens, got[1])
+
+
+def test_the_gate_reports_to_the_status_word(monkeypatch):
+    # a wait that runs out cannot be had without a broken kernel: what is checked is where the calls would report it
+    from dynakv_b200 import _lib
+    from dynakv_b200.kernels import _common
+    from dynakv_b200.kernels.compressed_attention import gate_lengths, gate_lengths_pair, kv_process_fused
+    dev = torch.device("cuda")
+    word, seen, lib = _common.status_word(dev).data_ptr(), [], _lib.load()
+    for name in ("dkv_gate_lengths", "dkv_gate_lengths_pair"):
+        real = getattr(lib, name)
+        monkeypatch.setattr(lib, name, lambda *a, real=real: (seen.extend(x._obj.status for x in a), real(*a))[1])
+    x, w, b = torch.randn(200, 128, device=dev).bfloat16(), torch.randn(128, 128, device=dev).bfloat16(), torch.zeros(128, device=dev).bfloat16()
+    lens = torch.empty(200, dtype=torch.int32, device=dev)
+    gate_lengths(x, w, b, 128, out_lengths=lens)
+    gate_lengths_pair(x, w, b, x, w, b, 128, lens, lens.clone())
+    assert seen == [word] * 3
+    gate_lengths(x, w, b, 128)
+    kv_process_fused(x[None], x[None], w, b, w, b, 128)
+    assert _common.read_status(dev) == 0
