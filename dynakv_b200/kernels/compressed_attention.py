@@ -81,7 +81,7 @@ def gate_lengths(states: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
     if not states.is_cuda:
         raise RuntimeError("dynakv_b200 has no CPU path: the gate needs CUDA tensors")
     if out_lengths is None:
-        done = _lib.host().gate(states, weight, bias, low_rank, threshold, return_masked, len_multiple, bool(native_rounding))
+        done = _lib.host().gate(states, weight, bias, int(low_rank), threshold, bool(return_masked), int(len_multiple), bool(native_rounding))
         if done is not None:        # else: tensors that have to be copied first, or refused
             return done
     d = states.shape[-1]
@@ -155,7 +155,7 @@ def kv_process_fused(key_states: torch.Tensor, value_states: torch.Tensor, Wk, b
     """Drop-in for the reference module method of the same name (kernels/compressed_attention.py:84-119):
     returns (k_out, v_out, len_k, len_v, 1, 1) for key_states / value_states [B, S, d]."""
     if key_states.is_cuda:
-        done = _lib.host().gate_both(key_states, Wk, bk, value_states, Wv, bv, low_rank, 0.1, len_multiple)
+        done = _lib.host().gate_both(key_states, Wk, bk, value_states, Wv, bv, int(low_rank), 0.1, int(len_multiple))
         if done is not None:        # else: tensors that have to be copied first, or refused
             return *done, 1, 1
     k_out, len_k = gate_lengths(key_states, Wk, bk, low_rank, len_multiple=len_multiple)

@@ -28,7 +28,7 @@ def fused_attention_dispatch(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, 
     tensor-core kernel; the default makes no assumption and uses the generic kernel.
     """
     done = _lib.host().attend(q, k_flat, k_up, v_flat, v_up, l_k, o_k, l_v, o_v, theta, out, seq_lens, batch_index,
-                              k_norm_weight, k_norm_eps, len_multiple, route_min_tokens, route_max_tokens, False)
+                              k_norm_weight, k_norm_eps, int(len_multiple), int(route_min_tokens), int(route_max_tokens), False)
     if done is not None:        # else: tensors that have to be copied first, or refused
         return done
     q3 = q.squeeze(2) if q.dim() == 4 else q

@@ -68,7 +68,7 @@ def compressed_decode_attention(
         short, long_ = policy.partition(seq_lens_host)
         any_short, any_long = bool(short), bool(long_)
     if any_short and any_long and q.is_cuda:
-        done = _lib.host().attend(*args, None, seq_lens, None, k_norm_weight, k_norm_eps, len_multiple, 0, 0, int(policy.switch_tokens))
+        done = _lib.host().attend(*args, None, seq_lens, None, k_norm_weight, k_norm_eps, int(len_multiple), 0, 0, int(policy.switch_tokens))
         if done is not None:        # else: tensors that have to be copied first, or refused
             return done
     q3 = q.squeeze(2) if q.dim() == 4 else q

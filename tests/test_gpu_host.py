@@ -1,0 +1,33 @@
+"""The native host side takes the calls that the Python side took: numbers of any kind, refusals and fallbacks alike."""
+import pytest
+import torch
+
+from dynakv_b200 import synthetic
+from dynakv_b200.kernels import _common
+from dynakv_b200.kernels.fused import fused_attention_dispatch
+from dynakv_b200.kernels.two_stage import two_stage_attention
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def test_numbers_of_any_kind():
+    from dynakv_b200.kernels.compressed_attention import gate_lengths, kv_process_fused
+    gen = torch.Generator().manual_seed(1)
+    x, w, b = torch.randn(1, 5, 64, generator=gen).to(DEV), torch.randn(64, 64, generator=gen).to(DEV), torch.randn(64, generator=gen).to(DEV)
+    masked, lens = gate_lengths(x, w, b, 48, len_multiple=8)
+    for rank, yes, step in ((48.0, 1, 8.0), (torch.tensor(48), [0], 8), (torch.tensor(48.0), True, torch.tensor(8))):
+        got, n = gate_lengths(x, w, b, rank, return_masked=yes, len_multiple=step)
+        assert torch.equal(got, masked) and torch.equal(n, lens)
+        assert torch.equal(kv_process_fused(x, x, w, b, w, b, rank, len_multiple=step)[2], lens)
+    assert gate_lengths(x, w, b, 48, return_masked=0)[0] is None
+    seq = [100, 700]
+    c = synthetic.make_layer_case(5, seq, "beta:2,5", 5e5, torch.bfloat16, DEV)
+    fk, fv, lk, lv, ok, ov = c.views()
+    args = (c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov)
+    rows = torch.tensor(seq, dtype=torch.int32, device=DEV)
+    for fn in (fused_attention_dispatch, two_stage_attention):
+        want = fn(*args, 5e5, seq_lens=rows, len_multiple=8, route_max_tokens=800)
+        got = fn(*args, torch.tensor(5e5), seq_lens=rows, len_multiple=8.0, route_min_tokens=0.0, route_max_tokens=torch.tensor(800.0))
+        assert torch.equal(got, want)
+    assert _common.read_status(torch.device(DEV)) == 0
