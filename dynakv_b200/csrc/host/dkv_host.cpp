@@ -195,7 +195,8 @@ PyObject* append_token(PyObject*, PyObject* const* v, Py_ssize_t n) {
   if (ks.dim() != 3 || ks.size(1) != 1 || ks.size(2) % A != 0 || vs.sizes() != ks.sizes() || !ks.is_contiguous() || !vs.is_contiguous()) Py_RETURN_NONE;
   const int64_t B = ks.size(0), rows = B * A;
   for (const at::Tensor* t : {&kl, &vl})
-    if (t->scalar_type() != at::kInt || t->numel() != rows || !t->is_contiguous() || !(t->dim() == 2 || t->dim() == 3)) Py_RETURN_NONE;
+    // (without an axis for the arenas: one per row, or refused by the general path)
+    if (t->scalar_type() != at::kInt || t->numel() != rows || !t->is_contiguous() || !(t->dim() == 3 || (t->dim() == 2 && A == 1))) Py_RETURN_NONE;
   dkv_append_args a = {};
   a.dtype = dtype_code(ks.scalar_type());
   if (a.dtype < 0 || vs.scalar_type() != ks.scalar_type()) Py_RETURN_NONE;

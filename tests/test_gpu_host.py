@@ -4,6 +4,7 @@ import torch
 
 from dynakv_b200 import synthetic
 from dynakv_b200.kernels import _common
+from dynakv_b200.kernels.compressed_cache import CustomDynamicCache
 from dynakv_b200.kernels.fused import fused_attention_dispatch
 from dynakv_b200.kernels.two_stage import two_stage_attention
 
@@ -30,4 +31,22 @@ def test_numbers_of_any_kind():
         want = fn(*args, 5e5, seq_lens=rows, len_multiple=8, route_max_tokens=800)
         got = fn(*args, torch.tensor(5e5), seq_lens=rows, len_multiple=8.0, route_min_tokens=0.0, route_max_tokens=torch.tensor(800.0))
         assert torch.equal(got, want)
+    assert _common.read_status(torch.device(DEV)) == 0
+
+
+@pytest.mark.parametrize("arenas,shape,taken", [(1, (3, 1), True), (1, (3,), True), (1, (3, 1, 1), True), (2, (3, 2, 1), True), (2, (3, 2), False),
+                                                (2, (6,), False)], ids=str)
+def test_lengths_of_a_new_token(arenas, shape, taken):
+    cache = CustomDynamicCache(arenas_per_batch=arenas, len_multiple=8)
+    x = torch.randn(3, 4, arenas * 128, device=DEV).bfloat16()
+    lens = torch.full((3, arenas, 4), 8, dtype=torch.int32, device=DEV)
+    cache.reserve(0, 3, 1024, 64, torch.bfloat16, DEV)
+    cache.update_sp(x, lens, x, lens, arenas * 128, 0, 128)
+    new, one = x[:, :1].contiguous(), torch.full(shape, 16, dtype=torch.int32, device=DEV)
+    if taken:
+        cache.update_sp(new, one, new, one, arenas * 128, 0, 128)
+    else:
+        with pytest.raises((RuntimeError, ValueError)):
+            cache.update_sp(new, one, new, one, arenas * 128, 0, 128)
+    assert cache.get_seq_length(0) == 4 + taken and cache.key_cache_sp[0][3].tolist() == [32 + 16 * taken] * 3 * arenas
     assert _common.read_status(torch.device(DEV)) == 0
