@@ -79,6 +79,12 @@ at::Tensor rows_view(const at::Tensor& base, int64_t offset, at::IntArrayRef siz
   return t;
 }
 
+// a runtime call that failed here: raised once, and not found again by the launch check of the next call
+PyObject* fail(const char* what, cudaError_t e) {
+  cudaGetLastError();
+  PyErr_Format(PyExc_RuntimeError, "%s failed: %s", what, cudaGetErrorString(e));
+  return nullptr;
+}
 PyObject* fail(const char* what, int rc) {
   PyErr_Format(PyExc_RuntimeError, "%s failed (code %d): %s", what, rc, dkv_last_error());
   return nullptr;
@@ -275,10 +281,7 @@ PyObject* new_state(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const at::Tensor ints = empty({2 * rows * seq + rows}, at::kInt, flat.device());
   cudaError_t e = cudaMemsetAsync(flat.data_ptr(), 0, flat.nbytes(), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(ints.data_ptr(), 0, ints.nbytes(), st);
-  if (e != cudaSuccess) {
-    PyErr_Format(PyExc_RuntimeError, "zeroing a new cache layer failed: %s", cudaGetErrorString(e));
-    return nullptr;
-  }
+  if (e != cudaSuccess) return fail("zeroing a new cache layer", e);
   PyObject* zeros = PyList_New(rows);
   for (int64_t i = 0; i < rows; ++i) PyList_SET_ITEM(zeros, i, PyLong_FromLong(0));
   PyObject* r = PyList_New(6);
@@ -300,16 +303,16 @@ PyObject* grow(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const int64_t cols = PyLong_AsLong(v[1]);
   if (PyErr_Occurred()) return nullptr;
   if (t.dim() != 2 || t.stride(1) != 1 || t.requires_grad() || cols < t.size(1) || t.numel() == 0) Py_RETURN_NONE;
+  // what a two-dimensional copy cannot express: rows that overlap (one row may have any stride), pitches past 2^31 - 1 bytes
+  constexpr int64_t MAX_PITCH = 2147483647;
+  if (t.stride(0) < t.size(1) || (int64_t)t.element_size() * std::max(t.stride(0), cols) > MAX_PITCH) Py_RETURN_NONE;
   c10::cuda::CUDAGuard guard(t.device());
   cudaStream_t st = at::cuda::getCurrentCUDAStream(t.get_device()).stream();
   const at::Tensor r = empty({t.size(0), cols}, t.scalar_type(), t.device());
   const size_t es = t.element_size(), had = t.size(1) * es, pitch = cols * es;
   cudaError_t e = cudaMemcpy2DAsync(r.data_ptr(), pitch, t.data_ptr(), t.stride(0) * es, had, t.size(0), cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess && pitch > had) e = cudaMemset2DAsync(static_cast<char*>(r.data_ptr()) + had, pitch, 0, pitch - had, t.size(0), st);
-  if (e != cudaSuccess) {
-    PyErr_Format(PyExc_RuntimeError, "growing a cache buffer failed: %s", cudaGetErrorString(e));
-    return nullptr;
-  }
+  if (e != cudaSuccess) return fail("growing a cache buffer", e);
   return THPVariable_Wrap(r);
   END_HANDLE_TH_ERRORS
 }
@@ -408,10 +411,7 @@ PyObject* block_begin(PyObject*, PyObject* const* v, Py_ssize_t n) {
   }
   if (here) cudaEventDestroy(here);
   if (rc) return fail("dkv_pack_bulk", rc);
-  if (e != cudaSuccess) {
-    PyErr_Format(PyExc_RuntimeError, "reading a block's totals failed: %s", cudaGetErrorString(e));
-    return nullptr;
-  }
+  if (e != cudaSuccess) return fail("reading a block's totals", e);
   PyObject* r = PyTuple_New(2);
   for (int sd = 0; sd < 2; ++sd) {
     const int32_t* t = static_cast<const int32_t*>(host.data_ptr()) + sd * rows * 4;

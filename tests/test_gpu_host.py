@@ -50,3 +50,22 @@ def test_lengths_of_a_new_token(arenas, shape, taken):
             cache.update_sp(new, one, new, one, arenas * 128, 0, 128)
     assert cache.get_seq_length(0) == 4 + taken and cache.key_cache_sp[0][3].tolist() == [32 + 16 * taken] * 3 * arenas
     assert _common.read_status(torch.device(DEV)) == 0
+
+
+def test_buffers_that_a_two_dimensional_copy_cannot_grow():
+    n = 64
+    one = torch.arange(n, device=DEV, dtype=torch.float32).bfloat16()
+    odd = one.as_strided((1, n), (1, 1))              # one row: its stride says nothing
+    ints = torch.zeros(1, 8, dtype=torch.int32, device=DEV)
+    cache = CustomDynamicCache(len_multiple=8)
+    cache.adopt(0, (odd, ints.clone(), ints.clone(), ints[:, 0].clone()), (odd.clone(), ints.clone(), ints.clone(), ints[:, 0].clone()), [0])
+    x = torch.randn(1, 4, 128, device=DEV).bfloat16()
+    lens = torch.full((1, 4), 64, dtype=torch.int32, device=DEV)
+    cache.update_sp(x, lens, x, lens, 128, 0, 128, token_counts=[4])
+    for state in (cache.key_cache_sp[0], cache.value_cache_sp[0]):
+        assert state[3].tolist() == [256] and torch.equal(state[0][0, :256], x[0, :, :64].reshape(-1))
+    big = torch.zeros(2, (1 << 30) - 8, dtype=torch.bfloat16, device=DEV)     # rows of 2 GiB less 16 bytes
+    big[:, -1] = 3.0
+    grown = CustomDynamicCache._grown(big, (1 << 30) + 8)
+    assert grown.shape == (2, (1 << 30) + 8) and grown[:, (1 << 30) - 9].tolist() == [3.0, 3.0] and int(grown.count_nonzero()) == 2
+    assert _common.read_status(torch.device(DEV)) == 0
