@@ -1,4 +1,5 @@
-// Generic decode attention in one kernel, one CTA per (row, query head): the path of callers that give no workspace.
+// Generic decode attention in one kernel, one CTA per (row, query head): the path of callers that give no workspace and of
+// calls of a few tokens (the rules are beside tiles_ok in dkv_tiles.cu).
 //
 // Handles every layout the reference API can express: any element type, rank R up to 1024,
 // any integer lengths, lens/offs as strided views, joint latent rows shared by all heads or
@@ -17,7 +18,7 @@
 
 namespace dkv {
 
-enum { MODE_ATTN = 0, MODE_SOFTMAX_V = 2 };
+enum { MODE_ATTN = 0, MODE_SCORES = 1, MODE_SOFTMAX_V = 2 };
 
 constexpr int GD = 128;       // head_dim
 constexpr int GTT = 32;       // tokens per tile
@@ -47,7 +48,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
   if (MODE == MODE_ATTN && row_routed_out(p, b)) return;   // the row belongs to the other kernel
   int S = p.seq_len;
   if (p.seq_lens) S = min(S, max(p.seq_lens[b], 0));
-  const int t_begin = 0, t_end = S;
+  const int t_begin = 0, t_end = MODE == MODE_SCORES ? p.seq_len : S;     // the score operator writes every column
 
   const T* kflat = reinterpret_cast<const T*>(p.k.flat) + (size_t)a * p.k.flat_stride;
   const T* vflat = reinterpret_cast<const T*>(p.v.flat) + (size_t)a * p.v.flat_stride;
@@ -88,7 +89,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
             lk = 0; ok = 0;
           }
         }
-        {
+        if (MODE != MODE_SCORES) {
           lv = p.v.lens[(size_t)a * p.v.lens_stride_a + (size_t)s * p.v.lens_stride_s];
           ov = p.v.offs[(size_t)a * p.v.offs_stride_a + (size_t)s * p.v.offs_stride_s];
           lv = min(max(lv, 0), R);
@@ -142,10 +143,8 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
               if (vec) {
                 v = __ldg(reinterpret_cast<const uint4*>(kup + (size_t)r * GD) + c);
               } else {
-                __align__(16) T tmp[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) tmp[i] = kup[(size_t)r * GD + 8 * c + i];
-                v = *reinterpret_cast<const uint4*>(tmp);
+                const uint16_t* e = reinterpret_cast<const uint16_t*>(kup + (size_t)r * GD + 8 * c);
+                v = make_uint4(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16, e[4] | (uint32_t)e[5] << 16, e[6] | (uint32_t)e[7] << 16);
               }
             }
             br[u] = v;
@@ -257,7 +256,9 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
         part = warp_sum(part);
         if (lane == 0) {
           const bool in = s < t_end;
-          {
+          if (MODE == MODE_SCORES) {
+            if (in) (reinterpret_cast<T*>(p.out) + (size_t)b * p.out_stride_b + (size_t)h * p.out_stride_h)[s] = from_f32<T>((lenk_s[t] > 0 ? part : -1.0e4f) * scale);
+          } else {
             sc_s[t] = (in && lenk_s[t] > 0) ? part * scale : -INFINITY;
           }
         }
@@ -271,7 +272,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
       __syncthreads();
     }
 
-    {
+    if (MODE != MODE_SCORES) {
       // ---- online softmax over the tile (warp 0) ----
       if (warp == 0) {
         const float sc = sc_s[lane];
@@ -313,6 +314,7 @@ generic_decode_kernel(dkv_attn_args p, const T* __restrict__ scores_in, int64_t 
     }
   }
 
+  if (MODE == MODE_SCORES) return;
   // ---- normalise and project the latent accumulator through Bv ----
   float* lat_s = &k_s[0][0];  // >= 1024 floats
   const float l = l_s;
@@ -366,9 +368,9 @@ static int launch_generic(const dkv_attn_args* a, const void* scores, int64_t sb
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const dim3 grid(a->batch, a->n_q_heads);
   const float log_theta = (float)log((double)a->theta);
-  if (a->dtype == DKV_F32)
-    generic_decode_kernel<float, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const float*)scores, sb, sh, log_theta);
-  else if (a->dtype == DKV_F16)
+  if (a->dtype == DKV_F32) {
+    if constexpr (MODE != MODE_SCORES) generic_decode_kernel<float, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const float*)scores, sb, sh, log_theta);
+  } else if (a->dtype == DKV_F16)
     generic_decode_kernel<__half, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const __half*)scores, sb, sh, log_theta);
   else
     generic_decode_kernel<__nv_bfloat16, MODE><<<grid, GTHREADS, 0, st>>>(*a, (const __nv_bfloat16*)scores, sb, sh, log_theta);
@@ -377,14 +379,17 @@ static int launch_generic(const dkv_attn_args* a, const void* scores, int64_t sb
 }
 
 // implemented in dkv_tiles.cu
-bool tiles_ok(const dkv_attn_args* a, bool with_scores);
+bool tiles_ok(const dkv_attn_args* a);
+bool tiles_scores_ok(const dkv_attn_args* a);
+bool tiles_softmax_ok(const dkv_attn_args* a);
+size_t tiles_softmax_workspace_bytes(const dkv_attn_args* a);
 int tiles_scores(const dkv_attn_args* a);
 int tiles_attention(const dkv_attn_args* a);
 int tiles_softmax_v(const dkv_attn_args* a, const void* scores, int64_t sb, int64_t sh);
 
 // Both entries on caches that take this path: tile kernels when the caller's workspace holds their scores and records.
 int generic_attention(const dkv_attn_args* a) {
-  return tiles_ok(a, true) ? tiles_attention(a) : launch_generic<MODE_ATTN>(a, nullptr, 0, 0);
+  return tiles_ok(a) ? tiles_attention(a) : launch_generic<MODE_ATTN>(a, nullptr, 0, 0);
 }
 
 }  // namespace dkv
@@ -393,12 +398,14 @@ using namespace dkv;
 
 extern "C" int dkv_scores(const dkv_attn_args* a) {
   if (int rc = check_attn_args(a, "dkv_scores", true, true, false)) return rc;
-  return tiles_scores(a);
+  return tiles_scores_ok(a) ? tiles_scores(a) : launch_generic<MODE_SCORES>(a, nullptr, 0, 0);
 }
 
 extern "C" int dkv_softmax_v(const dkv_attn_args* a, const void* scores, int64_t sc_stride_b, int64_t sc_stride_h) {
   if (int rc = check_attn_args(a, "dkv_softmax_v", false, false, true)) return rc;
   DKV_REQUIRE(scores != nullptr, DKV_E_ARG, "dkv_softmax_v: null scores");
-  if (tiles_ok(a, false)) return tiles_softmax_v(a, scores, sc_stride_b, sc_stride_h);
+  if (tiles_softmax_ok(a)) return tiles_softmax_v(a, scores, sc_stride_b, sc_stride_h);
   return launch_generic<MODE_SOFTMAX_V>(a, scores, sc_stride_b, sc_stride_h);
 }
+
+extern "C" size_t dkv_softmax_v_workspace_bytes(const dkv_attn_args* a) { return a == nullptr ? 0 : tiles_softmax_workspace_bytes(a); }

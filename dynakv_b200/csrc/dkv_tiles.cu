@@ -914,20 +914,36 @@ int softmax_v(const dkv_attn_args* a, const void* scores, int64_t sb, int64_t sh
 
 }  // namespace
 
-// the workspace of the attention (scores and records); the softmax operator needs the records only
+// the workspace of the attention (scores and records)
 size_t tiles_workspace_bytes(const dkv_attn_args* a) {
   if (a->batch <= 0 || a->seq_len <= 0) return 0;
   return score_bytes(a) + record_bytes(a);
 }
-// Whether a call takes the tile kernels: it has the workspace, and is not one of the small calls where three kernels cost
-// more than one -- a single 32-token tile of the one-kernel path, CTAs enough for every (row, head) at once (measured,
-// bf16: 8.7-13 us against 18-22 at up to 32 tokens, 19-20 against 18-23 at 48; B * Hq = 1024: 42-51 against 28), and for
-// fp32 a rank up to 256 (1024: 57 against 41).
-bool tiles_ok(const dkv_attn_args* a, bool with_scores) {
-  if (with_scores && a->seq_len <= 32 && (long long)a->batch * a->n_q_heads <= 4LL * sm_count() && (a->dtype != DKV_F32 || a->rank <= 256))
-    return false;
+// Whether a call takes the tile kernels.  Small calls do not, where a chain of kernels costs more than the one-kernel path of
+// dkv_generic.cu: a few tokens, and CTAs enough for every (row, head) at once.
+static bool one_kernel_call(const dkv_attn_args* a, int tokens) {
+  return a->seq_len <= tokens && (long long)a->batch * a->n_q_heads <= 4LL * sm_count();
+}
+// The attention, with its workspace: up to a tile of 32 tokens (measured, bf16: 8.7-13 us against 18-22 at up to 32 tokens,
+// 19-20 against 18-23 at 48; B * Hq = 1024: 42-51 against 28), for fp32 at a rank up to 256 (1024: 57 against 41).
+bool tiles_ok(const dkv_attn_args* a) {
+  if (one_kernel_call(a, 32) && (a->dtype != DKV_F32 || a->rank <= 256)) return false;
   return a->batch > 0 && a->seq_len > 0 && a->workspace != nullptr && ((uintptr_t)a->workspace & 15) == 0 &&
-         a->workspace_bytes >= record_bytes(a) + (with_scores ? score_bytes(a) : 0);
+         a->workspace_bytes >= record_bytes(a) + score_bytes(a);
+}
+// The scores alone, 32 heads: 16-bit types up to 32 tokens (rank 256: 6.2 us against 8.6, 48 tokens 9.7 against 8.4; rank 1024:
+// 14.6 against 16.2, 48 tokens 25 against 17).  fp32 never (16 tokens, rank 256: 20.5 against 11).
+bool tiles_scores_ok(const dkv_attn_args* a) { return a->dtype == DKV_F32 || !one_kernel_call(a, 32); }
+// The softmax over given scores, 32 heads: 16-bit types up to 32 tokens (rank 256: 9 us against 13, 48 tokens 12.3-13.1 against
+// 14; rank 1024: 15-16 against 14-17), fp32 up to 64 (rank 256: 9.4 against 13.5, 128 tokens 14.5 against 13.6; rank 1024: 16
+// against 14-23).
+static bool softmax_in_one_kernel(const dkv_attn_args* a) { return one_kernel_call(a, a->dtype == DKV_F32 ? 64 : 32); }
+size_t tiles_softmax_workspace_bytes(const dkv_attn_args* a) {
+  return a->batch <= 0 || a->seq_len <= 0 || softmax_in_one_kernel(a) ? 0 : record_bytes(a);
+}
+bool tiles_softmax_ok(const dkv_attn_args* a) {
+  return !softmax_in_one_kernel(a) && a->batch > 0 && a->seq_len > 0 && a->workspace != nullptr && ((uintptr_t)a->workspace & 15) == 0 &&
+         a->workspace_bytes >= record_bytes(a);
 }
 int tiles_scores(const dkv_attn_args* a) { return launch_scores(a, nullptr); }
 int tiles_attention(const dkv_attn_args* a) {

@@ -179,6 +179,84 @@ PyObject* attend(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// The arguments that the two stage operators share: one side of the cache and its basis, [B, Hq] rows of type `like`.
+bool operator_args(dkv_attn_args& a, const at::Tensor& like, dkv_side& side, PyObject* flat, PyObject* lens, PyObject* offs, const at::Tensor& up, int dev) {
+  a.dtype = dtype_code(like.scalar_type());
+  if (a.dtype < 0 || up.dim() != 3 || !up.is_contiguous() || up.scalar_type() != like.scalar_type() || unpack(flat).scalar_type() != like.scalar_type())
+    return false;
+  const int64_t B = like.size(0);
+  int64_t rows, tokens;
+  if (B == 0 || !fill_side(side, unpack(flat), unpack(lens), unpack(offs), rows, tokens) || rows % B != 0 || tokens == 0) return false;
+  a.n_q_heads = (int32_t)like.size(1);
+  a.n_basis_groups = (int32_t)up.size(0);
+  a.rank = (int32_t)up.size(1);
+  a.head_dim = (int32_t)up.size(2);
+  a.arenas_per_batch = (int32_t)(rows / B);
+  a.batch = (int32_t)B;
+  a.seq_len = (int32_t)tokens;
+  a.theta = 10000.f;
+  a.len_multiple = 1;
+  a.status = g_status[dev];
+  a.stream = stream_of(dev);
+  return true;
+}
+// whether the first argument is a CUDA tensor and all of them are plain tensors on its device, whose status word is known
+int operator_device(PyObject* const* v, int n) {
+  if (!is_tensor(v[0]) || !unpack(v[0]).is_cuda()) return -1;
+  const int dev = unpack(v[0]).get_device();
+  if (dev < 0 || dev >= MAX_DEVICES || g_status[dev] == nullptr) return -1;
+  for (int i = 0; i < n; ++i)
+    if (!plain(v[i], dev)) return -1;
+  return dev;
+}
+
+// scores(q, k_up, k_flat, lens, offs, theta) -> scaled scores [B, Hq, S]
+PyObject* scores(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const int dev = n == 6 ? operator_device(v, 5) : -1;
+  if (dev < 0) Py_RETURN_NONE;
+  const at::Tensor &q = unpack(v[0]), &up = unpack(v[1]);
+  dkv_attn_args a = {};
+  if (q.dim() != 3 || q.stride(2) != 1 || !operator_args(a, q, a.k, v[2], v[3], v[4], up, dev) || q.size(2) != up.size(2)) Py_RETURN_NONE;
+  a.q = q.data_ptr();
+  a.q_stride_b = q.stride(0);
+  a.q_stride_h = q.stride(1);
+  a.k_up = up.data_ptr();
+  a.theta = (float)PyFloat_AsDouble(v[5]);
+  if (PyErr_Occurred()) return nullptr;
+  const at::Tensor out = empty({q.size(0), q.size(1), a.seq_len}, q.scalar_type(), q.device());
+  a.out = out.data_ptr();
+  a.out_stride_b = out.stride(0);
+  a.out_stride_h = out.stride(1);
+  if (int rc = dkv_scores(&a)) return fail("dkv_scores", rc);
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// softmax_v(scores, v_flat, v_up, lens, offs) -> [B, Hq, D]
+PyObject* softmax_v(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const int dev = n == 5 ? operator_device(v, 5) : -1;
+  if (dev < 0) Py_RETURN_NONE;
+  const at::Tensor &sc = unpack(v[0]), &up = unpack(v[2]);
+  dkv_attn_args a = {};
+  if (sc.dim() != 3 || sc.stride(2) != 1 || !operator_args(a, sc, a.v, v[1], v[3], v[4], up, dev)) Py_RETURN_NONE;
+  a.v_up = up.data_ptr();
+  const at::Tensor out = empty({sc.size(0), sc.size(1), up.size(2)}, sc.scalar_type(), sc.device());
+  a.out = out.data_ptr();
+  a.out_stride_b = out.stride(0);
+  a.out_stride_h = out.stride(1);
+  at::Tensor ws;
+  if (const size_t need = dkv_softmax_v_workspace_bytes(&a)) {
+    ws = empty({(int64_t)need}, at::kByte, sc.device());
+    a.workspace = ws.data_ptr();
+    a.workspace_bytes = need;
+  }
+  if (int rc = dkv_softmax_v(&a, sc.data_ptr(), sc.stride(0), sc.stride(1))) return fail("dkv_softmax_v", rc);
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
 long long_max(PyObject* list) {
   long m = 0;
   for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) m = std::max(m, PyLong_AsLong(PyList_GET_ITEM(list, i)));
@@ -583,6 +661,8 @@ PyObject* set_status_word(PyObject*, PyObject* const* v, Py_ssize_t n) {
 
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)), METH_FASTCALL
 PyMethodDef methods[] = {{"attend", FAST(attend), "decode attention"},
+                         {"scores", FAST(scores), "scaled scores of a query"},
+                         {"softmax_v", FAST(softmax_v), "softmax over scores applied to the values"},
                          {"append_token", FAST(append_token), "decode append"},
                          {"new_state", FAST(new_state), "buffers of a new cache layer"},
                          {"grow", FAST(grow), "a cache buffer with more columns"},

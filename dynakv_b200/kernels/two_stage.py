@@ -63,6 +63,9 @@ def abx_sparse(a: torch.Tensor, b: torch.Tensor, x_flat: torch.Tensor, l_vec: to
     """Scaled scores [B, Hq, S] in a's dtype; a = rotated queries [B,Hq,D], b = K basis [groups,R,D]."""
     if offsets is None:
         raise ValueError("offsets are required for the variable-length key cache")
+    done = _lib.host().scores(a, b, x_flat, l_vec, offsets, theta)
+    if done is not None:        # else: tensors that have to be copied first, or refused
+        return done
     batch, heads, _ = a.shape
     seq_len = l_vec.shape[-1]
     out = torch.empty((batch, heads, seq_len), dtype=a.dtype, device=a.device)
@@ -81,10 +84,16 @@ def avx(a: torch.Tensor, x_flat: torch.Tensor, v_up: torch.Tensor, l_vec: torch.
         raise ValueError("offsets are required for the variable-length value cache")
     if a.stride(-1) != 1:
         a = a.contiguous()
+    done = _lib.host().softmax_v(a, x_flat, v_up, l_vec, offsets)
+    if done is not None:        # else: tensors that have to be copied first, or refused
+        return done
     batch, heads, _ = a.shape
     out = torch.empty((batch, heads, v_up.shape[-1]), dtype=a.dtype, device=a.device)
-    args, keep = build_attn_args(None, None, None, x_flat, v_up, None, None, l_vec, offsets, 10000.0, out=out,
-                                 need_workspace=True)
-    _lib.check(_lib.load().dkv_softmax_v(C.byref(args), a.data_ptr(), a.stride(0), a.stride(1)), "dkv_softmax_v")
+    args, keep = build_attn_args(None, None, None, x_flat, v_up, None, None, l_vec, offsets, 10000.0, out=out)
+    lib = _lib.load()
+    if need := lib.dkv_softmax_v_workspace_bytes(C.byref(args)):
+        keep.append(torch.empty(need, dtype=torch.uint8, device=out.device))
+        args.workspace, args.workspace_bytes = keep[-1].data_ptr(), need
+    _lib.check(lib.dkv_softmax_v(C.byref(args), a.data_ptr(), a.stride(0), a.stride(1)), "dkv_softmax_v")
     del keep
     return out

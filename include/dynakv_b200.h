@@ -149,8 +149,11 @@ int dkv_two_stage_decode_noalloc(const dkv_attn_args* a);
 int dkv_scores(const dkv_attn_args* a);
 
 /* Stage 2 as a standalone op: softmax over given scores, latent-space V accumulation, up-projection.
- * Replaces avx (two_stage.py:283-324). scores: [batch, Hq, S] in dtype a->dtype, S contiguous. */
+ * Replaces avx (two_stage.py:283-324). scores: [batch, Hq, S] in dtype a->dtype, S contiguous.  With a workspace of
+ * dkv_softmax_v_workspace_bytes (0: the call is too small to use one; dkv_split_workspace_bytes is enough for any call) the
+ * tokens are cut into slices, without one a CTA takes a (row, head). */
 int dkv_softmax_v(const dkv_attn_args* a, const void* scores, int64_t sc_stride_b, int64_t sc_stride_h);
+size_t dkv_softmax_v_workspace_bytes(const dkv_attn_args* a);
 
 /* ---- cache update ------------------------------------------------------ */
 

@@ -6,7 +6,7 @@ from dynakv_b200 import synthetic
 from dynakv_b200.kernels import _common
 from dynakv_b200.kernels.compressed_cache import CustomDynamicCache
 from dynakv_b200.kernels.fused import fused_attention_dispatch
-from dynakv_b200.kernels.two_stage import two_stage_attention
+from dynakv_b200.kernels.two_stage import abx_sparse, avx, two_stage_attention
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -68,4 +68,28 @@ def test_buffers_that_a_two_dimensional_copy_cannot_grow():
     big[:, -1] = 3.0
     grown = CustomDynamicCache._grown(big, (1 << 30) + 8)
     assert grown.shape == (2, (1 << 30) + 8) and grown[:, (1 << 30) - 9].tolist() == [3.0, 3.0] and int(grown.count_nonzero()) == 2
+    assert _common.read_status(torch.device(DEV)) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("tokens", [1, 20, 90, 700])
+def test_operators_give_what_the_general_path_gives(tokens, dtype):
+    # a basis that records gradients, strided queries and scores, lengths as columns of a wider buffer, a heads axis of one
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    B, R, A = 2, 96, 2
+    lens = torch.randint(1, R + 1, (B * A, tokens + 5), generator=gen, device=DEV, dtype=torch.int32)
+    offs = (torch.cumsum(lens, 1) - lens).to(torch.int32)
+    flat = torch.randn(B * A, int(lens.sum(1).max()), generator=gen, device=DEV).to(dtype)
+    up = (torch.randn(4, R, 128, generator=gen, device=DEV) / R ** 0.5).to(dtype)
+    q = torch.randn(B, 8, 256, generator=gen, device=DEV).to(dtype)[:, :, ::2]
+    lens, offs = lens[:, :tokens], offs[:, :tokens]
+    want = abx_sparse(q.contiguous(), up, flat, lens, offsets=offs, theta=5e5)
+    general = abx_sparse(q.contiguous(), up.clone().requires_grad_(), flat, lens, offsets=offs, theta=5e5)
+    assert torch.equal(want, general) and torch.equal(want, abx_sparse(q, up, flat, lens.view(B, A, -1), offsets=offs.view(B, A, -1), theta=5e5))
+    out = avx(want, flat, up, lens, offs)
+    wide = torch.zeros(B, 8, 2 * tokens, dtype=dtype, device=DEV)
+    wide[:, :, ::2] = want
+    for got in (avx(want, flat, up.clone().requires_grad_(), lens, offs), avx(want.unsqueeze(2), flat.view(B, A, -1), up, lens, offs),
+                avx(wide[:, :, ::2], flat, up, lens, offs)):
+        assert torch.equal(got, out)
     assert _common.read_status(torch.device(DEV)) == 0

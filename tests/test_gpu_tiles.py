@@ -40,6 +40,8 @@ def _dev(t, shift):
 @pytest.mark.parametrize("B,S,R,Hq,groups,arenas,shift", [
     (1, 1, 8, 4, 1, 1, 0), (2, 127, 63, 8, 2, 2, 0), (1, 129, 64, 12, 1, 1, 1), (3, 33, 819, 32, 8, 1, 0), (1, 300, 1024, 40, 40, 1, 0),
     (1, 130, 513, 36, 4, 1, 1),
+    # around the lines below which the operators take one kernel (32 tokens; 64 for the fp32 softmax; 592 rows x heads)
+    (2, 32, 256, 32, 8, 1, 0), (1, 64, 100, 16, 4, 4, 0), (1, 65, 40, 16, 16, 2, 0), (19, 32, 72, 32, 8, 1, 0), (18, 31, 72, 32, 32, 1, 1),
     # one basis for several arenas, basis groups that straddle arenas
     (2, 70, 24, 8, 1, 4, 0), (1, 150, 100, 12, 2, 3, 0), (2, 129, 64, 24, 4, 3, 1), (1, 260, 128, 32, 2, 32, 0)])
 def test_tile_kernels_against_oracle(B, S, R, Hq, groups, arenas, shift, dtype):
