@@ -731,6 +731,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_combine_kernel(dkv_attn_args 
     for (int k = tid; k < n_split; k += 32) M = fmaxf(M, rec0[(size_t)k * (2 + R)]);
     M = warp_max(M);
     float L = 0.f;
+#pragma unroll 1
     for (int k = tid; k < n_split; k += 32) {
       // (a slice whose scores are all NaN leaves the maximum of no score and a sum that is NaN, which its weight takes on)
       const float m = rec0[(size_t)k * (2 + R)], l = rec0[(size_t)k * (2 + R) + 1];
