@@ -964,18 +964,20 @@ __global__ void __launch_bounds__(512, 2) split_combine_kernel(dkv_attn_args p) 
   uint4 bv[4];
   {
     const T* vup = reinterpret_cast<const T*>(p.v_up) + (size_t)g * R * D;
-    const bool vec = (reinterpret_cast<uintptr_t>(p.v_up) & 15) == 0;
+    if ((reinterpret_cast<uintptr_t>(p.v_up) & 15) == 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int row = row0 + 32 * j;
-      bv[j] = make_uint4(0u, 0u, 0u, 0u);
-      if (row < R) {
-        if (vec) {
-          bv[j] = __ldg(reinterpret_cast<const uint4*>(vup + (size_t)row * D) + c8);
-        } else {
-          const uint16_t* e = reinterpret_cast<const uint16_t*>(vup + (size_t)row * D + 8 * c8);
-          bv[j] = make_uint4(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16, e[4] | (uint32_t)e[5] << 16, e[6] | (uint32_t)e[7] << 16);
-        }
+      for (int j = 0; j < 4; ++j) {
+        const int row = row0 + 32 * j;
+        bv[j] = row < R ? __ldg(reinterpret_cast<const uint4*>(vup + (size_t)row * D) + c8) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const int row = row0 + 32 * j;
+        const uint16_t* e = reinterpret_cast<const uint16_t*>(vup + (size_t)row * D + 8 * c8);
+        const uint4 v = row < R ? make_uint4(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16, e[4] | (uint32_t)e[5] << 16, e[6] | (uint32_t)e[7] << 16)
+                                : make_uint4(0u, 0u, 0u, 0u);
+        if (j == 0) bv[0] = v; else if (j == 1) bv[1] = v; else if (j == 2) bv[2] = v; else bv[3] = v;
       }
     }
   }

@@ -119,11 +119,12 @@ __device__ __forceinline__ void token_meta(const dkv_attn_args& p, const dkv_sid
   }
 }
 
-// where the scores of (call row i, head h, token s) go
+// Where the scores of (call row i, head h, token s) go.  The score kernels are given units in place of basis groups in
+// p.n_basis_groups: consecutive query heads that share a basis and an arena, a basis group or an equal part of one.
 struct ScoreSink {
   float* ws;             // fp32 workspace [batch, Hq, pitch], or NULL: out in the query type, masked as the reference does
   int64_t pitch;
-  int heads;             // consecutive query heads of a CTA, all of one basis group and one arena
+  int per_basis;         // units of a basis group
 };
 
 // --------------------------------------------------------------- 1. scores, 16-bit types
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tile = (p.seq_len + TS_TOK - 1) / TS_TOK, i_row = blockIdx.x / n_tile, g = blockIdx.y, t0 = (blockIdx.x - i_row * n_tile) * TS_TOK;
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
-  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = sink.heads;
+  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = Hq / p.n_basis_groups;
   if (sink.ws && row_routed_out(p, b)) return;
   const int t_end = sink.ws ? row_len(p, b) : p.seq_len;     // the operator writes every column
   if (t0 >= t_end) return;
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
   const uint32_t tmem = sm.tmem;
   const int rmax = sm.rmax, n_chunk = (rmax + TS_CHUNK - 1) / TS_CHUNK;
   const T* flat = reinterpret_cast<const T*>(p.k.flat) + (size_t)a * p.k.flat_stride;
-  const T* kup = reinterpret_cast<const T*>(p.k_up) + (size_t)(g * G / (Hq / p.n_basis_groups)) * R * TD;
+  const T* kup = reinterpret_cast<const T*>(p.k_up) + (size_t)(g / sink.per_basis) * R * TD;
   const bool b_vec = (reinterpret_cast<uintptr_t>(p.k_up) & 15) == 0;
   // X pieces of this thread: tokens (tid & 7) + 8 * (tid >> 5) + 64 u', pieces ((tid >> 3) & 3) + 4 u: eight lanes with
   // consecutive tokens write 128 consecutive bytes, four lanes read 64 consecutive bytes of a row
@@ -530,7 +531,10 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
 
 // --------------------------------------------------------------- fp32: the same two steps on the FMA units
 // 16 tokens per CTA: thread = (dim, 8 tokens), coefficients staged transposed so that a load serves four tokens; the
-// rotation's (cos, sin) once per CTA for all heads of the group, exact sincosf as in the single-kernel path.
+// rotation's (cos, sin) once per CTA for all heads of the unit, exact sincosf as in the single-kernel path.  PARTS: units that
+// are parts of basis groups (an instance of its own: with the division in it the compiler keeps 48 registers and not 62, and
+// one sequence of 256 tokens takes 23.5 us in place of 22.6).
+template <bool PARTS>
 __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_args p, ScoreSink sink, float log_theta) {
   __shared__ __align__(16) float x_s[TS_CHUNK][TF_TOK];
   __shared__ float k_s[TF_TOK][TD + 4];
@@ -541,7 +545,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tile = (p.seq_len + TF_TOK - 1) / TF_TOK, i_row = blockIdx.x / n_tile, g = blockIdx.y, t0 = (blockIdx.x - i_row * n_tile) * TF_TOK;
   const int b = p.batch_index ? p.batch_index[i_row] : i_row;
-  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = sink.heads;
+  const int A = p.arenas_per_batch, Hq = p.n_q_heads, R = p.rank, G = Hq / p.n_basis_groups;
   if (sink.ws && row_routed_out(p, b)) return;
   const int t_end = sink.ws ? row_len(p, b) : p.seq_len;
   if (t0 >= t_end) return;
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   }
   __syncthreads();
   const float* flat = reinterpret_cast<const float*>(p.k.flat) + (size_t)a * p.k.flat_stride;
-  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(g * G / (Hq / p.n_basis_groups)) * R * TD;
+  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(PARTS ? g / sink.per_basis : g) * R * TD;
   const int d = tid & 127, th = tid >> 7, rmax = rmax_s;
   float acc[8];
 #pragma unroll
@@ -726,18 +730,21 @@ __global__ void __launch_bounds__(TS_THREADS) tile_combine_kernel(dkv_attn_args 
   const int g = h / (Hq / p.n_basis_groups);
   pdl_wait();
   const float* rec0 = rec + (((size_t)blockIdx.x * Hq + h) * n_split) * (size_t)(2 + R);
-  if (tid < 32) {
-    float M = -INFINITY;
-    for (int k = tid; k < n_split; k += 32) M = fmaxf(M, rec0[(size_t)k * (2 + R)]);
-    M = warp_max(M);
-    float L = 0.f;
-#pragma unroll 1
-    for (int k = tid; k < n_split; k += 32) {
+  if (tid < 32) {      // maxima and sums of up to 64 records, asked for at once
+    float m[2], l[2], M, L = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = tid + 32 * u;
+      m[u] = k < n_split ? rec0[(size_t)k * (2 + R)] : -INFINITY;
+      l[u] = k < n_split ? rec0[(size_t)k * (2 + R) + 1] : 0.f;
+    }
+    M = warp_max(fmaxf(m[0], m[1]));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
       // (a slice whose scores are all NaN leaves the maximum of no score and a sum that is NaN, which its weight takes on)
-      const float m = rec0[(size_t)k * (2 + R)], l = rec0[(size_t)k * (2 + R) + 1];
-      const float w = l != l ? l : m == -INFINITY ? 0.f : __expf(m - M);
-      w_s[k] = w;
-      L = fmaf(w, l, L);
+      const float w = l[u] != l[u] ? l[u] : m[u] == -INFINITY ? 0.f : __expf(m[u] - M);
+      w_s[tid + 32 * u] = w;
+      L = fmaf(w, l[u], L);
     }
     L = warp_sum(L);
     if (tid == 0) L_s = L;
@@ -833,20 +840,23 @@ int launch_scores(const dkv_attn_args* a, float* ws) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const float log_theta = (float)log((double)a->theta);
   const int heads = std::gcd(a->n_q_heads / a->n_basis_groups, a->n_q_heads / a->arenas_per_batch);
-  const ScoreSink sink{ws, score_pitch(a), heads};
+  dkv_attn_args u = *a;
+  u.n_basis_groups = a->n_q_heads / heads;
+  const ScoreSink sink{ws, score_pitch(a), u.n_basis_groups / a->n_basis_groups};
   const int tok = a->dtype == DKV_F32 ? TF_TOK : TS_TOK;
   const long long ctas = (long long)a->batch * ((a->seq_len + tok - 1) / tok);
   DKV_REQUIRE(ctas <= 2147483647LL, DKV_E_LIMIT, "too many tokens");
-  const dim3 grid((unsigned)ctas, a->n_q_heads / heads);      // (n_q_heads <= 65535)
+  const dim3 grid((unsigned)ctas, u.n_basis_groups);      // (n_q_heads <= 65535)
   const int smem = (int)sizeof(ScoreSmem) + 128;
   if (a->dtype == DKV_F32) {
-    tile_scores_f32_kernel<<<grid, TS_THREADS, 0, st>>>(*a, sink, log_theta);
+    if (sink.per_basis > 1) tile_scores_f32_kernel<true><<<grid, TS_THREADS, 0, st>>>(u, sink, log_theta);
+    else tile_scores_f32_kernel<false><<<grid, TS_THREADS, 0, st>>>(u, sink, log_theta);
   } else if (a->dtype == DKV_F16) {
     if (int rc = opt_in(tile_scores_kernel<__half>, smem)) return rc;
-    tile_scores_kernel<__half><<<grid, TS_THREADS, smem, st>>>(*a, sink, log_theta);
+    tile_scores_kernel<__half><<<grid, TS_THREADS, smem, st>>>(u, sink, log_theta);
   } else {
     if (int rc = opt_in(tile_scores_kernel<__nv_bfloat16>, smem)) return rc;
-    tile_scores_kernel<__nv_bfloat16><<<grid, TS_THREADS, smem, st>>>(*a, sink, log_theta);
+    tile_scores_kernel<__nv_bfloat16><<<grid, TS_THREADS, smem, st>>>(u, sink, log_theta);
   }
   DKV_CHECK_LAUNCH();
   return DKV_OK;
