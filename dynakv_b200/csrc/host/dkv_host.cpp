@@ -559,11 +559,22 @@ PyObject* expand(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// One side of the gate: argument struct from tensors, outputs and scratch allocated; false for anything but the plain case.
+// One side of the gate: argument struct from tensors, outputs allocated; false for anything but the plain case.
 struct GateSide {
   dkv_gate_args a = {};
-  at::Tensor lengths, masked, ws;
+  at::Tensor lengths, masked;
 };
+// scratch of one side or of both, in one allocation
+at::Tensor gate_scratch(GateSide* g, int sides) {
+  size_t at[3] = {0, 0, 0};
+  for (int i = 0; i < sides; ++i) at[i + 1] = at[i] + std::max<size_t>((dkv_gate_workspace_bytes(&g[i].a) + 255) / 256 * 256, 256);
+  const at::Tensor ws = empty({(int64_t)at[sides]}, at::kByte, g[0].lengths.device());
+  for (int i = 0; i < sides; ++i) {
+    g[i].a.workspace = static_cast<char*>(ws.data_ptr()) + at[i];
+    g[i].a.workspace_bytes = at[i + 1] - at[i];
+  }
+  return ws;
+}
 bool gate_side(GateSide& g, PyObject* const* t, long low_rank, double threshold, bool want, long len_multiple, bool native) {
   if (!is_tensor(t[0]) || !unpack(t[0]).is_cuda()) return false;
   const int dev = unpack(t[0]).get_device();
@@ -595,10 +606,6 @@ bool gate_side(GateSide& g, PyObject* const* t, long low_rank, double threshold,
     a.masked = g.masked.data_ptr();
     a.masked_stride = d;
   }
-  const size_t need = std::max<size_t>(dkv_gate_workspace_bytes(&a), 16);
-  g.ws = empty({(int64_t)need}, at::kByte, x.device());
-  a.workspace = g.ws.data_ptr();
-  a.workspace_bytes = need;
   a.stream = stream_of(dev);
   return true;
 }
@@ -613,6 +620,7 @@ PyObject* gate(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const bool want = v[5] == Py_True;
   GateSide g;
   if (!gate_side(g, v, low_rank, threshold, want, len_multiple, v[7] == Py_True)) Py_RETURN_NONE;
+  const at::Tensor ws = gate_scratch(&g, 1);
   if (int rc = dkv_gate_lengths(&g.a)) return fail("dkv_gate_lengths", rc);
   PyObject* r = PyTuple_New(2);
   if (want) {
@@ -636,6 +644,9 @@ PyObject* gate_both(PyObject*, PyObject* const* v, Py_ssize_t n) {
   GateSide g[2];
   for (int i = 0; i < 2; ++i)
     if (!gate_side(g[i], v + 3 * i, low_rank, threshold, true, len_multiple, true)) Py_RETURN_NONE;
+  // (the sides may be on two devices, though no one launch takes both then)
+  const bool one_device = g[0].lengths.device() == g[1].lengths.device();
+  const at::Tensor ws = gate_scratch(g, one_device ? 2 : 1), ws2 = one_device ? at::Tensor() : gate_scratch(g + 1, 1);
   if (int rc = dkv_gate_lengths_both(&g[0].a, &g[1].a)) return fail("dkv_gate_lengths_both", rc);
   PyObject* r = PyTuple_New(4);
   for (int i = 0; i < 2; ++i) {
