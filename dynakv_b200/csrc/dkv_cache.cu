@@ -231,14 +231,15 @@ __global__ void __launch_bounds__(256) append_project_grid_kernel(dkv_append_arg
 }
 
 // Bulk (prefill) pack, two kernels on the caller's stream.
-//  1. pack_scan_kernel, one CTA per (block of 1024 new tokens, arena row): validates the row's new lengths, adds
+//  1. pack_scan_kernel, one CTA per (block of 4096 new tokens, arena row): validates the row's new lengths, adds
 //     them up (the whole for the fits test, the part before its block for its first offset) and writes lens / offs
 //     of its tokens.  A block whose payload does not fit is flagged and its tokens are recorded as empty (lens 0,
 //     offs = the write pointer: the rule of the decode append), so that attention never reads stale metadata for
 //     them; a block whose positions do not fit the metadata row is flagged and nothing is written.  The write
 //     pointer is read by every CTA of the row, so it is not advanced here.
 //  2. pack_copy_kernel, one CTA per (block of 256 new tokens, arena row): reads the metadata just written, copies
-//     the payload, and the CTA that holds the row's last new token advances the write pointer to that token's end.  A warp's 32 rows land back to back in the arena, so its payload is one run; with 16-bit elements,
+//     the payload, and the CTA that holds the row's last new token advances the write pointer to that token's end.  A warp's
+//     32 rows land back to back in the arena, so its payload is one run; with 16-bit elements,
 //     lengths multiples of 8 and aligned bases and strides the run moves as 16-byte pieces, one per lane whatever
 //     the rows' lengths (the source of a piece is found by a binary search over the rows' piece prefixes, held
 //     one per lane), four pieces per lane in flight; element by element otherwise.

@@ -120,8 +120,9 @@ def gate_lengths_pair(k_rows: torch.Tensor, Wk: torch.Tensor, bk: torch.Tensor, 
                       bv: torch.Tensor, low_rank: int, out_len_k: torch.Tensor, out_len_v: torch.Tensor,
                       threshold: float = 0.1, len_multiple: int = 1, native_rounding: bool = True) -> None:
     """The cutoffs of the K rows and of the V rows in one launch, for rows of at most 128 coefficients (the decode
-    shape of the per-head layout): the lengths ``gate_lengths`` gives for each side, written into the caller's int32
-    tensors.  Nothing is allocated."""
+    shape of the per-head layout): the lengths ``gate_lengths`` gives for each side (above 64 16-bit rows of 128 up to the
+    order of its sums: a tie with the threshold may fall the other way), written into the caller's int32 tensors.  Nothing
+    is allocated."""
     if not k_rows.is_cuda:
         raise RuntimeError("dynakv_b200 has no CPU path: the gate needs CUDA tensors")
     d = k_rows.shape[-1]

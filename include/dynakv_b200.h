@@ -300,9 +300,10 @@ int dkv_gate_lengths(const dkv_gate_args* args);
 int dkv_gate_lengths_both(const dkv_gate_args* k, const dkv_gate_args* v);
 
 /* The gate for narrow rows (dim <= 128: one row per (sequence, KV head), the decode shape of the per-head layout),
- * K and V sides in ONE launch and without a workspace: same arithmetic, in the same order, as dkv_gate_lengths on
- * each side (kv_process_fused computes both sides in one call too, compressed_attention.py:92-114).  The two
- * argument blocks must agree in dtype, dim, n_rows and stream; workspace fields are ignored. */
+ * K and V sides in ONE launch and without a workspace: same arithmetic, in the same order, as dkv_gate_lengths on each
+ * side up to 64 rows and in fp32 (kv_process_fused computes both sides in one call too, compressed_attention.py:92-114).
+ * Above 64 16-bit rows dkv_gate_lengths takes the logits of rows of 128 from the tensor core: fp32 sums in another order, so a
+ * length may differ where a running sum ties with the threshold.  The two argument blocks must agree in dtype, dim, n_rows and stream; workspace fields are ignored. */
 int dkv_gate_lengths_pair(const dkv_gate_args* k, const dkv_gate_args* v);
 
 /* ---- row operators of a Llama-shaped decode step ------------------------ */

@@ -57,3 +57,28 @@ def test_the_gate_reports_to_the_status_word(monkeypatch):
     gate_lengths(x, w, b, 128)
     kv_process_fused(x[None], x[None], w, b, w, b, 128)
     assert _common.read_status(dev) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("rows", [64, 65, 512])
+def test_pair_and_prompt_paths_differ_by_summation_order_only(rows, dtype):
+    # dkv_gate_lengths takes more than 64 16-bit rows of 128 from the tensor core, the pair adds up in ascending order
+    from dynakv_b200.kernels.compressed_attention import gate_lengths, gate_lengths_pair
+    gen, d, thr = torch.Generator().manual_seed(rows), 128, 0.1
+    x, v = ((torch.randn(rows, d, generator=gen) * 2).to(dtype).cuda() for _ in range(2))
+    w, b = (torch.randn(d, d, generator=gen) / d ** 0.5).to(dtype).cuda(), (torch.randn(d, generator=gen) * 0.5).to(dtype).cuda()
+    lk, lv = (torch.empty(rows, dtype=torch.int32, device="cuda") for _ in range(2))
+    gate_lengths_pair(x, w, b, v, w, b, d, lk, lv, native_rounding=False)
+    for states, pair in ((x, lk), (v, lv)):
+        _, lens = gate_lengths(states, w, b, d, native_rounding=False)
+        if rows <= 64 or dtype == torch.float32:
+            assert torch.equal(lens, pair)
+            continue
+        logits = states.double() @ w.double() + b.double()
+        sums = torch.cumsum(torch.softmax(logits, -1), -1)
+        # a logit is a sum of 129 terms: off by at most 129 units of 2^-23 of the terms' sum (2^-24 if rounded, twice that if cut);
+        # a probability by twice the largest of these, relative, and a running sum of them by as much of itself and 256 roundings
+        off = 129 * 2.0 ** -23 * (states.double().abs() @ w.double().abs() + b.double().abs()).amax(-1, keepdim=True)
+        tie = (sums - thr).abs() <= sums * (2 * off + 256 * 2.0 ** -23)
+        differ = lens != pair
+        assert bool(tie.any(-1)[differ].all()) and int((lens - pair).abs().max()) <= int(tie.sum(-1).max())

@@ -118,3 +118,37 @@ def test_a_block_whose_growth_fails_leaves_the_layer_as_it_was(fresh, monkeypatc
         for r in range(B * A):
             assert np.array_equal(state[0][r, : lay.ptr[r]].float().cpu().numpy(), lay.flat[r])
     assert _common.read_status(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("grows", ["both", "values"])
+def test_ragged_blocks_grow_like_the_layout_oracle(grows):
+    # rows of other counts in every block: at a growth some rows fit the old buffers (and moved on in the first attempt), some do not
+    gen = torch.Generator().manual_seed(6)
+    B, A, R = 3, 2, 128
+    cache = CustomDynamicCache(arenas_per_batch=A, len_multiple=8)
+    cache.reserve(0, B, 1 << 17 if grows == "values" else 1500, 8, torch.bfloat16, "cuda")
+    if grows == "values":
+        cache.value_cache_sp[0] = cache._new_state(B * A, 1500, 8, torch.bfloat16, "cuda")
+    lays = [[O.LayoutOracle(A, np.float32) for _ in range(B)] for _ in range(2)]
+    caps = []
+    for n_new, counts in ((12, [12, 3, 0]), (70, [2, 70, 9]), (1, [1, 0, 1]), (300, [300, 1, 0]), (40, [40, 40, 40]), (5000, [17, 5000, 4097])):
+        rows = [torch.randn(B, n_new, A * R, generator=gen).to(torch.bfloat16) for _ in range(2)]
+        lens = [(torch.randint(0, 17, (B, A, n_new), generator=gen) * 8).to(torch.int32) for _ in range(2)]
+        cache.update_sp(rows[0].cuda(), lens[0].cuda(), rows[1].cuda(), lens[1].cuda(), A * R, 0, R, token_counts=counts)
+        for side in range(2):
+            for b, c in enumerate(counts):
+                lays[side][b].update(rows[side][b, :c].float().view(c, A, R).permute(1, 0, 2).numpy(), lens[side][b, :, :c].numpy())
+        caps.append((cache.key_cache_sp[0][0].shape[1], cache.value_cache_sp[0][0].shape[1]))
+    growths = [(a[0] != b[0], a[1] != b[1]) for a, b in zip(caps, caps[1:])]
+    assert ((True, True) if grows == "both" else (False, True)) in growths
+    stored = [lays[0][b].seq for b in range(B)]
+    assert cache.seq_lens(0).tolist() == stored == cache.seq_lens_host(0)
+    for side, state in enumerate((cache.key_cache_sp[0], cache.value_cache_sp[0])):
+        assert state[5] == state[3].tolist() == [int(x) for b in range(B) for x in lays[side][b].ptr]
+        for b in range(B):
+            lay, n = lays[side][b], stored[b]
+            assert np.array_equal(state[1][b * A:(b + 1) * A, :n].cpu().numpy(), lay.lens)
+            assert np.array_equal(state[2][b * A:(b + 1) * A, :n].cpu().numpy(), lay.offs)
+            for j in range(A):
+                assert np.array_equal(state[0][b * A + j, : lay.ptr[j]].float().cpu().numpy(), lay.flat[j])
+    assert _common.read_status(torch.device("cuda")) == 0
