@@ -10,7 +10,7 @@
 // (a piece of 8 coefficients may start at any element, it is put together from two aligned 16-byte loads), the softmax
 // weights as two 16-bit terms so that nothing is lost against fp32 weights.  fp32 stays on the FMA units.
 // The first version (one CTA per (row, query head, slice), K reconstructed per query head on mma.sync) took 281 us on
-// B = 2, S = 2048, R = 1024, 8 groups, bf16, and 13 us for the merge; now 25 (scores) + 13 (latent sums) + 8 us (merge).
+// B = 2, S = 2048, R = 1024, 8 groups, bf16, and 13 us for the merge; now 25 (scores) + 13 (latent sums) + 7 us (merge).
 // fp32, B = 1, S = 256, 8 arenas: 131 us in one kernel of 32 CTAs, now 12 + 6.5 + 5 us.
 //
 // Math (reference: src/dynakv/kernels/fused.py:28-142, two_stage.py:52-157, 211-281): as in dkv_generic.cu, which keeps
