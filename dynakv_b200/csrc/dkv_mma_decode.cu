@@ -10,25 +10,36 @@
 //   4+4 gather warps : copy each token's ragged K / V coefficient row (16-byte cp.async, zero fill past the
 //                      row's length) into K-major, unswizzled 128 x 128 operand tiles in shared memory; the
 //                      copy engine itself signals the tile's barrier when a lane's copies have landed;
-//   2 MMA threads    : per tile  (1) K = X . Bk          M=128 tokens, N=128, K=128 (A, B from shared memory)
+//   3 MMA warps      : per tile  (1) K = X . Bk          M=128 tokens, N=128, K=128 (A, B from shared memory)
 //                                (2) S = K' . Q~^T       M=128 tokens, N=16,  K=128 (A = K' in tensor memory)
 //                                (3) O^T += XV^T . P     M=128 latent, N=16,  K=128 tokens (accumulates per row);
-//                      one thread issues (1) and (2) from an event loop over barrier probes, another issues (3);
-//                      completion of each product is signalled by tcgen05.commit on mbarriers;
+//                      one product each, issued by an elected lane; completion is signalled by tcgen05.commit on mbarriers;
 //   1 rotator warp   : Q~ = scale . R(-s0) q for the tile's base position s0 (the B operand of (2)), so K is
 //                      rotated only by the in-tile offset 0..127;
-//   4 RoPE warps     : a thread reads its token's K row from one of three accumulator buffers (tcgen05.ld.32x32b),
-//                      applies [RMSNorm and] RoPE in fp32 with its 64 (cos, sin) pairs, which also live in tensor
-//                      memory (fp16 pairs; they depend on the lane only), and writes K' back in place as packed
+//   8 RoPE warps     : a thread reads half of its token's K row from one of three accumulator buffers
+//                      (tcgen05.ld.32x32b), applies [RMSNorm and] RoPE in fp32 with its (cos, sin) pairs, which also live in
+//                      tensor memory (fp16 pairs; they depend on the lane only), and writes K' back in place as packed
 //                      16-bit pairs (tcgen05.st) for product (2);
-//   4 softmax warps  : a thread reads its token's four scores, takes p = exp2(s - m_ref) against a reference
-//                      maximum shared by the four warps, which is only raised (with a rescale of O in tensor
-//                      memory) when a tile exceeds it by more than 2^8, and stores P for product (3); these
-//                      warps follow the batch rows and write each row's partial (split) or projected (fused)
-//                      result.
+//   2 x 4 softmax warps : even and odd tiles, each with its own reference maximum, sum and O.  A thread reads its token's
+//                      four scores, takes p = exp2(s - m_ref) against the reference maximum shared by the four warps,
+//                      which is only raised (with a rescale of O in tensor memory) when a tile exceeds it by more than
+//                      2^8, and stores P for product (3); these warps follow the batch rows, merge the even and the odd
+//                      tiles' sums at a row's end and write its partial (split) or projected (fused) result.
+//
+// What bounds it: no unit is saturated; a tile passes through a ring of latencies, and every stage is a chain of dependent
+// instructions on a warp that shares its issue slots with six others and its instruction cache with all of them.  Measured
+// with clock64 at every hand-over (8 rows of 32768 tokens, cycles per tile): one lane that issued (1) and (2) was the period
+// (620 + 600 of issue, 770 of barrier probes and commits: 1980).  A product's eight instructions took 75 cycles each because
+// a lane's operands are not known to be uniform: 38 instructions per tcgen05.mma.  Issued from converged warps through
+// elect.sync they take 20, and the kernel 58 KB of code instead of 84.  Now the gather loop is the period (1600: 600 of copies,
+// the rest before them).
+// Split kernel, 8 KV heads, start -> now in us, in a chain of launches with the merge: 8 rows of 32768 tokens, lengths beta(2,8)
+// 139 -> 106; 32 rows of 8192, beta(2,5) 151 -> 119; 32 rows of 513 28.6 -> 25.2; 30 rows of 300, 600 and 2500 with K-RMSNorm
+// 37.5 -> 33.3; one row of 1100 / 4096 / 16000 tokens 16.3 / 17.4 / 22.9 -> 15.4 / 16.1 / 20.0.
 //
 // Reference math: src/dynakv/kernels/fused.py:28-142 (fused), two_stage.py:52-157,211-281 (two-stage;
 // the latent-space V accumulation with one up-projection at the end is two_stage.py:261-277).
+#include <limits.h>
 #include <math.h>
 
 #include <type_traits>
@@ -38,32 +49,33 @@
 namespace dkv {
 
 constexpr int D = 128;
-constexpr int NGROUP = 2;              // score tiles / P tiles in flight (tile parity)
-constexpr int NCW = 8;                 // warps 0-3: RoPE stage, warps 4-7: softmax stage
-// Service warps.  Warp w runs on SM sub-partition w % 4, next to RoPE warp w % 4 and softmax warp 4 + w % 4; the roles are
-// placed so that the sub-partitions of the two issuer threads do not also hold the (large) gather code: the
-// instruction caches are small and the issuers' instruction stream is the serial part of the pipeline.
-constexpr int W_KG0 = 8;               // K gather warps 8, 12 (32 tokens of the tile each; two more below)
-constexpr int W_VG0 = 9;               // V gather warps 9, 13
-constexpr int W_MMA = 10;              // tcgen05.mma issuer for products (1), (2); owns the tensor-memory allocation
-constexpr int W_ROT = 14;              // query rotator
-constexpr int W_MMA2 = 11;             // tcgen05.mma issuer for product (3)
-constexpr int W_G2 = 16;               // gather warps 16, 17 (K) and 18, 19 (V): the second half of each side's four
+constexpr int NGROUP = 2;              // even and odd tiles: score tiles, P tiles, O accumulators, softmax warps
+constexpr int NCW = 8;                 // warps 0-3: RoPE stage, warps 4-7: softmax stage of the even tiles
+// Service warps 8-19.  Warp w runs on SM sub-partition w % 4, next to RoPE warps w % 4 and 20 + w % 4 and softmax warps 4 + w % 4
+// and 24 + w % 4: two gather warps and one of the four others on each.
+constexpr int W_KG0 = 8;               // K gather warps 8-11 (32 tokens of the tile each)
+constexpr int W_VG0 = 12;              // V gather warps 12-15
+constexpr int W_MMA = 16;              // tcgen05.mma issuer for product (1); owns the tensor-memory allocation
+constexpr int W_MMA2 = 17;             // tcgen05.mma issuer for product (2)
+constexpr int W_MMA3 = 18;             // tcgen05.mma issuer for product (3)
+constexpr int W_ROT = 19;              // query rotator
 constexpr int W_ROPE2 = 20;            // RoPE warps 20-23: the second half of each token's pairs (sub-partition w % 4 again)
-constexpr int NTHREADS = 24 * 32;      // at most 85 registers per thread
+constexpr int W_SM2 = 24;              // softmax warps 24-27: the odd tiles
+constexpr int NTHREADS = 28 * 32;      // at most 72 registers per thread
 constexpr int ST_TOK = 128;            // tokens per tile = rows of one UMMA
 constexpr int NBUF_A = 3;              // K operand tiles in shared memory (on the critical ring: three in flight)
 constexpr int NBUF_T = 3;              // K accumulator buffers in tensor memory (held from product (1) to product (2))
 constexpr int NBUF_V = 2;              // V operand tiles
 constexpr int NQ = 2;                  // rotated-query tiles
-constexpr int PD = 2;                  // prefetch distance of the gather warps' metadata (tiles)
-constexpr int MSLOT = PD + 1;          // metadata staging slots (private to the lane that fetched them)
 constexpr int KV_RING = 8;             // tiles of token-validity masks kept
 // 1/rms ring: a RoPE write for tile c only implies that the softmax warps have finished tile c-5 (product (1) of c
-// needs product (2) of c-3 issued, which needs the P tile of c-5), so tiles c-4 .. c may be unread
+// needs product (2) of c-3, which needs the P tile of c-5), so tiles c-4 .. c may be unread
 constexpr int RS_RING = 5;
 static_assert(RS_RING >= 5, "1/rms ring must cover the RoPE warps' lead over the softmax warps");
-constexpr int TILE_BYTES = ST_TOK * 128 * 2;   // 128 tokens x 128 coefficients, chunk-major
+// Operand tiles: chunk c (8 coefficients) of token t at c*CHUNK_PITCH + t*16.  The 32 bytes beyond 128 rows of 16 put a token's
+// neighbouring chunks on other banks: the four lanes that copy them would otherwise all write to one bank group.
+constexpr int CHUNK_PITCH = ST_TOK * 16 + 32;
+constexpr int TILE_BYTES = 16 * CHUNK_PITCH;
 constexpr int Q_LBO = 272;             // byte distance of the 8-dim chunks of the rotated-query tile (bank spread)
 constexpr int Q_TILE_BYTES = 16 * Q_LBO;
 constexpr int HP = 4;                  // query heads per KV head supported by this kernel
@@ -71,36 +83,45 @@ constexpr int MAX_BATCH = 1024;
 constexpr int PART_STRIDE = 2 + 128;   // floats per (head) partial record: m, l, latent[128]
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 constexpr float M_SLACK = 8.f;         // a tile may exceed the reference maximum by 2^8 before O is rescaled
-// tensor-memory columns (32-bit cells): three K accumulators, the RoPE table (fp16 pairs), two score tiles, one O
-// accumulator
+// tensor-memory columns (32-bit cells): three K accumulators, the RoPE table (fp16 pairs), two score tiles, O of
+// the even and of the odd tiles
 constexpr uint32_t TM_K = 0, TM_TRIG = 384, TM_S = 448, TM_O = 480, TMEM_COLS = 512;
 
 struct SmemLayout {
-  alignas(1024) unsigned char a_tile[NBUF_A][TILE_BYTES];   // chunk c (8 coefficients) of token t at c*2048 + t*16
-  alignas(1024) unsigned char v_tile[NBUF_V][TILE_BYTES];   // same layout; [NBUF_V-1] stages the RoPE table in the prologue
-  alignas(1024) unsigned char basis[128 * 256];             // Bk[r][d] at (r/8)*2048 + (d/8)*128 + (r%8)*16 + (d%8)*2
+  alignas(1024) unsigned char a_tile[NBUF_A][TILE_BYTES];
+  alignas(128) unsigned char v_tile[NBUF_V][TILE_BYTES];   // both together stage the RoPE table in the prologue
+  alignas(128) unsigned char basis[128 * 256];             // Bk[r][d] at (r/8)*2048 + (d/8)*128 + (r%8)*16 + (d%8)*2
   alignas(128) unsigned char qrot[NQ][Q_TILE_BYTES];        // Q~[n][d] at (d/8)*272 + (n/8)*128 + (n%8)*16 + (d%8)*2
   alignas(128) unsigned char p_tile[NGROUP][ST_TOK * 16];   // P[t][n < 8] at t*16
-  alignas(16) int meta[2][MSLOT][2][ST_TOK];                // [K|V][slot][lens|offs][token]
-  alignas(16) float lat[HP][128];                           // fused path: normalised latent result of a row
-  alignas(16) float tmax[4][4];                             // [warp][head]
-  alignas(16) float lsum[4][4];                             // [warp][head]
-  alignas(16) float rs_buf[RS_RING][2][ST_TOK];             // K-RMSNorm: sum of squares of each half of the tokens' K rows, last tiles
+  alignas(16) int kmax[NBUF_A][4];                          // chunks of the longest row of each 32 tokens
+  alignas(16) float4 dep_o[2][ST_TOK];                        // what one group hands to the other at a row's end: latent sums ([1]: also the fused path's result),
+  alignas(16) float dep_l[2][HP][4];                        // sums of weights [head][warp],
+  alignas(16) float4 dep_m[2];                              // reference maxima
+  alignas(16) float tmax[NGROUP][4][4];                     // [warp][head]
+  alignas(16) float factor[NGROUP][2][HP];                  // of the two groups' sums in the row's
+  alignas(16) float fused_l[HP];                            // fused path: the row's sums of weights
+  alignas(16) float lsum[NGROUP][HP][4];                    // [head][warp]
+  alignas(16) float rs_buf[RS_RING][2][ST_TOK];             // K-RMSNorm: sums of squares of the halves of the tokens' K rows, last tiles
   alignas(16) float knorm_w[D];
   uint32_t kvalid[KV_RING][4];                              // bit l of word w: token 32w + l of the tile has a K row
-  alignas(8) unsigned long long a_full[NBUF_A];    // K operand tile written (128 gather lanes)
+  alignas(8) unsigned long long basis_full;        // Bk written (every thread's copies)
+  alignas(8) unsigned long long a_full[NBUF_A];    // K operand tile written (128 gather lanes, and the 4 warps' kmax)
   alignas(8) unsigned long long v_full[NBUF_V];    // V operand tile written (128 gather lanes)
-  alignas(8) unsigned long long v_free[NBUF_V];    // product (3) done with it (commit)
   alignas(8) unsigned long long q_full[NQ];        // rotated queries written (rotator)
   alignas(8) unsigned long long t_ready[NBUF_T];   // K accumulator written (commit)
   alignas(8) unsigned long long kp_ready[NBUF_T];  // K' written back to tensor memory (8 RoPE warps)
-  alignas(8) unsigned long long s_ready[NGROUP];   // scores written (commit)
+  alignas(8) unsigned long long s_ready[NBUF_T];   // scores written (commit): product (2) of the K accumulator's tile is done
   alignas(8) unsigned long long p_ready[NGROUP];   // P tile written (4 token warps)
-  alignas(8) unsigned long long pv_done[NGROUP];   // product (3) done: O updated, P tile free (commit)
+  alignas(8) unsigned long long pv_done[NGROUP];   // product (3) done: O updated, P tile and V operand tile free (commit)
+  alignas(8) unsigned long long dep_full[2];       // a row's end handed over (4 warps)
+  alignas(8) unsigned long long dep_free[2];       // and taken (4 warps)
   int prefix[MAX_BATCH + 1];
+  int tokens[MAX_BATCH];                           // of each row in this call
   int abort_flag;
   uint32_t tmem_base;
 };
+static_assert(NBUF_V == NGROUP && NQ == NGROUP, "rings of two share index and phase");
+static_assert(NBUF_A == NBUF_T, "the K operand tiles and the K accumulators share ring index and phase");
 static_assert(sizeof(SmemLayout) <= 227 * 1024, "shared memory budget");
 static_assert(ST_TOK * 65 * 4 <= NBUF_V * TILE_BYTES, "RoPE staging table must fit in the V tiles");
 
@@ -127,6 +148,7 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // polling lane the other lanes' later shared-memory loads are not ordered behind the wait and can be scheduled
 // ahead of it.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
   for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
     if (mbar_test(bar, parity)) return true;
     if ((it & 1023u) == 1023u && *abort_flag) return false;
@@ -134,67 +156,45 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
-// Non-blocking probe of a barrier phase.
-__device__ __forceinline__ bool mbar_probe(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
+// The same answer in all lanes (the tensor-core issuers elect a lane afterwards).
+__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
-// The same for a single thread (the tensor-core issuers run on one lane).
-__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
-    if (mbar_test(bar, parity)) return true;
-    if ((it & 1023u) == 1023u && *abort_flag) return false;
-  }
-  *abort_flag = 1;
-  return false;
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, int src_bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+// 16 bytes, or zeros without a read
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool zero) {
+  asm volatile("{\n.reg .pred z;\nsetp.ne.u32 z, %2, 0;\ncp.async.ca.shared.global [%0], [%1], 16, z;\n}" ::"r"(dst), "l"(src), "r"((uint32_t)zero) : "memory");
 }
 // The barrier receives one arrival from this thread once all of its earlier cp.async copies have landed.
 __device__ __forceinline__ void cp_async_arrive_when_landed(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // tcgen05 (5th generation tensor core) helpers ---------------------------------------------------------
 // Shared-memory matrix descriptors are unswizzled: start address, leading and stride byte offsets in 16-byte
 // units, descriptor version 1.
 // tcgen05.mma with the shared-memory operand descriptors passed as two 32-bit words (low = (address >> 4) |
-// (LBO >> 4) << 16, high = (SBO >> 4) | version bit 46): the issuer threads keep the words of each ring slot ready
-// and add the (compile-time) k-step offset to the low word, so that nothing but that add stands between two
-// tcgen05.mma of a product.  Building the 64-bit descriptor with shifts, masks and ors per step (~15 dependent
-// instructions on a lone thread) was what an issue block waited on.
+// (LBO >> 4) << 16, high = (SBO >> 4) | version bit 46).  Called by a converged warp with operands that are the same in all
+// lanes, and issued by one elected lane: what stands in a branch of a single lane is built lane by lane, at twice the
+// instructions.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) { return ((addr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16); }
 __device__ __forceinline__ uint32_t desc_hi(uint32_t sbo) { return ((sbo >> 4) & 0x3FFFu) | (1u << 14); }
 __device__ __forceinline__ void umma_f16_w(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                            uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n.reg .b64 da, db;\n.reg .pred p;\nmov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\nsetp.ne.b32 p, %6, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}"
+      "{\n.reg .b64 da, db;\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nmov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\nsetp.ne.b32 p, %6, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}"
       ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 // the same with the A operand in tensor memory (16-bit pairs packed in 32-bit cells, lane = row)
 __device__ __forceinline__ void umma_f16_ta_w(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
-      "{\n.reg .b64 db;\n.reg .pred p;\nmov.b64 db, {%2, %3};\nsetp.ne.b32 p, %5, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
+      "{\n.reg .b64 db;\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nmov.b64 db, {%2, %3};\nsetp.ne.b32 p, %5, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
       ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -246,14 +246,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const float (&v)[16]) {
 
 // whether any thread of the 4 softmax warps says so.  (All four pass the same sequence of these barriers whatever their
 // bounded waits return.)
-__device__ __forceinline__ bool consumer_any(bool v) {
+__device__ __forceinline__ bool consumer_any(int grp, bool v) {
   uint32_t r;
-  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred q, 1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
-               : "=r"(r) : "r"((uint32_t)v), "n"(4 * 32) : "memory");
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred q, %3, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
+               : "=r"(r) : "r"((uint32_t)v), "n"(4 * 32), "r"(1 + grp) : "memory");
   return r != 0;
 }
-__device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, %0;" ::"n"(4 * 32) : "memory"); }   // the 4 softmax warps
-
+__device__ __forceinline__ void consumer_bar(int grp) { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(4 * 32) : "memory"); }   // the 4 softmax warps of a group
 // order-preserving map float -> int (and back: the map is its own inverse), for redux.sync
 __device__ __forceinline__ int float_key(float f) {
   const int i = __float_as_int(f);
@@ -261,6 +260,17 @@ __device__ __forceinline__ int float_key(float f) {
 }
 __device__ __forceinline__ float key_float(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
 __device__ __forceinline__ float warp_max_redux(float v) { return key_float(__reduce_max_sync(0xffffffffu, float_key(v))); }
+
+// Sums over the warp of four values at once: lane l gets that of value l / 8 (6 shuffles; 20 one by one).
+__device__ __forceinline__ float warp_sum4(const float (&v)[4], int lane) {
+  const bool hi = lane & 16, odd = lane & 8;
+  float a = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+  float b = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+  float s = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
 
 template <typename T>
 struct Pack;
@@ -278,6 +288,9 @@ struct Pack<__half> {
     return *reinterpret_cast<uint32_t*>(&v);
   }
 };
+
+// One copy of the library function for all its uses here (each inlined copy brings its slow path for large arguments).
+__device__ __noinline__ void sincos_call(float x, float* s, float* c) { sincosf(x, s, c); }
 
 // --------------------------------------------------------------- work partition
 // Token space of one KV head: batch rows back to back, each rounded up to whole 128-token tiles.
@@ -310,7 +323,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   SmemLayout& sm = *reinterpret_cast<SmemLayout*>(smem_raw);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // (known to be the same in all lanes)
   const int g = blockIdx.y;                        // KV head == basis group == arena within the batch row
   const int G = p.n_q_heads / p.n_basis_groups;    // query heads sharing this KV head (<= HP)
   const int R = p.rank;
@@ -336,26 +349,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
   if (tid == 0) {
     sm.prefix[0] = 0;
     sm.abort_flag = 0;
-    for (int s = 0; s < NBUF_A; ++s) mbar_init(smem_u32(&sm.a_full[s]), ST_TOK);   // one arrival per gather lane
-    for (int s = 0; s < NBUF_V; ++s) { mbar_init(smem_u32(&sm.v_full[s]), ST_TOK); mbar_init(smem_u32(&sm.v_free[s]), 1); }
+    mbar_init(smem_u32(&sm.basis_full), NTHREADS);
+    for (int s = 0; s < NBUF_A; ++s) mbar_init(smem_u32(&sm.a_full[s]), ST_TOK + 4);   // one arrival per gather lane when its copies have landed, one per warp for kmax
+    for (int s = 0; s < NBUF_V; ++s) { mbar_init(smem_u32(&sm.v_full[s]), ST_TOK); }
     for (int s = 0; s < NQ; ++s) mbar_init(smem_u32(&sm.q_full[s]), 1);
+    for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&sm.dep_full[s]), 4); mbar_init(smem_u32(&sm.dep_free[s]), 4); }
     for (int s = 0; s < NGROUP; ++s) {
-      mbar_init(smem_u32(&sm.s_ready[s]), 1);
       mbar_init(smem_u32(&sm.p_ready[s]), 4);
       mbar_init(smem_u32(&sm.pv_done[s]), 1);
     }
-    for (int s = 0; s < NBUF_T; ++s) { mbar_init(smem_u32(&sm.t_ready[s]), 1); mbar_init(smem_u32(&sm.kp_ready[s]), 8); }
+    for (int s = 0; s < NBUF_T; ++s) { mbar_init(smem_u32(&sm.t_ready[s]), 1); mbar_init(smem_u32(&sm.s_ready[s]), 1); mbar_init(smem_u32(&sm.kp_ready[s]), 8); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   {
     // basis rows [R][128] -> the MN-major unswizzled operand layout of the tensor core: 8x8 core matrices,
     // element (r, d) at (r/8)*2048 + (d/8)*128 + (r%8)*16 + (d%8)*2; rows >= R are zero
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.k_up) + (size_t)g * R * D);
+    // (asked for all at once; the first tiles' metadata and copies need not wait for it)
+    const T* src = reinterpret_cast<const T*>(p.k_up) + (size_t)g * R * D;
     for (int e = tid; e < 128 * 16; e += NTHREADS) {
       const int r = e >> 4, c = e & 15;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (r < R) v = src[r * 16 + c];
-      *reinterpret_cast<uint4*>(sm.basis + (r >> 3) * 2048 + c * 128 + (r & 7) * 16) = v;
+      cp_async16_or_zero(smem_u32(sm.basis + (r >> 3) * 2048 + c * 128 + (r & 7) * 16), src + (size_t)min(r, R - 1) * D + 8 * c, r >= R);
     }
     if (warp == W_MMA) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
@@ -373,8 +386,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     const int j = tid & 63;
     const float f = expf(-((float)(2 * j) / (float)D) * log_theta);
     float sn, cs, ds, dc;
-    sincosf((float)(tid >> 6) * f, &sn, &cs);
-    sincosf((float)TSTEP * f, &ds, &dc);
+    sincos_call((float)(tid >> 6) * f, &sn, &cs);
+    sincos_call((float)TSTEP * f, &ds, &dc);
     for (int t = tid >> 6; t < ST_TOK; t += TSTEP) {
       const int idx = t * 130 + 4 * (j >> 1) + (j & 1);
       tr[idx] = __float2half_rn(cs);
@@ -393,20 +406,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     int carry = 0;
     for (int base = 0; base < p.batch; base += 32) {
       const int i = base + lane;
-      int v = (i < p.batch) ? (row_tokens(p, i) + ST_TOK - 1) / ST_TOK : 0;
+      const int tokens = i < p.batch ? row_tokens(p, i) : 0;
+      int v = (tokens + ST_TOK - 1) / ST_TOK;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int t = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += t;
       }
-      if (i < p.batch) sm.prefix[i + 1] = carry + v;
+      if (i < p.batch) { sm.prefix[i + 1] = carry + v; sm.tokens[i] = tokens; }
       carry += __shfl_sync(0xffffffffu, v, 31);
     }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = sm.tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
   if (warp < 4) {
     // the table row of this thread's in-tile offset goes to its tensor-memory lane
     const float* tr = reinterpret_cast<const float*>(sm.v_tile[0]) + tid * 65;   // 64 packed words of this row
@@ -420,7 +434,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     }
     tmem_wait_st();
   }
-  proxy_fence_async();     // the basis was written with ordinary stores and is read by the tensor core
+  cp_async_arrive_when_landed(smem_u32(&sm.basis_full));     // the basis: only product (1) waits for it
+  proxy_fence_async();     // the query tiles' zeros are read by the tensor core
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -467,12 +482,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     while (u >= sm.prefix[ri.row + 1]) ++ri.row;
     const int b = p.batch_index ? p.batch_index[ri.row] : ri.row;
     ri.arena = b * p.arenas_per_batch + g;
-    ri.tokens = row_tokens(p, ri.row);
+    ri.tokens = sm.tokens[ri.row];
     ri.first_unit = sm.prefix[ri.row];
   };
 
   if (n_stages <= 0) {
     // nothing to do for this CTA (fewer tiles than CTAs, or an empty row): straight to the epilogue
+    cp_async_wait_all();
   }
   else if (warp == W_ROT) {
     // =========================== query rotator warp ===========================
@@ -482,35 +498,52 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     const float f0 = expf(-((float)(4 * lane) / (float)D) * log_theta);
     const float f1 = expf(-((float)(4 * lane + 2) / (float)D) * log_theta);
     float cd0, sd0, cd1, sd1;     // rotation by one tile
-    sincosf((float)ST_TOK * f0, &sd0, &cd0);
-    sincosf((float)ST_TOK * f1, &sd1, &cd1);
+    sincos_call((float)ST_TOK * f0, &sd0, &cd0);
+    sincos_call((float)ST_TOK * f1, &sd1, &cd1);
     const float qscale = rsqrtf((float)D) * 1.4426950408889634f;  // softmax scale and log2(e) folded into q
     float a0[HP], b0[HP], a1[HP], b1[HP];   // (q~_j, q~_{j+64}) for j = 2l and j = 2l+1
-    int row = row0;
+    // The queries of the CTA's next row are asked for when a row begins: read at its own start they hold product (2) back by
+    // the latency of memory (1100 tokens: 16.0 -> 15.9 us with the merge, 30 rows of 300 to 2500 with K-RMSNorm 41.1 -> 40.5).
+    T next[HP][4];
+    int row = row0, next_row = row0;
+    auto ask_queries = [&](int r) {       // of the first row from r on that has tiles here
+      while (r < p.batch && sm.prefix[r + 1] == sm.prefix[r]) ++r;
+      next_row = r;
+      if (r >= p.batch || sm.prefix[r] >= u_end) return;
+      const int b = p.batch_index ? p.batch_index[r] : r;
+#pragma unroll
+      for (int h = 0; h < HP; ++h) {
+        if (h < G) {
+          const T* qp = reinterpret_cast<const T*>(p.q) + (size_t)b * p.q_stride_b + (size_t)(g * G + h) * p.q_stride_h;
+          next[h][0] = qp[2 * lane]; next[h][1] = qp[2 * lane + 64]; next[h][2] = qp[2 * lane + 1]; next[h][3] = qp[2 * lane + 65];
+        }
+      }
+    };
+    ask_queries(row0);
     for (int c = 0; c < n_stages; ++c) {
       const int slot = c % NQ;
       // the slot was read by product (2) of tile c-2, whose completion is s_ready of that tile
-      if (c >= NQ && !mbar_wait(smem_u32(&sm.s_ready[slot]), (uint32_t)(((c / NQ) - 1) & 1), abort_flag)) break;
+      if (c >= NQ && !mbar_wait(smem_u32(&sm.s_ready[(c - NQ) % NBUF_T]), (uint32_t)(((c - NQ) / NBUF_T) & 1), abort_flag)) break;
       const int u = u_begin + c;
-      while (u >= sm.prefix[row + 1]) ++row;
-      const bool row_start = (c == 0) || (u == sm.prefix[row]);
-      if (row_start) {
-        const int b = p.batch_index ? p.batch_index[row] : row;
-        const int s0 = (u - sm.prefix[row]) * ST_TOK;
-        float sa, ca, sb, cb;
-        sincosf((float)s0 * f0, &sa, &ca);
-        sincosf((float)s0 * f1, &sb, &cb);
+      if (c == 0 || u >= sm.prefix[row + 1]) {
+        row = next_row;
+        float sa = 0.f, ca = 1.f, sb = 0.f, cb = 1.f;
+        if (u != sm.prefix[row]) {        // (the CTA's first tile: the others begin at their row's first token)
+          const int s0 = (u - sm.prefix[row]) * ST_TOK;
+          sincos_call((float)s0 * f0, &sa, &ca);
+          sincos_call((float)s0 * f1, &sb, &cb);
+        }
 #pragma unroll
         for (int h = 0; h < HP; ++h) {
           float x0 = 0.f, x1 = 0.f, y0 = 0.f, y1 = 0.f;
           if (h < G) {
-            const T* qp = reinterpret_cast<const T*>(p.q) + (size_t)b * p.q_stride_b + (size_t)(g * G + h) * p.q_stride_h;
-            x0 = to_f32(qp[2 * lane]) * qscale; x1 = to_f32(qp[2 * lane + 64]) * qscale;
-            y0 = to_f32(qp[2 * lane + 1]) * qscale; y1 = to_f32(qp[2 * lane + 65]) * qscale;
+            x0 = to_f32(next[h][0]) * qscale; x1 = to_f32(next[h][1]) * qscale;
+            y0 = to_f32(next[h][2]) * qscale; y1 = to_f32(next[h][3]) * qscale;
           }
           a0[h] = x0 * ca + x1 * sa; b0[h] = x1 * ca - x0 * sa;
           a1[h] = y0 * cb + y1 * sb; b1[h] = y1 * cb - y0 * sb;
         }
+        ask_queries(row + 1);
       } else {
 #pragma unroll
         for (int h = 0; h < HP; ++h) {
@@ -531,165 +564,171 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     }
   }
 
-  else if (warp == W_KG0 || warp == W_KG0 + 4 || warp == W_VG0 || warp == W_VG0 + 4 || (warp >= W_G2 && warp < W_ROPE2)) {
+  else if (warp >= W_KG0 && warp < W_MMA) {
     // =========================== gather warps ===========================
-    // Four warps per side; lane l of gather warp j owns token 32j + l of every tile: it stages the token's length
-    // and offset (cp.async, PD tiles ahead, slots private to the lane) and copies the coefficient row into the
-    // operand tile, one 16-byte chunk per cp.async, chunk c of token t at c*2048 + t*16.  Chunks past the row's
-    // length are zero-filled (source size 0), but only those that the row before in this buffer had reached: what lies
-    // past both is zero already, and the tensor core always sees a full 128 x 128 tile.  (8 rows of 32768 tokens: 151.6 us
-    // with all 16 chunks written each time, 146.2 so; a loop up to the warp's longest row instead of predicates: 154.)
-    const bool is_v = warp >= W_G2 ? warp >= W_G2 + 2 : (warp & 3) == (W_VG0 & 3);
-    const int gw = warp >= W_G2 ? 2 + ((warp - W_G2) & 1) : (warp >> 2) & 1;
+    // Four warps per side, 32 tokens of every tile each.  Lane l reads the length and offset of token l (a tile ahead, into
+    // registers) and checks them; then four lanes copy a token's row together, 64 contiguous bytes of it per instruction for
+    // eight tokens, which come back to back: a few cache lines, where a lane per token touches one per token (lengths uniform
+    // in 8..128, 8 rows of 32768: 206 -> 164 us).  Chunk c of token t goes to c*CHUNK_PITCH + t*16.  Chunks past the row's
+    // length are zero-filled without a read, but only those that the row before in this buffer had reached: what lies past
+    // both is zero already.  Everything that does not need the buffer is done before the wait for it, and the copies are
+    // unrolled twice, for rows of up to 8 chunks and for all: the latency of this loop is what counts, not its bytes.
+    const bool is_v = warp >= W_VG0;
+    const int gw = warp & 3;
     const dkv_side& sd = is_v ? p.v : p.k;
-    const int side = is_v ? 1 : 0;
     const int NB = is_v ? NBUF_V : NBUF_A;
-    const int t = 32 * gw + lane;
+    const int t = 32 * gw + lane, sub = lane & 3, tl = lane >> 2;      // reads token t's metadata, copies pieces sub, sub + 4, .. of tokens tl + 8 r
+    const unsigned limit = (unsigned)min(sd.flat_stride, (int64_t)INT_MAX);
+    const uint32_t tile0 = smem_u32(is_v ? sm.v_tile[0] : sm.a_tile[0]) + (32 * gw + tl) * 16 + sub * CHUNK_PITCH;
+    const uint32_t full0 = smem_u32(is_v ? &sm.v_full[0] : &sm.a_full[0]), free0 = smem_u32(is_v ? &sm.pv_done[0] : &sm.t_ready[0]);
     uint32_t held = 0x10101010u;      // chunks that the buffers' rows hold, a byte per buffer (at first: anything)
-    RowInfo pre{row0, 0, 0, 0}, cur{row0, 0, 0, 0};
-    int pre_end = -1, cur_end = -1;
-    auto prefetch_meta = [&](int c) {   // no commit: the caller groups it with the tile's data copies
-      if (c < n_stages) {
-        const int u = u_begin + c;
-        if (u >= pre_end) { enter_row(pre, u); pre_end = sm.prefix[pre.row + 1]; }
-        const int s0 = (u - pre.first_unit) * ST_TOK;
-        int(*dst)[ST_TOK] = sm.meta[side][c % MSLOT];
-        if (s0 + t < pre.tokens) {
-          cp_async4(smem_u32(&dst[0][t]), sd.lens + (size_t)pre.arena * sd.lens_stride_a + s0 + t);
-          cp_async4(smem_u32(&dst[1][t]), sd.offs + (size_t)pre.arena * sd.offs_stride_a + s0 + t);
-        } else {
-          dst[0][t] = 0; dst[1][t] = 0;
-        }
-      }
-    };
-    for (int c = 0; c < PD; ++c) { prefetch_meta(c); cp_async_commit(); }   // groups 0..PD-1
-    for (int c = 0; c < n_stages; ++c) {
-      const int buf = c % NB;
-      cp_async_wait<PD - 1>();   // group c (this tile's metadata) is complete
+    int len = 0, off = 0;             // of this lane's token of the next tile, asked for a tile ahead
+    const unsigned char* arena_next = nullptr;
+    const int32_t *lens_at = nullptr, *offs_at = nullptr;
+    RowInfo row{row0, 0, 0, 0};
+    int row_end = -1, left = 0;
+    auto ask_meta = [&](int c) {
+      if (c >= n_stages) return;
       const int u = u_begin + c;
-      if (u >= cur_end) { enter_row(cur, u); cur_end = sm.prefix[cur.row + 1]; }
-      int(*mt)[ST_TOK] = sm.meta[side][c % MSLOT];
-      int len = mt[0][t];
-      const int off = mt[1][t];
-      if (((len | off) & 7) != 0 || len < 0 || len > R || off < 0 || (int64_t)off + len > sd.flat_stride) {
+      if (u >= row_end) {
+        enter_row(row, u);
+        row_end = sm.prefix[row.row + 1];
+        const int s = (u - row.first_unit) * ST_TOK + t;
+        left = row.tokens - s;
+        lens_at = sd.lens + (size_t)row.arena * sd.lens_stride_a + s;
+        offs_at = sd.offs + (size_t)row.arena * sd.offs_stride_a + s;
+        arena_next = reinterpret_cast<const unsigned char*>(reinterpret_cast<const T*>(sd.flat) + (size_t)row.arena * sd.flat_stride) + 16 * sub;
+      }
+      len = off = 0;
+      if (left > 0) { len = __ldg(lens_at); off = __ldg(offs_at); }
+      left -= ST_TOK; lens_at += ST_TOK; offs_at += ST_TOK;
+    };
+    ask_meta(0);
+    int buf = 0;
+    uint32_t par = 1;                 // of the buffer's last release (none in the first round)
+    for (int c = 0; c < n_stages; ++c) {
+      int nc = len >> 3, o = off;
+      if (((len | off) & 0x80000007) != 0 || len > R || (unsigned)len + (unsigned)off > limit) {
         set_status(p.status, DKV_ST_BAD_LENGTH);   // breaks the layout contract: token dropped, call flagged
-        len = 0;
+        nc = o = 0;
       }
-      const unsigned char* row_src = reinterpret_cast<const unsigned char*>(
-          reinterpret_cast<const T*>(sd.flat) + (size_t)cur.arena * sd.flat_stride + (len > 0 ? off : 0));
+      const int sh = 8 * buf;
+      const int n_write = max(nc, (int)((held >> sh) & 0xff));
+      held = (held & ~(0xffu << sh)) | ((uint32_t)nc << sh);
+      const int both = nc | n_write << 8;
+      int n[4], n_w[4];
+      const unsigned char* src[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int w = __shfl_sync(0xffffffffu, both, 8 * r + tl), from = __shfl_sync(0xffffffffu, o, 8 * r + tl);
+        n[r] = (w & 0xff) - sub;
+        n_w[r] = (w >> 8) - sub;
+        src[r] = arena_next + (size_t)(unsigned)from * sizeof(T);
+      }
+      const bool far = __any_sync(0xffffffffu, n_write > 8);
+      ask_meta(c + 1);
       // the tensor core must be done with the tile that was in this buffer NB tiles ago
-      // (K: product (1) of tile c-2 read this buffer; its completion is t_ready of that tile, ring of NBUF_T)
-      if (c >= NB) {
-        const uint32_t bar = is_v ? smem_u32(&sm.v_free[buf]) : smem_u32(&sm.t_ready[(c - NBUF_A) % NBUF_T]);
-        const uint32_t par = is_v ? (uint32_t)(((c / NBUF_V) - 1) & 1) : (uint32_t)(((c - NBUF_A) / NBUF_T) & 1);
-        if (!mbar_wait(bar, par, abort_flag)) break;
-      }
+      // (K: product (1) of tile c-3 read this buffer; its completion is t_ready of that tile, same ring)
+      if (c >= NB && !mbar_wait(free0 + 8 * buf, par, abort_flag)) break;
       if (!is_v) {
         // written after the wait: product (1) of tile c-3 is complete, so product (2) of tile c-6 has been issued,
         // which needed the P tile of tile c-8 written -- the softmax warps are past the mask of tile c-8 (same slot)
-        const uint32_t m = __ballot_sync(0xffffffffu, len > 0);
-        if (lane == 0) sm.kvalid[c % KV_RING][gw] = m;
+        const uint32_t m = __ballot_sync(0xffffffffu, nc > 0);
+        const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)nc);
+        if (lane == 0) {
+          sm.kvalid[c % KV_RING][gw] = m;
+          sm.kmax[buf][gw] = longest;
+          mbar_arrive(full0 + 8 * buf);
+        }
       }
-      const uint32_t dst = smem_u32(is_v ? sm.v_tile[buf] : sm.a_tile[buf]) + t * 16;
-      const int nc = len >> 3, had = (held >> (8 * buf)) & 0xff;
-      held = (held & ~(0xffu << (8 * buf))) | ((uint32_t)nc << (8 * buf));
-      const int n_write = max(nc, had);
+      const uint32_t dst = tile0 + buf * TILE_BYTES;
+      // past the row's length nothing is read: zeros are written
+      auto copy_rows = [&](auto pieces) {
 #pragma unroll
-      for (int ch = 0; ch < 16; ++ch) {
-        // past the row's length the source size is 0: nothing is read from the (then meaningless) address
-        if (ch < n_write) cp_async16_zfill(dst + ch * 2048, row_src + ch * 16, ch < nc ? 16 : 0);
-      }
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int i = 0; i < decltype(pieces)::value; ++i)
+            if (4 * i < n_w[r]) cp_async16_or_zero(dst + 128 * r + 4 * i * CHUNK_PITCH, src[r] + 64 * i, 4 * i >= n[r]);
+      };
+      if (far) copy_rows(std::integral_constant<int, 4>()); else copy_rows(std::integral_constant<int, 2>());
       // The tile is handed over by the copy engine itself: each lane's arrival on the tile's barrier fires when
       // its copies have landed, so the warp neither waits for the data nor delays the hand-over until it comes
       // round again (which would put the next tile's wait for a free buffer into the serial loop
       // buffer free -> copies -> product (1) -> buffer free).  The consumer issues the proxy fence.
-      cp_async_arrive_when_landed(smem_u32(is_v ? &sm.v_full[buf] : &sm.a_full[buf]));
-      prefetch_meta(c + PD);
-      cp_async_commit();                       // group PD + c
+      cp_async_arrive_when_landed(full0 + 8 * buf);
+      if (++buf == NB) { buf = 0; par ^= 1u; }
     }
-    cp_async_wait<0>();
+    cp_async_wait_all();
   }
 
   else if (warp == W_MMA) {
-    // =========================== tensor-core issuer A: products (1) and (2) ===========================
-    // One lane issues both products.  It never blocks on one barrier: it probes whether the next product (1) or
-    // (2) has its operands in place and issues what is ready, so that one group's RoPE pass does not hold back
-    // the other group's products.  The tensor core executes one thread's instructions in issue order, which also
-    // orders the re-use of the accumulator buffers: product (1) of tile i+3 is only issued after product (2) of
-    // tile i, which reads K' from the same buffer.  This thread is the serial part of the pipeline, so its code
-    // is kept short: fully unrolled issue loops over constant descriptors, probes issued back to back.
-    if (lane == 0) {
+    // =========================== tensor-core issuer A: product (1) ===========================
+    // K-steps past the tile's longest row are left out: they would add zeros (lengths beta(2,8): 5.3 of 8 are issued).
+    {
       const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;   // 0 = f16, 1 = bf16
       const uint32_t idesc_k = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-      const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
       // descriptor words: low = (address >> 4) | (LBO >> 4) << 16, high = (SBO >> 4) | version bit
-      const uint32_t a_lo0 = desc_lo(smem_u32(sm.a_tile[0]), 2048), b_lo0 = desc_lo(smem_u32(sm.basis), 2048);
-      const uint32_t q_lo0 = desc_lo(smem_u32(sm.qrot[0]), Q_LBO), hi_128 = desc_hi(128);
-      static_assert(TILE_BYTES % 16 == 0 && Q_TILE_BYTES % 16 == 0 && (2 * Q_LBO) % 16 == 0, "descriptor steps are whole 16-byte units");
-      int ri = 0, qi = 0;     // next tile of products (1), (2)
-      int rt = 0, qt = 0;     // their accumulator buffers ri % 3, qi % 3 ...
-      uint32_t rtp = 0, qtp = 0;   // ... and phases (ri / 3) & 1, (qi / 3) & 1
-      uint32_t idle = 0;
-      while (qi < n_stages) {
-        static_assert(NBUF_A == NBUF_T, "the K operand tiles and the K accumulators share ring index and phase");
-        const int rb = rt, qg = qi & 1;
-        const bool r_ok = mbar_probe(smem_u32(&sm.a_full[rb]), rtp);
-        const bool k_ok = mbar_probe(smem_u32(&sm.kp_ready[qt]), qtp);
-        const bool q_ok = mbar_probe(smem_u32(&sm.q_full[qg]), (uint32_t)((qi >> 1) & 1)) &&
-                          (qi < 2 || mbar_probe(smem_u32(&sm.p_ready[qg]), (uint32_t)(((qi >> 1) - 1) & 1)));   // score tile read out
-        bool progress = false;
-        if (ri < n_stages && ri - qi < NBUF_T && r_ok) {
-          proxy_fence_async();   // the tile was written by cp.async (generic proxy), the tensor core reads it through the async proxy
-          tc_fence_after();
-          const uint32_t a_lo = a_lo0 + (uint32_t)rb * (TILE_BYTES >> 4), d_k = tmem_base + TM_K + rt * 128;
+      const uint32_t a_lo0 = desc_lo(smem_u32(sm.a_tile[0]), CHUNK_PITCH), b_lo0 = desc_lo(smem_u32(sm.basis), 2048);
+      const uint32_t hi_128 = desc_hi(128);
+      const bool have_basis = mbar_wait_all(smem_u32(&sm.basis_full), 0u, abort_flag);
+      for (int c = 0; have_basis && c < n_stages; ++c) {
+        const int buf = c % NBUF_T;
+        const uint32_t par = (uint32_t)((c / NBUF_T) & 1);
+        if (c >= NBUF_T && !mbar_wait_all(smem_u32(&sm.s_ready[buf]), par ^ 1u, abort_flag)) break;   // product (2) of tile c-3 has read the accumulator
+        if (!mbar_wait_all(smem_u32(&sm.a_full[buf]), par, abort_flag)) break;
+        proxy_fence_async();   // the tile was written by cp.async (generic proxy), the tensor core reads it through the async proxy
+        tc_fence_after();
+        const int4 km = *reinterpret_cast<const int4*>(sm.kmax[buf]);
+        const int n_ks = __shfl_sync(0xffffffffu, (max(max(km.x, km.y), max(km.z, km.w)) + 1) >> 1, 0);     // k-steps that hold coefficients (the first is always taken: it clears the accumulator)
+        const uint32_t a_lo = a_lo0 + (uint32_t)buf * (TILE_BYTES >> 4), d_k = tmem_base + TM_K + buf * 128;
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            // A: K-major, 8-row core matrices 128 B apart (SBO), the two 8-coefficient chunks 2048 B apart (LBO)
-            // B: MN-major, 8-column core matrices 128 B apart (SBO), the two 8-row groups 2048 B apart (LBO)
-            // a k-step is 4096 B further in both tiles
-            umma_f16_w(d_k, a_lo + ks * 256, hi_128, b_lo0 + ks * 256, hi_128, idesc_k, ks > 0 ? 1u : 0u);
-          }
-          umma_commit(smem_u32(&sm.t_ready[rt]));   // also frees the operand tile (the K gather warps wait on it too)
-          ++ri;
-          if (++rt == NBUF_T) { rt = 0; rtp ^= 1u; }
-          progress = true;
+        for (int ks = 0; ks < 8; ++ks) {
+          // A: K-major, 8-row core matrices 128 B apart (SBO), the two 8-coefficient chunks CHUNK_PITCH apart (LBO)
+          // B: MN-major, 8-column core matrices 128 B apart (SBO), the two 8-row groups 2048 B apart (LBO)
+          // a k-step is two chunks further in both tiles
+          if (ks == 0 || ks < n_ks) umma_f16_w(d_k, a_lo + ks * (2 * CHUNK_PITCH >> 4), hi_128, b_lo0 + ks * 256, hi_128, idesc_k, ks > 0 ? 1u : 0u);
         }
-        if (qi < ri && k_ok && q_ok && !(progress && qi + 1 == ri)) {
-          tc_fence_after();
-          const uint32_t q_lo = q_lo0 + (uint32_t)qg * (Q_TILE_BYTES >> 4), d_s = tmem_base + TM_S + 16 * qg;
-          const uint32_t kp = tmem_base + TM_K + qt * 128;
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            // A: K' of the tile, dims 16ks..16ks+15 = 8 packed columns; each 32-dim quarter of the row starts its
-            // 16 packed columns at the quarter's own first column (0, 32, 64, 96)
-            // B: K-major, head rows 16 B apart inside a core matrix, 8-row groups 128 B (SBO), dim chunks Q_LBO apart
-            umma_f16_ta_w(d_s, kp + 32 * (ks >> 1) + 8 * (ks & 1), q_lo + ks * ((2 * Q_LBO) >> 4), hi_128, idesc_s,
-                          ks > 0 ? 1u : 0u);
-          }
-          umma_commit(smem_u32(&sm.s_ready[qg]));   // also frees the rotated queries (the rotator waits on it too)
-          ++qi;
-          if (++qt == NBUF_T) { qt = 0; qtp ^= 1u; }
-          progress = true;
-        }
-        if (progress) {
-          idle = 0;
-        } else {
-          ++idle;
-          if ((idle & 1023u) == 0u && *abort_flag) break;
-          if (idle >= SPIN_LIMIT) { *abort_flag = 1; break; }
-        }
+        umma_commit(smem_u32(&sm.t_ready[buf]));   // also frees the operand tile (the K gather warps wait on it too)
       }
     }
   }
 
   else if (warp == W_MMA2) {
-    // =========================== tensor-core issuer B: product (3) ===========================
-    // A thread of its own (on another SM sub-partition), so that product (3) costs issuer A no time.
-    if (lane == 0) {
+    // =========================== tensor-core issuer B: product (2) ===========================
+    // A warp of its own, so that its waits and commits cost product (1) no time.
+    {
+      const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+      const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
+      const uint32_t q_lo0 = desc_lo(smem_u32(sm.qrot[0]), Q_LBO), hi_128 = desc_hi(128);
+      static_assert(TILE_BYTES % 16 == 0 && Q_TILE_BYTES % 16 == 0 && (2 * Q_LBO) % 16 == 0, "descriptor steps are whole 16-byte units");
+      for (int c = 0; c < n_stages; ++c) {
+        const int buf = c % NBUF_T, qg = c & 1;
+        if (!mbar_wait_all(smem_u32(&sm.q_full[qg]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
+        if (c >= 2 && !mbar_wait_all(smem_u32(&sm.p_ready[qg]), (uint32_t)(((c >> 1) - 1) & 1), abort_flag)) break;   // score tile read out
+        if (!mbar_wait_all(smem_u32(&sm.kp_ready[buf]), (uint32_t)((c / NBUF_T) & 1), abort_flag)) break;
+        tc_fence_after();
+        const uint32_t q_lo = q_lo0 + (uint32_t)qg * (Q_TILE_BYTES >> 4), d_s = tmem_base + TM_S + 16 * qg;
+        const uint32_t kp = tmem_base + TM_K + buf * 128;
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          // A: K' of the tile, dims 16ks..16ks+15 = 8 packed columns; each 32-dim quarter of the row starts its
+          // 16 packed columns at the quarter's own first column (0, 32, 64, 96)
+          // B: K-major, head rows 16 B apart inside a core matrix, 8-row groups 128 B (SBO), dim chunks Q_LBO apart
+          umma_f16_ta_w(d_s, kp + 32 * (ks >> 1) + 8 * (ks & 1), q_lo + ks * ((2 * Q_LBO) >> 4), hi_128, idesc_s,
+                        ks > 0 ? 1u : 0u);
+        }
+        umma_commit(smem_u32(&sm.s_ready[buf]));   // also frees the rotated queries and the K accumulator
+      }
+    }
+  }
+
+  else if (warp == W_MMA3) {
+    // =========================== tensor-core issuer C: product (3) ===========================
+    {
       const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
       const uint32_t idesc_o = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
       const uint32_t v_lo0 = desc_lo(smem_u32(sm.v_tile[0]), 128), p_lo0 = desc_lo(smem_u32(sm.p_tile[0]), 128);
-      const uint32_t hi_2048 = desc_hi(2048), hi_0 = desc_hi(0), d_o = tmem_base + TM_O;
+      const uint32_t hi_pitch = desc_hi(CHUNK_PITCH), hi_0 = desc_hi(0), d_o = tmem_base + TM_O;
       int row_pv = row0;
       int c_row_lo = 0, c_row_hi = 0;   // tiles of the current batch row in this CTA: [c_row_lo, c_row_hi)
       for (int c = 0; c < n_stages; ++c) {
@@ -700,9 +739,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
           c_row_lo = max(sm.prefix[row_pv], u_begin) - u_begin;
           c_row_hi = sm.prefix[row_pv + 1] - u_begin;
         }
-        const bool first = c == c_row_lo;   // the first tile of a row starts a new sum
-        if (!mbar_wait_thread(smem_u32(&sm.v_full[vb]), (uint32_t)((c / NBUF_V) & 1), abort_flag)) break;
-        if (!mbar_wait_thread(smem_u32(&sm.p_ready[grp]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
+        const bool first = c - c_row_lo < NGROUP;   // the first even and the first odd tile of a row start new sums
+        if (!mbar_wait_all(smem_u32(&sm.v_full[vb]), (uint32_t)((c / NBUF_V) & 1), abort_flag)) break;
+        if (!mbar_wait_all(smem_u32(&sm.p_ready[grp]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
         proxy_fence_async();   // V tile written by cp.async
         tc_fence_after();
         const uint32_t v_lo = v_lo0 + (uint32_t)vb * (TILE_BYTES >> 4), p_lo = p_lo0 + (uint32_t)grp * ((ST_TOK * 16) >> 4);
@@ -710,25 +749,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           // A = XV^T: MN-major, 16 tokens per step (256 B), token groups of 8 are 128 B apart (LBO), latent
-          //     chunks 2048 B apart (SBO)
+          //     chunks CHUNK_PITCH apart (SBO)
           // B = P:    MN-major, token groups of 8 are 128 B apart (LBO); the second group of 8 columns aliases
           //     the first (SBO 0): columns 8..15 of the result duplicate 0..7 and are never read
-          umma_f16_w(d_o, v_lo + ks * 16, hi_2048, p_lo + ks * 16, hi_0, idesc_o, ks > 0 ? 1u : acc0);
+          umma_f16_w(d_o + 16 * grp, v_lo + ks * 16, hi_pitch, p_lo + ks * 16, hi_0, idesc_o, ks > 0 ? 1u : acc0);
         }
         umma_commit(smem_u32(&sm.pv_done[grp]));
-        umma_commit(smem_u32(&sm.v_free[vb]));
       }
     }
   }
 
-  else if (warp < 4 || warp >= W_ROPE2) {
+  else if (warp < 4 || (warp >= W_ROPE2 && warp < W_SM2)) {
     // ============================= RoPE warps =============================
     // Two threads per token: threads (w, lane) and (W_ROPE2 + w, lane) own token 32 w + lane of every tile, which is
     // tensor-memory lane 32 w + lane -- the lanes a warp in SM sub-partition w may access.  The first takes the
     // rotation pairs j = 0..31 (dims j and 64 + j), the second j = 32..63.  They turn the K row of product (1) into
     // K' for product (2) in place: each 32-dim quarter of the row is packed into the first 16 columns of the
     // quarter, columns its own thread has read before, so the two threads never touch each other's columns.
-    // They know nothing about batch rows.
+    // They know nothing about batch rows.  (Whole rows of alternate tiles per thread instead: the same time.)
     const int w4 = warp & 3, half = warp >= W_ROPE2 ? 1 : 0;
     const int tok = 32 * w4 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * w4) << 16);
@@ -742,9 +780,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       float ss = 0.f;
 #pragma unroll 1   // kept rolled: the warp roles of an SM sub-partition share a small instruction cache
       for (int ii = 0; ii < 4; ++ii) {
+        const int i = 4 * half + ii;
         // pairs j = 8i..8i+7: dims j (columns 8i..) and j+64 (columns 64+8i..); table cells 8i..: per two pairs
         // one word {cos_j, cos_j+1} and one word {sin_j, sin_j+1} in fp16
-        const int i = 4 * half + ii;
         float lo[8], hi[8];
         uint32_t tg[8];
         tmem_ld_rope_chunk(lo, hi, tg, k_addr + 8 * i, k_addr + 64 + 8 * i, lane_addr + TM_TRIG + 8 * i);
@@ -789,32 +827,34 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     }
   }
 
-  else if (warp < NCW) {
+  else if (warp < NCW || warp >= W_SM2) {
   // ============================= softmax warps =============================
   // Thread (wq, lane) owns token 32 wq + lane of every tile: it reads the token's scores from product (2),
   // forms the softmax weights against the reference maximum m_ref shared by the four warps, and stores P for
   // product (3).  These warps follow the batch rows and write each row's result.
-  const int wq = warp & 3;
+  const int wq = warp & 3, grp = warp >= W_SM2 ? 1 : 0;
   const int tok = 32 * wq + lane;
   const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * wq) << 16);
-  const uint32_t o_addr = lane_addr + TM_O;
+  const uint32_t o_addr = lane_addr + TM_O + 16 * grp;
 
   int row = row0;
+  int n_shared = 0;      // rows so far that both groups had tiles of
   while (row < p.batch && sm.prefix[row] < u_end) {
     const int c_lo = max(sm.prefix[row], u_begin) - u_begin;     // tiles of this row in this CTA: [c_lo, c_hi)
     const int c_hi = min(sm.prefix[row + 1], u_end) - u_begin;
+    const bool alone = c_hi - c_lo == 1;                         // one tile: its warps have the whole sum
+    if (alone && ((c_lo ^ grp) & 1)) { ++row; continue; }
     float m_ref[HP], l_part[HP];
 #pragma unroll
     for (int h = 0; h < HP; ++h) { m_ref[h] = -INFINITY; l_part[h] = 0.f; }
     int c_last = -1;            // last tile of the row that was processed
     bool dead = false;
 
-    for (int c = c_lo; c < c_hi; ++c) {
-      const int buf = c & 1;
-      const uint32_t par = (uint32_t)((c >> 1) & 1);
-      const bool first = c == c_lo;     // O holds nothing of this row yet
+    for (int c = c_lo + ((c_lo ^ grp) & 1); c < c_hi; c += NGROUP) {
+      const int buf = grp;
+      const bool first = c_last < 0;    // this group's O holds nothing of this row yet
       // ---------------- scores of this token for the group's heads ----------------
-      if (!dead) dead = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&sm.s_ready[buf]), par, abort_flag));
+      if (!dead) dead = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&sm.s_ready[c % NBUF_T]), (uint32_t)((c / NBUF_T) & 1), abort_flag));
       tc_fence_after();
       float s[HP];
       tmem_ld4(s, lane_addr + TM_S + 16 * buf);
@@ -835,20 +875,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
         over |= s[h] > m_ref[h] + M_SLACK;
         pr[h] = exp2f(s[h] - (m_ref[h] == -INFINITY ? 0.f : m_ref[h]));
       }
-      const bool grow = consumer_any(over);
+      const bool grow = consumer_any(grp, over);
       // the P tile of this parity was read by product (3) of tile c-2
       if (!dead && c >= 2) dead = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&sm.pv_done[buf]), (uint32_t)(((c >> 1) - 1) & 1), abort_flag));
       if (grow) {
 #pragma unroll
         for (int h = 0; h < HP; ++h) {
           const float mx = warp_max_redux(s[h]);
-          if (lane == 0) sm.tmax[wq][h] = mx;
+          if (lane == 0) sm.tmax[grp][wq][h] = mx;
         }
-        consumer_bar();
+        consumer_bar(grp);
         float factor[HP];
 #pragma unroll
         for (int h = 0; h < HP; ++h) {
-          const float tm = fmaxf(fmaxf(sm.tmax[0][h], sm.tmax[1][h]), fmaxf(sm.tmax[2][h], sm.tmax[3][h]));   // (written again behind the next tile's barrier)
+          const float tm = fmaxf(fmaxf(sm.tmax[grp][0][h], sm.tmax[grp][1][h]), fmaxf(sm.tmax[grp][2][h], sm.tmax[grp][3][h]));   // (written again behind the next tile's barrier)
           const float m_new = fmaxf(m_ref[h], tm);
           factor[h] = m_new == -INFINITY ? 1.f : exp2f(m_ref[h] - m_new);   // 0 when there was no reference yet
           m_ref[h] = m_new;
@@ -856,8 +896,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
           pr[h] = exp2f(s[h] - (m_new == -INFINITY ? 0.f : m_new));
         }
         if (!first) {
-          // O is rescaled in tensor memory: product (3) of tile c-1 must be complete as well
-          if (!dead) dead = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&sm.pv_done[buf ^ 1]), (uint32_t)(((c - 1) >> 1) & 1), abort_flag));
+          // O is rescaled in tensor memory: product (3) of tile c-2, the last one into it, is complete
           tc_fence_after();
           float o[4];
           tmem_ld4(o, o_addr);
@@ -876,39 +915,76 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       c_last = c;
     }
 
-    // ---------------- row flush ----------------
+    // ---------------- row end: the group that had the row's last tile takes over the other's sums ----------------
+    // (the other one goes on with the next row as soon as it has handed them over)
     float o[4] = {0.f, 0.f, 0.f, 0.f};
-    if (c_last >= 0 && !dead && mbar_wait(smem_u32(&sm.pv_done[c_last & 1]), (uint32_t)((c_last >> 1) & 1), abort_flag)) {
+    if (c_last >= 0 && !dead && mbar_wait(smem_u32(&sm.pv_done[grp]), (uint32_t)((c_last >> 1) & 1), abort_flag)) {
       tc_fence_after();
       tmem_ld4(o, o_addr);   // O^T[r = tok][head]
     }
-#pragma unroll
-    for (int h = 0; h < HP; ++h) {
-      const float l = warp_sum(l_part[h]);
-      if (lane == 0) sm.lsum[wq][h] = l;
-    }
-    consumer_bar();
-    float L[HP];
-#pragma unroll
-    for (int h = 0; h < HP; ++h) L[h] = (sm.lsum[0][h] + sm.lsum[1][h]) + (sm.lsum[2][h] + sm.lsum[3][h]);
-    if (!FUSED) {
-      // partial record (row, cta) -> entry row + blockIdx.x of this KV head
-      float* ws = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.workspace) + ws_header_bytes());
-      const size_t entries_per_group = (size_t)p.batch + n_cta;
-      float* rec = ws + (((size_t)g * entries_per_group + (size_t)row + blockIdx.x) * HP) * PART_STRIDE;
-#pragma unroll
-      for (int h = 0; h < HP; ++h) {
-        rec[h * PART_STRIDE + 2 + tok] = o[h];
-        if (tok == 0) { rec[h * PART_STRIDE] = m_ref[h]; rec[h * PART_STRIDE + 1] = L[h]; }
-      }
-      consumer_bar();   // lsum may be rewritten by the next row
+    const int slot = n_shared & 1;
+    const uint32_t slot_par = (uint32_t)((n_shared >> 1) & 1);
+    const bool gives = !alone && ((c_hi - 1) & 1) != grp;
+    if (!alone) ++n_shared;
+    const float l_sum = warp_sum4(l_part, lane);      // of head lane / 8
+    if (gives) {
+      if (n_shared > 2) mbar_wait(smem_u32(&sm.dep_free[slot]), slot_par ^ 1u, abort_flag);
+      sm.dep_o[slot][tok] = make_float4(o[0], o[1], o[2], o[3]);
+      if ((lane & 7) == 0) sm.dep_l[slot][lane >> 3][wq] = l_sum;
+      if (tok == 0) sm.dep_m[slot] = make_float4(m_ref[0], m_ref[1], m_ref[2], m_ref[3]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm.dep_full[slot]));
     } else {
+      // partial record (row, cta) -> entry row + blockIdx.x of this KV head
+      float* rec = nullptr;
+      if (!FUSED) {
+        float* ws = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.workspace) + ws_header_bytes());
+        const size_t entries_per_group = (size_t)p.batch + n_cta;
+        rec = ws + (((size_t)g * entries_per_group + (size_t)row + blockIdx.x) * HP) * PART_STRIDE;
+      }
+      // One thread per head has the maxima, sums and factors; code that runs once a row is kept short, for its first run
+      // waits for its instructions (with these in every thread, unrolled over the heads, 3800 cycles).  What is written here is
+      // written again only behind the barrier of a further tile, where all four warps have read it.
+      if ((lane & 7) == 0) sm.lsum[grp][lane >> 3][wq] = l_sum;
+      if (!alone) mbar_wait(smem_u32(&sm.dep_full[slot]), slot_par, abort_flag);
+      consumer_bar(grp);
+      if (tok < HP) {
+        const float4 w = *reinterpret_cast<const float4*>(sm.lsum[grp][tok]);
+        float m = tok == 0 ? m_ref[0] : tok == 1 ? m_ref[1] : tok == 2 ? m_ref[2] : m_ref[3];
+        float l = (w.x + w.y) + (w.z + w.w);
+        if (!alone) {
+          const float4 w1 = *reinterpret_cast<const float4*>(sm.dep_l[slot][tok]);
+          const float m0 = m, m1 = reinterpret_cast<const float*>(&sm.dep_m[slot])[tok];
+          m = fmaxf(m0, m1);
+          const float f0 = m0 == -INFINITY ? 0.f : exp2f(m0 - m), f1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m);
+          l = f0 * l + f1 * ((w1.x + w1.y) + (w1.z + w1.w));
+          sm.factor[grp][0][tok] = f0;
+          sm.factor[grp][1][tok] = f1;
+        }
+        if (FUSED) {
+          sm.fused_l[tok] = l;
+          if (l <= 0.f && tok < G) set_status(p.status, DKV_ST_EMPTY_ROW);
+        } else {
+          rec[tok * PART_STRIDE] = m;
+          rec[tok * PART_STRIDE + 1] = l;
+        }
+      }
+      if (FUSED || !alone) consumer_bar(grp);
+      if (!alone) {
+        const float4 f0 = *reinterpret_cast<const float4*>(sm.factor[grp][0]), f1 = *reinterpret_cast<const float4*>(sm.factor[grp][1]);
+        const float4 d = sm.dep_o[slot][tok];
+        o[0] = f0.x * o[0] + f1.x * d.x; o[1] = f0.y * o[1] + f1.y * d.y;
+        o[2] = f0.z * o[2] + f1.z * d.z; o[3] = f0.w * o[3] + f1.w * d.w;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm.dep_free[slot]));
+      }
 #pragma unroll
       for (int h = 0; h < HP; ++h) {
-        sm.lat[h][tok] = L[h] > 0.f ? o[h] / L[h] : 0.f;
-        if (L[h] <= 0.f && tok == 0 && h < G) set_status(p.status, DKV_ST_EMPTY_ROW);
+        if (FUSED) o[h] = sm.fused_l[h] > 0.f ? o[h] / sm.fused_l[h] : 0.f;
+        else rec[h * PART_STRIDE + 2 + tok] = o[h];
       }
-      // the up-projection is done by the whole block after the pipeline has drained (a fused CTA has one row)
+      // (the up-projection is done by the whole block after the pipeline has drained: a fused CTA has one row)
+      if (FUSED) sm.dep_o[1][tok] = make_float4(o[0], o[1], o[2], o[3]);
     }
     ++row;
   }
@@ -923,13 +999,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     if (h < HP && h < G) {
       const int b = p.batch_index ? p.batch_index[blockIdx.x] : blockIdx.x;
       const T* vup = reinterpret_cast<const T*>(p.v_up) + (size_t)g * R * D + d;
+      const float* lat = reinterpret_cast<const float*>(sm.dep_o[1]);
       float acc0 = 0.f, acc1 = 0.f;
       int r = 0;
       for (; r + 1 < R; r += 2) {
-        acc0 = fmaf(sm.lat[h][r], to_f32(vup[(size_t)r * D]), acc0);
-        acc1 = fmaf(sm.lat[h][r + 1], to_f32(vup[(size_t)(r + 1) * D]), acc1);
+        acc0 = fmaf(lat[4 * r + h], to_f32(vup[(size_t)r * D]), acc0);
+        acc1 = fmaf(lat[4 * (r + 1) + h], to_f32(vup[(size_t)(r + 1) * D]), acc1);
       }
-      if (r < R) acc0 = fmaf(sm.lat[h][r], to_f32(vup[(size_t)r * D]), acc0);
+      if (r < R) acc0 = fmaf(lat[4 * r + h], to_f32(vup[(size_t)r * D]), acc0);
       T* op = reinterpret_cast<T*>(p.out) + (size_t)b * p.out_stride_b + (size_t)(g * G + h) * p.out_stride_h;
       op[d] = from_f32<T>(acc0 + acc1);
     }

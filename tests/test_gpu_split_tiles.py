@@ -1,0 +1,69 @@
+"""Packed decode pipeline: even and odd tiles of a row on warp groups of their own, k-steps and copies cut at the tile's longest
+row.  Rows of one to five tiles per CTA in every phase of the rings, tiles of short rows only, tiles whose K or V rows are all
+empty, single long rows among short ones, scores that raise the reference maximum in one group only."""
+import ctypes
+
+import pytest
+import torch
+
+from dynakv_b200 import _lib, synthetic
+from dynakv_b200.kernels import _common
+from oracle import dynakv_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _decode(c, lens_k, lens_v, n_sm, theta=5e5, knorm=None):
+    """dkv_two_stage_decode on `n_sm` SMs: the fewer, the more tiles a CTA walks."""
+    gen = torch.Generator().manual_seed(3)
+    k, v = (synthetic.ragged_side(x, gen, c.q.dtype) for x in (lens_k, lens_v))
+    args = [c.q, k.flat, c.k_up, v.flat, c.v_up, k.lens, k.offs, v.lens, v.offs]
+    ref = O.compact_attention(*args[:5], *args[5:], theta, seq_lens=c.seq_lens, k_norm_weight=knorm)
+    d = [t.cuda() for t in args]
+    out = torch.zeros(c.q.shape, dtype=c.q.dtype, device="cuda")
+    a, keep = _common.build_attn_args(d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7], d[8], theta, out=out, len_multiple=8, need_workspace=True,
+                                      seq_lens=torch.tensor(c.seq_lens, dtype=torch.int32, device="cuda"),
+                                      k_norm_weight=None if knorm is None else knorm.cuda())
+    a.n_sm = n_sm
+    need = int(_lib.load().dkv_split_workspace_bytes(ctypes.byref(a)))
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    _lib.check(_lib.load().dkv_two_stage_decode(ctypes.byref(a)), "dkv_two_stage_decode")
+    torch.cuda.synchronize()
+    del keep
+    ref = torch.nan_to_num(ref)
+    assert float((out.float().cpu() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
+    assert _common.read_status(torch.device("cuda")) == 0
+
+
+def _lengths(kind, rows, S, gen):
+    lens = torch.randint(1, 17, (rows, S), generator=gen, dtype=torch.int32) * 8
+    if kind == "short":
+        lens = lens.clamp(max=16)
+    elif kind == "one long":
+        lens = lens.clamp(max=24)
+        lens[:, S // 2] = 128
+    elif kind == "empty tiles":
+        lens[:, 128:256] = 0
+        lens[:, 300:] = 0
+    return lens
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("kind", ["any", "short", "one long", "empty tiles"])
+@pytest.mark.parametrize("seq,n_sm", [([640], 2), ([1, 128, 129, 257, 513], 2), ([385, 1, 640, 256, 3], 6)], ids=str)
+def test_tiles_of_both_groups(seq, n_sm, kind, dtype):
+    gen = torch.Generator().manual_seed(len(seq) + n_sm)
+    c = synthetic.make_layer_case(7, seq, "uniform", 5e5, dtype, "cpu", n_q_heads=8, n_kv_heads=2)
+    lens_k, lens_v = (_lengths(kind, 2 * len(seq), max(seq), gen) for _ in range(2))
+    _decode(c, lens_k, lens_v, n_sm, knorm=1.0 + 0.1 * torch.randn(128, generator=gen) if kind == "any" else None)
+
+
+@pytest.mark.parametrize("tile", [0, 1, 3, 4])
+def test_reference_maximum_raised_in_one_group(tile):
+    gen = torch.Generator().manual_seed(11)
+    c = synthetic.make_layer_case(9, [640], "uniform", 5e5, torch.bfloat16, "cpu", n_q_heads=8, n_kv_heads=2)
+    c.q[:, :] *= 4
+    lens = torch.full((2, 640), 8, dtype=torch.int32)
+    lens[:, 128 * tile:128 * tile + 128] = 128
+    _decode(c, lens, lens.flip(1).contiguous(), 2)
