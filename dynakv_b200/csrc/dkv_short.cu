@@ -51,6 +51,7 @@ static_assert(2 * (sizeof(ShortSmem) + 128 + 1024) <= 228 * 1024, "two CTAs per 
 
 __device__ __forceinline__ uint32_t ss_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool ss_wait(unsigned long long* bar, uint32_t parity) {
+#pragma unroll 1
   for (uint32_t it = 0; it < SSPIN; ++it) {
     uint32_t r;
     asm volatile("{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\nselp.u32 %0, 1, 0, q;\n}"
@@ -62,12 +63,14 @@ __device__ __forceinline__ bool ss_wait(unsigned long long* bar, uint32_t parity
 __device__ __forceinline__ uint64_t ss_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
+// Called by a converged warp with operands that are the same in all lanes; an elected lane issues (in a branch of a single lane
+// the operands are built lane by lane, at twice the instructions: a decode step of 4 short rows through 32 layers 793 -> 733 us).
 __device__ __forceinline__ void ss_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
-  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n}"
+  asm volatile("{\n.reg .pred q, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 q, %4, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n}"
                ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u) : "memory");
 }
 __device__ __forceinline__ void ss_commit(unsigned long long* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(ss_addr(bar)) : "memory");
+  asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(ss_addr(bar)) : "memory");
 }
 // columns c .. c+7 and c+64 .. c+71 of this thread's lane
 __device__ __forceinline__ void ss_ld_pairs(float (&lo)[8], float (&hi)[8], uint32_t addr) {
@@ -116,7 +119,7 @@ template <typename T, bool KNORM>
 __global__ void __launch_bounds__(STHREADS, 2) short_decode_kernel(dkv_attn_args p, float log_theta) {
   extern __shared__ unsigned char ss_raw[];
   ShortSmem& sm = *reinterpret_cast<ShortSmem*>(ss_raw + ((128u - (ss_addr(ss_raw) & 127u)) & 127u));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;     // (the warp: known to be the same in all lanes)
   const int tok = tid & 127, quarter = tid >> 7;
   const int CS = (int)(gridDim.x / p.batch), rank = (int)cluster_rank();
   const int i_row = blockIdx.x / CS, g = blockIdx.y;
@@ -219,8 +222,8 @@ __global__ void __launch_bounds__(STHREADS, 2) short_decode_kernel(dkv_attn_args
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = sm.tmem;
-    if (tid == 0) {
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem, 0);
+    if (warp == 0) {
       // K = X Bk
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks)
@@ -298,7 +301,7 @@ __global__ void __launch_bounds__(STHREADS, 2) short_decode_kernel(dkv_attn_args
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // O^T = XV^T P: columns 0..3 values, 4..7 remainders, 8..15 alias them
 #pragma unroll
@@ -396,11 +399,11 @@ __global__ void __launch_bounds__(STHREADS, 2) short_decode_kernel(dkv_attn_args
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
-      if (tid == 0) {
+      if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          ss_mma(sm.tmem + S_TM_O, ss_desc(ss_addr(sm.x) + ks * 256, 128, 2048), ss_desc(ss_addr(sm.p) + ks * 256, 128, 0), idesc_o, ks > 0);
+          ss_mma(__shfl_sync(0xffffffffu, sm.tmem, 0) + S_TM_O, ss_desc(ss_addr(sm.x) + ks * 256, 128, 2048), ss_desc(ss_addr(sm.p) + ks * 256, 128, 0), idesc_o, ks > 0);
         ss_commit(&sm.bar[2]);
       }
       __syncwarp();
