@@ -20,7 +20,7 @@ ST_OVERFLOW, ST_BAD_LENGTH, ST_EMPTY_ROW, ST_TIMEOUT = 1, 2, 4, 8
 _DTYPES = {torch.float32: DKV_F32, torch.float16: DKV_F16, torch.bfloat16: DKV_BF16}
 
 EXPORTS = (
-    "dkv_version", "dkv_last_error", "dkv_fused_decode", "dkv_split_workspace_bytes", "dkv_fused_workspace_bytes", "dkv_routed_decode", "dkv_split_decode",
+    "dkv_version", "dkv_last_error", "dkv_fused_decode", "dkv_split_workspace_bytes", "dkv_fused_workspace_bytes", "dkv_routed_decode", "dkv_routed_launches", "dkv_split_decode",
     "dkv_split_combine", "dkv_two_stage_decode", "dkv_two_stage_decode_noalloc", "dkv_scores", "dkv_softmax_v", "dkv_softmax_v_workspace_bytes", "dkv_append_decode",
     "dkv_pack_bulk", "dkv_pack_pair", "dkv_row_totals", "dkv_decompress", "dkv_gate_lengths", "dkv_gate_lengths_both", "dkv_gate_workspace_bytes", "dkv_gate_lengths_pair", "dkv_project_bulk", "dkv_probe_tensor_pipe",
     "dkv_norm_rows", "dkv_split_qkv", "dkv_silu_mul", "dkv_argmax_rows",
@@ -144,6 +144,8 @@ def load() -> C.CDLL:
         fn.restype = C.c_int
     lib.dkv_routed_decode.argtypes = [C.POINTER(AttnArgs), C.c_int32]
     lib.dkv_routed_decode.restype = C.c_int
+    lib.dkv_routed_launches.argtypes = [C.POINTER(AttnArgs), C.c_int32]
+    lib.dkv_routed_launches.restype = C.c_int
     for fn in (lib.dkv_split_workspace_bytes, lib.dkv_fused_workspace_bytes, lib.dkv_softmax_v_workspace_bytes):
         fn.argtypes = [C.POINTER(AttnArgs)]
         fn.restype = C.c_size_t

@@ -35,6 +35,7 @@ bool mma_path_ok(const dkv_attn_args* a);
 size_t mma_split_workspace_bytes(const dkv_attn_args* a);
 int mma_fused(const dkv_attn_args* a);
 bool short_ok(const dkv_attn_args* a);
+bool short_takes_all(const dkv_attn_args* a);
 int short_fused(const dkv_attn_args* a);
 int mma_split(const dkv_attn_args* a);
 int mma_combine(const dkv_attn_args* a);
@@ -109,18 +110,21 @@ extern "C" int dkv_routed_decode(const dkv_attn_args* a, int32_t switch_tokens) 
   if (int rc = check_attn_args(a, "dkv_routed_decode", true, true, true)) return rc;
   DKV_REQUIRE(a->seq_lens != nullptr, DKV_E_ARG, "dkv_routed_decode: needs seq_lens");
   dkv_attn_args s = *a, l = *a;
-  s.route_min_tokens = l.route_max_tokens = 0;
-  if (switch_tokens <= 0) {      // no row is short
-    l.route_min_tokens = 0;
-    return dkv_two_stage_decode(&l);
-  }
+  s.route_min_tokens = l.route_min_tokens = l.route_max_tokens = 0;
+  if (switch_tokens <= 0) return dkv_two_stage_decode(&l);      // no row is short
+  // On the packed path one route takes all rows, whatever their lengths: a launch of a kernel whose rows are all someone else's
+  // costs 2 us, and short rows beside long ones are a few tiles more of the split (8 KV heads, split + merge for all against
+  // the short kernel for short rows and split + merge for the others: 1 row of 2000 tokens 15.1 / 19.5 us, 4 rows 16.5 / 21.2,
+  // 8 rows of 500 15.1 / 18.0).  Only where all rows happen to be short under a bound that allows longer ones is it 1 us more.
+  if (mma_path_ok(a)) return short_takes_all(&l) ? short_fused(&l) : dkv_two_stage_decode(&l);
   s.route_max_tokens = l.route_min_tokens = switch_tokens;
-  if (mma_path_ok(a) && fused_by_split(&s)) {      // the short rows would go through split and merge as well: one pass for all
-    l.route_min_tokens = 0;
-    return dkv_two_stage_decode(&l);
-  }
   if (int rc = dkv_fused_decode(&s)) return rc;
   return dkv_two_stage_decode(&l);
+}
+
+extern "C" int dkv_routed_launches(const dkv_attn_args* a, int32_t switch_tokens) {
+  if (a == nullptr || !mma_path_ok(a)) return 0;
+  return switch_tokens > 0 && short_takes_all(a) ? 1 : 2;
 }
 
 extern "C" int dkv_two_stage_decode_noalloc(const dkv_attn_args* a) {

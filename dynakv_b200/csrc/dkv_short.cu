@@ -27,6 +27,9 @@ constexpr int ST = 128;                 // tokens per tile
 constexpr int STHREADS = 512;
 constexpr int SHP = 4;                  // query heads per KV head
 constexpr int SCLUSTER = 4;             // CTAs per row at most
+// A routed call whose rows cannot be longer is one launch of this kernel, two rounds of tiles per CTA (us, against split and
+// merge: 1 row of 499 / 600 / 1024 / 1400 tokens 9.4 / 13.7 / 14.0 / 18.6 and 14.6 / 14.5 / 14.7 / 15.1; 4 rows of 1024 15.1 and 15.0).
+constexpr int SHORT_ALL_TOKENS = 1024;
 constexpr uint32_t SSPIN = 1u << 22;
 constexpr uint32_t S_TM_K = 0, S_TM_O = 128, S_TMEM_COLS = 256;
 
@@ -474,6 +477,13 @@ int launch_short(const dkv_attn_args* a) {
 bool short_ok(const dkv_attn_args* a) {
   const int cs = short_cluster(a), n_sm = a->n_sm > 0 ? a->n_sm : sm_count();
   return cs == 1 || (long long)a->batch * a->n_basis_groups * cs <= n_sm;
+}
+
+// Whether a routed call leaves its rows to this kernel, also those at or past the switch point.
+bool short_takes_all(const dkv_attn_args* a) {
+  dkv_attn_args all = *a;
+  all.route_min_tokens = all.route_max_tokens = 0;
+  return a->seq_len <= SHORT_ALL_TOKENS && short_ok(&all);
 }
 
 int short_fused(const dkv_attn_args* a) {

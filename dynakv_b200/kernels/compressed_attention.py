@@ -239,10 +239,9 @@ class CompressedDecodeLayer:
         lib = _lib.load()
         if prepare_only:
             need = int(lib.dkv_split_workspace_bytes(C.byref(args)))
-            if route == "routed":
-                args.route_max_tokens = self.policy.switch_tokens
+            launches = int(lib.dkv_routed_launches(C.byref(args), self.policy.switch_tokens)) if route == "routed" else 0
             by_split = lib.dkv_fused_workspace_bytes(C.byref(args)) > 0       # short rows through split and merge
-            return need, {"long_two_stage": 2, "short_fused": 2 if by_split else 1, "routed": 2 if by_split else 3}[route]
+            return need, launches or {"long_two_stage": 2, "short_fused": 2 if by_split else 1, "routed": 3}[route]
         if route == "routed":
             _lib.check(lib.dkv_routed_decode(C.byref(args), self.policy.switch_tokens), "dkv_routed_decode")
         elif route == "short_fused":
