@@ -468,11 +468,33 @@ __global__ void __launch_bounds__(GG_THREADS) gate_gemm_kernel(const __grid_cons
   }
 }
 
+// The least float whose rounding to T reaches thr (itself a value of T): rounding is monotonic, so comparing an unrounded sum
+// with this bound is comparing the rounded one with thr.  The bound is the middle between thr and the value of T below it,
+// which rounds to thr when thr's last bit is even, or the float after it.  (Sums are not negative: bounds <= 0 stay.)
+template <typename T>
+__device__ __forceinline__ float rounded_bound(float thr) {
+  if (!(thr > 0.f) || isinf(thr)) return thr;
+  const T t = from_f32<T>(thr);
+  uint16_t u = *reinterpret_cast<const uint16_t*>(&t);
+  const bool even = (u & 1) == 0;
+  --u;
+  const float mid = 0.5f * (thr + to_f32(*reinterpret_cast<const T*>(&u)));     // exact
+  return even ? mid : __uint_as_float(__float_as_uint(mid) + 1);
+}
+// a / b for y = 1 / b correctly rounded, two at a time: a quotient within one last place and two exact remainders (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): the result of the division.
+__device__ __forceinline__ float2 quotient2(float2 a, float2 neg_b, float2 y) {
+  float2 q = __fmul2_rn(a, y);
+  q = __ffma2_rn(__ffma2_rn(q, neg_b, a), y, q);
+  return __ffma2_rn(__ffma2_rn(q, neg_b, a), y, q);
+}
+
 // gate_rows_kernel: softmax, running sum, count and masked copy of a row whose logits gate_gemm_kernel left in the
 // workspace; lane l holds columns PER l .. PER l + PER - 1 in registers.  The work is one read of the logits, one of x
-// and one write of the masked row.  Both sides of 8192 rows x
-// 1024, bf16: 2 x 98 us with the columns in (bank-conflicted) shared memory, 2 x 15.6 in registers, 30 us in one launch;
-// bound by the ~900 instructions of a row (exp, division and the roundings that the reference makes).
+// and one write of the masked row; bound by the instructions of a row.  Both sides of 8192 rows x 1024, bf16: 2 x 98 us with
+// the columns in (bank-conflicted) shared memory, 27 us in registers and one launch (1230 instructions a row, 0.69 of the issue
+// slots), now 22: one reciprocal and exact remainders for the divisions by the row's sum, the bound compared instead of each
+// sum rounded, roundings of pairs.  (Call with the logits: 61.5 -> 57.5 us.)
 template <typename T, bool NATIVE, int PER>
 __global__ void __launch_bounds__(256) gate_rows_kernel(const __grid_constant__ dkv_gate_args pk, const __grid_constant__ dkv_gate_args pv) {
   const dkv_gate_args& p = blockIdx.y ? pv : pk;
@@ -480,7 +502,8 @@ __global__ void __launch_bounds__(256) gate_rows_kernel(const __grid_constant__ 
   if (row >= p.n_rows) return;
   pdl_wait();       // the logits come from gate_gemm_kernel
   constexpr int d = 32 * PER;
-  const float thr = NATIVE ? to_f32(from_f32<T>(p.threshold)) : p.threshold;   // the comparison converts the scalar
+  // the comparison converts the scalar; cumsum writes every running sum in the storage type
+  const float thr = NATIVE ? rounded_bound<T>(to_f32(from_f32<T>(p.threshold))) : p.threshold;
   float e[PER];
   if (NATIVE) {
     constexpr int W = PER < 8 ? PER : 8;           // columns of a load
@@ -509,11 +532,20 @@ __global__ void __launch_bounds__(256) gate_rows_kernel(const __grid_constant__ 
   for (int i = 0; i < PER; ++i) { e[i] = expf(e[i] - mx); z += e[i]; }
   z = warp_sum(z);
   float local = 0.f;
+  const float y = __frcp_rn(z);
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    e[i] = e[i] / z;
-    if (NATIVE) e[i] = to_f32(from_f32<T>(e[i]));      // softmax writes the probabilities in the storage type
+  for (int i = 0; i < PER; i += 2) {
+    const float2 q = quotient2(make_float2(e[i], e[i + 1]), make_float2(-z, -z), make_float2(y, y));
+    e[i] = q.x;
+    e[i + 1] = q.y;
+    if (NATIVE) {      // softmax writes the probabilities in the storage type
+      const uint32_t w = gg_pack<T>(q.x, q.y);
+      const T* const t = reinterpret_cast<const T*>(&w);
+      e[i] = to_f32(t[0]);
+      e[i + 1] = to_f32(t[1]);
+    }
     local += e[i];
+    local += e[i + 1];
   }
   float incl = local;
 #pragma unroll
@@ -523,13 +555,13 @@ __global__ void __launch_bounds__(256) gate_rows_kernel(const __grid_constant__ 
   }
   float run = incl - local;
   const int lo = d - min(max(p.low_rank, 0), d);   // only columns >= lo can count
-  int cnt = 0;
+  int below = 0;      // the lane's sums do not fall: those that do not reach the bound (or are no numbers) come first
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     run += e[i];
-    const float c = NATIVE ? to_f32(from_f32<T>(run)) : run;   // cumsum writes every running sum in the storage type
-    cnt += PER * lane + i >= lo && c >= thr;
+    below += !(run >= thr);
   }
+  int cnt = PER - max(below, min(max(lo - PER * lane, 0), PER));
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   if (p.len_multiple > 1) cnt = min((cnt + p.len_multiple - 1) / p.len_multiple * p.len_multiple, d - d % p.len_multiple);
   if (lane == 0) p.lengths[row] = cnt;

@@ -82,3 +82,23 @@ def test_pair_and_prompt_paths_differ_by_summation_order_only(rows, dtype):
         tie = (sums - thr).abs() <= sums * (2 * off + 256 * 2.0 ** -23)
         differ = lens != pair
         assert bool(tie.any(-1)[differ].all()) and int((lens - pair).abs().max()) <= int(tie.sum(-1).max())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("d", [128, 1024])
+@pytest.mark.parametrize("thr", [0.1, 0.5, 0.50390625, 0.7529296875, 0.998046875, 1.0, 1.5, 0.0, -1.0, 1e-30, float("inf"), float("nan")])
+def test_bound_of_rounded_sums(thr, d, native, dtype):
+    """Equal logits: probabilities 1/d and sums j/d are exact, and for d = 1024 their roundings are not: ties on both sides."""
+    from dynakv_b200.kernels.compressed_attention import gate_lengths
+    rows = 65
+    x = torch.randn(rows, d, device="cuda").to(dtype)
+    w, b = torch.zeros(d, d, device="cuda", dtype=dtype), torch.full((d,), 0.5, device="cuda", dtype=dtype)
+    sums = torch.arange(1, d + 1, dtype=torch.float32) / d
+    bound = torch.tensor(thr, dtype=torch.float32)
+    if native:
+        sums, bound = sums.to(dtype).float(), bound.to(dtype).float()
+    for low_rank in (d, d - 37):
+        want = int((sums[d - low_rank:] >= bound).sum())
+        got = gate_lengths(x, w, b, low_rank, threshold=thr, return_masked=False, native_rounding=native)[1]
+        assert got.cpu().tolist() == [want] * rows
