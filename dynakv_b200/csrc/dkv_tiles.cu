@@ -10,7 +10,8 @@
 // (a piece of 8 coefficients may start at any element, it is put together from two aligned 16-byte loads), the softmax
 // weights as two 16-bit terms so that nothing is lost against fp32 weights.  fp32 stays on the FMA units.
 // The first version (one CTA per (row, query head, slice), K reconstructed per query head on mma.sync) took 281 us on
-// B = 2, S = 2048, R = 1024, 8 groups, bf16, and 13 us for the merge; now 25 (scores) + 13 (latent sums) + 7 us (merge).
+// B = 2, S = 2048, R = 1024, 8 groups, bf16, and 13 us for the merge; the three took 25 (scores) + 13 (latent sums) + 7 us (merge),
+// the call 48.0; 43.1 since a thread's pieces are asked for together and the V rows before the scores are waited for.
 // fp32, B = 1, S = 256, 8 arenas: 131 us in one kernel of 32 CTAs, now 12 + 6.5 + 5 us.
 //
 // Math (reference: src/dynakv/kernels/fused.py:28-142, two_stage.py:52-157, 211-281): as in dkv_generic.cu, which keeps
@@ -67,39 +68,39 @@ __device__ __forceinline__ void ts_ld8(float (&v)[8], uint32_t addr) {      // (
 }
 
 // Elements e0 .. e0+7 of a row of `len` 16-bit elements (zeros past its end), whatever the row's alignment: a piece that
-// does not start on a 16-byte boundary is cut out of two aligned loads.  Only 16-byte blocks that hold an element of the
-// row are touched.
-__device__ __forceinline__ uint4 load_piece(const uint16_t* row, int e0, int len) {
-  uint4 o = make_uint4(0u, 0u, 0u, 0u);
-  const int n = len - e0;
-  if (n <= 0) return o;
+// does not start on a 16-byte boundary is cut out of two aligned blocks.  Only 16-byte blocks that hold an element of the
+// row are touched.  Asking for the blocks and cutting the piece are two steps without a branch around the loads: in one
+// function the pieces of a thread were read one after the other, a trip to memory each.
+struct RawPiece {
+  uint4 v0, v1;
+  int shift, n;          // elements of v0 before the piece; elements of the piece that exist
+};
+__device__ __forceinline__ RawPiece ask_piece(const uint16_t* row, int e0, int len) {
+  RawPiece r;
+  r.n = min(max(len - e0, 0), 8);
   const uintptr_t a = reinterpret_cast<uintptr_t>(row + e0);
   const uint4* base = reinterpret_cast<const uint4*>(a & ~(uintptr_t)15);
-  const int sh = (int)(a & 15) >> 1;          // elements to skip
-  const uint4 v0 = __ldg(base);
-  if (sh == 0) {
-    o = v0;
-  } else {
-    uint4 v1 = make_uint4(0u, 0u, 0u, 0u);
-    if (sh + min(n, 8) > 8) v1 = __ldg(base + 1);
-    uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-    if (sh & 4) {
+  r.shift = (int)(a & 15) >> 1;
+  r.v0 = r.v1 = make_uint4(0u, 0u, 0u, 0u);
+  if (r.n > 0) r.v0 = __ldg(base);
+  if (r.shift + r.n > 8) r.v1 = __ldg(base + 1);       // (only with r.n > 0: shift is at most 7)
+  return r;
+}
+__device__ __forceinline__ uint4 cut_piece(const RawPiece& r) {
+  uint32_t w[8] = {r.v0.x, r.v0.y, r.v0.z, r.v0.w, r.v1.x, r.v1.y, r.v1.z, r.v1.w};
+  if (r.shift & 4) {
 #pragma unroll
-      for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
-    }
-    if (sh & 2) {
-#pragma unroll
-      for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
-    }
-    const uint32_t sel = (sh & 1) ? 0x5432u : 0x3210u;
-    o = make_uint4(__byte_perm(w[0], w[1], sel), __byte_perm(w[1], w[2], sel), __byte_perm(w[2], w[3], sel), __byte_perm(w[3], w[4], sel));
+    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
   }
-  if (n < 8) {
-    uint32_t* t = reinterpret_cast<uint32_t*>(&o);
+  if (r.shift & 2) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = n >= 2 * i + 2 ? t[i] : (n == 2 * i + 1 ? t[i] & 0xffffu : 0u);
+    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
   }
-  return o;
+  const uint32_t sel = (r.shift & 1) ? 0x5432u : 0x3210u;
+  uint32_t t[4] = {__byte_perm(w[0], w[1], sel), __byte_perm(w[1], w[2], sel), __byte_perm(w[2], w[3], sel), __byte_perm(w[3], w[4], sel)};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = r.n >= 2 * i + 2 ? t[i] : (r.n == 2 * i + 1 ? t[i] & 0xffffu : 0u);
+  return make_uint4(t[0], t[1], t[2], t[3]);
 }
 
 __device__ __forceinline__ int row_len(const dkv_attn_args& p, int b) {
@@ -193,12 +194,12 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
   // X pieces of this thread: tokens (tid & 7) + 8 * (tid >> 5) + 64 u', pieces ((tid >> 3) & 3) + 4 u: eight lanes with
   // consecutive tokens write 128 consecutive bytes, four lanes read 64 consecutive bytes of a row
   const int x_t = (tid & 7) + 8 * warp, x_c = (tid >> 3) & 3;
-  uint4 xr[4];
+  RawPiece xr[4];
   auto load_x = [&](int c) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int t = x_t + 64 * (u & 1), e = c * TS_CHUNK + 8 * (x_c + 4 * (u >> 1));
-      xr[u] = load_piece(reinterpret_cast<const uint16_t*>(flat) + sm.off[t], e, sm.len[t]);
+      xr[u] = ask_piece(reinterpret_cast<const uint16_t*>(flat) + sm.off[t], e, sm.len[t]);
     }
   };
   auto copy_b = [&](int c) {
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_kernel(dkv_attn_args p
     // (the products of stage c - 3, the last user of this buffer, were waited for in the round before)
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      *reinterpret_cast<uint4*>(sm.x[buf] + (x_c + 4 * (u >> 1)) * 2048 + (x_t + 64 * (u & 1)) * 16) = xr[u];
+      *reinterpret_cast<uint4*>(sm.x[buf] + (x_c + 4 * (u >> 1)) * 2048 + (x_t + 64 * (u & 1)) * 16) = cut_piece(xr[u]);
     if (c + 1 < n_chunk) {
       if (c >= 2) ok = ts_wait(&sm.done[(c + 1) % TS_STAGES], (uint32_t)(((c - 2) / TS_STAGES) & 1)) && ok;
       load_x(c + 1);
@@ -426,12 +427,6 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
   }
   if (tid < NH) sm.l[tid] = 0.f;
   for (int e = tid; e < 2 * TS_TOK * NH; e += TS_THREADS) reinterpret_cast<uint32_t*>(sm.pt)[e] = 0u;     // columns of heads that are not there
-  pdl_wait();        // the scores (and, in a chain of layers, the workspace) are the kernel's before this one
-  slice_maxima(src, i_row, b, Hq, head0, nh, t0, t1, sm.m);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = sm.tmem;
   const T* flat = reinterpret_cast<const T*>(p.v.flat) + (size_t)a * p.v.flat_stride;
   const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
   // D fp32, A = V^T (MN-major: bit 15), B = P (MN-major: bit 16), M = 128, N = 2 NH
@@ -442,7 +437,8 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
   for (int tt = t0; tt < t1; tt += TS_TOK) {
     const int buf = n_done & 1;
     if (n_done >= 2) ok = ts_wait(&sm.done[buf], (uint32_t)(((n_done - 2) >> 1) & 1)) && ok;
-    if (tid == 0) sm.rmax[buf] = 0;
+    const int par = ((tt - t0) / TS_TOK) & 1;      // (not buf, which an unused tile leaves to the next one, whose reset could overtake a reader)
+    if (tid == 0) sm.rmax[par] = 0;
     __syncthreads();
     if (tid < TS_TOK) {
       int len = 0, off = 0;
@@ -450,7 +446,25 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
       sm.len[buf][tid] = len;
       sm.off[buf][tid] = off;
       const int mx = __reduce_max_sync(0xffffffffu, len);
-      if (lane == 0) atomicMax(&sm.rmax[buf], mx);
+      if (lane == 0) atomicMax(&sm.rmax[par], mx);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // The V rows are asked for before the weights are formed, the first tile's before the scores are waited for.
+    const bool use = sm.rmax[par] > 128 * rb;
+    RawPiece v[8];
+    if (use) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int t = x_t + 64 * (u & 1);
+        v[u] = ask_piece(reinterpret_cast<const uint16_t*>(flat) + sm.off[buf][t], 128 * rb + 8 * (x_c + 4 * (u >> 1)), sm.len[buf][t]);
+      }
+    }
+    if (tt == t0) {
+      pdl_wait();        // the scores (and, in a chain of layers, the workspace) are the kernel's before this one
+      slice_maxima(src, i_row, b, Hq, head0, nh, t0, t1, sm.m);
+      __syncthreads();
     }
     // weights: a warp takes a head at a time, four tokens per lane
     for (int h = warp; h < nh; h += TS_THREADS / 32) {
@@ -470,27 +484,17 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
       l = warp_sum(l);
       if (lane == 0) sm.l[h] += l;
     }
-    __syncthreads();
-    if (sm.rmax[buf] > 128 * rb) {
+    if (use) {
 #pragma unroll
-      for (int u0 = 0; u0 < 8; u0 += 4) {
-        uint4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int t = x_t + 64 * (u & 1), e = 128 * rb + 8 * (x_c + 4 * ((u0 + u) >> 1));
-          v[u] = load_piece(reinterpret_cast<const uint16_t*>(flat) + sm.off[buf][t], e, sm.len[buf][t]);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          *reinterpret_cast<uint4*>(sm.v[buf] + (x_c + 4 * ((u0 + u) >> 1)) * 2048 + (x_t + 64 * (u & 1)) * 16) = v[u];
-      }
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<uint4*>(sm.v[buf] + (x_c + 4 * (u >> 1)) * 2048 + (x_t + 64 * (u & 1)) * 16) = cut_piece(v[u]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
       if (tid == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          ts_mma(tmem, ts_desc(ts_smem(sm.v[buf]) + ks * 256, 128, 2048), ts_desc(ts_smem(sm.pt[buf]) + ks * 256, 128, 2048), idesc, n_done > 0 || ks > 0);
+          ts_mma(sm.tmem, ts_desc(ts_smem(sm.v[buf]) + ks * 256, 128, 2048), ts_desc(ts_smem(sm.pt[buf]) + ks * 256, 128, 2048), idesc, n_done > 0 || ks > 0);
         ts_commit(&sm.done[buf]);
       }
       ++n_done;
@@ -502,6 +506,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
   if (!ok && tid == 0) set_status(p.status, DKV_ST_TIMEOUT);
   if (rb == 0 && tid < nh) { my_rec[tid * rec_h] = sm.m[tid]; my_rec[tid * rec_h + 1] = sm.l[tid]; }
   // thread = (latent, half of the heads)
+  const uint32_t tmem = sm.tmem;
   const int r = 128 * rb + (tid & 127), half = tid >> 7;
   const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
 #pragma unroll
