@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   __shared__ __align__(16) float x_s[TS_CHUNK][TF_TOK];
   __shared__ float k_s[TF_TOK][TD + 4];
   __shared__ float cs_s[TF_TOK][64], sn_s[TF_TOK][64];
-  __shared__ float q_s[TD];
+  __shared__ float q_s[TS_HB][TD];
   __shared__ int len_s[TF_TOK], off_s[TF_TOK];
   __shared__ int rmax_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -556,6 +556,15 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   if (t0 >= t_end) return;
   const int a = b * A + (g * G * A) / Hq;
   pdl_launch_dependents();
+  // the queries of up to TS_HB heads are on their way from the start (asked for head by head they were a trip to memory each)
+  auto ask_queries = [&](int h0) {
+    const int n = min(TS_HB, G - h0) * TD;
+    for (int e = tid; e < n; e += TS_THREADS) {
+      const float* qp = reinterpret_cast<const float*>(p.q) + (size_t)b * p.q_stride_b + (size_t)(g * G + h0 + (e >> 7)) * p.q_stride_h + (e & 127);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ts_smem(&q_s[e >> 7][e & 127])), "l"(qp) : "memory");
+    }
+  };
+  ask_queries(0);
   if (warp == 0) {
     int len = 0, off = 0;
     if (lane < TF_TOK) {
@@ -600,6 +609,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) k_s[8 * th + i][d] = acc[i];
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const float scale = rsqrtf((float)TD);
   // a warp rotates its two tokens in place, then multiplies them with every head
@@ -622,14 +632,17 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
     k_s[t][lane + 96] = k1b * cb + k0b * sb;
   }
   for (int h = 0; h < G; ++h) {
-    const int head = g * G + h;
-    __syncthreads();
-    if (tid < TD) q_s[tid] = (reinterpret_cast<const float*>(p.q) + (size_t)b * p.q_stride_b + (size_t)head * p.q_stride_h)[tid];
-    __syncthreads();
+    const int head = g * G + h, hs = h % TS_HB;
+    if (h > 0 && hs == 0) {
+      __syncthreads();
+      ask_queries(h);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+    }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int t = warp + 8 * u, s = t0 + t;
-      float part = q_s[lane] * k_s[t][lane] + q_s[lane + 64] * k_s[t][lane + 64] + q_s[lane + 32] * k_s[t][lane + 32] + q_s[lane + 96] * k_s[t][lane + 96];
+      float part = q_s[hs][lane] * k_s[t][lane] + q_s[hs][lane + 64] * k_s[t][lane + 64] + q_s[hs][lane + 32] * k_s[t][lane + 32] + q_s[hs][lane + 96] * k_s[t][lane + 96];
       part = warp_sum(part);
       if (lane == 0 && s < t_end) {
         if (sink.ws) sink.ws[((size_t)i_row * Hq + head) * sink.pitch + s] = len_s[t] > 0 ? part * scale : -INFINITY;
@@ -665,8 +678,6 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_f32_kernel(dkv_attn_args p
   }
   const int a = b * A + j;
   if (tid < NH) l_s[tid] = 0.f;
-  pdl_wait();
-  slice_maxima(src, i_row, b, Hq, head0, nh, t0, t1, m_s);
   const float* flat = reinterpret_cast<const float*>(p.v.flat) + (size_t)a * p.v.flat_stride;
   const int r = 128 * rb + (tid & 127), half = tid >> 7;
   float acc[NH];
@@ -680,6 +691,20 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_f32_kernel(dkv_attn_args p
       len_s[lane] = len;
       off_s[lane] = off;
     }
+    __syncthreads();
+    // V is asked for before the weights are formed, the first tile's before the scores are waited for
+    float v[TF_SLICE / 2];
+#pragma unroll
+    for (int k = 0; k < TF_SLICE / 2; ++k) {
+      const int t = half + 2 * k;
+      v[k] = 0.f;
+      if (r < len_s[t]) v[k] = __ldg(flat + (size_t)off_s[t] + r);
+    }
+    if (tt == t0) {
+      pdl_wait();
+      slice_maxima(src, i_row, b, Hq, head0, nh, t0, t1, m_s);
+      __syncthreads();
+    }
     for (int h = warp; h < NH; h += TS_THREADS / 32) {
       float pv = 0.f;
       if (h < nh && tt + lane < t1) {
@@ -691,16 +716,15 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_f32_kernel(dkv_attn_args p
       if (lane == 0) l_s[h] += l;
     }
     __syncthreads();
-#pragma unroll 8
-    for (int t = half; t < TF_SLICE; t += 2) {
-      const float v = r < len_s[t] ? flat[(size_t)off_s[t] + r] : 0.f;
+#pragma unroll
+    for (int k = 0; k < TF_SLICE / 2; ++k) {
 #pragma unroll
       for (int h = 0; h < NH; h += 4) {
-        const float4 w = *reinterpret_cast<const float4*>(&p_s[t][h]);
-        acc[h] = fmaf(w.x, v, acc[h]);
-        acc[h + 1] = fmaf(w.y, v, acc[h + 1]);
-        acc[h + 2] = fmaf(w.z, v, acc[h + 2]);
-        acc[h + 3] = fmaf(w.w, v, acc[h + 3]);
+        const float4 w = *reinterpret_cast<const float4*>(&p_s[half + 2 * k][h]);
+        acc[h] = fmaf(w.x, v[k], acc[h]);
+        acc[h + 1] = fmaf(w.y, v[k], acc[h + 1]);
+        acc[h + 2] = fmaf(w.z, v[k], acc[h + 2]);
+        acc[h + 3] = fmaf(w.w, v[k], acc[h + 3]);
       }
     }
   }

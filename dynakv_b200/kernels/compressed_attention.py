@@ -224,8 +224,8 @@ class CompressedDecodeLayer:
     def attend(self, cache: CustomDynamicCache, q: torch.Tensor, out: torch.Tensor, row_counter: torch.Tensor,
                seq_columns: int, route: str, route_min_tokens: int = 0, route_max_tokens: int = 0,
                prepare_only: bool = False, workspace: Optional[torch.Tensor] = None):
-        """Attention of all batch rows through one kernel (``route``), or with ``"routed"`` every row through the kernel of
-        its current length (read from ``row_counter`` on the device) by the policy's switch point.  With routing bounds a
+        """Attention of all batch rows through one kernel (``route``), or with ``"routed"`` as ``dkv_routed_decode`` chooses
+        for rows on both sides of the policy's switch point (lengths read from ``row_counter`` on the device).  With routing bounds a
         single kernel skips the rows that belong to the other one.  ``workspace`` is
         scratch the caller keeps for calls that follow one another on one stream; the bytes the call needs are returned
         (``prepare_only``: nothing is launched, and the number of launches is returned beside them)."""
@@ -256,8 +256,8 @@ class DecodeGraph:
     """CUDA-graph replay of append + routed attention over a stack of layers.
 
     The caches must have been filled (prefill) with ``token_counts`` so that every layer owns a device
-    row counter; the graph reads the current cache lengths from those counters and the kernels route every
-    row on its own length (``KernelPolicy.switch_tokens``) on the device, so one capture serves every later
+    row counter; the graph reads the current cache lengths from those counters on the device, and where rows on
+    both sides of ``KernelPolicy.switch_tokens`` are possible the route takes rows of any length, so one capture serves every later
     step -- also when a row crosses the switch point -- as long as no row outgrows ``seq_capacity``.
     ``horizon`` = number of steps the capture must stay valid for (default: until the cache is full); it only
     decides whether the long-cache kernels have to be in the graph at all.
