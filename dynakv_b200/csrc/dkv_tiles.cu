@@ -575,14 +575,18 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
     const int mx = __reduce_max_sync(0xffffffffu, len);
     if (lane == 0) rmax_s = mx;
   }
+  const int d = tid & 127, th = tid >> 7;
+  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(PARTS ? g / sink.per_basis : g) * R * TD;
+  float w[16];           // the first basis rows too
+#pragma unroll
+  for (int u = 0; u < 16; ++u) w[u] = u < R ? __ldg(kup + (size_t)u * TD + d) : 0.f;
   for (int e = tid; e < TF_TOK * 64; e += TS_THREADS) {
     const int t = e >> 6, j = e & 63;
     sincosf((float)(t0 + t) * expf(-((float)(2 * j) / (float)TD) * log_theta), &sn_s[t][j], &cs_s[t][j]);
   }
   __syncthreads();
   const float* flat = reinterpret_cast<const float*>(p.k.flat) + (size_t)a * p.k.flat_stride;
-  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(PARTS ? g / sink.per_basis : g) * R * TD;
-  const int d = tid & 127, th = tid >> 7, rmax = rmax_s;
+  const int rmax = rmax_s;
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -595,9 +599,10 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
     __syncthreads();
 #pragma unroll 1
     for (int rr = 0; rr < nr; rr += 16) {
-      float w[16];
+      if (r0 + rr > 0) {
 #pragma unroll
-      for (int u = 0; u < 16; ++u) w[u] = r0 + rr + u < rmax ? __ldg(kup + (size_t)(r0 + rr + u) * TD + d) : 0.f;
+        for (int u = 0; u < 16; ++u) w[u] = r0 + rr + u < rmax ? __ldg(kup + (size_t)(r0 + rr + u) * TD + d) : 0.f;
+      }
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const float4 x0 = *reinterpret_cast<const float4*>(&x_s[rr + u][8 * th]), x1 = *reinterpret_cast<const float4*>(&x_s[rr + u][8 * th + 4]);
