@@ -250,7 +250,7 @@ def ragged_strong_leg(dev, world, rank, steps, warmup, timed, dist):
            "value": r["n_seq"] / (ms_step * 1e-3), "unit": "tokens/s", "ms_per_step": ms_step,
            "us_per_layer": ms_step * 1e3 / r["layers"],
            "hbm_gbs_all_ranks": float(comp_t.item()) / (ms_step * 1e-3) / 1e9,
-           "routing": "per row on the device, KernelPolicy(switch_tokens=500); %d of %d sequences below the switch point"
+           "routing": "lengths read per row on the device, KernelPolicy(switch_tokens=500); %d of %d sequences below the switch point"
                       % (sum(1 for n in lengths if n < 500), r["n_seq"])}
     del cache, layers
     torch.cuda.empty_cache()
