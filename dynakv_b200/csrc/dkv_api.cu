@@ -58,6 +58,18 @@ static bool fused_by_split(const dkv_attn_args* a) {
   const int n_sm = a->n_sm > 0 ? a->n_sm : sm_count();
   return (long long)a->batch * a->n_basis_groups > (short_ok(a) ? 2LL : 1LL) * n_sm;
 }
+// Kernels of a routed call on the packed path: 1 = the short kernel for rows of any length, 2 = split + merge for all rows, 3 = the
+// short kernel for short rows and split + merge for the others.  A launch of a kernel whose rows are all someone else's costs
+// 2 us, so all rows take one route (8 rows of 500 tokens: 18.0 us with three kernels, 15.1 with two) unless it would be less
+// exact: the short kernel keeps scores in fp32 and weights as value and remainder, the pipeline, which is what short rows take in
+// batches past short_ok, does what the split does.
+static int routed_launches(const dkv_attn_args* a, int switch_tokens) {
+  dkv_attn_args s = *a, all = *a;
+  all.route_min_tokens = all.route_max_tokens = s.route_min_tokens = 0;
+  s.route_max_tokens = switch_tokens;
+  if (short_takes_all(&all) && !fused_by_split(&all)) return 1;
+  return !short_ok(&s) || fused_by_split(&s) ? 2 : 3;
+}
 }  // namespace dkv
 
 extern "C" int dkv_fused_decode(const dkv_attn_args* a) {
@@ -112,19 +124,20 @@ extern "C" int dkv_routed_decode(const dkv_attn_args* a, int32_t switch_tokens) 
   dkv_attn_args s = *a, l = *a;
   s.route_min_tokens = l.route_min_tokens = l.route_max_tokens = 0;
   if (switch_tokens <= 0) return dkv_two_stage_decode(&l);      // no row is short
-  // On the packed path one route takes all rows, whatever their lengths: a launch of a kernel whose rows are all someone else's
-  // costs 2 us, and short rows beside long ones are a few tiles more of the split (8 KV heads, split + merge for all against
-  // the short kernel for short rows and split + merge for the others: 1 row of 2000 tokens 15.1 / 19.5 us, 4 rows 16.5 / 21.2,
-  // 8 rows of 500 15.1 / 18.0).  Only where all rows happen to be short under a bound that allows longer ones is it 1 us more.
-  if (mma_path_ok(a)) return short_takes_all(&l) ? short_fused(&l) : dkv_two_stage_decode(&l);
   s.route_max_tokens = l.route_min_tokens = switch_tokens;
+  if (mma_path_ok(a)) {
+    const int n = routed_launches(a, switch_tokens);
+    l.route_min_tokens = n < 3 ? 0 : switch_tokens;
+    if (n == 1) return short_fused(&l);
+    if (n == 2) return dkv_two_stage_decode(&l);
+  }
   if (int rc = dkv_fused_decode(&s)) return rc;
   return dkv_two_stage_decode(&l);
 }
 
 extern "C" int dkv_routed_launches(const dkv_attn_args* a, int32_t switch_tokens) {
   if (a == nullptr || !mma_path_ok(a)) return 0;
-  return switch_tokens > 0 && short_takes_all(a) ? 1 : 2;
+  return switch_tokens > 0 ? routed_launches(a, switch_tokens) : 2;
 }
 
 extern "C" int dkv_two_stage_decode_noalloc(const dkv_attn_args* a) {

@@ -257,7 +257,7 @@ class DecodeGraph:
 
     The caches must have been filled (prefill) with ``token_counts`` so that every layer owns a device
     row counter; the graph reads the current cache lengths from those counters on the device, and where rows on
-    both sides of ``KernelPolicy.switch_tokens`` are possible the route takes rows of any length, so one capture serves every later
+    both sides of ``KernelPolicy.switch_tokens`` are possible its kernels serve rows of any length, so one capture serves every later
     step -- also when a row crosses the switch point -- as long as no row outgrows ``seq_capacity``.
     ``horizon`` = number of steps the capture must stay valid for (default: until the cache is full); it only
     decides whether the long-cache kernels have to be in the graph at all.

@@ -4,10 +4,9 @@ Mirrors src/dynakv/kernels/router.py of the reference: ``KernelPolicy(switch_tok
 keyword-only ``compressed_decode_attention``.  Extension: with ``seq_lens`` (one cache length per batch
 row, on the device) every sequence has its own length, read by the kernels themselves, and nothing is
 copied to or from the host -- so a ragged batch that straddles the switch point, or a row that crosses it
-between two steps of a captured graph, is handled without re-partitioning.  On the packed path all rows of
-such a call take one route, which the row width of the metadata decides; on other caches both kernels are
-launched over the whole batch with the policy's switch point as a bound, and each skips the rows that
-belong to the other.  ``seq_lens_host`` (the same lengths as python ints) only lets the call skip a kernel
+between two steps of a captured graph, is handled without re-partitioning.  Where that loses no precision
+all rows of such a call take one route (``dkv_routed_decode``); else both kernels are launched over the whole
+batch with the policy's switch point as a bound, and each skips the rows that belong to the other.  ``seq_lens_host`` (the same lengths as python ints) only lets the call skip a kernel
 that has no row to process.
 """
 from __future__ import annotations
