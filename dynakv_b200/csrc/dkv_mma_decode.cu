@@ -67,6 +67,7 @@ constexpr int NBUF_A = 3;              // K operand tiles in shared memory (on t
 constexpr int NBUF_T = 3;              // K accumulator buffers in tensor memory (held from product (1) to product (2))
 constexpr int NBUF_V = 2;              // V operand tiles
 constexpr int NQ = 2;                  // rotated-query tiles
+constexpr int META_AHEAD = 4;          // tiles
 constexpr int KV_RING = 8;             // tiles of token-validity masks kept
 // 1/rms ring: a RoPE write for tile c only implies that the softmax warps have finished tile c-5 (product (1) of c
 // needs product (2) of c-3, which needs the P tile of c-5), so tiles c-4 .. c may be unread
@@ -601,6 +602,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       }
       len = off = 0;
       if (left > 0) { len = __ldg(lens_at); off = __ldg(offs_at); }
+      // a line of each, META_AHEAD tiles on, into L2: a tile ahead is less than a trip to memory since the loop got faster
+      // (8 rows of 32768 tokens 107.9 -> 104.3 us, 32 of 8192 124.7 -> 120.9)
+      if (lane < 2 && left > META_AHEAD * ST_TOK)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"((lane ? offs_at : lens_at) + META_AHEAD * ST_TOK));
       left -= ST_TOK; lens_at += ST_TOK; offs_at += ST_TOK;
     };
     ask_meta(0);
