@@ -847,6 +847,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
   while (row < p.batch && sm.prefix[row] < u_end) {
     const int c_lo = max(sm.prefix[row], u_begin) - u_begin;     // tiles of this row in this CTA: [c_lo, c_hi)
     const int c_hi = min(sm.prefix[row + 1], u_end) - u_begin;
+    if (c_hi <= c_lo) { ++row; continue; }                       // a row without tiles passes no barrier, so it may not touch what the warps share
     const bool alone = c_hi - c_lo == 1;                         // one tile: its warps have the whole sum
     if (alone && ((c_lo ^ grp) & 1)) { ++row; continue; }
     float m_ref[HP], l_part[HP];

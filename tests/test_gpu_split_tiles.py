@@ -85,3 +85,56 @@ def test_routes_of_a_routed_call(seq, switch):
     assert float((out.float().cpu() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
     assert _common.read_status(torch.device("cuda")) == (4 if 0 in seq else 0)      # an empty row is reported
     del keep
+
+
+def _row_errors(out, ref):
+    """Relative 2-norm of the error of each (row, head)."""
+    return (out.float().cpu() - ref).norm(dim=-1) / ref.norm(dim=-1).clamp_min(1e-30)
+
+
+# A result is off by the roundings of the result, the weights and the rotated keys and queries, each of them half a unit u in the
+# last place at most and independent over the tokens: about u (1 + 1 + 2 s) for scores that spread by s, here about 1.
+ROW_LIMIT = {torch.bfloat16: 8 * 2.0 ** -9, torch.float16: 8 * 2.0 ** -11}
+
+
+def _run(c, entry, n_sm, switch=None, repeats=30, **more):
+    """An entry on `n_sm` SMs, its result and the status; repeated runs have to agree bit for bit."""
+    fk, fv, lk, lv, ok, ov = c.views()
+    ref = torch.nan_to_num(O.compact_attention(c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov, c.theta, seq_lens=c.seq_lens))
+    d = [t.cuda() for t in (c.q, fk, c.k_up, fv, c.v_up, lk, ok, lv, ov)]
+    out = torch.full(c.q.shape, 7.0, dtype=c.q.dtype, device="cuda")
+    a, keep = _common.build_attn_args(*d, c.theta, out=out, len_multiple=8, need_workspace=True,
+                                      seq_lens=torch.tensor(c.seq_lens, dtype=torch.int32, device="cuda"), **more)
+    a.n_sm = n_sm
+    ws = torch.empty(int(_lib.load().dkv_split_workspace_bytes(ctypes.byref(a))), dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    first = None
+    for _ in range(repeats):
+        out.fill_(7.0)
+        _lib.check(entry(ctypes.byref(a)) if switch is None else entry(ctypes.byref(a), switch), "attention")
+        first = out.clone() if first is None else first
+        assert torch.equal(out, first)
+    del keep
+    return a, first, ref, _common.read_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("n_sm", [2, 4, 6])
+@pytest.mark.parametrize("seq", [[100, 0, 300], [0, 0, 700], [129, 0, 0, 1, 0, 257], [640, 0, 128, 0, 0, 384, 0], [256, 0, 90, 0, 1000, 0, 0, 5] * 2], ids=str)
+def test_rows_without_tiles_between_others(seq, n_sm, dtype):
+    """A CTA that goes from one row over rows without tiles to another one, or to its end."""
+    c = synthetic.make_layer_case(13, seq, "beta:2,5", 5e5, dtype, "cpu", n_q_heads=8, n_kv_heads=2)
+    _, out, ref, status = _run(c, _lib.load().dkv_two_stage_decode, n_sm)
+    empty = torch.tensor(seq) == 0
+    assert float(out[empty.cuda()].abs().max()) == 0 and status == 4      # an empty row is reported
+    assert float(_row_errors(out, ref)[~empty].max()) <= ROW_LIMIT[dtype]
+
+
+@pytest.mark.parametrize("n_sm", [8, 10, 14])
+@pytest.mark.parametrize("seq", [[1300, 40, 500, 63, 7, 1200, 128, 1], [1, 64, 63, 1500, 2, 100, 3, 3], [130, 5, 1030, 5, 128, 5, 300, 5]], ids=str)
+def test_short_rows_between_long_ones(seq, n_sm):
+    """The route of three kernels: the split walks over the rows that the short kernel takes."""
+    c = synthetic.make_layer_case(17, seq, "beta:2,5", 5e5, torch.bfloat16, "cpu", n_q_heads=8, n_kv_heads=2)
+    a, out, ref, status = _run(c, _lib.load().dkv_routed_decode, n_sm, switch=64)
+    assert _lib.load().dkv_routed_launches(ctypes.byref(a), 64) == 3
+    assert status == 0 and float(_row_errors(out, ref).max()) <= ROW_LIMIT[torch.bfloat16]
