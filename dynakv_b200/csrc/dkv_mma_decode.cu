@@ -579,7 +579,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     const dkv_side& sd = is_v ? p.v : p.k;
     const int NB = is_v ? NBUF_V : NBUF_A;
     const int t = 32 * gw + lane, sub = lane & 3, tl = lane >> 2;      // reads token t's metadata, copies pieces sub, sub + 4, .. of tokens tl + 8 r
-    const unsigned limit = (unsigned)min(sd.flat_stride, (int64_t)INT_MAX);
+    // (off + len of two non-negative ints, as unsigned: exact.  An arena row of negative size holds no token, not even an empty one.)
+    const unsigned limit = (unsigned)max(min(sd.flat_stride, (int64_t)UINT_MAX), (int64_t)0);
+    const int longest_ok = sd.flat_stride < 0 ? -1 : R;
     const uint32_t tile0 = smem_u32(is_v ? sm.v_tile[0] : sm.a_tile[0]) + (32 * gw + tl) * 16 + sub * CHUNK_PITCH;
     const uint32_t full0 = smem_u32(is_v ? &sm.v_full[0] : &sm.a_full[0]), free0 = smem_u32(is_v ? &sm.pv_done[0] : &sm.t_ready[0]);
     uint32_t held = 0x10101010u;      // chunks that the buffers' rows hold, a byte per buffer (at first: anything)
@@ -613,7 +615,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     uint32_t par = 1;                 // of the buffer's last release (none in the first round)
     for (int c = 0; c < n_stages; ++c) {
       int nc = len >> 3, o = off;
-      if (((len | off) & 0x80000007) != 0 || len > R || (unsigned)len + (unsigned)off > limit) {
+      if (((len | off) & 0x80000007) != 0 || len > longest_ok || (unsigned)len + (unsigned)off > limit) {
         set_status(p.status, DKV_ST_BAD_LENGTH);   // breaks the layout contract: token dropped, call flagged
         nc = o = 0;
       }

@@ -138,3 +138,45 @@ def test_short_rows_between_long_ones(seq, n_sm):
     a, out, ref, status = _run(c, _lib.load().dkv_routed_decode, n_sm, switch=64)
     assert _lib.load().dkv_routed_launches(ctypes.byref(a), 64) == 3
     assert status == 0 and float(_row_errors(out, ref).max()) <= ROW_LIMIT[torch.bfloat16]
+
+
+def _raw_call(q, k_up, v_up, flat, lens, offs, stride):
+    """dkv_two_stage_decode with K and V rows in one arena that is said to be `stride` elements wide."""
+    out = torch.full(q.shape, 7.0, dtype=q.dtype, device="cuda")
+    a, keep = _common.build_attn_args(q, flat, k_up, flat, v_up, lens, offs, lens, offs, 5e5, out=out, len_multiple=8, need_workspace=True)
+    a.k.flat_stride = a.v.flat_stride = stride
+    _lib.check(_lib.load().dkv_two_stage_decode(ctypes.byref(a)), "dkv_two_stage_decode")
+    torch.cuda.synchronize()
+    del keep
+    return out, _common.read_status(torch.device("cuda"))
+
+
+def _one_arena():
+    c = synthetic.make_layer_case(23, [300], "uniform", 5e5, torch.bfloat16, "cuda", n_q_heads=4, n_kv_heads=1)
+    gen = torch.Generator().manual_seed(23)
+    lens = torch.randint(1, 17, (1, 300), generator=gen, dtype=torch.int32) * 8
+    lens[0, -1] = 128
+    side = synthetic.ragged_side(lens.cuda(), torch.Generator("cuda").manual_seed(23), torch.bfloat16)
+    return (c.q, c.k_up, c.v_up), side.flat, side.lens[:, :300], side.offs[:, :300], int(lens.sum())
+
+
+@pytest.mark.parametrize("end", [2 ** 31 - 8, 2 ** 31, 2 ** 31 + 120])
+def test_arena_of_more_than_2_31_elements(end):
+    """A row may end behind the largest int, as long as its arena goes on: the same result as from an arena of its own."""
+    head, small, lens, offs, n = _one_arena()
+    want, status = _raw_call(*head, small, lens, offs, n)
+    assert status == 0
+    flat = torch.empty(1, end, dtype=torch.bfloat16, device="cuda")
+    shift = end - n
+    flat[0, shift:] = small[0, :n]
+    assert int(offs.max()) + shift <= 2 ** 31 - 1
+    got, status = _raw_call(*head, flat, lens, offs + shift, end)
+    assert status == 0 and torch.equal(got, want)
+    cut, status = _raw_call(*head, flat, lens, offs + shift, end - 8)      # the last row does not fit
+    assert status == 2 and not torch.equal(cut, want)
+
+
+def test_arena_of_negative_size_holds_nothing():
+    head, flat, lens, offs, _ = _one_arena()
+    out, status = _raw_call(*head, flat, lens, offs, -8)
+    assert status == 6 and float(out.abs().max()) == 0
