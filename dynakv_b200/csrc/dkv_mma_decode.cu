@@ -144,22 +144,19 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait for a whole warp: returns false (and raises the CTA's abort flag) instead of spinning forever.
-// Every lane tests the barrier itself (one instruction for the warp), so each has its own acquire: with a single
-// polling lane the other lanes' later shared-memory loads are not ordered behind the wait and can be scheduled
-// ahead of it.
+// Bounded wait of a whole, converged warp: false (and the CTA's abort flag raised) instead of spinning forever, and the same
+// answer in all lanes -- what follows is shuffles, votes, tensor-memory accesses and an elected lane, which a lane that has left
+// alone would hold up for good.  Every lane tests the barrier itself (one instruction for the warp), so each has its own
+// acquire: with a single polling lane the other lanes' later shared-memory loads are not ordered behind the wait and can be
+// scheduled ahead of it.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
 #pragma unroll 1
   for (uint32_t it = 0; it < SPIN_LIMIT; ++it) {
-    if (mbar_test(bar, parity)) return true;
-    if ((it & 1023u) == 1023u && *abort_flag) return false;
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    if ((it & 1023u) == 1023u && __any_sync(0xffffffffu, *abort_flag)) return false;
   }
   *abort_flag = 1;
   return false;
-}
-// The same answer in all lanes (the tensor-core issuers elect a lane afterwards).
-__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 // 16 bytes, or zeros without a read
 __device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool zero) {
@@ -677,12 +674,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       // descriptor words: low = (address >> 4) | (LBO >> 4) << 16, high = (SBO >> 4) | version bit
       const uint32_t a_lo0 = desc_lo(smem_u32(sm.a_tile[0]), CHUNK_PITCH), b_lo0 = desc_lo(smem_u32(sm.basis), 2048);
       const uint32_t hi_128 = desc_hi(128);
-      const bool have_basis = mbar_wait_all(smem_u32(&sm.basis_full), 0u, abort_flag);
+      const bool have_basis = mbar_wait(smem_u32(&sm.basis_full), 0u, abort_flag);
       for (int c = 0; have_basis && c < n_stages; ++c) {
         const int buf = c % NBUF_T;
         const uint32_t par = (uint32_t)((c / NBUF_T) & 1);
-        if (c >= NBUF_T && !mbar_wait_all(smem_u32(&sm.s_ready[buf]), par ^ 1u, abort_flag)) break;   // product (2) of tile c-3 has read the accumulator
-        if (!mbar_wait_all(smem_u32(&sm.a_full[buf]), par, abort_flag)) break;
+        if (c >= NBUF_T && !mbar_wait(smem_u32(&sm.s_ready[buf]), par ^ 1u, abort_flag)) break;   // product (2) of tile c-3 has read the accumulator
+        if (!mbar_wait(smem_u32(&sm.a_full[buf]), par, abort_flag)) break;
         proxy_fence_async();   // the tile was written by cp.async (generic proxy), the tensor core reads it through the async proxy
         tc_fence_after();
         const int4 km = *reinterpret_cast<const int4*>(sm.kmax[buf]);
@@ -710,9 +707,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       static_assert(TILE_BYTES % 16 == 0 && Q_TILE_BYTES % 16 == 0 && (2 * Q_LBO) % 16 == 0, "descriptor steps are whole 16-byte units");
       for (int c = 0; c < n_stages; ++c) {
         const int buf = c % NBUF_T, qg = c & 1;
-        if (!mbar_wait_all(smem_u32(&sm.q_full[qg]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
-        if (c >= 2 && !mbar_wait_all(smem_u32(&sm.p_ready[qg]), (uint32_t)(((c >> 1) - 1) & 1), abort_flag)) break;   // score tile read out
-        if (!mbar_wait_all(smem_u32(&sm.kp_ready[buf]), (uint32_t)((c / NBUF_T) & 1), abort_flag)) break;
+        if (!mbar_wait(smem_u32(&sm.q_full[qg]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
+        if (c >= 2 && !mbar_wait(smem_u32(&sm.p_ready[qg]), (uint32_t)(((c >> 1) - 1) & 1), abort_flag)) break;   // score tile read out
+        if (!mbar_wait(smem_u32(&sm.kp_ready[buf]), (uint32_t)((c / NBUF_T) & 1), abort_flag)) break;
         tc_fence_after();
         const uint32_t q_lo = q_lo0 + (uint32_t)qg * (Q_TILE_BYTES >> 4), d_s = tmem_base + TM_S + 16 * qg;
         const uint32_t kp = tmem_base + TM_K + buf * 128;
@@ -747,8 +744,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
           c_row_hi = sm.prefix[row_pv + 1] - u_begin;
         }
         const bool first = c - c_row_lo < NGROUP;   // the first even and the first odd tile of a row start new sums
-        if (!mbar_wait_all(smem_u32(&sm.v_full[vb]), (uint32_t)((c / NBUF_V) & 1), abort_flag)) break;
-        if (!mbar_wait_all(smem_u32(&sm.p_ready[grp]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
+        if (!mbar_wait(smem_u32(&sm.v_full[vb]), (uint32_t)((c / NBUF_V) & 1), abort_flag)) break;
+        if (!mbar_wait(smem_u32(&sm.p_ready[grp]), (uint32_t)((c >> 1) & 1), abort_flag)) break;
         proxy_fence_async();   // V tile written by cp.async
         tc_fence_after();
         const uint32_t v_lo = v_lo0 + (uint32_t)vb * (TILE_BYTES >> 4), p_lo = p_lo0 + (uint32_t)grp * ((ST_TOK * 16) >> 4);
@@ -862,7 +859,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       const int buf = grp;
       const bool first = c_last < 0;    // this group's O holds nothing of this row yet
       // ---------------- scores of this token for the group's heads ----------------
-      if (!dead) dead = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&sm.s_ready[c % NBUF_T]), (uint32_t)((c / NBUF_T) & 1), abort_flag));
+      if (!dead) dead = !mbar_wait(smem_u32(&sm.s_ready[c % NBUF_T]), (uint32_t)((c / NBUF_T) & 1), abort_flag);
       tc_fence_after();
       float s[HP];
       tmem_ld4(s, lane_addr + TM_S + 16 * buf);
@@ -885,7 +882,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       }
       const bool grow = consumer_any(grp, over);
       // the P tile of this parity was read by product (3) of tile c-2
-      if (!dead && c >= 2) dead = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&sm.pv_done[buf]), (uint32_t)(((c >> 1) - 1) & 1), abort_flag));
+      if (!dead && c >= 2) dead = !mbar_wait(smem_u32(&sm.pv_done[buf]), (uint32_t)(((c >> 1) - 1) & 1), abort_flag);
       if (grow) {
 #pragma unroll
         for (int h = 0; h < HP; ++h) {

@@ -150,3 +150,15 @@ def test_ctypes_mirrors_have_the_c_compilers_layout(tmp_path):
             assert getattr(cls, what).offset == int(value), (cname, what)
         seen += 1
     assert seen == sum(len(c._fields_) + 1 for c in pairs.values())
+
+
+def test_waits_of_the_decode_pipeline_answer_for_a_whole_warp():
+    """Shuffles, votes, tensor-memory accesses and elected lanes follow the waits: no lane may leave one, or go on, by itself."""
+    source = open(os.path.join(ROOT, "dynakv_b200", "csrc", "dkv_mma_decode.cu")).read()
+    waits = dict(re.findall(r"__device__ __forceinline__ bool (mbar_wait\w*)\([^)]*\) \{\n(.*?)\n\}", source, flags=re.S))
+    assert waits
+    for name, body in waits.items():
+        exits = re.findall(r"[^\n]*\breturn (?:true|ok)\b[^\n]*|if \([^\n]*abort_flag[^\n]*", body)
+        assert len(exits) >= 2 and all("_sync(0xffffffffu" in e for e in exits), name
+    # and nothing else polls a barrier
+    assert source.count("mbar_test(") == 1 + len(waits)
