@@ -116,6 +116,7 @@ struct SmemLayout {
   alignas(8) unsigned long long pv_done[NGROUP];   // product (3) done: O updated, P tile and V operand tile free (commit)
   alignas(8) unsigned long long dep_full[2];       // a row's end handed over (4 warps)
   alignas(8) unsigned long long dep_free[2];       // and taken (4 warps)
+  alignas(8) unsigned long long drained[3];        // a warp's products are done (commit); only when waits have run out
   int prefix[MAX_BATCH + 1];
   int tokens[MAX_BATCH];                           // of each row in this call
   int abort_flag;
@@ -352,6 +353,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     for (int s = 0; s < NBUF_V; ++s) { mbar_init(smem_u32(&sm.v_full[s]), ST_TOK); }
     for (int s = 0; s < NQ; ++s) mbar_init(smem_u32(&sm.q_full[s]), 1);
     for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&sm.dep_full[s]), 4); mbar_init(smem_u32(&sm.dep_free[s]), 4); }
+    for (int s = 0; s < 3; ++s) mbar_init(smem_u32(&sm.drained[s]), 1);
     for (int s = 0; s < NGROUP; ++s) {
       mbar_init(smem_u32(&sm.p_ready[s]), 4);
       mbar_init(smem_u32(&sm.pv_done[s]), 1);
@@ -998,6 +1000,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
   // ---- epilogue: every warp arrives here; the tensor memory is returned by the warp that allocated it ----
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag) {        // waits have run out: copies and products may be in flight, and end before their operands and sums go
+    if (tid == 0) set_status(p.status, DKV_ST_TIMEOUT);
+    cp_async_wait_all();
+    if (warp >= W_MMA && warp <= W_MMA3) {
+      umma_commit(smem_u32(&sm.drained[warp - W_MMA]));
+      mbar_wait(smem_u32(&sm.drained[warp - W_MMA]), 0u, abort_flag);      // (1024 probes)
+    }
+    __syncthreads();
+  }
   if (project) {
     // out[head][d] = sum_r latent[head][r] * Bv[r][d]: one output element per thread
     const int h = tid >> 7, d = tid & 127;
@@ -1020,7 +1031,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
   }
-  if (*abort_flag && tid == 0) set_status(p.status, DKV_ST_TIMEOUT);
 }
 
 // Merge the split partials of one (batch row, KV head) for its query heads and project through Bv.
