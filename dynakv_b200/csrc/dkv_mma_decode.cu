@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
         arena_next = reinterpret_cast<const unsigned char*>(reinterpret_cast<const T*>(sd.flat) + (size_t)row.arena * sd.flat_stride) + 16 * sub;
       }
       len = off = 0;
-      if (left > 0) { len = __ldg(lens_at); off = __ldg(offs_at); }
+      if (left > 0) { len = *lens_at; off = *offs_at; }      // (not read-only loads: the append that writes them may overlap this kernel's beginning)
       // a line of each, META_AHEAD tiles on, into L2: a tile ahead is less than a trip to memory since the loop got faster
       // (8 rows of 32768 tokens 107.9 -> 104.3 us, 32 of 8192 124.7 -> 120.9)
       if (lane < 2 && left > META_AHEAD * ST_TOK)

@@ -171,3 +171,11 @@ def test_a_decode_kernel_that_gives_up_waits_for_what_is_in_flight():
     given_up = re.search(r"if \(\*abort_flag\) \{(.*?)\n  \}\n", end, flags=re.S).group(1)
     order = [given_up.index(w) for w in ("cp_async_wait_all()", "umma_commit(", "mbar_wait(", "__syncthreads()")]
     assert order == sorted(order)
+
+
+def test_kernels_that_overlap_the_append_read_its_cache_with_ordinary_loads():
+    """A read-only load is for data that nothing writes in the kernel's lifetime: here the V basis alone."""
+    for name in ("dkv_mma_decode.cu", "dkv_short.cu"):
+        source = open(os.path.join(ROOT, "dynakv_b200", "csrc", name)).read()
+        loads = re.findall(r"[^\n]*(?:__ldg\(|ld\.global\.nc)[^\n]*", source)
+        assert all("vup" in line for line in loads), loads
