@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
   }
   const int d = tid & 127, th = tid >> 7;
   const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(PARTS ? g / sink.per_basis : g) * R * TD;
-  float w[16];           // the first basis rows too
+  float w[16];           // the first basis rows too, before it is known how many are needed
 #pragma unroll
   for (int u = 0; u < 16; ++u) w[u] = u < R ? __ldg(kup + (size_t)u * TD + d) : 0.f;
   for (int e = tid; e < TF_TOK * 64; e += TS_THREADS) {
@@ -602,6 +602,9 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
       if (r0 + rr > 0) {
 #pragma unroll
         for (int u = 0; u < 16; ++u) w[u] = r0 + rr + u < rmax ? __ldg(kup + (size_t)(r0 + rr + u) * TD + d) : 0.f;
+      } else if (rmax < 16) {      // rows that no token of the tile reaches take no part, whatever they hold (here, where they have arrived)
+#pragma unroll
+        for (int u = 0; u < 16; ++u) w[u] = u < rmax ? w[u] : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < 16; ++u) {

@@ -133,3 +133,21 @@ def test_what_is_not_finite_stays_so(poison, dtype):
     for out in outs:
         assert torch.equal(out[0].isnan().any(-1).cpu(), want)
     _common.read_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("longest", [1, 7, 15, 16, 17, 70])
+@pytest.mark.parametrize("value", ["nan", "inf"])
+def test_fp32_basis_rows_that_no_token_reaches_take_no_part(value, longest):
+    t = _case(4, 1, 100, 96, 8, 2, 1, torch.float32)
+    for side in "kv":
+        t["lens_" + side] = t["lens_" + side].clamp(min=1, max=longest)
+        t["offs_" + side] = (torch.cumsum(t["lens_" + side], 1) - t["lens_" + side]).to(torch.int32)
+    outs = []
+    for fill in (0.0, float(value)):
+        t["k_up"][:, longest:] = fill
+        d = _dev(t, 0)
+        args = [d[k] for k in ("q", "flat_k", "k_up", "flat_v", "v_up", "lens_k", "offs_k", "lens_v", "offs_v")]
+        outs.append([fn(*args, 10000.0) for fn in (fused_attention_dispatch, two_stage_attention)]
+                    + [abx_sparse(d["q"], d["k_up"], d["flat_k"], d["lens_k"], offsets=d["offs_k"], theta=10000.0)])
+    assert all(torch.equal(a, b) and bool(b.isfinite().all()) for a, b in zip(*outs))
+    assert _common.read_status(torch.device("cuda")) == 0
