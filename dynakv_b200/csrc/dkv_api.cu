@@ -35,7 +35,7 @@ bool mma_path_ok(const dkv_attn_args* a);
 size_t mma_split_workspace_bytes(const dkv_attn_args* a);
 int mma_fused(const dkv_attn_args* a);
 bool short_ok(const dkv_attn_args* a);
-bool short_takes_all(const dkv_attn_args* a);
+bool short_takes_all(const dkv_attn_args* a, int switch_tokens);
 int short_fused(const dkv_attn_args* a);
 int mma_split(const dkv_attn_args* a);
 int mma_combine(const dkv_attn_args* a);
@@ -67,7 +67,7 @@ static int routed_launches(const dkv_attn_args* a, int switch_tokens) {
   dkv_attn_args s = *a, all = *a;
   all.route_min_tokens = all.route_max_tokens = s.route_min_tokens = 0;
   s.route_max_tokens = switch_tokens;
-  if (short_takes_all(&all) && !fused_by_split(&all)) return 1;
+  if (short_takes_all(&all, switch_tokens) && !fused_by_split(&all)) return 1;
   return !short_ok(&s) || fused_by_split(&s) ? 2 : 3;
 }
 }  // namespace dkv

@@ -27,8 +27,9 @@ constexpr int ST = 128;                 // tokens per tile
 constexpr int STHREADS = 512;
 constexpr int SHP = 4;                  // query heads per KV head
 constexpr int SCLUSTER = 4;             // CTAs per row at most
-// A routed call whose rows cannot be longer is one launch of this kernel, two rounds of tiles per CTA (us, against split and
-// merge: 1 row of 499 / 600 / 1024 / 1400 tokens 9.4 / 13.7 / 14.0 / 18.6 and 14.6 / 14.5 / 14.7 / 15.1; 4 rows of 1024 15.1 and 15.0).
+// A routed call whose rows can be no longer is one launch of this kernel: two rounds of tiles per CTA at most.  Measured (us,
+// against split and merge for all rows; 1, 2, 4, 8 KV heads and every batch that short_ok admits): 600 to 1024 tokens 13.7-15.4
+// and 14.6-24, at 128 CTAs 15.1-16.0 and 15.5-15.8, 32 rows of one KV head 16.1-18.8 and 15.8; 1 row of 1400 tokens 18.6 and 15.1.
 constexpr int SHORT_ALL_TOKENS = 1024;
 constexpr uint32_t SSPIN = 1u << 22;
 constexpr uint32_t S_TM_K = 0, S_TM_O = 128, S_TMEM_COLS = 256;
@@ -479,11 +480,14 @@ bool short_ok(const dkv_attn_args* a) {
   return cs == 1 || (long long)a->batch * a->n_basis_groups * cs <= n_sm;
 }
 
-// Whether a routed call leaves its rows to this kernel, also those at or past the switch point.
-bool short_takes_all(const dkv_attn_args* a) {
+// Whether a routed call leaves its rows to this kernel, also those at or past the switch point.  The policy's switch point
+// decides with them: only while no row has more than twice the tiles of the longest row that it calls short (500: 1024 tokens,
+// 64: 256) -- a caller with a low switch point asks for the long rows' kernel where this one would still be taken.
+bool short_takes_all(const dkv_attn_args* a, int switch_tokens) {
   dkv_attn_args all = *a;
   all.route_min_tokens = all.route_max_tokens = 0;
-  return a->seq_len <= SHORT_ALL_TOKENS && short_ok(&all);
+  const int tiles = (a->seq_len + ST - 1) / ST, short_tiles = (int)(((long long)switch_tokens - 1 + ST - 1) / ST);
+  return a->seq_len <= SHORT_ALL_TOKENS && tiles <= 2LL * short_tiles && short_ok(&all);
 }
 
 int short_fused(const dkv_attn_args* a) {

@@ -116,7 +116,8 @@ size_t dkv_split_workspace_bytes(const dkv_attn_args* a);
 
 /* Per-row routing (router.py:20-59) in one call.  Rows below switch_tokens cached tokens (seq_lens, read on the device)
  * go as dkv_fused_decode takes them, the others as dkv_two_stage_decode; on the packed path all rows take one route where that
- * loses no precision: the short kernel where seq_len allows nothing long, split + merge in larger batches.
+ * loses no precision: the short kernel where seq_len allows at most 1024 tokens and no row of more than twice the tiles of 128
+ * tokens that the longest short row has, split + merge in larger batches.
  * switch_tokens <= 0: no row is short.  route_min_tokens / route_max_tokens are ignored.  Workspace as for dkv_two_stage_decode. */
 int dkv_routed_decode(const dkv_attn_args* a, int32_t switch_tokens);
 /* Kernels that the call launches on the packed path; 0 on other caches. */

@@ -81,7 +81,7 @@ def test_routes_of_a_routed_call(seq, switch):
     a, keep = _common.build_attn_args(*d, c.theta, out=out, len_multiple=8, need_workspace=True, route_min_tokens=5, route_max_tokens=9,
                                       seq_lens=torch.tensor(seq, dtype=torch.int32, device="cuda"))
     _lib.check(_lib.load().dkv_routed_decode(ctypes.byref(a), switch), "dkv_routed_decode")
-    assert _lib.load().dkv_routed_launches(ctypes.byref(a), switch) == (1 if max(seq) <= 1024 and len(seq) < 9 else 2 if len(seq) > 9 and switch == 500 else 3)
+    assert _lib.load().dkv_routed_launches(ctypes.byref(a), switch) == (1 if max(seq) <= {500: 1024, 64: 256}[switch] and len(seq) < 9 else 2 if len(seq) > 9 and switch == 500 else 3)
     assert float((out.float().cpu() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
     assert _common.read_status(torch.device("cuda")) == (4 if 0 in seq else 0)      # an empty row is reported
     del keep

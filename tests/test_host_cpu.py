@@ -179,3 +179,18 @@ def test_kernels_that_overlap_the_append_read_its_cache_with_ordinary_loads():
         source = open(os.path.join(ROOT, "dynakv_b200", "csrc", name)).read()
         loads = re.findall(r"[^\n]*(?:__ldg\(|ld\.global\.nc)[^\n]*", source)
         assert all("vup" in line for line in loads), loads
+
+
+@pytest.mark.parametrize("switch,longest", [(1, 0), (2, 256), (64, 256), (129, 256), (130, 512), (300, 768), (385, 768), (386, 1024), (500, 1024),
+                                            (2000, 1024), (2 ** 31 - 1, 1024)])
+def test_switch_point_decides_in_a_routed_call(switch, longest):
+    """One kernel for rows of any length only up to twice the tiles of the longest row that the policy calls short."""
+    a = _lib.AttnArgs()
+    a.dtype, a.batch, a.n_q_heads, a.n_basis_groups, a.arenas_per_batch, a.head_dim, a.rank, a.len_multiple = _lib.DKV_BF16, 4, 32, 8, 8, 128, 128, 8
+    for side in (a.k, a.v):
+        side.flat_stride, side.lens_stride_s, side.offs_stride_s = 8, 1, 1
+    a.n_sm = 148
+    for columns in (1, 128, 129, 256, 257, 499, 512, 513, 768, 769, 1000, 1024, 1025, 4096):
+        a.seq_len = columns
+        n = _lib.load().dkv_routed_launches(ctypes.byref(a), switch)
+        assert (n == 1) == (columns <= longest), (columns, n)
