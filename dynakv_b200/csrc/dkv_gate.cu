@@ -481,8 +481,10 @@ __device__ __forceinline__ float rounded_bound(float thr) {
   const float mid = 0.5f * (thr + to_f32(*reinterpret_cast<const T*>(&u)));     // exact
   return even ? mid : __uint_as_float(__float_as_uint(mid) + 1);
 }
-// a / b for y = 1 / b correctly rounded, two at a time: a quotient within one last place and two exact remainders (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): the result of the division.
+// a / b for y = 1 / b correctly rounded, two at a time: a quotient within one last place and two remainders (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  It is the result of the division as long
+// as the remainders are exact, that is down to about a = 2^-102 for b in 1..1024; below (exponentials of logits 71 or more under the
+// row's largest) it may be off in the last place, of terms too small to change a sum that holds the largest.
 __device__ __forceinline__ float2 quotient2(float2 a, float2 neg_b, float2 y) {
   float2 q = __fmul2_rn(a, y);
   q = __ffma2_rn(__ffma2_rn(q, neg_b, a), y, q);

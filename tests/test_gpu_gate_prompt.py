@@ -102,3 +102,39 @@ def test_bound_of_rounded_sums(thr, d, native, dtype):
         want = int((sums[d - low_rank:] >= bound).sum())
         got = gate_lengths(x, w, b, low_rank, threshold=thr, return_masked=False, native_rounding=native)[1]
         assert got.cpu().tolist() == [want] * rows
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("d", [128, 256, 512, 1024])
+@pytest.mark.parametrize("thr", [0.1, 0.6, 0.97])
+def test_lengths_of_unequal_logits(thr, d, native, dtype):
+    """Identity weights: a row's logits are its own elements, spread by 0.5 to 120.  The lengths are those of 64-bit sums of the
+    softmax, with the roundings to the storage type that `native` asks for, except where a sum ties with the threshold."""
+    from dynakv_b200.kernels.compressed_attention import gate_lengths
+    rows = 600
+    gen = torch.Generator().manual_seed(d)
+    spread = torch.tensor([0.5, 3.0, 10.0, 40.0, 120.0]).repeat(rows // 5)[:, None]
+    x = (-torch.rand(rows, d, generator=gen) * spread).to(dtype)
+    got = gate_lengths(x.cuda(), torch.eye(d, dtype=dtype, device="cuda"), torch.zeros(d, dtype=dtype, device="cuda"), d, threshold=thr,
+                       return_masked=False, native_rounding=native)[1].cpu().long()
+    p = torch.softmax(x.double(), -1)
+    # relative error of a probability, and of a sum of them: 2 units of the exponential, 30 / 2 of its argument (smaller ones do not
+    # count), a half for each of the 37 additions of the sum, the quotient and another 37: below 64 units of 2^-23
+    err = 64 * 2.0 ** -23
+    slack = torch.zeros(rows, 1, dtype=torch.float64)
+    bound = float(torch.tensor(thr, dtype=torch.float32))
+    if native:
+        digits, least = (8, -133) if dtype == torch.bfloat16 else (11, -24)
+        ulp = torch.ldexp(torch.ones_like(p), (torch.frexp(p).exponent - digits).clamp_min(least))
+        near = ((p / ulp - torch.floor(p / ulp) - 0.5).abs() <= err * p / ulp)      # may be rounded to either side
+        slack = (near * ulp).cumsum(-1)
+        p = p.to(dtype).double()
+        bound = float(torch.tensor(thr, dtype=dtype))
+    sums = p.cumsum(-1)
+    lo, hi = sums * (1 - err) - slack, sums * (1 + err) + slack
+    if native:
+        lo, hi = lo.to(dtype).double(), hi.to(dtype).double()
+    least, most = (lo >= bound).sum(-1), (hi >= bound).sum(-1)
+    assert bool(((least <= got) & (got <= most)).all())
+    assert float((most > least).double().mean()) <= 0.1        # ties are few: nearly every row is held to one length

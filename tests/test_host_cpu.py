@@ -194,3 +194,35 @@ def test_switch_point_decides_in_a_routed_call(switch, longest):
         a.seq_len = columns
         n = _lib.load().dkv_routed_launches(ctypes.byref(a), switch)
         assert (n == 1) == (columns <= longest), (columns, n)
+
+
+def test_quotient_from_a_reciprocal_and_two_remainders_is_the_division():
+    """The gate's division of exponentials by their row's sum, step by step in exact arithmetic."""
+    from fractions import Fraction
+
+    import numpy as np
+
+    def rn(f):          # to the nearest float32, ties to even
+        if f == 0:
+            return Fraction(0)
+        n, e = abs(f), 0
+        while n >= 2 ** 24:
+            n, e = n / 2, e + 1
+        while n < 2 ** 23 and e > -149:
+            n, e = n * 2, e - 1
+        return (1 if f > 0 else -1) * Fraction(round(n)) * Fraction(2) ** e
+
+    def quotient(a, b):
+        y = rn(1 / b)
+        q = rn(a * y)
+        for _ in range(2):
+            q = rn(rn(a - q * b) * y + q)
+        return q
+
+    rng = np.random.default_rng(5)
+    for lowest, exact in ((-100, True), (-148, False)):
+        for _ in range(1500):
+            a = rn(Fraction(float(rng.uniform(1, 2))) * Fraction(2) ** int(rng.integers(lowest, 0)))
+            b = rn(Fraction(float(rng.uniform(1, 1024))))
+            want, got = rn(a / b), quotient(a, b)
+            assert got == want if exact else abs(got - want) <= max(want / 2 ** 23, Fraction(2) ** -149)
