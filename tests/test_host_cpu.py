@@ -226,3 +226,15 @@ def test_quotient_from_a_reciprocal_and_two_remainders_is_the_division():
             b = rn(Fraction(float(rng.uniform(1, 1024))))
             want, got = rn(a / b), quotient(a, b)
             assert got == want if exact else abs(got - want) <= max(want / 2 ** 23, Fraction(2) ** -149)
+
+
+def test_smoke_check_reaches_the_split_kernel():
+    import __graft_entry__ as entry
+    a = _lib.AttnArgs()
+    a.dtype, a.batch, a.n_q_heads, a.n_basis_groups, a.arenas_per_batch, a.head_dim, a.rank, a.len_multiple = _lib.DKV_BF16, 2, 32, 8, 8, 128, 128, 8
+    for side in (a.k, a.v):
+        side.flat_stride, side.lens_stride_s, side.offs_stride_s = 8, 1, 1
+    a.n_sm, a.seq_len = 148, max(entry.SMOKE_TOKENS) + 8
+    switch = KernelPolicy().switch_tokens
+    assert len(entry.SMOKE_TOKENS) == 2 and min(entry.SMOKE_TOKENS) + 1 < switch <= max(entry.SMOKE_TOKENS)
+    assert 1 + _lib.load().dkv_routed_launches(ctypes.byref(a), switch) == entry.SMOKE_LAUNCHES
