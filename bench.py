@@ -354,8 +354,8 @@ def prefill_compress_leg(dev, reps=200):
 
 def joint_layout_leg(dev):
     """The reference's literal layout next to the headline: one joint latent row per batch row (R = 1024 over all
-    heads), bases [Hq, 1024, 128], any integer length (len_multiple 1).  It runs on the generic CUDA-core kernels
-    (the tensor-core kernels need per-KV-head arenas and lengths in multiples of 8); with the reference's own
+    heads), bases [Hq, 1024, 128], any integer length (len_multiple 1).  It runs on the tile kernels
+    (the packed pipeline needs per-KV-head arenas and lengths in multiples of 8); with the reference's own
     Triton kernels on the same tensors beside it when the installed copy is there."""
     from dynakv_b200.kernels.fused import fused_attention_dispatch
     from dynakv_b200.kernels.two_stage import two_stage_attention
@@ -416,25 +416,23 @@ def joint_layout_leg(dev):
 
 def tensor_pipe_probe(dev, tiles=100):
     """Cycles per 128-token tile that one SM's tensor pipe is held by the decode kernel's three tcgen05.mma chains
-    (issued back to back by one thread, nothing else on the SM): the floor under the split kernel's time per tile."""
+    (issued back to back, nothing else on the SM): a floor under the split kernel's time per tile."""
     from dynakv_b200 import _lib
     from dynakv_b200.kernels._common import status_word, read_status
     lib = _lib.load()
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
-    cyc = torch.zeros(2 * n_sm, dtype=torch.int64, device=dev)
+    cyc = torch.zeros(3, n_sm, dtype=torch.int64, device=dev)
     out = {}
-    for name, mask in (("k_reconstruction", 1), ("scores", 2), ("latent_accumulation", 4), ("all_three", 7),
-                       ("all_three_commit_per_chain", 23), ("all_three_nonzero_operands", 39),
-                       ("two_issuers_nonzero_thread_1_2", 43), ("two_issuers_thread_1_2", 11)):
+    for name, mask, warps in (("k_reconstruction", 1, 1), ("scores", 2, 1), ("latent_accumulation", 4, 1), ("all_three", 7, 1),
+                              ("all_three_commit_per_chain", 23, 1), ("all_three_nonzero_operands", 39, 1),
+                              ("two_warps", 11, 2), ("two_warps_nonzero_operands", 43, 2),
+                              ("warp_per_product", 71, 3), ("warp_per_product_nonzero_operands", 103, 3)):
         for _ in range(2):
             _lib.check(lib.dkv_probe_tensor_pipe(mask, tiles, n_sm, cyc.data_ptr(), status_word(dev).data_ptr(),
                                                  _lib.stream_ptr(dev)), "dkv_probe_tensor_pipe")
         torch.cuda.synchronize()
-        out[name] = float(cyc[:n_sm].double().median().item()) / tiles
-        if mask == 11:
-            out["two_issuers_thread_3"] = float(cyc[n_sm:].double().median().item()) / tiles
-        if mask == 43:
-            out["two_issuers_nonzero_thread_3"] = float(cyc[n_sm:].double().median().item()) / tiles
+        per_warp = [float(cyc[i].double().median().item()) / tiles for i in range(warps)]
+        out[name] = per_warp[0] if warps == 1 else per_warp
     out["status"] = read_status(dev)
     return {"cycles_per_tile": out, "tiles": tiles, "ctas": n_sm}
 

@@ -229,14 +229,13 @@ int dkv_pack_pair(const dkv_pack_args* k, const dkv_pack_args* v);
 int dkv_row_totals(const dkv_pack_args* k, const dkv_pack_args* v, int32_t* totals /* [2, n_arena, 4], 16-byte aligned */);
 
 /* Diagnostic, no counterpart in the reference: clock cycles per 128-token tile that the tensor pipe of one SM is
- * held by the decode kernel's tcgen05.mma chains, issued back to back by one thread over zero operands with nothing
- * else running on the SM.  `products` is a mask: 1 = K reconstruction (8 x M128 N128 K16), 2 = scores (8 x M128 N16
- * K16, A in tensor memory), 4 = latent accumulation (8 x M128 N16 K16); 11 = products 1 and 2 from one thread with
- * product 4's chain issued concurrently by a thread of another warp, as the decode kernel does; 23 = all three from
- * one thread with a tcgen05.commit behind every chain (the kernel's four commits per tile); 39 and 43 = 7 and 11
- * over non-zero operands.  Launches n_cta
- * CTAs (one per SM when n_cta <= the SM count) of `tiles` tiles each and writes cycles[c] = elapsed clock64 of CTA c
- * for all its tiles (and, for 11, cycles[n_cta + c] for the second thread: `cycles` holds 2 * n_cta values).
+ * held by the decode kernel's tcgen05.mma chains, issued as that kernel issues them (a converged warp, an elected lane), back to
+ * back over zero operands with nothing else running on the SM.  `products` is a mask: 1 = K reconstruction (8 x M128 N128 K16),
+ * 2 = scores (8 x M128 N16 K16, A in tensor memory), 4 = latent accumulation (8 x M128 N16 K16), all from one warp; 11 = products 1
+ * and 2 from one warp with product 4's chain issued concurrently by another; 23 = all three from one warp with a tcgen05.commit behind
+ * every chain; 71 = a warp per product, as the decode kernel does; 39, 43 and 103 = 7, 11 and 71 over non-zero operands.  Launches
+ * n_cta CTAs (one per SM when n_cta <= the SM count) of `tiles` tiles each and writes cycles[c] = elapsed clock64 of CTA c for all
+ * its tiles (for 11 and 43 also cycles[n_cta + c] for the second warp, for 71 and 103 cycles[w * n_cta + c] for the three).
  * The wait for the products is bounded; DKV_ST_TIMEOUT is set in *status when it runs out. */
 int dkv_probe_tensor_pipe(int32_t products, int32_t tiles, int32_t n_cta, int64_t* cycles, int32_t* status, void* stream);
 

@@ -180,3 +180,17 @@ def test_arena_of_negative_size_holds_nothing():
     head, flat, lens, offs, _ = _one_arena()
     out, status = _raw_call(*head, flat, lens, offs, -8)
     assert status == 6 and float(out.abs().max()) == 0
+
+
+def test_probe_of_the_tensor_pipe():
+    """Every form ends in time; 8 x (M128 N128 K16) cannot take less than 512 cycles (4096 multiply-adds a cycle and SM)."""
+    n, tiles, dev = 4, 50, torch.device("cuda")
+    word = _common.status_word(dev)
+    for mask, warps in ((1, 1), (2, 1), (3, 1), (4, 1), (5, 1), (6, 1), (7, 1), (11, 2), (23, 1), (39, 1), (43, 2), (71, 3), (103, 3)):
+        cyc = torch.zeros(3, n, dtype=torch.int64, device=dev)
+        _lib.check(_lib.load().dkv_probe_tensor_pipe(mask, tiles, n, cyc.data_ptr(), word.data_ptr(), _lib.stream_ptr(dev)), "dkv_probe_tensor_pipe")
+        assert _common.read_status(dev) == 0
+        assert bool((cyc[:warps] > 0).all()) and not cyc[warps:].any()
+        if mask & 1:
+            assert float(cyc[0].min()) >= 0.98 * 512 * tiles
+    assert _lib.load().dkv_probe_tensor_pipe(8, tiles, n, cyc.data_ptr(), word.data_ptr(), _lib.stream_ptr(dev)) != 0
