@@ -291,6 +291,18 @@ struct Pack<__half> {
 // One copy of the library function for all its uses here (each inlined copy brings its slow path for large arguments).
 __device__ __noinline__ void sincos_call(float x, float* s, float* c) { sincosf(x, s, c); }
 
+// Waits have run out: copies and products may be in flight, and end before their operands and sums go.  (Out of line: the
+// kernel's code is not to grow by what never runs.)
+__device__ __noinline__ void end_what_is_in_flight(SmemLayout& sm, int warp, int32_t* status) {
+  if (threadIdx.x == 0) set_status(status, DKV_ST_TIMEOUT);
+  cp_async_wait_all();
+  if (warp >= W_MMA && warp <= W_MMA3) {
+    umma_commit(smem_u32(&sm.drained[warp - W_MMA]));
+    mbar_wait(smem_u32(&sm.drained[warp - W_MMA]), 0u, &sm.abort_flag);      // (1024 probes)
+  }
+  __syncthreads();
+}
+
 // --------------------------------------------------------------- work partition
 // Token space of one KV head: batch rows back to back, each rounded up to whole 128-token tiles.
 __device__ __forceinline__ int row_tokens(const dkv_attn_args& p, int i) {
@@ -1000,15 +1012,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
   // ---- epilogue: every warp arrives here; the tensor memory is returned by the warp that allocated it ----
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) {        // waits have run out: copies and products may be in flight, and end before their operands and sums go
-    if (tid == 0) set_status(p.status, DKV_ST_TIMEOUT);
-    cp_async_wait_all();
-    if (warp >= W_MMA && warp <= W_MMA3) {
-      umma_commit(smem_u32(&sm.drained[warp - W_MMA]));
-      mbar_wait(smem_u32(&sm.drained[warp - W_MMA]), 0u, abort_flag);      // (1024 probes)
-    }
-    __syncthreads();
-  }
+  if (*abort_flag) end_what_is_in_flight(sm, warp, p.status);
   if (project) {
     // out[head][d] = sum_r latent[head][r] * Bv[r][d]: one output element per thread
     const int h = tid >> 7, d = tid & 127;

@@ -167,10 +167,11 @@ def test_waits_of_the_decode_pipeline_answer_for_a_whole_warp():
 def test_a_decode_kernel_that_gives_up_waits_for_what_is_in_flight():
     """Copies and products end before shared memory and tensor memory go, also when the loops were left by waits that ran out."""
     source = open(os.path.join(ROOT, "dynakv_b200", "csrc", "dkv_mma_decode.cu")).read()
-    end = source[source.index("// ---- epilogue"):source.index("tcgen05.dealloc")]
-    given_up = re.search(r"if \(\*abort_flag\) \{(.*?)\n  \}\n", end, flags=re.S).group(1)
-    order = [given_up.index(w) for w in ("cp_async_wait_all()", "umma_commit(", "mbar_wait(", "__syncthreads()")]
+    body = re.search(r"void end_what_is_in_flight\([^)]*\) \{(.*?)\n\}\n", source, flags=re.S).group(1)
+    order = [body.index(w) for w in ("cp_async_wait_all()", "umma_commit(", "mbar_wait(", "__syncthreads()")]
     assert order == sorted(order)
+    end = source[source.index("// ---- epilogue"):source.index("tcgen05.dealloc")]
+    assert re.search(r"__syncthreads\(\);\n  if \(\*abort_flag\) end_what_is_in_flight\(", end)
 
 
 def test_kernels_that_overlap_the_append_read_its_cache_with_ordinary_loads():
