@@ -536,10 +536,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_pv_kernel(dkv_attn_args p, Sc
 
 // --------------------------------------------------------------- fp32: the same two steps on the FMA units
 // 16 tokens per CTA: thread = (dim, 8 tokens), coefficients staged transposed so that a load serves four tokens; the
-// rotation's (cos, sin) once per CTA for all heads of the unit, exact sincosf as in the single-kernel path.  PARTS: units that
-// are parts of basis groups (an instance of its own: with the division in it the compiler keeps 48 registers and not 62, and
-// one sequence of 256 tokens takes 23.5 us in place of 22.6).
-template <bool PARTS>
+// rotation's (cos, sin) once per CTA for all heads of the unit, exact sincosf as in the single-kernel path.
 __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_args p, ScoreSink sink, float log_theta) {
   __shared__ __align__(16) float x_s[TS_CHUNK][TF_TOK];
   __shared__ float k_s[TF_TOK][TD + 4];
@@ -576,7 +573,7 @@ __global__ void __launch_bounds__(TS_THREADS) tile_scores_f32_kernel(dkv_attn_ar
     if (lane == 0) rmax_s = mx;
   }
   const int d = tid & 127, th = tid >> 7;
-  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(PARTS ? g / sink.per_basis : g) * R * TD;
+  const float* kup = reinterpret_cast<const float*>(p.k_up) + (size_t)(g / sink.per_basis) * R * TD;
   float w[16];           // the first basis rows too, before it is known how many are needed
 #pragma unroll
   for (int u = 0; u < 16; ++u) w[u] = u < R ? __ldg(kup + (size_t)u * TD + d) : 0.f;
@@ -886,8 +883,7 @@ int launch_scores(const dkv_attn_args* a, float* ws) {
   const dim3 grid((unsigned)ctas, u.n_basis_groups);      // (n_q_heads <= 65535)
   const int smem = (int)sizeof(ScoreSmem) + 128;
   if (a->dtype == DKV_F32) {
-    if (sink.per_basis > 1) tile_scores_f32_kernel<true><<<grid, TS_THREADS, 0, st>>>(u, sink, log_theta);
-    else tile_scores_f32_kernel<false><<<grid, TS_THREADS, 0, st>>>(u, sink, log_theta);
+    tile_scores_f32_kernel<<<grid, TS_THREADS, 0, st>>>(u, sink, log_theta);
   } else if (a->dtype == DKV_F16) {
     if (int rc = opt_in(tile_scores_kernel<__half>, smem)) return rc;
     tile_scores_kernel<__half><<<grid, TS_THREADS, smem, st>>>(u, sink, log_theta);
