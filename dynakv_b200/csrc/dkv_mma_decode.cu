@@ -29,13 +29,14 @@
 // What bounds it: no unit is saturated; a tile passes through a ring of latencies, and every stage is a chain of dependent
 // instructions on a warp that shares its issue slots with six others and its instruction cache with all of them.  Measured
 // with clock64 at every hand-over (8 rows of 32768 tokens, cycles per tile): one lane that issued (1) and (2) was the period
-// (620 + 600 of issue, 770 of barrier probes and commits: 1980).  A product's eight instructions took 75 cycles each because
-// a lane's operands are not known to be uniform: 38 instructions per tcgen05.mma.  Issued from converged warps through
-// elect.sync they take 20, and the kernel 58 KB of code instead of 84.  Now the gather loop is the period (1600: 600 of copies,
-// the rest before them).
-// Split kernel, 8 KV heads, start -> now in us, in a chain of launches with the merge: 8 rows of 32768 tokens, lengths beta(2,8)
-// 139 -> 106; 32 rows of 8192, beta(2,5) 151 -> 119; 32 rows of 513 28.6 -> 25.2; 30 rows of 300, 600 and 2500 with K-RMSNorm
-// 37.5 -> 33.3; one row of 1100 / 4096 / 16000 tokens 16.3 / 17.4 / 22.9 -> 15.4 / 16.1 / 20.0.
+// (620 + 600 of issue, 770 of barrier probes and commits: 1980), a product's eight instructions taking 75 cycles each.  From a
+// converged warp through elect.sync the chain of product (2) alone takes 76 cycles where a lane in a branch took 377
+// (dkv_probe_tensor_pipe).  Now the gather loop is the period (about 1550: 600 of copies, the rest before them); the three
+// chains by themselves take 934 from one warp and 1169 from three, with all eight k-steps of product (1).
+// Split kernel and merge in a chain of launches, 8 KV heads, us, with 24 warps and one lane for two products -> as it is: 8 rows of
+// 32768 tokens, lengths beta(2,8) 133.6 -> 98.5, uniform 204.5 -> 144.7, beta(2,8) with K-RMSNorm 145.9 -> 129.6; 32 rows of 8192,
+// beta(2,5) 141.5 -> 110.5; 32 rows of 513 30.1 -> 26.4; 30 rows of 300, 600 and 2500 with K-RMSNorm 40.3 -> 35.3; one row of
+// 1100 / 4096 / 16000 tokens 15.8 / 17.0 / 23.4 -> 15.1 / 15.8 / 22.4.
 //
 // Reference math: src/dynakv/kernels/fused.py:28-142 (fused), two_stage.py:52-157,211-281 (two-stage;
 // the latent-space V accumulation with one up-projection at the end is two_stage.py:261-277).
@@ -173,8 +174,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // units, descriptor version 1.
 // tcgen05.mma with the shared-memory operand descriptors passed as two 32-bit words (low = (address >> 4) |
 // (LBO >> 4) << 16, high = (SBO >> 4) | version bit 46).  Called by a converged warp with operands that are the same in all
-// lanes, and issued by one elected lane: what stands in a branch of a single lane is built lane by lane, at twice the
-// instructions.
+// lanes, and issued by one elected lane: from a branch of a single lane, whose operands are not known to be uniform, eight
+// instructions of N = 16 took 377 cycles, so they take 76.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) { return ((addr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16); }
 __device__ __forceinline__ uint32_t desc_hi(uint32_t sbo) { return ((sbo >> 4) & 0x3FFFu) | (1u << 14); }
 __device__ __forceinline__ void umma_f16_w(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
@@ -581,7 +582,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
     // Four warps per side, 32 tokens of every tile each.  Lane l reads the length and offset of token l (a tile ahead, into
     // registers) and checks them; then four lanes copy a token's row together, 64 contiguous bytes of it per instruction for
     // eight tokens, which come back to back: a few cache lines, where a lane per token touches one per token (lengths uniform
-    // in 8..128, 8 rows of 32768: 206 -> 164 us).  Chunk c of token t goes to c*CHUNK_PITCH + t*16.  Chunks past the row's
+    // in 8..128, 8 rows of 32768: 206 -> 164 us when it came).  Chunk c of token t goes to c*CHUNK_PITCH + t*16.  Chunks past the row's
     // length are zero-filled without a read, but only those that the row before in this buffer had reached: what lies past
     // both is zero already.  Everything that does not need the buffer is done before the wait for it, and the copies are
     // unrolled twice, for rows of up to 8 chunks and for all: the latency of this loop is what counts, not its bytes.
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mma_decode_kernel(dkv_attn_args p
       len = off = 0;
       if (left > 0) { len = *lens_at; off = *offs_at; }      // (not read-only loads: the append that writes them may overlap this kernel's beginning)
       // a line of each, META_AHEAD tiles on, into L2: a tile ahead is less than a trip to memory since the loop got faster
-      // (8 rows of 32768 tokens 107.9 -> 104.3 us, 32 of 8192 124.7 -> 120.9)
+      // (a step of two layers, 8 rows of 32768 tokens: 223 -> 217 us)
       if (lane < 2 && left > META_AHEAD * ST_TOK)
         asm volatile("prefetch.global.L2 [%0];" ::"l"((lane ? offs_at : lens_at) + META_AHEAD * ST_TOK));
       left -= ST_TOK; lens_at += ST_TOK; offs_at += ST_TOK;

@@ -12,7 +12,8 @@
 // The first version (one CTA per (row, query head, slice), K reconstructed per query head on mma.sync) took 281 us on
 // B = 2, S = 2048, R = 1024, 8 groups, bf16, and 13 us for the merge; the three took 25 (scores) + 13 (latent sums) + 7 us (merge),
 // the call 48.0; 43.1 since a thread's pieces are asked for together and the V rows before the scores are waited for.
-// fp32, B = 1, S = 256, 8 arenas: 131 us in one kernel of 32 CTAs, now 12 + 6.5 + 5 us.
+// fp32, B = 1, S = 256, 8 arenas: 131 us in one kernel of 32 CTAs, in three kernels 22.5, 19.1 since queries, basis
+// rows and V are asked for ahead.
 //
 // Math (reference: src/dynakv/kernels/fused.py:28-142, two_stage.py:52-157, 211-281): as in dkv_generic.cu, which keeps
 // the single-kernel path for callers without a workspace.
